@@ -5,111 +5,273 @@
 // the tile shape and however many rows the launch has, so a row's result does not depend on what
 // else is in the batch (bitwise). Both operands are contiguous along K.
 //
-// Tiles BM x BN x 16 through shared memory (stored k-major so the inner loop reads vectors), each
-// thread a TM x TN micro-tile. Three shapes: 128x128 (8x8) for prompts, 32x64 (2x4) and 16x64 (1x4)
-// for few rows; and a kernel of its own for up to 16 rows against a wide w, which streams w once. kreasof-ai/akas's plain float32 `linear` is a per-row tree reduction
-// (src/akas/ops/linear/kernel.py:403-447).
+// Four kernels: pipelined tiles for more than 16 rows; a warp per 8 rows of w, or a block per 32 of a wide w, for fewer,
+// which stream w once; and a plain tiled kernel for operands whose rows do not start on 16 bytes. kreasof-ai/akas's plain float32
+// `linear` is a per-row tree reduction (src/akas/ops/linear/kernel.py:403-447).
 #include "common.cuh"
 
 using namespace akas;
 
-#define AKAS_BK 16
+namespace {
+
+// 16 bytes from global to shared memory, or zeros where `live` is false (the source is then not read).
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool live) {
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// Tiles of BM x BN outputs, kBK of K a stage, two stages in shared memory, stored k-major (the next stage is on its way to
+// registers while one is multiplied, and transposed on the way into shared memory). A warp owns 4 TM x 8 TN outputs, lane
+// (ty, tx) of 4 x 8 takes the rows 4 ty .. 4 ty + 3 of every 16 and the columns 4 tx .. 4 tx + 3 of every 32, so that its
+// operands of a k are 16-byte loads. Two neighbouring columns are one packed pair: fma.rn.f32x2 does the two chains'
+// steps in one instruction, each rounded as fmaf rounds it.
+constexpr int kBK = 16;
+
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 parts_of(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma_pair(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
 
 template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-sgemm_tn_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
-                const float* __restrict__ residual, int N, int O, int K, int vec_ok) {
-  constexpr int NT = (BM / TM) * (BN / TN);
-  __shared__ float As[AKAS_BK][BM + 4];
-  __shared__ float Bs[AKAS_BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+__global__ void __launch_bounds__((BM / (4 * TM)) * (BN / (8 * TN)) * 32)
+sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, float* y, const float* residual, int N, int O, int K) {
+  constexpr int NT = (BM / (4 * TM)) * (BN / (8 * TN)) * 32;
+  constexpr int PA = BM + 4, PB = BN + 4, GA = TM / 4, GB = TN / 4;
+  constexpr int LA = BM * (kBK / 4) / NT, LB = BN * (kBK / 4) / NT;  // 16-byte loads of a stage per thread
+  static_assert(LA * NT == BM * (kBK / 4) && LB * NT == BN * (kBK / 4), "whole loads");
+  __shared__ __align__(16) float As[2][kBK][PA];
+  __shared__ __align__(16) float Bs[2][kBK][PB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = lane >> 3, tx = lane & 7;
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+  const int wm = (warp / (BN / (8 * TN))) * 4 * TM + 4 * ty, wn = (warp % (BN / (8 * TN))) * 8 * TN + 4 * tx;
+  const int lr = tid / (kBK / 4), lc = (tid % (kBK / 4)) * 4;  // a thread's loads: rows lr + i NT / 4, channels lc ..
 
-  float acc[TM][TN];
+  float4 ra[LA], rb[LB];
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto fetch_w = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < LB; ++i) {
+      const int r = col0 + lr + i * (NT / (kBK / 4));
+      rb[i] = r < O && k0 + lc < K ? *reinterpret_cast<const float4*>(w + (size_t)r * K + k0 + lc) : none;
+    }
+  };
+  auto fetch_x = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+      const int r = row0 + lr + i * (NT / (kBK / 4));
+      ra[i] = r < N && k0 + lc < K ? *reinterpret_cast<const float4*>(x + (size_t)r * K + k0 + lc) : none;
+    }
+  };
+  auto put = [&](int to) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+      const int r = lr + i * (NT / (kBK / 4));
+      As[to][lc][r] = ra[i].x; As[to][lc + 1][r] = ra[i].y; As[to][lc + 2][r] = ra[i].z; As[to][lc + 3][r] = ra[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < LB; ++i) {
+      const int r = lr + i * (NT / (kBK / 4));
+      Bs[to][lc][r] = rb[i].x; Bs[to][lc + 1][r] = rb[i].y; Bs[to][lc + 2][r] = rb[i].z; Bs[to][lc + 3][r] = rb[i].w;
+    }
+  };
+
+  uint64_t acc[TM][TN / 2];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
 
-  for (int k0 = 0; k0 < K; k0 += AKAS_BK) {
-    // each tile row has AKAS_BK / 4 = 4 groups of four consecutive k
-    for (int i = tid; i < BM * (AKAS_BK / 4); i += NT) {
-      const int r = i / (AKAS_BK / 4), kq = (i % (AKAS_BK / 4)) * 4;
-      const int gr = row0 + r, gk = k0 + kq;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (gr < N) {
-        const float* p = x + (size_t)gr * K + gk;
-        if (vec_ok && gk + 3 < K) {
-          const float4 f = *reinterpret_cast<const float4*>(p);
-          v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
+  float4 fa[2][GA], fb[2][GB];  // the operands of two k: one is multiplied while the next is loaded
+  auto load = [&](int slot, int stage, int k) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (gk + j < K) v[j] = p[j];
-        }
+    for (int g = 0; g < GA; ++g) fa[slot][g] = *reinterpret_cast<const float4*>(&As[stage][k][wm + 16 * g]);
+#pragma unroll
+    for (int g = 0; g < GB; ++g) fb[slot][g] = *reinterpret_cast<const float4*>(&Bs[stage][k][wn + 32 * g]);
+  };
+
+  const int steps = (K + kBK - 1) / kBK;
+  chain_release();
+  fetch_w(0);  // weights: no kernel writes them
+  chain_wait();
+  fetch_x(0);
+  put(0);
+  __syncthreads();
+  load(0, 0, 0);
+  for (int step = 0; step < steps; ++step) {
+    const int at = step & 1;
+    const bool more = step + 1 < steps;
+    if (more) {
+      fetch_w((step + 1) * kBK);
+      fetch_x((step + 1) * kBK);
+    }
+#pragma unroll
+    for (int k = 0; k < kBK; ++k) {
+      if (k + 1 < kBK) {
+        load((k + 1) & 1, at, k + 1);
+      } else if (more) {
+        put(at ^ 1);  // read last in the round before the last barrier
+        __syncthreads();
+        load(0, at ^ 1, 0);
+      }
+      const float4 *pa = fa[k & 1], *pb = fb[k & 1];
+      uint64_t bv[TN / 2];
+#pragma unroll
+      for (int g = 0; g < GB; ++g) {
+        bv[2 * g] = pair_of(pb[g].x, pb[g].y);
+        bv[2 * g + 1] = pair_of(pb[g].z, pb[g].w);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) As[kq + j][r] = v[j];
-    }
-    for (int i = tid; i < BN * (AKAS_BK / 4); i += NT) {
-      const int r = i / (AKAS_BK / 4), kq = (i % (AKAS_BK / 4)) * 4;
-      const int gr = col0 + r, gk = k0 + kq;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (gr < O) {
-        const float* p = w + (size_t)gr * K + gk;
-        if (vec_ok && gk + 3 < K) {
-          const float4 f = *reinterpret_cast<const float4*>(p);
-          v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
+      for (int g = 0; g < GA; ++g) {
+        const float av[4] = {pa[g].x, pa[g].y, pa[g].z, pa[g].w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (gk + j < K) v[j] = p[j];
+        for (int e = 0; e < 4; ++e) {
+          const uint64_t aa = pair_of(av[e], av[e]);
+#pragma unroll
+          for (int j = 0; j < TN / 2; ++j) fma_pair(acc[4 * g + e][j], aa, bv[j]);
         }
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) Bs[kq + j][r] = v[j];
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < AKAS_BK; ++k) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[k][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[k][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
   }
-
+  const bool four = O % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)residual % 16 == 0;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int gr = row0 + ty * TM + i;
+    const int gr = row0 + wm + 16 * (i / 4) + i % 4;
     if (gr >= N) continue;
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gc = col0 + tx * TN + j;
-      if (gc >= O) continue;
-      const size_t at = (size_t)gr * O + gc;
-      y[at] = residual ? residual[at] + acc[i][j] : acc[i][j];
+    for (int g = 0; g < GB; ++g) {
+      const int gc = col0 + wn + 32 * g;
+      const float2 lo = parts_of(acc[i][2 * g]), hi = parts_of(acc[i][2 * g + 1]);
+      float v[4] = {lo.x, lo.y, hi.x, hi.y};
+      const size_t place = (size_t)gr * O + gc;
+      if (four && gc < O) {
+        if (residual) {
+          const float4 h = *reinterpret_cast<const float4*>(residual + place);
+          v[0] = h.x + v[0]; v[1] = h.y + v[1]; v[2] = h.z + v[2]; v[3] = h.w + v[3];
+        }
+        *reinterpret_cast<float4*>(y + place) = make_float4(v[0], v[1], v[2], v[3]);
+        continue;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (gc + e < O) y[place + e] = residual ? residual[place + e] + v[e] : v[e];
     }
   }
 }
 
-// A handful of rows (decode steps): the time goes to reading w once. A block owns 32 rows of w (32 output
-// channels): its 128 threads fetch them 64 k at a time with coalesced 16-byte loads into a double-buffered
+// A handful of rows (decode steps): w is read once, and an output's chain of K dependent multiply-adds (four cycles each)
+// is what a warp cannot be faster than. So a block is one warp with 8 rows of w and up to 16 rows of x, lane (r, g) of
+// 8 x 4 holding row r against tokens g + 4 i: even the narrowest product of a model spreads over all SMs. STAGES of kFewK
+// channels are on their way by cp.async. The first stages of w are asked for before the wait for the kernel ahead.
+constexpr int kFewK = 64, kFewPitch = kFewK + 4, kFewRows = 8;
+
+template <int TOK, int STAGES>  // tokens per lane: a warp covers 4 * TOK tokens
+__global__ void __launch_bounds__(32)
+sgemm_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float* y, const float* residual, int N, int O, int K) {
+  extern __shared__ __align__(16) float ring[];  // [STAGES][kFewRows + 4 TOK][kFewPitch]
+  constexpr int kStageFloats = (kFewRows + 4 * TOK) * kFewPitch;
+  const int lane = threadIdx.x, r = lane >> 2, g = lane & 3;
+  const int row0 = blockIdx.x * kFewRows;
+  // a lane's copies of a stage: channel lc of rows lr, lr + 2, ..: its sources move on by kFewK a stage
+  const int lr = lane >> 4, lc = (lane & 15) * 4;
+  const float* wsrc = w + (size_t)(row0 + lr) * K + lc;
+  const float* xsrc = x + (size_t)lr * K + lc;
+  auto issue_w = [&](float* stage, int k0) {
+#pragma unroll
+    for (int i = 0; i < kFewRows / 2; ++i) {
+      const bool live = row0 + lr + 2 * i < O && k0 + lc < K;
+      copy16(stage + (lr + 2 * i) * kFewPitch + lc, live ? wsrc + (size_t)(2 * i) * K + k0 : w, live);
+    }
+  };
+  auto issue_x = [&](float* stage, int k0) {
+#pragma unroll
+    for (int i = 0; i < 2 * TOK; ++i) {
+      const bool live = lr + 2 * i < N && k0 + lc < K;
+      copy16(stage + (kFewRows + lr + 2 * i) * kFewPitch + lc, live ? xsrc + (size_t)(2 * i) * K + k0 : x, live);
+    }
+  };
+  float acc[TOK];
+#pragma unroll
+  for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
+  const int steps = (K + kFewK - 1) / kFewK;
+  chain_release();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) issue_w(ring + s * kStageFloats, s * kFewK);
+  chain_wait();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    issue_x(ring + s * kStageFloats, s * kFewK);
+    copies_commit();
+  }
+  int at = 0, to = STAGES - 1;
+  for (int step = 0; step < steps; ++step) {
+    copies_wait<STAGES - 2>();
+    __syncwarp();  // the stage has landed for every lane, and the one before it has been read
+    const int ahead = (step + STAGES - 1) * kFewK;
+    if (ahead < K) {
+      issue_w(ring + to * kStageFloats, ahead);
+      issue_x(ring + to * kStageFloats, ahead);
+    }
+    copies_commit();
+    const float* ws = ring + at * kStageFloats + r * kFewPitch;
+    const float* xs = ring + at * kStageFloats + (kFewRows + g) * kFewPitch;
+    constexpr int AHEAD = TOK == 1 ? 4 : 2;  // words of w and x that are loaded ahead of their use
+    float4 wv[2 * AHEAD], xv[2 * AHEAD][TOK];
+    auto load = [&](int slot, int kk) {
+      wv[slot] = *reinterpret_cast<const float4*>(ws + kk);
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) xv[slot][i] = *reinterpret_cast<const float4*>(xs + i * 4 * kFewPitch + kk);
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) load(u, 4 * u);
+#pragma unroll
+    for (int u = 0; u < kFewK / 4; ++u) {
+      if (u + AHEAD < kFewK / 4) load((u + AHEAD) % (2 * AHEAD), 4 * (u + AHEAD));
+      const float4 wu = wv[u % (2 * AHEAD)];
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) acc[i] = fmaf(xv[u % (2 * AHEAD)][i].x, wu.x, acc[i]);
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) acc[i] = fmaf(xv[u % (2 * AHEAD)][i].y, wu.y, acc[i]);
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) acc[i] = fmaf(xv[u % (2 * AHEAD)][i].z, wu.z, acc[i]);
+#pragma unroll
+      for (int i = 0; i < TOK; ++i) acc[i] = fmaf(xv[u % (2 * AHEAD)][i].w, wu.w, acc[i]);
+    }
+    at = at + 1 == STAGES ? 0 : at + 1;
+    to = to + 1 == STAGES ? 0 : to + 1;
+  }
+  const int row = row0 + r;
+  if (row >= O) return;
+#pragma unroll
+  for (int i = 0; i < TOK; ++i) {
+    const int t = g + 4 * i;
+    if (t >= N) continue;
+    const size_t place = (size_t)t * O + row;
+    y[place] = residual ? residual[place] + acc[i] : acc[i];
+  }
+}
+
+// Five to 16 rows against a wide w: the time goes to reading w once, and with the blocks many, more rows of w a block leave
+// fewer reads of x. A block owns 32 rows of w (32 output channels): its 128 threads fetch them 64 k at a time with coalesced 16-byte loads into a double-buffered
 // shared-memory tile (the next tile is on its way while the current one is multiplied); then lane l of every warp
 // reads row l of the tile, and the block's four warps split the tokens. x is staged in shared memory 256 k at a
 // time and read from there by broadcast. Each output is the same ascending chain of fused multiply-adds as in the
 // tiled kernel above, so the two give the same bits.
 template <int TOK>  // tokens per thread; the block's 4 warps cover 4 * TOK tokens
 __global__ void __launch_bounds__(128)
-sgemm_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
-                 const float* __restrict__ residual, int N, int O, int K) {
+sgemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, float* y,
+                  const float* residual, int N, int O, int K) {
   constexpr int KC = 256, KS = 64, PITCH = KS + 4;  // rows of the tile 16-byte aligned and conflict-free to read
   __shared__ __align__(16) float xs[4 * TOK][KC];
   __shared__ __align__(16) float tile[2][32][PITCH];
@@ -134,7 +296,9 @@ sgemm_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float
     for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&tile[buffer][load_row + 8 * j][load_k]) = next[j];
   };
 
-  fetch(0);
+  chain_release();
+  fetch(0);  // weights: no kernel writes them
+  chain_wait();
   int buffer = 0;
   for (int k0 = 0; k0 < K; k0 += KC) {
     __syncthreads();  // the last chunk's x has been read
@@ -174,26 +338,118 @@ sgemm_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float
   }
 }
 
+// Operands whose rows do not start on 16 bytes (K no multiple of 4, or an odd base): tiles BM x BN x 16 through registers,
+// stored k-major, a thread a TM x TN part.
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+sgemm_any_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
+                 const float* __restrict__ residual, int N, int O, int K) {
+  constexpr int NT = (BM / TM) * (BN / TN);
+  __shared__ float As[kBK][BM + 4];
+  __shared__ float Bs[kBK][BN + 4];
+  const int tid = threadIdx.x;
+  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+  const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+
+  for (int k0 = 0; k0 < K; k0 += kBK) {
+    for (int i = tid; i < BM * kBK; i += NT) {
+      const int r = i / kBK, c = i % kBK;
+      As[c][r] = row0 + r < N && k0 + c < K ? x[(size_t)(row0 + r) * K + k0 + c] : 0.f;
+    }
+    for (int i = tid; i < BN * kBK; i += NT) {
+      const int r = i / kBK, c = i % kBK;
+      Bs[c][r] = col0 + r < O && k0 + c < K ? w[(size_t)(col0 + r) * K + k0 + c] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kBK; ++k) {
+      float a[TM], b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = As[k][ty * TM + i];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[j] = Bs[k][tx * TN + j];
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gr = row0 + ty * TM + i;
+    if (gr >= N) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int gc = col0 + tx * TN + j;
+      if (gc >= O) continue;
+      const size_t at = (size_t)gr * O + gc;
+      y[at] = residual ? residual[at] + acc[i][j] : acc[i][j];
+    }
+  }
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_tile(const float* x, const float* w, float* y, const float* residual, int N, int O, int K, cudaStream_t stream) {
+  constexpr int NT = (BM / (4 * TM)) * (BN / (8 * TN)) * 32;
+  return launch_chained(sgemm_tile_kernel<BM, BN, TM, TN>, dim3((O + BN - 1) / BN, (N + BM - 1) / BM), dim3(NT), 0, stream, x, w, y,
+                        residual, N, O, K);
+}
+
+template <int TOK, int STAGES>
+int launch_few(const float* x, const float* w, float* y, const float* residual, int N, int O, int K, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)STAGES * (kFewRows + 4 * TOK) * kFewPitch * sizeof(float);
+  static_assert(smem <= 227 * 1024, "the ring fits a block");
+  if (smem > 48 * 1024) {
+    static bool configured[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
+    if (!configured[device]) {
+      const cudaError_t e = cudaFuncSetAttribute(sgemm_few_kernel<TOK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return (int)e;
+      configured[device] = true;
+    }
+  }
+  return launch_chained(sgemm_few_kernel<TOK, STAGES>, dim3((O + kFewRows - 1) / kFewRows), dim3(32), smem, stream, x, w, y, residual, N, O, K);
+}
+
+}  // namespace
+
 // residual may alias y (in-place accumulation into the residual stream) or be null.
+//
+// Which kernel, from times on a B200 (us; the kernels before were 128 x 128 tiles from 65 rows on, 32 x 64 tiles from 17, and
+// sgemm_wide_kernel up to 16 rows):
+//   up to 4 rows, a warp per 8 rows of w: w of 1,024 x 4,608 18.5 (58.6 before), 9,216 x 1,024 16.2 (17.4), 65,536 x 1,024 72
+//     (79). Eight rows: 30.6 (67), 30 (21), 109 (89), so from 5 rows on a wide w stays with the kernel of 32 rows a block.
+//   64 x 64 tiles up to 511 rows: 1,024 x 1,024 with 128 rows 38 (185), 300 rows 39 (185); 9,216 x 1,024 with 300 rows 141 (276;
+//     128 x 64 tiles 147). Tiles of 128 x 64 from there on: 9,216 x 1,024 with 723 rows 281 (524; 64 x 64 tiles 322), with
+//     2,048 rows 732 (1,056): 53 TFLOP/s. Up to 32 rows against a wide w, 32 x 32 tiles: 16,384 x 2,048 135 (197; 64 x 64 181).
 AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* residual, int N, int O, int K,
                         cudaStream_t stream) {
   if (N <= 0 || O <= 0) return 0;
   if (K <= 0) return (int)cudaErrorInvalidValue;
-  const int vec_ok = (K % 4 == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0);
-  if (N <= 16 && vec_ok && O >= 256) {
-    const dim3 grid((O + 31) / 32);
-    if (N <= 4) sgemm_few_kernel<1><<<grid, 128, 0, stream>>>(x, w, y, residual, N, O, K);
-    else if (N <= 8) sgemm_few_kernel<2><<<grid, 128, 0, stream>>>(x, w, y, residual, N, O, K);
-    else sgemm_few_kernel<4><<<grid, 128, 0, stream>>>(x, w, y, residual, N, O, K);
-  } else if (N > 64) {
-    const dim3 grid((O + 127) / 128, (N + 127) / 128);
-    sgemm_tn_kernel<128, 128, 8, 8><<<grid, 256, 0, stream>>>(x, w, y, residual, N, O, K, vec_ok);
-  } else if (N > 16) {
-    const dim3 grid((O + 63) / 64, (N + 31) / 32);
-    sgemm_tn_kernel<32, 64, 2, 4><<<grid, 256, 0, stream>>>(x, w, y, residual, N, O, K, vec_ok);
-  } else {
-    const dim3 grid((O + 63) / 64, 1);
-    sgemm_tn_kernel<16, 64, 1, 4><<<grid, 256, 0, stream>>>(x, w, y, residual, N, O, K, vec_ok);
+  const bool rows_on_16_bytes = (K % 4 == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0);
+  if (!rows_on_16_bytes) {
+    sgemm_any_kernel<32, 64, 2, 4><<<dim3((O + 63) / 64, (N + 31) / 32), 256, 0, stream>>>(x, w, y, residual, N, O, K);
+    return launch_status();
   }
-  return launch_status();
+  const bool wide = O >= 8192;
+  if (N <= 4) return launch_few<1, 12>(x, w, y, residual, N, O, K, stream);
+  if (N <= 16 && wide) {
+    const dim3 grid((O + 31) / 32);
+    if (N <= 8) return launch_chained(sgemm_wide_kernel<2>, grid, dim3(128), 0, stream, x, w, y, residual, N, O, K);
+    return launch_chained(sgemm_wide_kernel<4>, grid, dim3(128), 0, stream, x, w, y, residual, N, O, K);
+  }
+  if (N <= 8) return launch_few<2, 4>(x, w, y, residual, N, O, K, stream);
+  if (N <= 16) return launch_few<4, 4>(x, w, y, residual, N, O, K, stream);
+  if (N <= 32 && wide) return launch_tile<32, 32, 8, 4>(x, w, y, residual, N, O, K, stream);
+  if (N < 512) return launch_tile<64, 64, 8, 4>(x, w, y, residual, N, O, K, stream);
+  return launch_tile<128, 64, 8, 8>(x, w, y, residual, N, O, K, stream);
 }

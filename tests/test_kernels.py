@@ -105,6 +105,20 @@ def test_linear_float32_rows_do_not_depend_on_the_batch(ops):
             assert torch.equal(cuda.linear(x[rows].contiguous(), w, residual=res[rows].clone()), added[rows])
 
 
+@pytest.mark.parametrize("k,o", [(68, 8200), (132, 257), (1024, 72), (16, 65)])
+def test_linear_float32_every_kernel_gives_the_same_bits(ops, k, o):
+    """Row counts on both sides of every line between the float32 product's kernels (4, 8, 16, 32, 511 rows; a wide w and a
+    narrow one; remainders of tiles and of stages), against the kernel for operands whose rows do not start on 16 bytes."""
+    cuda, _ = ops
+    x, w, res = _rand((600, k), torch.float32, 11), _rand((o, k), torch.float32, 12), _rand((600, o), torch.float32, 13)
+    odd = torch.empty(o * k + 1, device=w.device)[1:].view(o, k).copy_(w)  # off the 16-byte boundary: the general kernel
+    want, added = cuda.linear(x, odd), cuda.linear(x, odd, residual=res.clone())
+    _close(want, x.double() @ w.double().T, torch.float32, "product")
+    for n in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 511, 512, 600):
+        assert torch.equal(cuda.linear(x[:n], w), want[:n]), n
+        assert torch.equal(cuda.linear(x[:n], w, residual=res[:n].clone()), added[:n]), n
+
+
 @pytest.mark.parametrize("n,k,o", [(1, 64, 50), (17, 104, 37), (70, 56, 130), (300, 96, 192), (8, 2048, 321)])
 def test_linear_bfloat16(ops, n, k, o):
     cuda, ref = ops
