@@ -65,9 +65,7 @@ __global__ void decay_gates_kernel(const T* __restrict__ low, long long ld, cons
 //           pass silu on their way in (the mixer's activations, applied in float32).
 //   GATE:   s <- g_t[kk] s + (1 - g_t[kk]) v_t[j], o_t[j] = sum_kk s silu(q_t[kk]), with the forget gate of a key channel
 //           g = low + (1 - low) sigmoid(z + b) from its logit z (k's place) and b, low [H * D] (decay's and beta's place);
-//           1 - g is computed as (1 - low) sigmoid(-(z + b)), which keeps its digits where the gate is nearly open. PART 1:
-//           a chunk's walk from an empty state, which leaves the state and the products of the gates per key channel in
-//           scratch, no outputs; PART 2: a chunk's walk from the state that scratch holds for its start, outputs only.
+//           1 - g is computed as (1 - low) sigmoid(-(z + b)), which keeps its digits where the gate is nearly open.
 //   DELTA:  s <- g_t s; u = beta_t (v_t[j] - sum_kk s k_t[kk]); s <- s + k_t[kk] u; o_t[j] = sum_kk s q_t[kk]
 constexpr int kPad = 4;  // floats between the R-blocks of a shared row: neighbouring lanes' 16-byte reads miss each other's banks
 
@@ -96,15 +94,14 @@ __device__ __forceinline__ bool find_chunk(const int* __restrict__ cu_seqlens, c
 
 enum { RULE_GLA = 0, RULE_DELTA = 1, RULE_FIXED = 2, RULE_GATE = 3 };
 
-template <typename T, int R, int KS, int CH, int TH, int RULE, int PART = 0>
+template <typename T, int R, int KS, int CH, int TH, int RULE>
 __global__ void __launch_bounds__(TH)
 scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk, const T* __restrict__ v,
             long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; DELTA: g [N, H] */,
             const float* __restrict__ beta /* DELTA: [N, H] */, float* __restrict__ state, long long slot_stride,
             const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ out, int H, int rep,
-            int D, int V, float q_scale, int write, int act, float* __restrict__ scratch, float* __restrict__ gates, int requests) {
+            int D, int V, float q_scale, int write, int act) {
   constexpr bool DELTA = RULE == RULE_DELTA, FIXED = RULE == RULE_FIXED, GATE = RULE == RULE_GATE;
-  static_assert(PART == 0 || GATE, "only the forget gate's recurrence is walked in chunks");
   constexpr int VT = TH / KS;           // value channels of a block
   constexpr int ROW = KS * (R + kPad);  // floats of a padded shared row of key channels
   __shared__ __align__(16) float sq[CH][ROW];
@@ -114,16 +111,9 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   __shared__ float sg[CH], sb[CH];
 
   const int h = blockIdx.x;
-  int req = blockIdx.y, t_begin, t_end;
-  if (PART == 0) {
-    t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
-    if (slots[req] < 0 || t_end <= t_begin) return;
-  } else {
-    int len, index;
-    if (!find_chunk(cu_seqlens, slots, requests, blockIdx.y, req, t_begin, len, index)) return;
-    t_end = t_begin + len;
-  }
+  const int req = blockIdx.y, t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
   const int slot = slots[req];
+  if (slot < 0 || t_end <= t_begin) return;
   const int ks = threadIdx.x % KS, jl = threadIdx.x / KS;
   const int j = blockIdx.z * VT + jl;
   const bool live = j < V;
@@ -131,16 +121,11 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   const int kk0 = ks * R;
 
   float s[R];
-  float* srow = (PART == 0 ? state + (size_t)slot * slot_stride : scratch + (size_t)blockIdx.y * H * V * D) + ((size_t)h * V + (live ? j : 0)) * D;
-  const bool vec = D % 4 == 0 && (PART != 0 || slot_stride % 4 == 0) && (reinterpret_cast<uintptr_t>(PART == 0 ? state : scratch) & 15) == 0;
-  float kept[PART == 1 ? R : 1];  // the products of the gates so far
-#pragma unroll
-  for (int r = 0; r < (PART == 1 ? R : 1); ++r) kept[r] = 1.f;
+  float* srow = state + (size_t)slot * slot_stride + ((size_t)h * V + (live ? j : 0)) * D;
+  const bool vec = D % 4 == 0 && slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
 #pragma unroll
   for (int r = 0; r < R; r += 4) {
-    if (PART == 1) {
-      s[r] = s[r + 1] = s[r + 2] = s[r + 3] = 0.f;
-    } else if (live && vec && kk0 + r + 3 < D) {
+    if (live && vec && kk0 + r + 3 < D) {
       const float4 x = *reinterpret_cast<const float4*>(srow + kk0 + r);
       s[r] = x.x; s[r + 1] = x.y; s[r + 2] = x.z; s[r + 3] = x.w;
     } else {
@@ -164,7 +149,7 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
       const int t = i / (KS * R), kk = i % (KS * R);
       const bool in = t < count && kk < D;
       const size_t n = (size_t)(c0 + t);
-      if (PART != 1) rq[u] = in ? q[n * ldq + (size_t)hk * D + kk] : zero;
+      rq[u] = in ? q[n * ldq + (size_t)hk * D + kk] : zero;
       rk[u] = in ? k[n * ldk + (size_t)hk * D + kk] : zero;
       if (RULE == RULE_GLA) ra[u] = in ? decay[n * ((size_t)H * D) + (size_t)h * D + kk] : 0.f;
     }
@@ -189,7 +174,7 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
       if (i < CH * KS * R) {
         const int t = i / (KS * R), kk = i % (KS * R);
         const int at = kk + (kk / R) * kPad;
-        float qv = PART != 1 ? to_f32(rq[u]) : 0.f, kv = to_f32(rk[u]);
+        float qv = to_f32(rq[u]), kv = to_f32(rk[u]);
         if (FIXED && act) { qv *= sigmoid_f(qv); kv *= sigmoid_f(kv); }
         if (GATE) {
           const float low = kk < D ? beta[(size_t)h * D + kk] : 1.f, z = kk < D ? kv + decay[(size_t)h * D + kk] : 0.f;
@@ -197,7 +182,7 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
           kv = (1.f - low) * sigmoid_f(-z);
           sa[t][at] = fmaf(1.f - low, sigmoid_f(z), low);
         }
-        if (PART != 1) sq[t][at] = qv * q_scale;
+        sq[t][at] = qv * q_scale;
         sk[t][at] = kv;
         if (RULE == RULE_GLA) sa[t][at] = ra[u];
       }
@@ -259,28 +244,15 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
           const float4 av = *reinterpret_cast<const float4*>(ar + r);
           s[r] = fmaf(av.x, s[r], kv.x * vj); s[r + 1] = fmaf(av.y, s[r + 1], kv.y * vj);
           s[r + 2] = fmaf(av.z, s[r + 2], kv.z * vj); s[r + 3] = fmaf(av.w, s[r + 3], kv.w * vj);
-          if (PART == 1) {
-            if (threadIdx.x < 32 && blockIdx.z == 0) {  // one warp holds every key channel's product
-              kept[r] *= av.x; kept[r + 1] *= av.y; kept[r + 2] *= av.z; kept[r + 3] *= av.w;
-            }
-            continue;
-          }
           const float4 qv = *reinterpret_cast<const float4*>(qr + r);
           acc = fmaf(s[r], qv.x, acc); acc2 = fmaf(s[r + 1], qv.y, acc2); acc = fmaf(s[r + 2], qv.z, acc); acc2 = fmaf(s[r + 3], qv.w, acc2);
         }
       }
-      if (PART == 1) continue;
       acc = group_sum<KS>(acc + acc2);
       if (ks == 0 && live) out[(size_t)(c0 + t) * ((size_t)H * V) + (size_t)h * V + j] = acc;
     }
   }
-  if (PART == 1 && blockIdx.z == 0 && jl == 0) {
-    float* grow = gates + ((size_t)blockIdx.y * H + h) * D;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (kk0 + r < D) grow[kk0 + r] = kept[r];
-  }
-  if ((PART == 0 ? write != 0 : PART == 1) && live) {
+  if (write && live) {
 #pragma unroll
     for (int r = 0; r < R; r += 4) {
       if (vec && kk0 + r + 3 < D) {
@@ -294,14 +266,13 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   }
 }
 
-template <typename T, int RULE, int PART = 0>
+template <typename T, int RULE>
 int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v, long long ldv, const float* decay,
                 const float* beta, float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out,
                 int tokens, int requests, int H, int rep, int D, int V, float q_scale, int write, cudaStream_t stream,
-                int act = 0, float* scratch = nullptr, float* gates = nullptr, int chunks = 0) {
+                int act = 0) {
   if (requests <= 0 || H <= 0) return 0;
-  const int walks = PART == 0 ? requests : chunks;  // what the blocks of one head and tile of value channels walk each
-  if (walks > 65535) return (int)cudaErrorInvalidValue;
+  if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (D > 1024) return (int)cudaErrorInvalidValue;
   // (Blocks of 64 threads, which spread a head's value channels over four times as many SMs when a step holds few
   // long portions, were measured and dropped: a token's cost is the latency of its chain of shared-memory reads, sums
@@ -309,17 +280,15 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
   (void)tokens;
 #define AKAS_SCAN(R, KS, CH)                                                                                              \
   {                                                                                                                       \
-    const dim3 grid(H, walks, (V + 256 / KS - 1) / (256 / KS));                                                           \
-    return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE, PART>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
-                          decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act,     \
-                          scratch, gates, requests);                                                                      \
+    const dim3 grid(H, requests, (V + 256 / KS - 1) / (256 / KS));                                                           \
+    return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
+                          decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act);       \
   }
   if (D <= 8) AKAS_SCAN(8, 1, 16)
   if (D <= 16) AKAS_SCAN(8, 2, 16)
   if (D <= 32) AKAS_SCAN(8, 4, 16)
   if (D <= 64) AKAS_SCAN(16, 4, 16)
   if (D <= 128) AKAS_SCAN(16, 8, 16)
-  if (PART != 0) return (int)cudaErrorInvalidValue;  // (the caller walks larger keys token by token)
   if (D <= 256) AKAS_SCAN(16, 16, 8)
   if (D <= 512) AKAS_SCAN(16, 32, 4)
   AKAS_SCAN(32, 32, 2)
@@ -576,13 +545,223 @@ int launch_chunks(const T* q, long long ldq, const T* k, long long ldk, const T*
                          cu_seqlens, slots, (const float*)scratch, out, requests, H, D, V, DP, q_scale, act);
 }
 
-// ------------------------------------------------------------------------------------------------ forget gates, in chunks
+// ------------------------------------------------------------------------------------------------ gates per key channel, in chunks
 //
-// The recurrence whose forget gate also writes, for prompt portions: every chunk of kChunk tokens is walked from an empty
-// state at once (scan_kernel, PART 1), gate_carry puts the chunks' ends together, S_(j+1) = diag(product of chunk j's
-// gates) S_j + U_j, leaving every chunk's start where its end stood and the last one in the slot, and every chunk is
-// walked again from its start (PART 2), for its outputs. No quotient of gate products is ever formed, so gates near zero
-// cost no digits; a result differs from the walk token by token, and between ways of cutting a prompt, by rounding only.
+// The recurrences with a decay per key channel (gated linear attention, and the forget gate that also writes), for prompt
+// portions: every chunk of kChunk tokens is walked from an empty state at once (PART 1: the state it ends with and the
+// products of the gates per key channel go to scratch, no outputs), gate_carry puts the chunks' ends together, S_(j+1) =
+// diag(product of chunk j's gates) S_j + U_j, leaving every chunk's start where its end stood and the last one in the
+// slot, and every chunk is walked again from its start (PART 2), for its outputs. No quotient of gate products is ever
+// formed, so gates near zero cost no digits; a result differs from the walk token by token, and between ways of cutting a
+// prompt, by rounding only.
+//
+// A walk is three multiply-adds per state element and token (two in PART 1), so the FFMA rate is what bounds it as long as
+// shared memory keeps up: a thread owns 16 key channels of FOUR value channels, 64 elements of state, and reads a token's
+// q, k and gate of its key channels once for all four. KS neighbouring lanes hold a value channel's D key channels and
+// exchange halves of their four sums until each holds one (the order of the additions is that of scan_kernel). A block's
+// 128 threads cover 512 / KS value channels of one (head, chunk).
+constexpr int kWalkThreads = 128, kWalkR = 16, kWalkNV = 4, kWalkTokens = 16;
+
+// Four neighbouring elements as they are in memory; `live` of them exist, the others are zero. Where the rows do not start
+// on four elements (`vec` false) they are fetched one by one.
+template <typename T> struct Four;
+template <> struct Four<float> {
+  float4 raw;
+  __device__ __forceinline__ void fetch(const float* p, int live, bool vec) {
+    if (vec && live >= 4) { raw = *reinterpret_cast<const float4*>(p); return; }
+    raw.x = live > 0 ? p[0] : 0.f; raw.y = live > 1 ? p[1] : 0.f; raw.z = live > 2 ? p[2] : 0.f; raw.w = live > 3 ? p[3] : 0.f;
+  }
+  __device__ __forceinline__ void widen(float (&v)[4]) const { v[0] = raw.x; v[1] = raw.y; v[2] = raw.z; v[3] = raw.w; }
+};
+template <> struct Four<bf16> {
+  uint2 raw;
+  __device__ __forceinline__ void fetch(const bf16* p, int live, bool vec) {
+    if (vec && live >= 4) { raw = *reinterpret_cast<const uint2*>(p); return; }
+    const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+    raw.x = (live > 0 ? u[0] : 0u) | (live > 1 ? (uint32_t)u[1] << 16 : 0u);
+    raw.y = (live > 2 ? u[2] : 0u) | (live > 3 ? (uint32_t)u[3] << 16 : 0u);
+  }
+  __device__ __forceinline__ void widen(float (&v)[4]) const {
+    v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xffff0000u);
+    v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xffff0000u);
+  }
+};
+
+template <typename T, int KS, int RULE, int PART>
+__global__ void __launch_bounds__(kWalkThreads)
+walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk, const T* __restrict__ v,
+                  long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; GATE: the logits' bias [H * D] */,
+                  const float* __restrict__ low /* GATE: the gates' lower bounds [H * D] */, const int* __restrict__ cu_seqlens,
+                  const int* __restrict__ slots, float* __restrict__ out, int H, int D, int V, float q_scale,
+                  float* __restrict__ scratch, float* __restrict__ gates, int requests, int vec) {
+  static_assert(RULE == RULE_GLA || RULE == RULE_GATE, "a decay per key channel");
+  constexpr int R = kWalkR, NV = kWalkNV, CH = kWalkTokens, TH = kWalkThreads;
+  constexpr int VT = TH / KS * NV, W = KS * R, ROW = KS * (R + kPad);
+  constexpr int NQ = (CH * W / 4 + TH - 1) / TH, NVL = CH * VT / 4 / TH;
+  __shared__ __align__(16) float sq[PART == 1 ? 1 : CH][ROW];
+  __shared__ __align__(16) float sk[CH][ROW];
+  __shared__ __align__(16) float sa[CH][ROW];
+  __shared__ __align__(16) float sv[CH][VT];
+
+  const int h = blockIdx.x;
+  int req, t_begin, len, index;
+  if (!find_chunk(cu_seqlens, slots, requests, blockIdx.y, req, t_begin, len, index)) return;
+  const int t_end = t_begin + len;
+  const int ks = threadIdx.x % KS, jl = threadIdx.x / KS, kk0 = ks * R;
+  const int v0 = blockIdx.z * VT, j0 = v0 + jl * NV;
+
+  // the state: rows of D key channels per value channel, in scratch
+  float s[NV][R];
+  float* srow = scratch + (((size_t)blockIdx.y * H + h) * V + j0) * D + kk0;
+  const bool whole = D % 4 == 0 && ((uintptr_t)scratch & 15) == 0;
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+#pragma unroll
+    for (int r = 0; r < R; r += 4) {
+      Four<float> x;
+      x.fetch(srow + (size_t)n * D + r, PART == 2 && j0 + n < V ? D - kk0 - r : 0, whole);
+      x.widen(reinterpret_cast<float(&)[4]>(s[n][r]));
+    }
+  float kept[PART == 1 ? R : 1];  // PART 1: the products of the gates so far (in one warp of the first tile)
+  const bool keeps = PART == 1 && threadIdx.x < 32 && blockIdx.z == 0;
+#pragma unroll
+  for (int r = 0; r < (PART == 1 ? R : 1); ++r) kept[r] = 1.f;
+
+  // the next tokens' inputs are on their way to registers while the tokens in shared memory are walked
+  Four<T> rq[PART == 1 ? 1 : NQ], rk[NQ], rv[NVL];
+  Four<float> ra[RULE == RULE_GLA ? NQ : 1];
+  auto fetch = [&](int c0) {
+    const int count = min(CH, t_end - c0);
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      const int i = threadIdx.x + u * TH, t = i / (W / 4), kk = (i % (W / 4)) * 4;
+      const int live = t < count ? D - kk : 0;
+      const size_t n = (size_t)(c0 + (t < count ? t : 0)), at = (size_t)h * D + (live > 0 ? kk : 0);
+      if (PART != 1) rq[u].fetch(q + n * ldq + at, live, vec);
+      rk[u].fetch(k + n * ldk + at, live, vec);
+      if (RULE == RULE_GLA) ra[u].fetch(decay + n * ((size_t)H * D) + at, live, vec);
+    }
+#pragma unroll
+    for (int u = 0; u < NVL; ++u) {
+      const int i = threadIdx.x + u * TH, t = i / (VT / 4), c = v0 + (i % (VT / 4)) * 4;
+      const int live = t < count ? V - c : 0;
+      rv[u].fetch(v + (size_t)(c0 + (t < count ? t : 0)) * ldv + (size_t)h * V + (live > 0 ? c : 0), live, vec);
+    }
+  };
+  fetch(t_begin);
+  for (int c0 = t_begin; c0 < t_end; c0 += CH) {
+    const int count = min(CH, t_end - c0);
+    __syncthreads();  // the tokens before have been read
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      const int i = threadIdx.x + u * TH, t = i / (W / 4), kk = (i % (W / 4)) * 4;
+      if (i >= CH * W / 4) continue;
+      const int at = kk + (kk / R) * kPad;
+      float kv[4], qv[4], av[4];
+      rk[u].widen(kv);
+      if (PART != 1) rq[u].widen(qv);
+      if (RULE == RULE_GLA) {
+        ra[u].widen(av);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool in = kk + e < D;
+          const float lo = in ? low[(size_t)h * D + kk + e] : 1.f, z = in ? kv[e] + decay[(size_t)h * D + kk + e] : 0.f;
+          if (PART != 1) qv[e] *= sigmoid_f(qv[e]);
+          kv[e] = (1.f - lo) * sigmoid_f(-z);
+          av[e] = fmaf(1.f - lo, sigmoid_f(z), lo);
+        }
+      }
+      if (PART != 1) *reinterpret_cast<float4*>(&sq[t][at]) = make_float4(qv[0] * q_scale, qv[1] * q_scale, qv[2] * q_scale, qv[3] * q_scale);
+      *reinterpret_cast<float4*>(&sk[t][at]) = make_float4(kv[0], kv[1], kv[2], kv[3]);
+      *reinterpret_cast<float4*>(&sa[t][at]) = make_float4(av[0], av[1], av[2], av[3]);
+    }
+#pragma unroll
+    for (int u = 0; u < NVL; ++u) {
+      const int i = threadIdx.x + u * TH;
+      float vv[4];
+      rv[u].widen(vv);
+      *reinterpret_cast<float4*>(&sv[i / (VT / 4)][(i % (VT / 4)) * 4]) = make_float4(vv[0], vv[1], vv[2], vv[3]);
+    }
+    __syncthreads();
+    if (c0 + CH < t_end) fetch(c0 + CH);
+    for (int t = 0; t < count; ++t) {
+      const float* kr = &sk[t][ks * (R + kPad)];
+      const float* ar = &sa[t][ks * (R + kPad)];
+      const float* qr = PART == 1 ? kr : &sq[t][ks * (R + kPad)];
+      const float4 v4 = *reinterpret_cast<const float4*>(&sv[t][jl * NV]);
+      const float vj[NV] = {v4.x, v4.y, v4.z, v4.w};
+      float acc[2][NV] = {};
+#pragma unroll
+      for (int r = 0; r < R; r += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(kr + r), a4 = *reinterpret_cast<const float4*>(ar + r);
+        const float4 q4 = *reinterpret_cast<const float4*>(qr + r);
+        const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, aa[4] = {a4.x, a4.y, a4.z, a4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+          for (int n = 0; n < NV; ++n) {
+            s[n][r + e] = fmaf(aa[e], s[n][r + e], kk[e] * vj[n]);
+            if (PART != 1) acc[e & 1][n] = fmaf(s[n][r + e], qq[e], acc[e & 1][n]);
+          }
+          if (keeps) kept[r + e] *= aa[e];
+        }
+      }
+      if (PART == 1) continue;
+      float o[NV];
+#pragma unroll
+      for (int n = 0; n < NV; ++n) o[n] = acc[0][n] + acc[1][n];
+      int left = NV, first = 0;  // the lane holds the sums of channels first .. first + left - 1 of its four
+      if constexpr (KS > 1)
+#pragma unroll
+      for (int off = KS / 2; off > 0; off >>= 1) {
+        if (left > 1) {
+          const bool upper = (ks & off) != 0;
+#pragma unroll
+          for (int i = 0; i < NV / 2; ++i) {
+            if (i < left / 2) {
+              const float send = upper ? o[i] : o[i + left / 2], mine = upper ? o[i + left / 2] : o[i];
+              o[i] = mine + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+          }
+          first += upper ? left / 2 : 0;
+          left /= 2;
+        } else {
+          o[0] += __shfl_xor_sync(0xffffffffu, o[0], off);
+        }
+      }
+      if (KS <= NV || ks % (KS / NV > 0 ? KS / NV : 1) == 0) {
+        float* dst = out + (size_t)(c0 + t) * ((size_t)H * V) + (size_t)h * V + j0 + first;
+#pragma unroll
+        for (int i = 0; i < (KS >= NV ? 1 : NV / KS); ++i)
+          if (j0 + first + i < V) dst[i] = o[i];
+      }
+    }
+  }
+  if (PART == 1) {
+    if (blockIdx.z == 0 && jl == 0) {
+      float* grow = gates + ((size_t)blockIdx.y * H + h) * D;
+#pragma unroll
+      for (int r = 0; r < (PART == 1 ? R : 1); ++r)
+        if (kk0 + r < D) grow[kk0 + r] = kept[r];
+    }
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      if (j0 + n >= V) continue;
+#pragma unroll
+      for (int r = 0; r < R; r += 4) {
+        if (whole && kk0 + r + 3 < D) {
+          *reinterpret_cast<float4*>(srow + (size_t)n * D + r) = make_float4(s[n][r], s[n][r + 1], s[n][r + 2], s[n][r + 3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (kk0 + r + e < D) srow[(size_t)n * D + r + e] = s[n][r + e];
+        }
+      }
+    }
+  }
+}
+
 __global__ void gate_carry_kernel(const float* __restrict__ gates, float* __restrict__ state, long long slot_stride,
                                   const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ scratch,
                                   int H, int D, int V, int write) {
@@ -613,6 +792,30 @@ __global__ void gate_carry_kernel(const float* __restrict__ gates, float* __rest
     }
     if (write && chunks > 0) srow[i] = s;
   }
+}
+
+template <typename T, int RULE>
+int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* v, long long ldv, const float* decay, const float* low,
+                 float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out, float* scratch, int tokens,
+                 int requests, int H, int D, int V, float q_scale, int write, cudaStream_t stream) {
+  const int chunks = (tokens + kChunk - 1) / kChunk + requests;  // at most: every request may end with a part of a chunk
+  float* gates = scratch + (size_t)chunks * H * D * V;
+  const size_t four = 4 * sizeof(T);
+  const int vec = D % 4 == 0 && V % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && (uintptr_t)q % four == 0 &&
+                  (uintptr_t)k % four == 0 && (uintptr_t)v % four == 0 && (RULE != RULE_GLA || (uintptr_t)decay % 16 == 0);
+#define AKAS_WALK(KS, PART)                                                                                                  \
+  launch_ordinary(walk_chunk_kernel<T, KS, RULE, PART>, dim3(H, chunks, (V + kWalkThreads / KS * kWalkNV - 1) / (kWalkThreads / KS * kWalkNV)), \
+                  dim3(kWalkThreads), 0, stream, q, ldq, k, ldk, v, ldv, decay, low, cu_seqlens, slots, out, H, D, V, q_scale,   \
+                  scratch, gates, requests, vec)
+#define AKAS_WALKS(PART) (D <= 16 ? AKAS_WALK(1, PART) : D <= 32 ? AKAS_WALK(2, PART) : D <= 64 ? AKAS_WALK(4, PART) : AKAS_WALK(8, PART))
+  int err = AKAS_WALKS(1);
+  if (err) return err;
+  err = launch_ordinary(gate_carry_kernel, dim3(requests, H, min(64, (V * D + 255) / 256)), dim3(256), 0, stream, (const float*)gates,
+                        state, slot_stride, cu_seqlens, slots, scratch, H, D, V, write);
+  if (err) return err;
+  return AKAS_WALKS(2);
+#undef AKAS_WALKS
+#undef AKAS_WALK
 }
 
 // ------------------------------------------------------------------------------------------------ causal convolution
@@ -888,7 +1091,7 @@ AKAS_API int akas_gate_scan(const float* q, long long ldq, const float* f, long 
                                        requests, H, 1, D, V, 1.f, write, stream);
 }
 
-// Floats of scratch that akas_gate_scan_chunked needs; 0 where it does not take the sizes (the token-by-token kernel does).
+// Floats of scratch that akas_gate_scan_chunked and akas_gla_scan_chunked need; 0 where it does not take the sizes (the token-by-token kernel does).
 AKAS_API long long akas_gate_chunk_scratch(int tokens, int requests, int H, int D, int V) {
   const long long chunks = (tokens + kChunk - 1) / kChunk + requests;
   if (D > kChunkMaxD || tokens <= 0 || requests <= 0 || chunks > 65535) return 0;
@@ -901,16 +1104,22 @@ AKAS_API int akas_gate_scan_chunked(const float* q, long long ldq, const float* 
                                     int H, int D, int V, int write, cudaStream_t stream) {
   if (tokens <= 0 || requests <= 0 || H <= 0) return 0;
   if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr) return (int)cudaErrorInvalidValue;
-  const int chunks = (tokens + kChunk - 1) / kChunk + requests;  // at most: every request may end with a part of a chunk
-  float* gates = scratch + (size_t)chunks * H * D * V;
-  int err = launch_scan<float, RULE_GATE, 1>(q, ldq, f, ldf, v, ldv, f_bias, lower, state, slot_stride, cu_seqlens, slots, out, tokens,
-                                             requests, H, 1, D, V, 1.f, 1, stream, 0, scratch, gates, chunks);
-  if (err) return err;
-  err = launch_ordinary(gate_carry_kernel, dim3(requests, H, min(64, (V * D + 255) / 256)), dim3(256), 0, stream, (const float*)gates,
-                        state, slot_stride, cu_seqlens, slots, scratch, H, D, V, write);
-  if (err) return err;
-  return launch_scan<float, RULE_GATE, 2>(q, ldq, f, ldf, v, ldv, f_bias, lower, state, slot_stride, cu_seqlens, slots, out, tokens,
-                                          requests, H, 1, D, V, 1.f, 0, stream, 0, scratch, gates, chunks);
+  return launch_walks<float, RULE_GATE>(q, ldq, f, ldf, v, ldv, f_bias, lower, state, slot_stride, cu_seqlens, slots, out, scratch,
+                                        tokens, requests, H, D, V, 1.f, write, stream);
+}
+
+// The gated linear attention of akas_gla_scan in chunks; scratch as for akas_gate_scan_chunked.
+AKAS_API int akas_gla_scan_chunked(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
+                                   const float* alpha, float* state, long long slot_stride, const int* cu_seqlens, const int* slots,
+                                   float* out, float* scratch, int tokens, int requests, int H, int D, int V, float q_scale, int write,
+                                   int dtype, cudaStream_t stream) {
+  if (tokens <= 0 || requests <= 0 || H <= 0) return 0;
+  if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr) return (int)cudaErrorInvalidValue;
+  if (dtype == AKAS_F32)
+    return launch_walks<float, RULE_GLA>((const float*)q, ldq, (const float*)k, ldk, (const float*)v, ldv, alpha, nullptr, state,
+                                         slot_stride, cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, write, stream);
+  return launch_walks<bf16, RULE_GLA>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state, slot_stride,
+                                      cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, write, stream);
 }
 
 AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv,

@@ -71,6 +71,8 @@ _SIGNATURES = {
         "akas_decay_gates": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "akas_gla_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
+        "akas_gla_scan_chunked": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
+                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
         "akas_delta_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_causal_conv_silu": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
@@ -1495,16 +1497,24 @@ def decay_gates(low, w_up, bias, tau):
 
 
 @_flushes
-def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True):
+def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True, longest=None):
+    """In chunks (three kernels, see csrc/recurrent.cu) when some request of the step brings at least _GATE_CHUNKED_FROM
+    tokens (``longest``) and the key size allows, token by token otherwise."""
     n = q.shape[0]
     if q.dtype != k.dtype or q.dtype != v.dtype or alpha.dtype != torch.float32 or not alpha.is_contiguous():
         raise ValueError("gla_scan takes q, k, v of one dtype and a dense float32 alpha")
     (qp, ldq), (kp, ldk), (vp, ldv) = _rows(q, "q"), _rows(k, "k"), _rows(v, "v")
     sp, stride = _slot_rows(state, "state")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
-    _check(_fn("recurrent", "akas_gla_scan")(qp, ldq, kp, ldk, vp, ldv, _ptr(alpha), sp, stride, _ptr(cu_seqlens), _ptr(slots),
-                                            _ptr(out), n, slots.numel(), heads, dim, vdim, float(q_scale), int(bool(write)),
-                                            _code(q), _stream()), "gla_scan")
+    head = (qp, ldq, kp, ldk, vp, ldv, _ptr(alpha), sp, stride, _ptr(cu_seqlens), _ptr(slots), _ptr(out))
+    tail = (n, slots.numel(), heads, dim, vdim, float(q_scale), int(bool(write)), _code(q), _stream())
+    if decay_scan_kernels == "auto" and longest is not None and longest >= _GATE_CHUNKED_FROM:
+        words = int(_fn("recurrent", "akas_gate_chunk_scratch")(n, slots.numel(), heads, dim, vdim))
+        if words:
+            scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+            _check(_fn("recurrent", "akas_gla_scan_chunked")(*head, _ptr(scratch), *tail), "gla_scan (chunks)", kernels=3)
+            return out
+    _check(_fn("recurrent", "akas_gla_scan")(*head, *tail), "gla_scan")
     return out
 
 

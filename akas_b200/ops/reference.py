@@ -339,7 +339,7 @@ def _requests(cu_seqlens, slots):
             yield slot, cu[r], cu[r + 1]
 
 
-def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True):
+def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True, longest=None):
     """Per request and head, token by token: S <- diag(alpha_t) S + k_t v_t^T; o_t = S^T (q_scale q_t).
     q, k, alpha [N, heads * dim], v [N, heads * vdim] -> o float32 [N, heads * vdim]."""
     n = q.shape[0]

@@ -85,7 +85,7 @@ class GatedLinearAttention(Mixer):
         low = proj[:, 2 * hd + 2 * hv : 2 * hd + 2 * hv + self.rank]
         alpha = ops.decay_gates(low, self.w_up, self.b_up, s.tau)
         o = ops.gla_scan(q, k, v, alpha, cache.state, ctx.cu_seqlens, ctx.slots, s.num_heads, s.key_dim, s.value_dim,
-                         s.key_dim ** -0.5, write=write)
+                         s.key_dim ** -0.5, write=write, longest=getattr(ctx, "max_query_len", None))
         y = ops.gated_rmsnorm(o, self.norm, s.norm_eps, gate, s.num_heads, s.value_dim, self.rt.dtype)
         return project(self.rt, y, self.w_out, residual=residual)
 

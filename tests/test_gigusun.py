@@ -288,6 +288,34 @@ def test_gla_scan_kernel(heads, dim, vdim, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim,vdim,pad", [(3, 20, 24, 3), (2, 72, 136, 0), (1, 8, 5, 3), (2, 128, 66, 4), (2, 64, 128, 0), (1, 16, 520, 0)])
+def test_gla_scan_in_chunks(heads, dim, vdim, pad, dtype):
+    """Portions around the edges of a chunk (64 tokens), rows that start on four elements and rows that do not, gates from
+    nearly closed to nearly open. The bounds are the token-by-token kernel's: both sum in float32, at most 300 tokens."""
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(heads * 1000 + dim)
+    lengths, slots = [300, 1, 0, 64, 65, 129], [2, 0, -1, 3, 1, 4]
+    n = sum(lengths)
+    proj = (torch.randn(n, 2 * heads * dim + heads * vdim + pad, generator=g) * 0.5).to(dtype).cuda()
+    q, k, v = proj[:, : heads * dim], proj[:, heads * dim : 2 * heads * dim], proj[:, 2 * heads * dim : 2 * heads * dim + heads * vdim]
+    alpha = torch.sigmoid(torch.randn(n, heads * dim, generator=g) * 4 + 3)
+    alpha[torch.rand(n, heads * dim, generator=g) < 0.01] = 0.0  # a gate that closes altogether
+    alpha = alpha.cuda()
+    state = (torch.randn(5, heads, vdim, dim, generator=g) * 0.3).cuda()
+    cu, _, sl = _batch(lengths, slots, "cuda")
+    for write in (True, False):
+        s_ref, s_got = state.clone(), state.clone()
+        want = reference.gla_scan(q, k, v, alpha, s_ref, cu, sl, heads, dim, vdim, dim ** -0.5, write=write)
+        got = cuda.gla_scan(q, k, v, alpha, s_got, cu, sl, heads, dim, vdim, dim ** -0.5, write=write, longest=300)
+        _close(got, want, 2e-5, "gla o")
+        _close(s_got, s_ref, 2e-5, "gla state")
+        assert write or torch.equal(s_got, state)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 4, 16, 12), (6, 2, 40, 20), (2, 1, 136, 72), (1, 1, 7, 3), (2, 2, 300, 33)])
 def test_delta_scan_kernel(heads, kv_heads, dim, vdim):
     from akas_b200.ops import cuda, reference
