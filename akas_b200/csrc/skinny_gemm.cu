@@ -652,9 +652,10 @@ struct SplitPlan {
   int ksplit, grid, smem;
 };
 
+// How a product is cut; not 0 where no cut fits (the whole K, or a part of it, does not fit a block's shared memory, or a
+// cluster would take more row tiles than it has room for).
 template <int NT, int IN, int OUTM>
-int launch_one(int num_tiles, const void* x, const int* rows, const float* norm_w, float eps, int zero_centered,
-               const void* W, void* y, int M, int O, int K, const ConvTail& tail, int groups, cudaStream_t stream) {
+int plan_for(SplitPlan& plan, int num_tiles, int K, int groups) {
   auto kernel = groups > 1 ? skinny_gemm_kernel<NT, IN, OUTM, true> : skinny_gemm_kernel<NT, IN, OUTM, false>;
   constexpr bool UNCUT = OUTM == OUT_SWIGLU || OUTM == OUT_CONV;  // read-outs that need a tile's whole K in one block
   if (block_smem<NT, OUTM>(K, 1) > kMaxSmemBytes && (UNCUT || block_smem<NT, OUTM>(K, MAX_KSPLIT) > kMaxSmemBytes))
@@ -665,7 +666,6 @@ int launch_one(int num_tiles, const void* x, const int* rows, const float* norm_
   static std::map<std::tuple<int, int, int>, int> cluster_room;  // (device, ksplit, smem) -> clusters resident at once
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
-  SplitPlan plan;
   {
     std::lock_guard<std::mutex> lock(mutex);
     if (sms_of[device] == 0) {
@@ -741,6 +741,17 @@ int launch_one(int num_tiles, const void* x, const int* rows, const float* norm_
       plan = found->second;
     }
   }
+  return 0;
+}
+
+template <int NT, int IN, int OUTM>
+int launch_one(int num_tiles, const void* x, const int* rows, const float* norm_w, float eps, int zero_centered,
+               const void* W, void* y, int M, int O, int K, const ConvTail& tail, int groups, cudaStream_t stream) {
+  auto kernel = groups > 1 ? skinny_gemm_kernel<NT, IN, OUTM, true> : skinny_gemm_kernel<NT, IN, OUTM, false>;
+  constexpr bool UNCUT = OUTM == OUT_SWIGLU || OUTM == OUT_CONV;
+  SplitPlan plan;
+  const int planned = plan_for<NT, IN, OUTM>(plan, num_tiles, K, groups);
+  if (planned) return planned;
   CUtensorMap map;
   const int err = weight_map(&map, W, O, K, UNCUT ? 8 : 16);
   if (err) return err;
@@ -817,6 +828,20 @@ static int skinny_dispatch(const void* x, const int* rows, const float* norm_w, 
   }
   if (in_mode == IN_BF16) return launch_out<2, IN_BF16>(out_mode, x, rows, norm_w, eps, zero_centered, W, y, M, O, K, tail, 1, stream);
   return launch_out<2, IN_NORM>(out_mode, x, rows, norm_w, eps, zero_centered, W, y, M, O, K, tail, 1, stream);
+}
+
+// Whether akas_skinny_gemm takes a bfloat16 x of M rows against [O, K] with a bfloat16, float32 or accumulating read-out: an
+// inner size whose activations do not fit a block's shared memory whole still runs where it can be cut into parts that do.
+AKAS_API int akas_skinny_gemm_takes(int M, int O, int K, int out_mode) {
+  if (M <= 0 || M > 16 || O <= 0 || K <= 0 || K % 64) return 0;
+  const int groups = M <= 8 ? 1 : 2, tiles = (O + 15) / 16;
+  SplitPlan plan;
+  switch (out_mode) {
+    case OUT_BF16: return plan_for<1, IN_BF16, OUT_BF16>(plan, tiles, K, groups) == 0;
+    case OUT_F32: return plan_for<1, IN_BF16, OUT_F32>(plan, tiles, K, groups) == 0;
+    case OUT_ACC: return plan_for<1, IN_BF16, OUT_ACC>(plan, tiles, K, groups) == 0;
+    default: return 0;
+  }
 }
 
 AKAS_API int akas_skinny_gemm(const void* x, const int* rows, const float* norm_w, float eps, int zero_centered,

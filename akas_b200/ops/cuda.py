@@ -206,6 +206,7 @@ _SIGNATURES = {
     "decode_chain": {
         "akas_chain_set_scratch": [c_void_p],
         "akas_chain_scratch_words": [],
+        "akas_skinny_gemm_takes": [c_int, c_int, c_int, c_int],
         "akas_chain_begin": [],
         "akas_chain_count": [],
         "akas_chain_takes": [c_int] * 5,
@@ -650,7 +651,7 @@ def linear(x, w, out_dtype=None, residual=None, bias=None):
         out = residual if residual is not None else torch.empty((n, o), dtype=target, device=x.device)
         _stream_product(x, None, None, 0.0, False, False, w, out, n, o, k, mode)
         return out
-    if _skinny_fits(n, k):
+    if _skinny_takes(n, o, k, mode):
         out = residual if residual is not None else torch.empty((n, o), dtype=target, device=x.device)
         _skinny(x, None, None, 0.0, False, w, out, n, o, k, 0, mode)
         return out
@@ -841,7 +842,17 @@ _SKINNY_ROWS = 16
 # Which kernels run the products of more than 16 tokens (prompt portions, mixed steps, large decode batches). "own"
 # (default; "auto" and "tcgen05" mean the same): the hand-written tcgen05 kernels everywhere: the kernel for pairs of
 # SMs (gemm_pair.cu, TMA-written read-outs) for every product whose output rows TMA can write, the one-block kernel
+def _skinny_takes(m: int, o: int, k: int, mode: int) -> bool:
+    """The same for a product without a norm in front and without a gated read-out, which may also be cut along K when
+    its activations do not fit a block whole."""
+    if _skinny_fits(m, k):
+        return True
+    return (decode_products == "skinny" and m <= _SKINNY_CUT_ROWS and k % 64 == 0
+            and bool(_fn("skinny_gemm", "akas_skinny_gemm_takes")(m, o, k, mode)))
+
+
 # (gemm_tcgen05.cu, masked read-outs) for the rest. "library": cuBLASLt everywhere, with SwiGLU as a kernel of its
+_SKINNY_CUT_ROWS = 8  # 2,048 x 12,288: 13.2 us against 17.0 of the weight-streaming kernel; 9 to 16 tokens, in two groups: 21.7
 # own: the arm that the hand-written kernels are measured against.
 products = os.environ.get("AKAS_B200_PRODUCTS", "own")
 if products not in ("own", "auto", "tcgen05", "library"):

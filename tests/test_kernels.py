@@ -133,6 +133,21 @@ def test_linear_bfloat16(ops, n, k, o):
     _close(cuda.linear(x, w, out_dtype=torch.float32), x.double() @ w.double().T, torch.float32, "padded inner size")
 
 
+@pytest.mark.parametrize("m,k,o", [(1, 12288, 2048), (8, 12288, 2040), (5, 10368, 1536), (8, 16384, 48), (3, 10240, 4096)])
+def test_skinny_products_of_a_long_inner_size(ops, m, k, o):
+    """Activations that do not fit a block whole: the product is cut along K. Float32 sums in another order than one block's
+    (the bound of the other kernels' float32 read-outs, over k terms)."""
+    cuda, _ = ops
+    x, w = _rand((m, k), torch.bfloat16, 31), _rand((o, k), torch.bfloat16, 32)
+    assert not cuda._skinny_fits(m, k) and cuda._skinny_takes(m, o, k, cuda._OUT_F32)
+    want = x.double() @ w.double().T
+    _close(cuda.linear(x, w), want, torch.bfloat16, "bf16 out")
+    _close(cuda.linear(x, w, out_dtype=torch.float32), want, torch.float32, "f32 out", k)
+    res = _rand((m, o), torch.float32, 33)
+    _close(cuda.linear(x, w, residual=res.clone()), res.double() + want, torch.float32, "accumulate", k)
+    assert cuda.skinny_status() == 0
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("k,o", [(64, 50), (192, 320), (2048, 37), (8192, 64), (96, 40)])
 def test_skinny_products_for_few_tokens(ops, m, k, o, monkeypatch):
