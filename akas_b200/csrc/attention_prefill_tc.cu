@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(THREADS, 2)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                             int max_blocks, const int* __restrict__ cu_seqlens, const int* __restrict__ positions,
-                            bf16* __restrict__ out, float scale, int window, int page_size, int H, int KH, int R) {
+                            bf16* __restrict__ out, float scale, int window, int page_size, int H, int KH, int R,
+                            const float* __restrict__ sinks, int unit_sink, float out_scale, long long ldo) {
   // The block has no static shared memory, so the dynamic array starts the block's window, 1024-byte aligned (the
   // swizzled tiles need that; it is checked below): with no bytes lost to alignment, two blocks fit an SM.
   chain_release();  // a kernel after this one that was launched as its programmatic dependent may set itself up meanwhile
@@ -435,8 +436,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     meet();
     l_run += sums[(half ^ 1) * 128 + row];
     if (row < rows && !*(volatile int*)&abort_s) {
-      const float inv = 1.f / l_run;
-      bf16* dst = out + ((size_t)(q0 + row) * H + head) * D + half * 32;
+      // a sink: one more term of the sum, exp(its logit), without a key or a value
+      if (sinks != nullptr || unit_sink) l_run += fast_exp2((sinks != nullptr ? sinks[head] * 1.4426950408889634f : 0.f) - m_ref * sl2);
+      const float inv = out_scale / l_run;
+      bf16* dst = out + (size_t)(q0 + row) * ldo + head * D + half * 32;
 #pragma unroll
       for (int c = 0; c < 32; c += 8) {
         float piece[8];
@@ -475,14 +478,14 @@ int rows_map(CUtensorMap* map, const void* base, long long rows, int row_elems, 
 }  // namespace
 
 // q: bfloat16 [N, H * 64]; pools: bfloat16 [pages, KH, page_size, 64] with page_size a multiple of 64; out: bfloat16
-// [N, H * 64]. tiles: an upper bound of the number of 128-token tiles (the sum over requests of ceil(tokens / 64)
-// will do). Returns 0, a CUDA error, 3000 + a driver error from building a tensor map, or 3999 if the kernel does
-// not take these sizes (nothing was launched).
-AKAS_API int akas_prefill_attention_tc(const void* q, const void* k_pool, const void* v_pool, long long pool_rows,
-                                       const int* block_table, int max_blocks, const int* cu_seqlens,
-                                       const int* positions, void* out, float scale, int window, int page_size, int tiles,
-                                       int N, int H, int KH, int head_dim, int R, cudaStream_t stream) {
-  if (head_dim != D || page_size % 64 || H % KH || tiles > 65535 || R <= 0 || N <= 0) return 3999;
+// rows of H * 64, ldo apart. tiles: an upper bound of the number of 128-token tiles (the sum over requests of
+// ceil(tokens / 64) will do). Returns 0, a CUDA error, 3000 + a driver error from building a tensor map, or 3999 if the
+// kernel does not take these sizes (nothing was launched).
+static int prefill_attention(bool chained, const void* q, const void* k_pool, const void* v_pool, long long pool_rows,
+                             const int* block_table, int max_blocks, const int* cu_seqlens, const int* positions, void* out,
+                             float scale, int window, int page_size, int tiles, int N, int H, int KH, int head_dim, int R,
+                             const float* sinks, int unit_sink, float out_scale, long long ldo, cudaStream_t stream) {
+  if (head_dim != D || page_size % 64 || H % KH || tiles > 65535 || R <= 0 || N <= 0 || ldo % 8) return 3999;
   if ((uintptr_t)q % 16 || (uintptr_t)k_pool % 16 || (uintptr_t)v_pool % 16 || (uintptr_t)out % 16) return 3999;
   if (tiles <= 0) return 0;
   static bool configured[64] = {};  // by device ordinal: the attribute belongs to a device's copy of the kernel
@@ -498,8 +501,33 @@ AKAS_API int akas_prefill_attention_tc(const void* q, const void* k_pool, const 
   if (!err) err = rows_map(&map_k, k_pool, pool_rows, D, D, 64);
   if (!err) err = rows_map(&map_v, v_pool, pool_rows, D, D, 64);
   if (err) return err;
-  return launch_chained(prefill_attention_tc_kernel, dim3(H, tiles), dim3(THREADS), SMEM_BYTES, stream,
-                        map_q, map_k, map_v, block_table, max_blocks, cu_seqlens, positions, (bf16*)out, scale, window, page_size, H, KH, R);
+  if (!chained)
+    return launch_ordinary(prefill_attention_tc_kernel, dim3(H, tiles), dim3(THREADS), SMEM_BYTES, stream, map_q, map_k, map_v,
+                           block_table, max_blocks, cu_seqlens, positions, (bf16*)out, scale, window, page_size, H, KH, R, sinks,
+                           unit_sink, out_scale, ldo);
+  return launch_chained(prefill_attention_tc_kernel, dim3(H, tiles), dim3(THREADS), SMEM_BYTES, stream, map_q, map_k, map_v,
+                        block_table, max_blocks, cu_seqlens, positions, (bf16*)out, scale, window, page_size, H, KH, R, sinks,
+                        unit_sink, out_scale, ldo);
+}
+
+AKAS_API int akas_prefill_attention_tc(const void* q, const void* k_pool, const void* v_pool, long long pool_rows,
+                                       const int* block_table, int max_blocks, const int* cu_seqlens,
+                                       const int* positions, void* out, float scale, int window, int page_size, int tiles,
+                                       int N, int H, int KH, int head_dim, int R, cudaStream_t stream) {
+  return prefill_attention(true, q, k_pool, v_pool, pool_rows, block_table, max_blocks, cu_seqlens, positions, out, scale, window,
+                           page_size, tiles, N, H, KH, head_dim, R, nullptr, 0, 1.f, (long long)H * D, stream);
+}
+
+// The same where the softmax has a sink per head (`sinks`, float32 logits, or `unit_sink`: the logit 0) or none, and the
+// result, times out_scale, goes to rows of a caller's pitch: the general attention's calls without a cap, a distance
+// penalty, kept first tokens, blocks or a gate. (Not a programmatic dependent: its neighbours there are ordinary launches.)
+AKAS_API int akas_prefill_attention_tc_sinks(const void* q, const void* k_pool, const void* v_pool, long long pool_rows,
+                                             const int* block_table, int max_blocks, const int* cu_seqlens, const int* positions,
+                                             void* out, float scale, int window, int page_size, int tiles, int N, int H, int KH,
+                                             int head_dim, int R, const float* sinks, int unit_sink, float out_scale,
+                                             long long ldo, cudaStream_t stream) {
+  return prefill_attention(false, q, k_pool, v_pool, pool_rows, block_table, max_blocks, cu_seqlens, positions, out, scale, window,
+                           page_size, tiles, N, H, KH, head_dim, R, sinks, unit_sink, out_scale, ldo, stream);
 }
 
 // 0 if no bounded wait of the kernel has ever run out on the current device (1: producer, 2: tensor cores,

@@ -152,6 +152,9 @@ _SIGNATURES = {
         "akas_prefill_attention_tc": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                       c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_prefill_attention_tc_status": [],
+        "akas_prefill_attention_tc_sinks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                            c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
+                                            c_longlong, c_void_p],
     },
     "attention_decode": {
         "akas_decode_attention_bf16": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -260,7 +263,7 @@ _PART_FILES = {
     "attention": lambda dtype: ["rope", "attention"] + (["attention_prefill", "attention_prefill_tc", "attention_decode"]
                                                         if dtype == torch.bfloat16 else []),
     "short_conv": lambda dtype: ["conv"],
-    "attention_general": lambda dtype: ["attention_general"] + (["attention_general_tc"] if dtype == torch.bfloat16 else []),
+    "attention_general": lambda dtype: ["attention_general"] + (["attention_general_tc", "attention_prefill_tc"] if dtype == torch.bfloat16 else []),
     "recurrent": lambda dtype: ["recurrent"],
     "moe": lambda dtype: ["moe"] + (["moe_grouped"] if dtype == torch.bfloat16 else []),
     "rope": lambda dtype: ["rope"],
@@ -1789,6 +1792,19 @@ def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, s
         if launches and all(0 < tiles <= 65535 for _, _, tiles, _ in launches):
             for start, requests, tiles, packed in launches:
                 # single tokens: every request's keys in parts, so that a few requests with long pasts fill the GPU; the
+                # A sink at most beside the plain softmax, and prompts of more than 64 tokens: the tensor-memory kernel of the
+                # plain attention (its rule for the tiles; 12 heads, 2,048 tokens: see attention_prefill_tc.cu)
+                if (not packed and not softcap and r1 is None and gate is None and blocks is None and not (window and keep_first)
+                        and d == 64 and vd == 64 and vpitch == 64 and page_size % 64 == 0
+                        and 0 < sum(-(-c // 128) for c in lens[start:]) <= 0.9 * tiles):
+                    err = _fn("attention_prefill_tc", "akas_prefill_attention_tc_sinks")(
+                        _ptr(q), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0] * k_pool.shape[1] * k_pool.shape[2],
+                        _ptr(block_table[start:]), block_table.shape[1], _ptr(ctx.cu_seqlens[start:]), _ptr(positions), op,
+                        float(scale), int(window or 0), page_size, tiles, n, heads, kh, d, requests, _ptr(sinks), int(bool(sink)),
+                        float(out_scale), ldo, _stream())
+                    if err != 3999:
+                        _check(err, "attention_general (tensor memory)")
+                        continue
                 # parts' sums meet in a merge kernel (the count comes from sizes the host knows, as for the plain decode path)
                 splits = decode_splits(requests, kh, 1, getattr(ctx, "max_context", 0) or 0) if packed and general_splits else 1
                 partial = torch.empty(requests * heads * splits * (vd + 2), dtype=torch.float32, device=q.device) if splits > 1 else None

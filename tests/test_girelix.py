@@ -567,6 +567,43 @@ def test_routed_experts_kernels(outputs, experts, count, keep, top, c, f, dtype)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lengths,starts,heads,kv_heads,page,window,sink", [
+    ([129, 300, 65], [0, 77, 301], 6, 2, 64, None, "learned"), ([1, 128, 257], [150, 0, 63], 4, 4, 128, None, "unit"),
+    ([200, 1, 66], [5, 9, 190], 3, 1, 64, 100, "learned"), ([130], [0], 2, 1, 192, 64, "none")])
+def test_sinks_on_the_tensor_memory_kernel(lengths, starts, heads, kv_heads, page, window, sink):
+    """Head size 64 and portions of more than 64 tokens: the tensor-memory kernel with a sink per head, a unit sink or none,
+    under a window, a request's single token in front, rows of the caller's pitch and a scale. A sink of 20 leaves a row
+    almost nothing, one of -20 everything. The bound is that of the kernel's plain calls (bfloat16 weights and values)."""
+    from types import SimpleNamespace
+
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["attention_general", "attention_general_tc", "attention_prefill_tc"])
+    g = torch.Generator().manual_seed(heads * 100 + page)
+    n, r, dim = sum(lengths), len(lengths), 64
+    blocks = -(-700 // page)
+    table = torch.randperm(r * blocks, generator=g).to(torch.int32).view(r, blocks).cuda()
+    k_pool, v_pool = (torch.randn(r * blocks, kv_heads, page, dim, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    cu, seq, _ = _batch(lengths, list(range(r)), "cuda")
+    pos = torch.cat([torch.arange(s, s + l) for s, l in zip(starts, lengths)]).to(torch.int32).cuda()
+    q = (torch.randn(n, heads * dim, generator=g) * 0.5).to(torch.bfloat16).cuda()
+    sinks = None
+    if sink == "learned":
+        sinks = torch.randn(heads, generator=g) * 2.0
+        sinks[0], sinks[-1] = 20.0, -20.0
+        sinks = sinks.cuda()
+    ctx = SimpleNamespace(query_lens=tuple(lengths), decode_only=False, cu_seqlens=cu, max_context=700)
+    args = (k_pool, v_pool, table, seq, pos, 0.3, window, 0, 0.0, None, None, sink == "unit", None, page)
+    want = reference.attention_general(q, *args, sinks=sinks, out_scale=1.2)
+    wide = torch.zeros(n, heads * dim + 16, dtype=torch.bfloat16, device="cuda")
+    view = wide[:, 8 : 8 + heads * dim]
+    cuda.attention_general(q, *args, ctx, sinks=sinks, out=view, out_scale=1.2)
+    _close(view, want, 1e-2, "sinks")
+    assert float(wide[:, :8].abs().max()) == 0.0 and float(wide[:, 8 + heads * dim :].abs().max()) == 0.0
+    assert cuda.prefill_attention_tc_status() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,dim,rot,page", [(6, 2, 24, 16, 8), (4, 4, 16, 16, 16), (3, 1, 20, 6, 4), (36, 2, 8, 0, 64),
                                                         (6, 1, 96, 64, 64), (2, 2, 128, 128, 32)])
