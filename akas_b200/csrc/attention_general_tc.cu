@@ -150,7 +150,15 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
     return i < kept_tiles ? i : kt0 + (i - kept_tiles);
   };
 
-  auto load_tile = [&](int kt, int stage) {
+  // A page that holds whole tiles (its size a multiple of 64) is looked up once per tile, an iteration before the tile's
+  // copies are issued; the copies then only step through it. (A look-up and a division per 16-byte copy, in front of
+  // every tile's products, took longer than the products.)
+  const bool whole_pages = page_size % BK == 0;
+  auto page_of = [&](int i) {
+    const int kt = tile_of(i);
+    return whole_pages && kt >= 0 ? block_table[(size_t)r * max_blocks + kt * BK / page_size] : -1;
+  };
+  auto load_tile = [&](int kt, int stage, int tile_page) {
     bf16* ks_ = k_s + stage * BK * KSTRIDE;
     bf16* vs_ = v_s + stage * BK * VSTRIDE;
     if (kt < 0) {
@@ -168,6 +176,27 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
         } else {
           const int col = (ch - KCH) * 8;
           cp_async16(vs_ + row * VSTRIDE + col, opt.v_blocks + base * V + min(col, V - 8), page >= 0 && col < V ? 16 : 0);
+        }
+      }
+      cp_async_commit();
+      return;
+    }
+    if (whole_pages) {
+      const size_t base = tile_page >= 0 ? ((size_t)tile_page * KH + kvh) * page_size + kt * BK % page_size : 0;
+      const bf16* kp = k_pool + base * D;
+      const bf16* vp = v_pool + base * opt.vpitch;
+#pragma unroll 4
+      for (int c = tid; c < BK * (KCH + VCH); c += WARPS * 32) {
+        const int row = c / (KCH + VCH), ch = c % (KCH + VCH);
+        const int key = kt * BK + row;
+        const bool live = tile_page >= 0 && key <= last_key && (key >= first_key || key < keep);
+        const int in = tile_page >= 0 ? row : 0;
+        if (ch < KCH) {
+          const int col = ch * 8;
+          cp_async16(ks_ + row * KSTRIDE + col, kp + in * D + min(col, D - 8), live && col < D ? 16 : 0);
+        } else {
+          const int col = (ch - KCH) * 8;
+          cp_async16(vs_ + row * VSTRIDE + col, vp + in * opt.vpitch + min(col, V - 8), live && col < V ? 16 : 0);
         }
       }
       cp_async_commit();
@@ -212,7 +241,9 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
   const float inv_cap = opt.cap > 0.f ? 1.f / opt.cap : 0.f;
   const float cap2 = opt.cap * kLog2e, scale2 = opt.scale * kLog2e;
 
-  if (i_begin < i_end) load_tile(tile_of(i_begin), 0);
+  int page_next = i_begin < i_end ? page_of(i_begin) : -1;
+  if (i_begin < i_end) load_tile(tile_of(i_begin), 0, page_next);
+  if (i_begin + 1 < i_end) page_next = page_of(i_begin + 1);
   if (table > 0) {
     for (int d = tid - kTableBefore; d < table + kTableAfter; d += WARPS * 32)
       penalty[d] = d > 0 ? r1[0] * fast_log2(fmaf(r2[0], (float)d, 1.f)) : 0.f;
@@ -224,7 +255,8 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
     const int kt = tile_of(i);
     const int stage = (i - i_begin) & 1;
     if (i + 1 < i_end) {
-      load_tile(tile_of(i + 1), stage ^ 1);
+      load_tile(tile_of(i + 1), stage ^ 1, page_next);
+      if (i + 2 < i_end) page_next = page_of(i + 2);
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
