@@ -129,6 +129,20 @@ paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
   }
 }
 
+// A lane's channels of a value row (zeros for row -1). A tile's rows are asked for eight (wide heads: four) at a time before the first is
+// used: one after another, every row of a tile was a trip to memory of its own (4 requests of 300 float32 keys, 16 heads: 39 us,
+// now 20). Not in the kernel above, whose many blocks hide the trips already (158 us, 167 in this form).
+template <typename T, int NE>
+__device__ __forceinline__ void load_row(const T* __restrict__ pool, int row, int lane, int D, float (&v)[NE]) {
+  const T* p = pool + (size_t)max(row, 0) * D;
+#pragma unroll
+  for (int i = 0; i < NE; ++i) {
+    const int e = lane + 32 * i;
+    const float x = to_f32(p[min(e, D - 1)]);
+    v[i] = row >= 0 && e < D ? x : 0.f;
+  }
+}
+
 // Decode: grid (token, kv_head * head_tiles, split). GT query heads of one kv head per block.
 template <typename T, int NE, int GT>
 __global__ void __launch_bounds__(AKAS_ATT_WARPS * 32)
@@ -178,6 +192,7 @@ decode_splitk_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, cons
     for (int g = 0; g < GT; ++g) s[g] = 0.f;
     if (row >= 0) {
       const T* kp = k_pool + (size_t)row * D;
+#pragma unroll 4
       for (int c = 0; c < D; c += Vec<T>::N) {
         float kv[Vec<T>::N];
         load_vec(kp + c, kv);
@@ -201,22 +216,19 @@ decode_splitk_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, cons
       m[g] = m_new;
     }
     const int keys = min(32, pos - tile * 32 + 1);
-    for (int j = 0; j < keys; ++j) {
-      const int rj = __shfl_sync(0xffffffffu, row, j);
-      if (rj < 0) continue;
-      const T* vp = v_pool + (size_t)rj * D;
-      float v[NE];
+    constexpr int kRowsAtOnce = NE <= 2 ? 8 : 4;
+    for (int j0 = 0; j0 < keys; j0 += kRowsAtOnce) {
+      float v[kRowsAtOnce][NE];
 #pragma unroll
-      for (int i = 0; i < NE; ++i) {
-        const int e = lane + 32 * i;
-        v[i] = e < D ? to_f32(vp[e]) : 0.f;
-      }
+      for (int u = 0; u < kRowsAtOnce; ++u) load_row<T, NE>(v_pool, __shfl_sync(0xffffffffu, row, j0 + u), lane, D, v[u]);
 #pragma unroll
-      for (int g = 0; g < GT; ++g) {
-        const float pj = __shfl_sync(0xffffffffu, p[g], j);
+      for (int u = 0; u < kRowsAtOnce; ++u)
 #pragma unroll
-        for (int i = 0; i < NE; ++i) acc[g][i] = fmaf(pj, v[i], acc[g][i]);
-      }
+        for (int g = 0; g < GT; ++g) {
+          const float pj = __shfl_sync(0xffffffffu, p[g], j0 + u);
+#pragma unroll
+          for (int i = 0; i < NE; ++i) acc[g][i] = fmaf(pj, v[u][i], acc[g][i]);
+        }
     }
   }
 
