@@ -151,10 +151,10 @@ _SIGNATURES = {
     "attention_prefill_tc": {
         "akas_prefill_attention_tc": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                       c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
-        "akas_prefill_attention_tc_status": [],
         "akas_prefill_attention_tc_sinks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                             c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
                                             c_longlong, c_void_p],
+        "akas_prefill_attention_tc_status": [],
     },
     "attention_decode": {
         "akas_decode_attention_bf16": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -205,11 +205,11 @@ _SIGNATURES = {
         "akas_skinny_gemm_norm_gated": [c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                         c_void_p, c_int, c_void_p],
         "akas_skinny_gemm_status": [],
+        "akas_skinny_gemm_takes": [c_int, c_int, c_int, c_int],
     },
     "decode_chain": {
         "akas_chain_set_scratch": [c_void_p],
         "akas_chain_scratch_words": [],
-        "akas_skinny_gemm_takes": [c_int, c_int, c_int, c_int],
         "akas_chain_begin": [],
         "akas_chain_count": [],
         "akas_chain_takes": [c_int] * 5,
@@ -841,10 +841,6 @@ def _skinny_fits(m: int, k: int) -> bool:
     return decode_products == "skinny" and m <= _SKINNY_ROWS and k % 64 == 0 and 1024 + 8 * 8192 + tokens * 512 + tokens * (k + 32) * 2 <= 226 * 1024
 
 
-_SKINNY_ROWS = 16
-# Which kernels run the products of more than 16 tokens (prompt portions, mixed steps, large decode batches). "own"
-# (default; "auto" and "tcgen05" mean the same): the hand-written tcgen05 kernels everywhere: the kernel for pairs of
-# SMs (gemm_pair.cu, TMA-written read-outs) for every product whose output rows TMA can write, the one-block kernel
 def _skinny_takes(m: int, o: int, k: int, mode: int) -> bool:
     """The same for a product without a norm in front and without a gated read-out, which may also be cut along K when
     its activations do not fit a block whole."""
@@ -854,8 +850,12 @@ def _skinny_takes(m: int, o: int, k: int, mode: int) -> bool:
             and bool(_fn("skinny_gemm", "akas_skinny_gemm_takes")(m, o, k, mode)))
 
 
-# (gemm_tcgen05.cu, masked read-outs) for the rest. "library": cuBLASLt everywhere, with SwiGLU as a kernel of its
+_SKINNY_ROWS = 16
 _SKINNY_CUT_ROWS = 8  # 2,048 x 12,288: 13.2 us against 17.0 of the weight-streaming kernel; 9 to 16 tokens, in two groups: 21.7
+# Which kernels run the products of more than 16 tokens (prompt portions, mixed steps, large decode batches). "own"
+# (default; "auto" and "tcgen05" mean the same): the hand-written tcgen05 kernels everywhere: the kernel for pairs of
+# SMs (gemm_pair.cu, TMA-written read-outs) for every product whose output rows TMA can write, the one-block kernel
+# (gemm_tcgen05.cu, masked read-outs) for the rest. "library": cuBLASLt everywhere, with SwiGLU as a kernel of its
 # own: the arm that the hand-written kernels are measured against.
 products = os.environ.get("AKAS_B200_PRODUCTS", "own")
 if products not in ("own", "auto", "tcgen05", "library"):
@@ -1791,7 +1791,6 @@ def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, s
             launches.append((first, len(lens) - first, tiles, 0))
         if launches and all(0 < tiles <= 65535 for _, _, tiles, _ in launches):
             for start, requests, tiles, packed in launches:
-                # single tokens: every request's keys in parts, so that a few requests with long pasts fill the GPU; the
                 # A sink at most beside the plain softmax, and prompts of more than 64 tokens: the tensor-memory kernel of the
                 # plain attention (its rule for the tiles; 12 heads, 2,048 tokens: see attention_prefill_tc.cu)
                 if (not packed and not softcap and r1 is None and gate is None and blocks is None and not (window and keep_first)
@@ -1805,6 +1804,7 @@ def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, s
                     if err != 3999:
                         _check(err, "attention_general (tensor memory)")
                         continue
+                # single tokens: every request's keys in parts, so that a few requests with long pasts fill the GPU; the
                 # parts' sums meet in a merge kernel (the count comes from sizes the host knows, as for the plain decode path)
                 splits = decode_splits(requests, kh, 1, getattr(ctx, "max_context", 0) or 0) if packed and general_splits else 1
                 partial = torch.empty(requests * heads * splits * (vd + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
