@@ -48,8 +48,8 @@ __global__ void __launch_bounds__((BM / (4 * TM)) * (BN / (8 * TN)) * 32)
 sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, float* y, const float* residual, int N, int O, int K) {
   constexpr int NT = (BM / (4 * TM)) * (BN / (8 * TN)) * 32;
   constexpr int PA = BM + 4, PB = BN + 4, GA = TM / 4, GB = TN / 4;
-  constexpr int RT = NT / (kBK / 4);                                      // rows that the threads load at a time
-  constexpr int LA = (BM + RT - 1) / RT, LB = (BN + RT - 1) / RT;          // 16-byte loads of a stage per thread
+  constexpr int LA = BM * (kBK / 4) / NT, LB = BN * (kBK / 4) / NT;  // 16-byte loads of a stage per thread
+  static_assert(LA * NT == BM * (kBK / 4) && LB * NT == BN * (kBK / 4), "whole loads");
   __shared__ __align__(16) float As[2][kBK][PA];
   __shared__ __align__(16) float Bs[2][kBK][PB];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -63,28 +63,26 @@ sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
   auto fetch_w = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < LB; ++i) {
-      const int r = col0 + lr + i * RT;
-      rb[i] = (BN % RT == 0 || lr + i * RT < BN) && r < O && k0 + lc < K ? *reinterpret_cast<const float4*>(w + (size_t)r * K + k0 + lc) : none;
+      const int r = col0 + lr + i * (NT / (kBK / 4));
+      rb[i] = r < O && k0 + lc < K ? *reinterpret_cast<const float4*>(w + (size_t)r * K + k0 + lc) : none;
     }
   };
   auto fetch_x = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
-      const int r = row0 + lr + i * RT;
-      ra[i] = (BM % RT == 0 || lr + i * RT < BM) && r < N && k0 + lc < K ? *reinterpret_cast<const float4*>(x + (size_t)r * K + k0 + lc) : none;
+      const int r = row0 + lr + i * (NT / (kBK / 4));
+      ra[i] = r < N && k0 + lc < K ? *reinterpret_cast<const float4*>(x + (size_t)r * K + k0 + lc) : none;
     }
   };
   auto put = [&](int to) {
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
-      const int r = lr + i * RT;
-      if (BM % RT != 0 && r >= BM) break;
+      const int r = lr + i * (NT / (kBK / 4));
       As[to][lc][r] = ra[i].x; As[to][lc + 1][r] = ra[i].y; As[to][lc + 2][r] = ra[i].z; As[to][lc + 3][r] = ra[i].w;
     }
 #pragma unroll
     for (int i = 0; i < LB; ++i) {
-      const int r = lr + i * RT;
-      if (BN % RT != 0 && r >= BN) break;
+      const int r = lr + i * (NT / (kBK / 4));
       Bs[to][lc][r] = rb[i].x; Bs[to][lc + 1][r] = rb[i].y; Bs[to][lc + 2][r] = rb[i].z; Bs[to][lc + 3][r] = rb[i].w;
     }
   };
@@ -104,6 +102,7 @@ sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
   };
 
   const int steps = (K + kBK - 1) / kBK;
+  chain_release();
   fetch_w(0);  // weights: no kernel writes them
   chain_wait();
   fetch_x(0);
@@ -145,9 +144,6 @@ sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
       }
     }
   }
-  // Only now may the next kernel's blocks come: while this one's run, they would all settle on the SMs that hold none of
-  // them, two to an SM, and stay there.
-  chain_release();
   const bool four = O % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)residual % 16 == 0;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
