@@ -39,124 +39,13 @@ __device__ __forceinline__ float plain_activation(float x, int act) {
   return act == AKAS_PLAIN_SILU ? silu_f(x) : x;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kRouteTokens * 32)
-moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ w, const float* __restrict__ correction,
-                 int* __restrict__ chosen, float* __restrict__ weights, int N, int C, int RC, int groups, int keep, int top,
-                 int sigmoid, int renorm, int extra, float* __restrict__ extras, int group_best, float wscale) {
-  extern __shared__ __align__(16) float smem[];
-  int R = RC + extra;                              // rows of the matrix: the RC outputs that compete, then the extra ones
-  float* rows = smem;                              // [kRouteTokens][kRouteChunk]
-  float* z = rows + kRouteTokens * kRouteChunk;    // [kRouteTokens][R] logits, then scores
-  float* pick = z + kRouteTokens * R;              // [kRouteTokens][R] choice scores
-  float* gbest = pick + kRouteTokens * R;          // [kRouteTokens][groups]
-  float* part = gbest + kRouteTokens * groups;     // [warps][kRouteOutputs][kRouteTokens] the warps' partial sums
-  const int n0 = blockIdx.x * kRouteTokens;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kRouteTokens * R; i += blockDim.x) z[i] = 0.f;
-  if (gridDim.x <= 16) {
-    // a step of few tokens is a few blocks that wait for memory: the whole matrix is asked into the L2 at once, so that
-    // the reads below, one group of outputs after another, do not each wait for DRAM
-    const char* bytes = reinterpret_cast<const char*>(w);
-    const size_t total = (size_t)R * C * sizeof(float);
-    for (size_t off = (size_t)threadIdx.x * 128; off < total; off += (size_t)blockDim.x * 128)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(bytes + off));
-  }
-  for (int c0 = 0; c0 < C; c0 += kRouteChunk) {
-    const int width = min(kRouteChunk, C - c0);
-    __syncthreads();
-    if (C % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)h % 16) == 0) {  // eight channels a load
-      const int per_row = width / 8;
-      for (int i = threadIdx.x; i < kRouteTokens * per_row; i += blockDim.x) {
-        const int t = i / per_row, c = (i % per_row) * 8;
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (n0 + t < N) load8(h + (size_t)(n0 + t) * ldh + c0 + c, v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) rows[t * kRouteChunk + c + j] = v[j];
-      }
-    } else {
-      for (int i = threadIdx.x; i < kRouteTokens * width; i += blockDim.x) {
-        const int t = i / width, c = i % width;
-        rows[t * kRouteChunk + c] = n0 + t < N ? to_f32(h[(size_t)(n0 + t) * ldh + c0 + c]) : 0.f;
-      }
-    }
-    __syncthreads();
-    // Warp w takes the w-th eighth of the staged channels for EVERY router output, so that all of a lane's loads of
-    // the matrix are in flight at once (one trip to memory instead of one per output); the warps' partial sums meet
-    // in shared memory and are added in the order of the warps: the order of a (token, output) sum depends on the
-    // width only.
-    const bool vec = C % 4 == 0 && ((uintptr_t)w % 16) == 0;
-    const int slice = ((width + kRouteTokens - 1) / kRouteTokens + 3) / 4 * 4;
-    const int s0 = min(width, warp * slice), s1 = min(width, s0 + slice);
-    for (int e0 = 0; e0 < R; e0 += kRouteOutputs) {
-      float acc[kRouteOutputs][kRouteTokens];
-#pragma unroll
-      for (int o = 0; o < kRouteOutputs; ++o)
-#pragma unroll
-        for (int t = 0; t < kRouteTokens; ++t) acc[o][t] = 0.f;
-      if (vec) {
-        for (int c = s0 + lane * 4; c < s1; c += 128) {
-          float4 wv[kRouteOutputs];
-#pragma unroll
-          for (int o = 0; o < kRouteOutputs; ++o)
-            wv[o] = e0 + o < R ? *reinterpret_cast<const float4*>(w + (size_t)(e0 + o) * C + c0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int t = 0; t < kRouteTokens; ++t) {
-            const float4 hv = *reinterpret_cast<const float4*>(rows + t * kRouteChunk + c);
-#pragma unroll
-            for (int o = 0; o < kRouteOutputs; ++o) {
-              acc[o][t] = fmaf(hv.x, wv[o].x, acc[o][t]); acc[o][t] = fmaf(hv.y, wv[o].y, acc[o][t]);
-              acc[o][t] = fmaf(hv.z, wv[o].z, acc[o][t]); acc[o][t] = fmaf(hv.w, wv[o].w, acc[o][t]);
-            }
-          }
-        }
-      } else {
-        for (int c = s0 + lane; c < s1; c += 32) {
-#pragma unroll
-          for (int o = 0; o < kRouteOutputs; ++o) {
-            const float wv = e0 + o < R ? w[(size_t)(e0 + o) * C + c0 + c] : 0.f;
-#pragma unroll
-            for (int t = 0; t < kRouteTokens; ++t) acc[o][t] = fmaf(rows[t * kRouteChunk + c], wv, acc[o][t]);
-          }
-        }
-      }
-      // the lanes' 32 sums each (4 outputs x 8 tokens) are added across the warp so that lane l ends with the total of
-      // sum number l: every round a lane hands one half of what it still holds to its partner and keeps the other
-      // (31 shuffles instead of 32 x 5); the order of the additions is the same for every token and batch
-      static_assert(kRouteOutputs * kRouteTokens == 32, "one sum per lane");
-      float* v = &acc[0][0];
-#pragma unroll
-      for (int off = 16, n = 32; off >= 1; off >>= 1, n >>= 1) {
-        const bool upper = (lane & off) != 0;
-#pragma unroll
-        for (int i = 0; i < n / 2; ++i) {
-          const float send = upper ? v[i] : v[i + n / 2];
-          const float keep = upper ? v[i + n / 2] : v[i];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-      }
-      part[warp * 32 + lane] = v[0];  // [warp][output][token]
-      __syncthreads();
-      for (int i = threadIdx.x; i < kRouteOutputs * kRouteTokens; i += blockDim.x) {
-        const int o = i / kRouteTokens, t = i % kRouteTokens;
-        if (e0 + o < R) {
-          float sum = z[t * R + e0 + o];
-          for (int ww = 0; ww < kRouteTokens; ++ww) sum += part[(ww * kRouteOutputs + o) * kRouteTokens + t];
-          z[t * R + e0 + o] = sum;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  // warp t chooses for token n0 + t
-  const int n = n0 + warp;
-  if (n >= N) return;
-  float* zt = z + warp * R;
-  float* pt = pick + warp * R;
-  float* gt = gbest + warp * groups;
+// One warp chooses for token n from its logits zt [RC + extra] (see above); zt and pt become scores, gt holds the groups'.
+__device__ __forceinline__ void choose_outputs(float* zt, float* pt, float* gt, const float* __restrict__ correction,
+                                               int* __restrict__ chosen, float* __restrict__ weights, int n, int lane, int RC,
+                                               int groups, int keep, int top, int sigmoid, int renorm, int extra,
+                                               float* __restrict__ extras, int group_best, float wscale) {
   for (int j = lane; j < extra; j += 32) extras[(size_t)n * extra + j] = 1.f / (1.f + expf(-zt[RC + j]));
-  R = RC;  // from here on: the outputs that compete
+  const int R = RC;  // from here on: the outputs that compete
   if (sigmoid) {
     // Without a correction the choice goes by the logits themselves: the same order as their sigmoids', and two large
     // logits whose sigmoids both round to one still compare.
@@ -214,7 +103,7 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
     }
     __syncwarp();
   }
-  float total = 0.f;
+  float total = 0.f, mine = 0.f;  // mine: the score of the lane-th choice
   for (int k = 0; k < top; ++k) {
     float best = -INFINITY;
     int at = 0x7fffffff;
@@ -229,16 +118,220 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
     if (at == 0x7fffffff) at = 0;  // fewer choosable outputs than `top`: cannot happen for a valid configuration
     if (lane == 0) {
       chosen[(size_t)n * top + k] = at;
-      weights[(size_t)n * top + k] = renorm ? zt[at] : zt[at] * wscale;
+      if (!renorm || k >= 32) weights[(size_t)n * top + k] = renorm ? zt[at] : zt[at] * wscale;
       pt[at] = -INFINITY;
     }
+    if (lane == k) mine = zt[at];
     total += zt[at];
     __syncwarp();
   }
-  if (lane == 0 && renorm) {
+  if (renorm) {
     const float norm = wscale / (total + 1e-20f);
-    for (int k = 0; k < top; ++k) weights[(size_t)n * top + k] *= norm;
+    if (lane < top) weights[(size_t)n * top + lane] = mine * norm;
+    for (int k = 32; lane == 0 && k < top; ++k) weights[(size_t)n * top + k] *= norm;
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRouteTokens * 32)
+moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ w, const float* __restrict__ correction,
+                 int* __restrict__ chosen, float* __restrict__ weights, int N, int C, int RC, int groups, int keep, int top,
+                 int sigmoid, int renorm, int extra, float* __restrict__ extras, int group_best, float wscale) {
+  extern __shared__ __align__(16) float smem[];
+  const int R = RC + extra;                        // rows of the matrix: the RC outputs that compete, then the extra ones
+  float* rows = smem;                              // [kRouteTokens][kRouteChunk]
+  float* z = rows + kRouteTokens * kRouteChunk;    // [kRouteTokens][R] logits, then scores
+  float* pick = z + kRouteTokens * R;              // [kRouteTokens][R] choice scores
+  float* gbest = pick + kRouteTokens * R;          // [kRouteTokens][groups]
+  float* part = gbest + kRouteTokens * groups;     // [warps][kRouteOutputs][kRouteTokens] the warps' partial sums
+  const int n0 = blockIdx.x * kRouteTokens;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < kRouteTokens * R; i += blockDim.x) z[i] = 0.f;
+  if (gridDim.x <= 16) {
+    // a step of few tokens is a few blocks that wait for memory: the whole matrix is asked into the L2 at once, so that
+    // the reads below, one group of outputs after another, do not each wait for DRAM
+    const char* bytes = reinterpret_cast<const char*>(w);
+    const size_t total = (size_t)R * C * sizeof(float);
+    for (size_t off = (size_t)threadIdx.x * 128; off < total; off += (size_t)blockDim.x * 128)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(bytes + off));
+  }
+  for (int c0 = 0; c0 < C; c0 += kRouteChunk) {
+    const int width = min(kRouteChunk, C - c0);
+    __syncthreads();
+    if (C % 8 == 0 && ldh % 8 == 0 && ((uintptr_t)h % 16) == 0) {  // eight channels a load
+      const int per_row = width / 8;
+      for (int i = threadIdx.x; i < kRouteTokens * per_row; i += blockDim.x) {
+        const int t = i / per_row, c = (i % per_row) * 8;
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (n0 + t < N) load8(h + (size_t)(n0 + t) * ldh + c0 + c, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) rows[t * kRouteChunk + c + j] = v[j];
+      }
+    } else {
+      for (int i = threadIdx.x; i < kRouteTokens * width; i += blockDim.x) {
+        const int t = i / width, c = i % width;
+        rows[t * kRouteChunk + c] = n0 + t < N ? to_f32(h[(size_t)(n0 + t) * ldh + c0 + c]) : 0.f;
+      }
+    }
+    __syncthreads();
+    // Warp w takes the w-th eighth of the staged channels for EVERY router output, so that all of a lane's loads of
+    // the matrix are in flight at once (one trip to memory instead of one per output); the warps' partial sums meet
+    // in shared memory and are added in the order of the warps: the order of a (token, output) sum depends on the
+    // width only.
+    const bool vec = C % 4 == 0 && ((uintptr_t)w % 16) == 0;
+    const int slice = ((width + kRouteTokens - 1) / kRouteTokens + 3) / 4 * 4;
+    const int s0 = min(width, warp * slice), s1 = min(width, s0 + slice);
+    for (int e0 = 0; e0 < R; e0 += kRouteOutputs) {
+      float acc[kRouteOutputs][kRouteTokens];
+#pragma unroll
+      for (int o = 0; o < kRouteOutputs; ++o)
+#pragma unroll
+        for (int t = 0; t < kRouteTokens; ++t) acc[o][t] = 0.f;
+      if (vec) {
+        for (int c = s0 + lane * 4; c < s1; c += 128) {
+          float4 wv[kRouteOutputs];
+#pragma unroll
+          for (int o = 0; o < kRouteOutputs; ++o)
+            wv[o] = *reinterpret_cast<const float4*>(w + (size_t)min(e0 + o, R - 1) * C + c0 + c);  // (no load hangs on a condition)
+#pragma unroll
+          for (int t = 0; t < kRouteTokens; ++t) {
+            const float4 hv = *reinterpret_cast<const float4*>(rows + t * kRouteChunk + c);
+#pragma unroll
+            for (int o = 0; o < kRouteOutputs; ++o) {
+              acc[o][t] = fmaf(hv.x, wv[o].x, acc[o][t]); acc[o][t] = fmaf(hv.y, wv[o].y, acc[o][t]);
+              acc[o][t] = fmaf(hv.z, wv[o].z, acc[o][t]); acc[o][t] = fmaf(hv.w, wv[o].w, acc[o][t]);
+            }
+          }
+        }
+      } else {
+        for (int c = s0 + lane; c < s1; c += 32) {
+#pragma unroll
+          for (int o = 0; o < kRouteOutputs; ++o) {
+            const float wv = e0 + o < R ? w[(size_t)(e0 + o) * C + c0 + c] : 0.f;
+#pragma unroll
+            for (int t = 0; t < kRouteTokens; ++t) acc[o][t] = fmaf(rows[t * kRouteChunk + c], wv, acc[o][t]);
+          }
+        }
+      }
+      // the lanes' 32 sums each (4 outputs x 8 tokens) are added across the warp so that lane l ends with the total of
+      // sum number l: every round a lane hands one half of what it still holds to its partner and keeps the other
+      // (31 shuffles instead of 32 x 5); the order of the additions is the same for every token and batch
+      static_assert(kRouteOutputs * kRouteTokens == 32, "one sum per lane");
+      float* v = &acc[0][0];
+#pragma unroll
+      for (int off = 16, n = 32; off >= 1; off >>= 1, n >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+          const float send = upper ? v[i] : v[i + n / 2];
+          const float keep = upper ? v[i + n / 2] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      }
+      part[warp * 32 + lane] = v[0];  // [warp][output][token]
+      __syncthreads();
+      for (int i = threadIdx.x; i < kRouteOutputs * kRouteTokens; i += blockDim.x) {
+        const int o = i / kRouteTokens, t = i % kRouteTokens;
+        if (e0 + o < R) {
+          float sum = z[t * R + e0 + o];
+          for (int ww = 0; ww < kRouteTokens; ++ww) sum += part[(ww * kRouteOutputs + o) * kRouteTokens + t];
+          z[t * R + e0 + o] = sum;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  // warp t chooses for token n0 + t
+  const int n = n0 + warp;
+  if (n >= N) return;
+  choose_outputs(z + warp * R, pick + warp * R, gbest + warp * groups, correction, chosen, weights, n, lane, RC, groups, keep, top,
+                 sigmoid, renorm, extra, extras, group_best, wscale);
+}
+
+// Four neighbouring elements as floats (16 bytes of float32, 8 of bfloat16).
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
+  const uint2 a = *reinterpret_cast<const uint2*>(p);
+  v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xffff0000u);
+  v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
+}
+
+// The router for steps of few tokens: a block per token instead of one per eight, because what such a step waits for is the
+// trip of the matrix's rows to one SM, again for every four outputs. Here a warp asks for its slice of sixteen outputs'
+// rows at once. Slices, chains and the order in which lanes and warps meet are those of the kernel above, so both give the
+// same bits. Rows of whole 16-byte words only. Up to two blocks an SM come at once; more of them wait for a second turn, and then
+// the rows' trips per token weigh as much. bfloat16 rows, us, the kernel above / this one: 16 outputs of 1,536 at 1, 8 and 296 tokens
+// 11.3 / 5.9, 12.3 / 6.1 and 12.3 / 6.7; 256 of 2,048 110 / 36, 111 / 37 and 104 / 42; at 512 tokens 12.3 / 11.6 and 104 / 82, but
+// 8 outputs of 512 7.3 / 10.0 (at 296 7.3 / 5.8).
+constexpr int kRouteFewOutputs = 16, kRouteFewMost = 296;
+
+template <typename T>
+__global__ void __launch_bounds__(kRouteTokens * 32)
+moe_route_few_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ w, const float* __restrict__ correction,
+                     int* __restrict__ chosen, float* __restrict__ weights, int C, int RC, int groups, int keep, int top,
+                     int sigmoid, int renorm, int extra, float* __restrict__ extras, int group_best, float wscale) {
+  extern __shared__ __align__(16) float smem[];
+  const int R = RC + extra, n = blockIdx.x;
+  float* z = smem;            // [R] logits, then scores
+  float* pick = z + R;        // [R] choice scores
+  float* gbest = pick + R;    // [groups]
+  float* part = gbest + groups;  // [warps][kRouteFewOutputs]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* row = h + (size_t)n * ldh;
+  for (int e0 = 0; e0 < R; e0 += kRouteFewOutputs) {
+    float sum = 0.f;  // thread o < kRouteFewOutputs: the logit of output e0 + o
+    for (int c0 = 0; c0 < C; c0 += kRouteChunk) {
+      const int width = min(kRouteChunk, C - c0);
+      const int slice = ((width + kRouteTokens - 1) / kRouteTokens + 3) / 4 * 4;
+      const int s0 = min(width, warp * slice), s1 = min(width, s0 + slice);
+      float v[kRouteFewOutputs];
+#pragma unroll
+      for (int o = 0; o < kRouteFewOutputs; ++o) v[o] = 0.f;
+      constexpr int kTrips = kRouteChunk / kRouteTokens / 128;
+#pragma unroll
+      for (int u = 0; u < kTrips; ++u) {
+        const int c = s0 + lane * 4 + u * 128;
+        if (c >= s1) break;
+        // all of the outputs' words in one trip to memory: no load hangs on a condition (outputs past the last take its row)
+        float4 wv[kRouteFewOutputs];
+#pragma unroll
+        for (int o = 0; o < kRouteFewOutputs; ++o)
+          wv[o] = *reinterpret_cast<const float4*>(w + (size_t)min(e0 + o, R - 1) * C + c0 + c);
+        float x[4];
+        load4(row + c0 + c, x);
+#pragma unroll
+        for (int o = 0; o < kRouteFewOutputs; ++o) {
+          v[o] = fmaf(x[0], wv[o].x, v[o]); v[o] = fmaf(x[1], wv[o].y, v[o]);
+          v[o] = fmaf(x[2], wv[o].z, v[o]); v[o] = fmaf(x[3], wv[o].w, v[o]);
+        }
+      }
+#pragma unroll
+      for (int off = 16, left = kRouteFewOutputs; off >= 2; off >>= 1, left >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < left / 2; ++i) {
+          const float send = upper ? v[i] : v[i + left / 2];
+          const float mine = upper ? v[i + left / 2] : v[i];
+          v[i] = mine + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      }
+      const float whole = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+      if ((lane & 1) == 0) part[warp * kRouteFewOutputs + (lane >> 1)] = whole;
+      __syncthreads();
+      if (threadIdx.x < kRouteFewOutputs)
+        for (int ww = 0; ww < kRouteTokens; ++ww) sum += part[ww * kRouteFewOutputs + threadIdx.x];
+      __syncthreads();
+    }
+    if (threadIdx.x < kRouteFewOutputs && e0 + (int)threadIdx.x < R) z[e0 + threadIdx.x] = sum;
+  }
+  __syncthreads();
+  if (warp == 0)
+    choose_outputs(z, pick, gbest, correction, chosen, weights, n, lane, RC, groups, keep, top, sigmoid, renorm, extra, extras,
+                   group_best, wscale);
 }
 
 // One warp per (pair, hidden channel f): both dots over C, act = silu(gate) * up. Pairs of identity experts do nothing.
@@ -363,6 +456,16 @@ AKAS_API int akas_moe_route(const void* h, long long ldh, const float* w, const 
   if (R <= 0 || groups <= 0 || R % groups || keep <= 0 || keep > groups || top <= 0 || top > keep * (R / groups) || extra < 0 || group_best < 1 ||
       (extra > 0 && extras == nullptr))
     return (int)cudaErrorInvalidValue;
+  const size_t elem = dtype == AKAS_F32 ? 4 : 2;
+  const size_t few_smem = sizeof(float) * (2 * (size_t)(R + extra) + groups + kRouteTokens * kRouteFewOutputs);
+  if (N <= kRouteFewMost && C % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)w % 16 == 0 &&
+      few_smem <= 48 * 1024) {
+    if (dtype == AKAS_F32)
+      return launch_ordinary(moe_route_few_kernel<float>, dim3(N), dim3(kRouteTokens * 32), few_smem, stream, (const float*)h, ldh, w,
+                             correction, chosen, weights, C, R, groups, keep, top, sigmoid, renorm, extra, extras, group_best, wscale);
+    return launch_ordinary(moe_route_few_kernel<bf16>, dim3(N), dim3(kRouteTokens * 32), few_smem, stream, (const bf16*)h, ldh, w,
+                           correction, chosen, weights, C, R, groups, keep, top, sigmoid, renorm, extra, extras, group_best, wscale);
+  }
   const size_t smem = sizeof(float) * ((size_t)kRouteTokens * kRouteChunk + 2 * (size_t)kRouteTokens * (R + extra) + (size_t)kRouteTokens * groups +
                                        (size_t)kRouteTokens * kRouteOutputs * kRouteTokens);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;

@@ -515,6 +515,24 @@ def test_gated_norm_options_and_scaled_add_kernels(dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("outputs,count,keep,top,c", [(16, 4, 2, 4, 1536), (20, 1, 1, 3, 2056), (6, 2, 1, 2, 264), (3, 1, 1, 1, 24)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_route_of_few_tokens_gives_the_bits_of_many(outputs, count, keep, top, c, dtype):
+    """A block per token where the tokens are few, four tokens a block where they are many: one order of sums, the same bits."""
+    from akas_b200.ops import cuda
+
+    cuda.require(["moe"])
+    g = torch.Generator().manual_seed(outputs * 100 + c)
+    h = torch.randn(700, c, generator=g).to(dtype).cuda()
+    w = (torch.randn(outputs, c, generator=g) * (3.0 / c ** 0.5)).cuda()
+    correction = (torch.randn(outputs, generator=g) * 0.2).cuda()
+    chosen, weights = cuda.moe_route(h, w, correction, count, keep, top)
+    for rows in (1, 37, 296):
+        few_c, few_w = cuda.moe_route(h[:rows], w, correction, count, keep, top)
+        assert torch.equal(few_c, chosen[:rows]) and torch.equal(few_w, weights[:rows])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("outputs,experts,count,keep,top,c,f", [(12, 10, 4, 2, 3, 80, 48), (9, 6, 3, 3, 4, 52, 20), (8, 8, 1, 1, 8, 64, 64),
                                                               (70, 64, 5, 2, 6, 1100, 24), (4, 3, 1, 1, 1, 24, 8)])
