@@ -15,15 +15,23 @@
 // Experts, token by token (moe_gate_up, moe_down): act[pair] = silu(W_gate h) * (W_up h) for every (token, chosen
 // real expert) pair, then out[n] = sum over the token's chosen outputs of weight * (W_down act, or h for an identity
 // expert), added in the order of the choice. Every output is one warp's sum over the inner size in a fixed order, so
-// a token's result does not depend on what else the step holds. Weights of all experts are stacked: gate and up as
+// a token's result does not depend on what else the step holds. (bfloat16 steps of few pairs and large matrices take an
+// expert's rows once for all of its pairs: "experts, few pairs".) Weights of all experts are stacked: gate and up as
 // [experts, 2 F, C] (gate rows first), down as [experts, C, F]. Where the weight multiplies the expert's INPUT
 // (out[n] = sum expert(w h)), moe_gate_up gets the weights and scales both of its float32 sums (W (w h) = w (W h))
 // before the activation, and moe_down gets none. Ungated experts (`plain`, an AKAS_PLAIN_* activation): the stack is
 // [experts, F, C] and act[pair] = act(W_up h). moe_down can also add a dense result of every token (a shared
 // expert's), times a gate per token.
 #include "common.cuh"
+#include "mma.cuh"
+#include "tcgen05.cuh"
 
 using namespace akas;
+using tc::mbar_arrive;
+using tc::mbar_expect_tx;
+using tc::mbar_init;
+using tc::mbar_wait;
+using tc::smem_u32;
 
 namespace {
 
@@ -446,6 +454,391 @@ moe_down_kernel(const T* __restrict__ h, long long ldh, const T* __restrict__ w_
   }
 }
 
+// ------------------------------------------------------------------------------------------------ experts, few pairs
+//
+// bfloat16 steps of at most kFewPairs (token, expert) pairs: what bounds them is reading the chosen experts' matrices, once
+// each. The kernels above walk pair by pair: an expert that two tokens chose is read twice (the second time from the L2), a
+// warp has the loads of one row in flight, and widening and multiplying every weight for every pair keeps the issue slots
+// busier than the memory (scalar warps behind the ring below still were: 31.9 and 23.0 us where these take 25.9 and 17.4).
+// Here a block per SM walks tiles of 16 rows of an EXPERT: a producer warp keeps a ring of row copies full (cp.async.bulk, a
+// lane a row, rows 16 bytes further apart than they are long, so that ldmatrix meets no bank twice; 150 to 200 KB on their
+// way per SM; whole rows, because halves of them take twice the copies: 25.8 us for the down projection), and a consumer
+// warp takes a whole tile against up to eight of the expert's pairs at a time by mma.sync m16n8k16, the rows as A, the
+// pairs' vectors as B. (tcgen05 wants 64 rows a tile at least, four times what a stage holds.) Sixteen products at a time
+// are summed by the tensor core and then added, rounded to nearest, by fours to one of four float32 sums: the core's own
+// running sum cuts off what it cannot hold, step after step. So the error against 64 bits is the older kernels' (the down
+// projection alone: 0.88e-7 to 0.92e-7 of the results' size at 1,536 x 1,728, 0.96e-7 to 0.98e-7 there). A (pair, row) sum is
+// the same chain whatever else the step holds. Waits are bounded (akas_moe_status).
+// 14 experts of 1,536 x 1,728, four a token, back to back (us: pair by pair / here / the bytes at 6.65 TB/s): gate and up at 1,
+// 8 and 16 tokens 12.0 / 10.0 / 6.4, 42.3 / 25.9 / 20.8 and 72.4 / 34.4 / 22.4; down 13.4 / 8.4 / 3.2, 25.4 / 17.4 / 10.4 and
+// 39.5 / 20.5 / 11.2. The rest is a launch's start: the choice sorted out, the first rows' way, the last tiles.
+constexpr int kFewPairs = 64, kTileRows = 16, kPad = 8;  // kPad: elements between a row's end and the next row in shared memory
+constexpr int kMostStages = 8, kStreamSmem = 225 * 1024;
+
+__device__ int g_moe_status = 0;
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+// What every block of a step derives from the choice: the real experts that were chosen, in the order of their first pair,
+// and every expert's pairs, one bit each.
+struct Chosen {
+  int picks[kFewPairs], experts[kFewPairs], used;
+  unsigned long long pairs[kFewPairs];
+  unsigned first[2];
+};
+
+__device__ __forceinline__ void sort_out(Chosen& c, const int* __restrict__ chosen, int pairs, int experts) {
+  const int tid = threadIdx.x;
+  if (tid < kFewPairs) c.picks[tid] = tid < pairs ? chosen[tid] : -1;
+  __syncthreads();
+  if (tid < kFewPairs) {
+    const int e = c.picks[tid];
+    unsigned long long mine = 0;
+    for (int p = 0; p < pairs; ++p) mine |= (unsigned long long)(c.picks[p] == e) << p;
+    const bool first = e >= 0 && e < experts && __ffsll((long long)mine) - 1 == tid;
+    const unsigned votes = __ballot_sync(0xffffffffu, first);
+    if ((tid & 31) == 0) c.first[tid >> 5] = votes;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    if (first) {
+      const int at = __popc(c.first[tid >> 5] & ((1u << (tid & 31)) - 1)) + (tid >= 32 ? __popc(c.first[0]) : 0);
+      c.experts[at] = e;
+      c.pairs[at] = mine;
+    }
+    if (tid == 0) c.used = __popc(c.first[0]) + __popc(c.first[1]);
+  }
+  __syncthreads();
+}
+
+// The ring of stages, one consumer warp a stage: a warp takes every consumers-th tile, and the ring's depth is the number of
+// consumers, so that a stage is always the same warp's (a warp that came to another's stage for a later filling before the
+// one in front of it had landed would find the barrier's parity as it wants it).
+struct Ring {
+  uint64_t full[kMostStages], empty[kMostStages];
+  int abort;
+};
+__device__ __forceinline__ void ring_init(Ring& ring, int stages) {
+  if (threadIdx.x == 0) {
+    ring.abort = 0;
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&ring.full[s], 1);
+      mbar_init(&ring.empty[s], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+}
+__device__ __forceinline__ bool ring_wait(Ring& ring, uint64_t* bar, unsigned parity, int code) {
+  if (*(volatile int*)&ring.abort) return false;
+  if (mbar_wait(bar, parity)) return true;
+  *(volatile int*)&ring.abort = 1;
+  atomicExch(&g_moe_status, code);
+  return false;
+}
+__device__ __forceinline__ void ring_lost(Ring& ring) {
+  if (*(volatile int*)&ring.abort)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // a lost launch: let copies in flight finish
+}
+
+// The fragments of 64 k, and their products: the tensor core's sums of 16 products, added in pairs.
+struct Fragments {
+  uint32_t a[4][4], b[2][4];
+  __device__ __forceinline__ void load(const bf16* rows, const bf16* vectors) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ldmatrix_x4(a[i], rows + i * 16);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) ldmatrix_x4(b[i], vectors + i * 32);
+  }
+  __device__ __forceinline__ void add_product(float (&sum)[4]) const {
+    float d[4][4] = {};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mma_bf16(d[i], a[i], b[i >> 1][(i & 1) * 2], b[i >> 1][(i & 1) * 2 + 1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += (d[0][i] + d[1][i]) + (d[2][i] + d[3][i]);
+  }
+};
+
+// acc = 16 rows (`tile`, `pitch` elements apart) times the eight vectors whose rows lie at the lanes' pointers (lane l: vector
+// l % 8), over K elements, a multiple of 32. The next 64 k are read while these are multiplied. Fragment layouts: see mma.cuh.
+__device__ __forceinline__ void tile_product(const bf16* tile, int pitch, const bf16* vector, int K, int lane, float (&acc)[4]) {
+  const bf16* a = tile + (lane & 15) * pitch + (lane >> 4) * 8;
+  const bf16* b = vector + (lane >> 3) * 8;  // the four 8-wide pieces of 32 k
+  float sum[4][4] = {};
+  const int blocks = K / 64;
+  int i = 0;
+  if (blocks >= 4) {
+    Fragments even, odd;
+    even.load(a, b);
+    const int last = blocks - 1;
+    for (; i + 4 <= blocks; i += 4) {
+      odd.load(a + (i + 1) * 64, b + (i + 1) * 64);
+      even.add_product(sum[0]);
+      even.load(a + (i + 2) * 64, b + (i + 2) * 64);
+      odd.add_product(sum[1]);
+      odd.load(a + (i + 3) * 64, b + (i + 3) * 64);
+      even.add_product(sum[2]);
+      even.load(a + min(i + 4, last) * 64, b + min(i + 4, last) * 64);
+      odd.add_product(sum[3]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    if (i + j >= blocks) break;
+    Fragments f;
+    f.load(a + (i + j) * 64, b + (i + j) * 64);
+    f.add_product(sum[j]);
+  }
+  if (K % 64) {
+    uint32_t a0[4], a1[4], bv[4];
+    ldmatrix_x4(a0, a + blocks * 64);
+    ldmatrix_x4(a1, a + blocks * 64 + 16);
+    ldmatrix_x4(bv, b + blocks * 64);
+    float d[2][4] = {};
+    mma_bf16(d[0], a0, bv[0], bv[1]);
+    mma_bf16(d[1], a1, bv[2], bv[3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[3][j] += d[0][j] + d[1][j];
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc[j] = (sum[0][j] + sum[1][j]) + (sum[2][j] + sum[3][j]);
+}
+
+// The next (up to) eight pairs out of the bits of `left`, packed a byte each.
+__device__ __forceinline__ unsigned long long take_eight(unsigned long long& left, int& count) {
+  unsigned long long list = 0;
+  for (count = 0; count < 8 && left != 0; ++count) {
+    list |= (unsigned long long)(__ffsll((long long)left) - 1) << (8 * count);
+    left &= left - 1;
+  }
+  return list;
+}
+__device__ __forceinline__ int pair_at(unsigned long long list, int i) { return (int)(list >> (8 * i)) & 63; }
+
+// act[pair] of every pair: tiles of eight hidden channels (the gate's rows, then the up projection's under them), or (PLAIN) of
+// sixteen, of a chosen expert.
+template <bool PLAIN>
+__global__ void __launch_bounds__((kMostStages + 1) * 32)
+moe_gate_up_stream_kernel(const bf16* __restrict__ h, long long ldh, const bf16* __restrict__ w_gate_up, const int* __restrict__ chosen,
+                          bf16* __restrict__ act, int pairs, int top, int C, int F, int experts, const float* __restrict__ in_weights,
+                          int plain, int stages) {
+  constexpr int WIDE = PLAIN ? kTileRows : kTileRows / 2;  // hidden channels of a tile
+  extern __shared__ __align__(128) unsigned char smem_bytes[];
+  __shared__ Chosen picked;
+  __shared__ Ring ring;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pitch = C + kPad, stage_elems = kTileRows * pitch, tokens = pairs / top;
+  bf16* stage0 = reinterpret_cast<bf16*>(smem_bytes);
+  bf16* x_s = stage0 + (size_t)stages * stage_elems;  // [tokens][pitch]
+  ring_init(ring, stages);
+  sort_out(picked, chosen, pairs, experts);
+  const int tiles_of = (F + WIDE - 1) / WIDE, total = picked.used * tiles_of;
+  if (warp == stages) {
+    int s = 0, turn = 0;
+    for (int id = blockIdx.x; id < total; id += gridDim.x) {
+      if (turn && !ring_wait(ring, &ring.empty[s], (turn & 1) ^ 1, 1)) break;
+      const int at = id / tiles_of, f0 = (id - at * tiles_of) * WIDE, live = min(WIDE, F - f0);
+      const bf16* src = w_gate_up + ((size_t)picked.experts[at] * (PLAIN ? F : 2 * F) + f0) * C;
+      if (lane == 0) mbar_expect_tx(&ring.full[s], (PLAIN ? 1 : 2) * live * C * (unsigned)sizeof(bf16));
+      __syncwarp();
+      const int row = lane % WIDE;
+      if (lane < kTileRows && row < live)
+        bulk_load(stage0 + (size_t)s * stage_elems + lane * pitch, src + ((size_t)row + (lane < WIDE ? 0 : F)) * C,
+                  C * (unsigned)sizeof(bf16), &ring.full[s]);
+      if (++s == stages) { s = 0; ++turn; }
+    }
+  } else {
+    const int per_row = C / 8;
+    for (int i = tid; i < tokens * per_row; i += stages * 32)
+      *reinterpret_cast<uint4*>(x_s + (size_t)(i / per_row) * pitch + (i % per_row) * 8) =
+          *reinterpret_cast<const uint4*>(h + (size_t)(i / per_row) * ldh + (i % per_row) * 8);
+    asm volatile("bar.sync 2, %0;" ::"r"(stages * 32) : "memory");
+    const int g = lane >> 2, t = lane & 3;
+    int turn = 0;
+    for (int id = blockIdx.x + warp * gridDim.x; id < total; id += stages * gridDim.x, ++turn) {
+      const int at = id / tiles_of, f0 = (id - at * tiles_of) * WIDE;
+      unsigned long long left = picked.pairs[at];
+      if (!ring_wait(ring, &ring.full[warp], turn & 1, 2)) break;
+      while (left != 0) {
+        int count;
+        const unsigned long long list = take_eight(left, count);
+        float acc[4];
+        tile_product(stage0 + (size_t)warp * stage_elems, pitch, x_s + (size_t)(pair_at(list, min(lane & 7, count - 1)) / top) * pitch, C,
+                     lane, acc);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int p = 2 * t + j, pair = pair_at(list, min(p, count - 1));
+          const float scale = in_weights != nullptr ? in_weights[pair] : 1.f;
+          const float upper = acc[j] * scale, lower = acc[2 + j] * scale;
+          bf16* dst = act + (size_t)pair * F + f0 + g;
+          if (p < count && f0 + g < F) dst[0] = from_f32<bf16>(PLAIN ? plain_activation(upper, plain) : silu_f(upper) * lower);
+          if (PLAIN && p < count && f0 + 8 + g < F) dst[8] = from_f32<bf16>(plain_activation(lower, plain));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ring.empty[warp]);
+    }
+  }
+  ring_lost(ring);
+}
+
+// The weighted sums of every token for the block's `channels` (at most 16) output channels: per chosen expert (and eight of its
+// pairs) a stage holds the channels' rows of its matrix and the pairs' activations; the pairs' sums stay in shared memory
+// until all experts have passed, and then a thread per (token, channel) adds them in the order of the choice.
+__global__ void __launch_bounds__((kMostStages + 1) * 32)
+moe_down_stream_kernel(const bf16* __restrict__ h, long long ldh, const bf16* __restrict__ w_down, const int* __restrict__ chosen,
+                       const float* __restrict__ weights, const bf16* __restrict__ act, float* __restrict__ out, int pairs, int top, int C,
+                       int F, int experts, float* __restrict__ x, const float* __restrict__ a_res, const float* __restrict__ ls_a,
+                       const float* __restrict__ ls_b, float mult, const float* __restrict__ shared,
+                       const float* __restrict__ shared_gate, long long ldsg, int channels, int stages) {
+  extern __shared__ __align__(128) unsigned char smem_bytes[];
+  __shared__ Chosen picked;
+  __shared__ Ring ring;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int c0 = blockIdx.x * channels, live = min(channels, C - c0);
+  // a stage: `channels` rows of the matrix, then eight rows for the pairs (the product's tile of 16 rows runs on into those
+  // where the channels are fewer: what it makes of them is not looked at)
+  const int pitch = F + kPad, stage_elems = max(channels + 8, kTileRows) * pitch;
+  bf16* stage0 = reinterpret_cast<bf16*>(smem_bytes);
+  float* dots = reinterpret_cast<float*>(stage0 + (size_t)stages * stage_elems);  // [pairs][channels]
+  ring_init(ring, stages);
+  sort_out(picked, chosen, pairs, experts);
+  if (warp == stages) {
+    int s = 0, turn = 0;
+    bool lost = false;
+    for (int at = 0; at < picked.used && !lost; ++at) {
+      unsigned long long left = picked.pairs[at];
+      while (left != 0) {
+        if (turn && !ring_wait(ring, &ring.empty[s], (turn & 1) ^ 1, 3)) { lost = true; break; }
+        int count;
+        const unsigned long long list = take_eight(left, count);
+        bf16* dst = stage0 + (size_t)s * stage_elems;
+        const unsigned row = F * (unsigned)sizeof(bf16);
+        if (lane == 0) mbar_expect_tx(&ring.full[s], (live + count) * row);
+        __syncwarp();
+        if (lane < live)
+          bulk_load(dst + (size_t)lane * pitch, w_down + ((size_t)picked.experts[at] * C + c0 + lane) * F, row, &ring.full[s]);
+        else if (lane >= 16 && lane - 16 < count)
+          bulk_load(dst + (size_t)(channels + lane - 16) * pitch, act + (size_t)pair_at(list, lane - 16) * F, row, &ring.full[s]);
+        if (++s == stages) { s = 0; ++turn; }
+      }
+    }
+  } else {
+    const int g = lane >> 2, t = lane & 3;
+    int next = 0, turn = 0;  // the stage that the next tile lies in
+    bool lost = false;
+    for (int at = 0; at < picked.used && !lost; ++at) {
+      unsigned long long left = picked.pairs[at];
+      while (left != 0) {
+        int count;
+        const unsigned long long list = take_eight(left, count);
+        const bool mine = next == warp;
+        if (++next == stages) next = 0;
+        if (!mine) continue;
+        if (!ring_wait(ring, &ring.full[warp], turn & 1, 4)) { lost = true; break; }
+        ++turn;
+        const bf16* tile = stage0 + (size_t)warp * stage_elems;
+        float acc[4];
+        tile_product(tile, pitch, tile + (size_t)(channels + min(lane & 7, count - 1)) * pitch, F, lane, acc);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int p = 2 * t + (j & 1), r = g + (j >> 1) * 8;
+          if (p < count && r < live) dots[pair_at(list, p) * channels + r] = acc[j];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ring.empty[warp]);
+      }
+    }
+  }
+  __syncthreads();
+  if (*(volatile int*)&ring.abort) {
+    ring_lost(ring);
+    return;
+  }
+  for (int i = tid; i < pairs / top * live; i += blockDim.x) {
+    const int n = i / live, j = i % live, c = c0 + j;
+    float total = 0.f;
+    for (int k = 0; k < top; ++k) {
+      const int pair = n * top + k;
+      const float g = weights != nullptr ? weights[pair] : 1.f;
+      total = fmaf(g, picked.picks[pair] >= experts ? to_f32(h[(size_t)n * ldh + c]) : dots[pair * channels + j], total);
+    }
+    if (shared != nullptr) total = fmaf(shared_gate != nullptr ? shared_gate[(size_t)n * ldsg] : 1.f, shared[(size_t)n * C + c], total);
+    const size_t place = (size_t)n * C + c;
+    if (x != nullptr) x[place] = fmaf(mult, fmaf(ls_b ? ls_b[c] : 1.f, total, a_res ? (ls_a ? ls_a[c] : 1.f) * a_res[place] : 0.f), x[place]);
+    else out[place] = total;
+  }
+}
+
+// The SMs of the current device, or 0; and the shared-memory limit of a kernel raised once per device.
+int sm_count() {
+  static int sms[64] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
+  if (sms[device] == 0) cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
+  return sms[device];
+}
+template <typename K>
+int allow_smem(K kernel, bool (&done)[64]) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
+  if (!done[device]) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+    if (e != cudaSuccess) return (int)e;
+    done[device] = true;
+  }
+  return 0;
+}
+
+// Where the two below are the faster ones (us, pair by pair / here, caches cold). A launch of theirs starts about 3 us later (the
+// choice sorted out, the first rows' way), so gate and up want work: 19 M products of 4 pairs of 2,048 x 2,304 9.7 / 11.5, 21 M
+// (1,536 x 3,456) 12.3 / 10.1, 23 M of 8 pairs of 1,024 x 2,816 10.8 / 10.7, 41 M (1,280 x 2,560) 20.1 / 16.1. The down projection also
+// wants long rows, a copy being 65 ns at least (64 experts of 2,048 x 768, 64 pairs: 39.6 / 42.3), and channels enough for every
+// SM that the matrix's rows outnumber the activations (16 pairs of 1,280 x 1,280 12.4 / 14.4, of 768 x 3,072 13.8 / 16.3; of
+// 2,048 x 1,152 20.5 / 17.1, of 1,536 x 1,728 17.7 / 14.7), the work of a second block per SM where they are more than 16 a
+// block (2 pairs of 4,096 x 1,536 11.0 / 11.7, 8 of them 22.4 / 20.3).
+constexpr long long kStreamWork = 20000000;
+inline bool stream_down(int pairs, int C, int F) {
+  return C >= 1536 && F >= 1152 && (long long)pairs * C * F >= kStreamWork / 2 * ((C + 16 * 148 - 1) / (16 * 148));
+}
+
+constexpr int kNotTaken = -1;  // the sizes do not fit: nothing was launched
+static_assert(kStreamSmem + sizeof(Chosen) + sizeof(Ring) + 256 <= 227 * 1024, "with the static arrays, what a block may have");
+
+template <bool PLAIN>
+int launch_gate_up_stream(const bf16* h, long long ldh, const bf16* w, const int* chosen, bf16* act, int pairs, int top, int C, int F,
+                          int experts, const float* in_weights, int plain, cudaStream_t stream) {
+  const size_t row = (size_t)(C + kPad) * sizeof(bf16), stage = kTileRows * row, xs = (size_t)(pairs / top) * row;
+  const int sms = sm_count();
+  if (sms <= 0 || xs + 3 * stage > kStreamSmem) return kNotTaken;
+  const int stages = (int)min((size_t)kMostStages, (kStreamSmem - xs) / stage);
+  static bool done[64] = {};
+  const int err = allow_smem(moe_gate_up_stream_kernel<PLAIN>, done);
+  if (err) return err;
+  const int wide = PLAIN ? kTileRows : kTileRows / 2;
+  const long long tiles = (long long)min(pairs, experts) * ((F + wide - 1) / wide);
+  return launch_ordinary(moe_gate_up_stream_kernel<PLAIN>, dim3((unsigned)min((long long)sms, tiles)), dim3((stages + 1) * 32),
+                         stages * stage + xs, stream, h, ldh, w, chosen, act, pairs, top, C, F, experts, in_weights, plain, stages);
+}
+
+int launch_down_stream(const bf16* h, long long ldh, const bf16* w, const int* chosen, const float* weights, const bf16* act, float* out,
+                       int pairs, int top, int C, int F, int experts, float* x, const float* a_res, const float* ls_a,
+                       const float* ls_b, float mult, const float* shared, const float* shared_gate, long long ldsg,
+                       cudaStream_t stream) {
+  const int sms = sm_count();
+  if (sms <= 0) return kNotTaken;
+  const int channels = min(16, (C + sms - 1) / sms);
+  const size_t stage = (size_t)max(channels + 8, kTileRows) * (F + kPad) * sizeof(bf16), dots = (size_t)pairs * channels * sizeof(float);
+  if (dots + 2 * stage > kStreamSmem) return kNotTaken;
+  const int stages = (int)min((size_t)kMostStages, (kStreamSmem - dots) / stage);
+  static bool done[64] = {};
+  const int err = allow_smem(moe_down_stream_kernel, done);
+  if (err) return err;
+  return launch_ordinary(moe_down_stream_kernel, dim3((C + channels - 1) / channels), dim3((stages + 1) * 32), stages * stage + dots,
+                         stream, h, ldh, w, chosen, weights, act, out, pairs, top, C, F, experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate,
+                         ldsg, channels, stages);
+}
+
 }  // namespace
 
 // R: the outputs that compete; the matrix has R + extra rows.
@@ -493,6 +886,16 @@ AKAS_API int akas_moe_gate_up(const void* h, long long ldh, const void* w_gate_u
   if (N <= 0 || top <= 0 || experts <= 0) return 0;
   if (plain < AKAS_PLAIN_NONE || plain > AKAS_PLAIN_SILU) return (int)cudaErrorInvalidValue;
   const int pairs = N * top;
+  // few pairs: every chosen expert's rows once through the tensor cores' older path (both sums of a pair, gate and up, end in
+  // one thread), where rows are whole steps of 32 channels and start on 16 bytes and there is enough to multiply
+  if (dtype == AKAS_BF16 && pairs <= kFewPairs && (long long)pairs * (plain ? F : 2 * F) * C >= kStreamWork && C % 32 == 0 &&
+      ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)w_gate_up % 16 == 0) {
+    const int err = plain ? launch_gate_up_stream<true>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
+                                                        experts, in_weights, plain, stream)
+                          : launch_gate_up_stream<false>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
+                                                         experts, in_weights, plain, stream);
+    if (err != kNotTaken) return err;
+  }
   // warps enough to fill the GPU when the pairs are few (a row of F per warp), fewer and longer-lived when they are many
   const dim3 grid(pairs, max(1, min((F + 7) / 8, pairs >= 4096 ? 2 : pairs >= 256 ? 16 : 256)));
   if (dtype == AKAS_F32)
@@ -507,10 +910,23 @@ AKAS_API int akas_moe_down(const void* h, long long ldh, const void* w_down, con
                            const float* a_res, const float* ls_a, const float* ls_b, float mult, const float* shared,
                            const float* shared_gate, long long ldsg, cudaStream_t stream) {
   if (N <= 0) return 0;
+  if (dtype == AKAS_BF16 && N * (long long)top <= kFewPairs && top > 0 && stream_down(N * top, C, F) && F % 32 == 0 &&
+      (uintptr_t)act % 16 == 0 && (uintptr_t)w_down % 16 == 0) {
+    const int err = launch_down_stream((const bf16*)h, ldh, (const bf16*)w_down, chosen, weights, (const bf16*)act, out, N * top, top, C, F,
+                                       experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg, stream);
+    if (err != kNotTaken) return err;
+  }
   const dim3 grid(N, max(1, min((C + 7) / 8, N >= 2048 ? 2 : N >= 64 ? 32 : 256)));
   if (dtype == AKAS_F32)
     return launch_ordinary(moe_down_kernel<float>, grid, dim3(256), 0, stream, (const float*)h, ldh, (const float*)w_down, chosen,
                            weights, (const float*)act, out, top, C, F, experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg);
   return launch_ordinary(moe_down_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)h, ldh, (const bf16*)w_down, chosen,
                          weights, (const bf16*)act, out, top, C, F, experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg);
+}
+
+// 0 unless a bounded wait of the kernels for few pairs has run out on the current device. Synchronises with the device.
+AKAS_API int akas_moe_status() {
+  int status = -1;
+  const cudaError_t e = cudaMemcpyFromSymbol(&status, g_moe_status, sizeof(int));
+  return e == cudaSuccess ? status : -(int)e;
 }

@@ -61,6 +61,7 @@ _SIGNATURES = {
     "moe": {
         "akas_moe_route": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p],
+        "akas_moe_status": [],
         "akas_moe_gate_up": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                              c_void_p, c_int, c_void_p],
         "akas_moe_down": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -1970,6 +1971,12 @@ moe_kernels = os.environ.get("AKAS_B200_MOE", "auto")
 if moe_kernels not in ("auto", "simple"):
     raise ValueError(f"AKAS_B200_MOE must be auto or simple, got {moe_kernels!r}")
 _MOE_SIMPLE_PAIRS = 64
+
+
+def moe_status() -> int:
+    """0 unless a bounded wait inside the experts' kernels for few pairs has run out on this device (then their results
+    since are not valid). Synchronises with the device."""
+    return int(_fn("moe", "akas_moe_status")())
 
 
 def moe_grouped_status() -> int:

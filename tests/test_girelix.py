@@ -533,6 +533,61 @@ def test_route_of_few_tokens_gives_the_bits_of_many(outputs, count, keep, top, c
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("outputs,experts,top,c,f", [(16, 14, 4, 1536, 1728), (20, 17, 3, 2080, 1152), (6, 5, 2, 2304, 1160), (70, 64, 1, 1536, 1152), (8, 8, 8, 1568, 1184),
+                                                   (6, 5, 4, 4100, 1568), (6, 6, 2, 32, 32)])
+@pytest.mark.parametrize("options", [dict(), dict(weight_input=True), dict(activation="relu2")], ids=["silu", "weighted", "relu2"])
+def test_experts_of_few_pairs(outputs, experts, top, c, f, options):
+    """bfloat16 steps of one to 64 (token, expert) pairs against the kernels that walk pair by pair (more pairs take those here),
+    with an expert that many tokens chose and outputs that are no experts; a token's results do not depend on its company. The
+    kernels' sums differ in order alone, so an activation can round to the neighbouring bfloat16 (2^-8 of itself at most)."""
+    from akas_b200.ops import cuda
+
+    cuda.require(["moe"])
+    g = torch.Generator().manual_seed(outputs * 100 + c)
+    n = 64 // top + 1
+    h = torch.randn(n, c, generator=g).to(torch.bfloat16).cuda()
+    chosen = torch.stack([torch.randperm(outputs, generator=g)[:top] for _ in range(n)]).int()
+    chosen[: n // 2] = chosen[0]
+    weights = torch.rand(n, top, generator=g).cuda()
+    w_gate_up = (torch.randn(experts, 2 * f, c, generator=g) * c ** -0.5).to(torch.bfloat16).cuda()
+    w_down = (torch.randn(experts, c, f, generator=g) * f ** -0.5).to(torch.bfloat16).cuda()
+    x0, a0, la, lb = (torch.randn(*s, generator=g).cuda() for s in ((n, c), (n, c), (c,), (c,)))
+    shared = (torch.randn(n, c, generator=g).cuda(), torch.rand(n, 1, generator=g).cuda())
+    up = w_gate_up[:, :f].contiguous() if "activation" in options else w_gate_up
+    size = torch.zeros(n, c, device="cuda")  # the sum of the down projection's terms, without their signs
+    for i in range(n):
+        for k in range(top):
+            e = int(chosen[i, k])
+            if e >= experts:
+                size[i] += weights[i, k] * h[i].float().abs()
+                continue
+            y = (up[e].float() @ h[i].float()) * (weights[i, k] if "weight_input" in options else 1.0)
+            a = y.clamp_min(0).square() if "activation" in options else torch.nn.functional.silu(y[:f]) * y[f:]
+            size[i] += (1.0 if "weight_input" in options else weights[i, k]) * (w_down[e].float().abs() @ a.abs())
+    chosen = chosen.cuda()
+    before = cuda.moe_kernels
+    cuda.moe_kernels = "simple"  # the token-by-token kernels for the whole of it
+    try:
+        whole = cuda.moe_experts(h, up, w_down, chosen, weights, shared=shared, **options)
+        updated = cuda.moe_experts(h, up, w_down, chosen, weights, update=(x0.clone(), a0, la, lb, 0.7), **options)
+    finally:
+        cuda.moe_kernels = before
+    results = []
+    for rows in (64 // top, max(1, 64 // top - 3), 1):
+        part = h[:rows], up, w_down, chosen[:rows].contiguous(), weights[:rows].contiguous()
+        got = cuda.moe_experts(*part, shared=(shared[0][:rows].contiguous(), shared[1][:rows].contiguous()), **options)
+        residual = cuda.moe_experts(*part, update=(x0[:rows].clone(), a0[:rows].contiguous(), la, lb, 0.7), **options)
+        assert cuda.moe_status() == 0
+        rounded = 1e-6 * (1 + whole[:rows].abs() + shared[0][:rows].abs())
+        assert ((got - whole[:rows]).abs() <= 2.0 ** -8 * size[:rows] + rounded).all()
+        rounded = 4e-6 * (1 + updated[:rows].abs() + x0[:rows].abs() + (la * a0[:rows]).abs() + (lb * whole[:rows]).abs())
+        assert ((residual - updated[:rows]).abs() <= 0.7 * lb.abs() * 2.0 ** -8 * size[:rows] + rounded).all()
+        results.append((got, residual))
+    rows = results[1][0].shape[0]  # (one row may be below the work that the kernels are for)
+    assert torch.equal(results[1][0], results[0][0][:rows]) and torch.equal(results[1][1], results[0][1][:rows])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("outputs,experts,count,keep,top,c,f", [(12, 10, 4, 2, 3, 80, 48), (9, 6, 3, 3, 4, 52, 20), (8, 8, 1, 1, 8, 64, 64),
                                                               (70, 64, 5, 2, 6, 1100, 24), (4, 3, 1, 1, 1, 24, 8)])
