@@ -25,31 +25,47 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-
 // out[n, o] = sigmoid(z)^(1 / tau), z = sum_r low[n, r] * wt[r, o] + bias[o]: the up projection of a low-rank pair in
 // float32 (one ascending chain of fused multiply-adds per output), then exp(log sigmoid(z) / tau). The matrix comes
 // transposed, [R, O], so that the threads of a warp read neighbouring words.
-constexpr int kGateTokens = 8;
-
-template <typename T>
-__global__ void decay_gates_kernel(const T* __restrict__ low, long long ld, const float* __restrict__ w,
-                                   const float* __restrict__ bias, float* __restrict__ out, int N, int O, int R,
-                                   float inv_tau) {
-  extern __shared__ float rows[];  // [kGateTokens][R]
-  const int n0 = blockIdx.x * kGateTokens;
-  for (int i = threadIdx.x; i < kGateTokens * R; i += blockDim.x) {
+template <typename T, int TOKENS>  // tokens a block
+__global__ void __launch_bounds__(128)
+decay_gates_kernel(const T* __restrict__ low, long long ld, const float* __restrict__ w, const float* __restrict__ bias,
+                   float* __restrict__ out, int N, int O, int R, float inv_tau) {
+  extern __shared__ __align__(16) float rows[];  // [TOKENS][R]
+  const int n0 = blockIdx.x * TOKENS;
+  for (int i = threadIdx.x; i < TOKENS * R; i += blockDim.x) {
     const int t = i / R, r = i % R;
     rows[i] = n0 + t < N ? to_f32(low[(size_t)(n0 + t) * ld + r]) : 0.f;
   }
   __syncthreads();
   for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < O; o += gridDim.y * blockDim.x) {
-    float acc[kGateTokens];
+    float acc[TOKENS];
 #pragma unroll
-    for (int t = 0; t < kGateTokens; ++t) acc[t] = 0.f;
-    for (int r = 0; r < R; ++r) {
+    for (int t = 0; t < TOKENS; ++t) acc[t] = 0.f;
+    // sixteen rows of the matrix are asked for at once: with one at a time a step of few tokens, a few blocks whose every
+    // load comes from DRAM, took 15 us for a rank of 64
+    int r = 0;
+    if (R % 4 == 0) {
+      for (; r + 16 <= R; r += 16) {
+        float wv[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) wv[j] = w[(size_t)(r + j) * O + o];
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t)
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(rows + t * R + r + j);
+            acc[t] = fmaf(x.x, wv[j], acc[t]); acc[t] = fmaf(x.y, wv[j + 1], acc[t]);
+            acc[t] = fmaf(x.z, wv[j + 2], acc[t]); acc[t] = fmaf(x.w, wv[j + 3], acc[t]);
+          }
+      }
+    }
+    for (; r < R; ++r) {
       const float wv = w[(size_t)r * O + o];
 #pragma unroll
-      for (int t = 0; t < kGateTokens; ++t) acc[t] = fmaf(rows[t * R + r], wv, acc[t]);
+      for (int t = 0; t < TOKENS; ++t) acc[t] = fmaf(rows[t * R + r], wv, acc[t]);
     }
     const float b = bias[o];
 #pragma unroll
-    for (int t = 0; t < kGateTokens; ++t)
+    for (int t = 0; t < TOKENS; ++t)
       if (n0 + t < N) out[(size_t)(n0 + t) * O + o] = expf(-softplus_f(-(acc[t] + b)) * inv_tau);
   }
 }
@@ -1029,12 +1045,20 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const float* _
 AKAS_API int akas_decay_gates(const void* low, long long ld, const float* w, const float* bias, float* out, int N, int O,
                               int R, float tau, int dtype, cudaStream_t stream) {
   if (N <= 0 || O <= 0) return 0;
-  const dim3 grid((N + kGateTokens - 1) / kGateTokens, min((O + 127) / 128, 64));
-  const size_t smem = (size_t)kGateTokens * R * sizeof(float);
-  if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-  if (dtype == AKAS_F32)
-    return launch_ordinary(decay_gates_kernel<float>, grid, dim3(128), smem, stream, (const float*)low, ld, w, bias, out, N, O, R, 1.f / tau);
-  return launch_ordinary(decay_gates_kernel<bf16>, grid, dim3(128), smem, stream, (const bf16*)low, ld, w, bias, out, N, O, R, 1.f / tau);
+  // eight tokens a block; sixteen, which read the matrix half as often, where that leaves enough blocks
+  const size_t row = (size_t)R * sizeof(float);
+  if (8 * row > 48 * 1024) return (int)cudaErrorInvalidValue;
+  const bool wide = 16 * row <= 48 * 1024 && (long long)((N + 15) / 16) * ((O + 127) / 128) >= 592;
+  const int tokens = wide ? 16 : 8;
+  const dim3 grid((N + tokens - 1) / tokens, min((O + 127) / 128, 64));
+#define AKAS_GATES(T, TOKENS)                                                                                                     \
+  return launch_ordinary(decay_gates_kernel<T, TOKENS>, grid, dim3(128), TOKENS * row, stream, (const T*)low, ld, w, bias, out, N, O, R, \
+                         1.f / tau)
+  if (dtype == AKAS_F32 && wide) AKAS_GATES(float, 16);
+  if (dtype == AKAS_F32) AKAS_GATES(float, 8);
+  if (wide) AKAS_GATES(bf16, 16);
+  AKAS_GATES(bf16, 8);
+#undef AKAS_GATES
 }
 
 AKAS_API int akas_gla_scan(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
