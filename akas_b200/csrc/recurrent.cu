@@ -300,11 +300,13 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
     return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
                           decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act);       \
   }
-  if (D <= 8) AKAS_SCAN(8, 1, 16)
-  if (D <= 16) AKAS_SCAN(8, 2, 16)
-  if (D <= 32) AKAS_SCAN(8, 4, 16)
-  if (D <= 64) AKAS_SCAN(16, 4, 16)
-  if (D <= 128) AKAS_SCAN(16, 8, 16)
+  if constexpr (RULE != RULE_DELTA) {  // (which walks such keys with delta_walk_kernel)
+    if (D <= 8) AKAS_SCAN(8, 1, 16)
+    if (D <= 16) AKAS_SCAN(8, 2, 16)
+    if (D <= 32) AKAS_SCAN(8, 4, 16)
+    if (D <= 64) AKAS_SCAN(16, 4, 16)
+    if (D <= 128) AKAS_SCAN(16, 8, 16)
+  }
   if (D <= 256) AKAS_SCAN(16, 16, 8)
   if (D <= 512) AKAS_SCAN(16, 32, 4)
   AKAS_SCAN(32, 32, 2)
@@ -728,9 +730,9 @@ walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ 
 #pragma unroll
       for (int n = 0; n < NV; ++n) o[n] = acc[0][n] + acc[1][n];
       int left = NV, first = 0;  // the lane holds the sums of channels first .. first + left - 1 of its four
-      if constexpr (KS > 1)
 #pragma unroll
-      for (int off = KS / 2; off > 0; off >>= 1) {
+      for (int off = 4; off > 0; off >>= 1) {
+        if (off >= KS) continue;
         if (left > 1) {
           const bool upper = (ks & off) != 0;
 #pragma unroll
@@ -832,6 +834,190 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
   return AKAS_WALKS(2);
 #undef AKAS_WALKS
 #undef AKAS_WALK
+}
+
+// ------------------------------------------------------------------------------------------------ delta rule, small keys
+//
+// The delta rule of scan_kernel for keys of up to 128 channels. A token's u waits for the sums over the keys, and the next
+// token's sums for its u: a walk is a chain of such rounds, so what a round holds beside its arithmetic is what costs.
+// A thread owns 16 key channels of NV value channels (see the launch); the decay is applied after the sums (S^T k of the state as it stands,
+// times g) and to the state while the lanes' sums meet; the read-out's sums are nobody's input and run under the next
+// token's. KS neighbouring lanes hold a value channel, lane ks the channels 4 (ks + KS i) .. + 3, so that rows of the state
+// and of a token's q and k are read in whole 128-byte lines.
+constexpr int kDeltaThreads = 128, kDeltaTokens = 16;
+
+template <int KS, int NV>
+__global__ void __launch_bounds__(kDeltaThreads)
+delta_walk_kernel(const float* __restrict__ q, long long ldq, const float* __restrict__ k, long long ldk, const float* __restrict__ v,
+                  long long ldv, const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ state,
+                  long long slot_stride, const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ out,
+                  int H, int rep, int D, int V, int write, int vec) {
+  constexpr int CH = kDeltaTokens, TH = kDeltaThreads, VT = TH / KS * NV, W = 16 * KS;
+  constexpr int NQ = (CH * W / 4 + TH - 1) / TH, NVL = (CH * VT / 4 + TH - 1) / TH;
+  __shared__ __align__(16) float sq[CH][W];
+  __shared__ __align__(16) float sk[CH][W];
+  __shared__ __align__(16) float sv[CH][VT];
+  __shared__ float sg[CH], sb[CH];
+  const int h = blockIdx.x, req = blockIdx.y, hk = h / rep;
+  const int t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
+  const int slot = slots[req];
+  if (slot < 0 || t_end <= t_begin) return;
+  const int ks = threadIdx.x % KS, jl = threadIdx.x / KS;
+  const int v0 = blockIdx.z * VT, j0 = v0 + jl * NV;
+
+  float s[NV][16];
+  float* srow = state + (size_t)slot * slot_stride + ((size_t)h * V + j0) * D;
+  const bool whole = D % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = 4 * (ks + KS * i);
+      Four<float> x;
+      x.fetch(srow + (size_t)n * D + c, j0 + n < V ? D - c : 0, whole);
+      x.widen(reinterpret_cast<float(&)[4]>(s[n][4 * i]));
+    }
+
+  Four<float> rq[NQ], rk[NQ], rv[NVL];  // the next tokens' inputs, on their way while the tokens in shared memory are walked
+  float rg = 0.f, rb = 0.f;
+  auto fetch = [&](int c0) {
+    const int count = min(CH, t_end - c0);
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      const int i = threadIdx.x + u * TH, t = i / (W / 4), c = (i % (W / 4)) * 4;
+      const int live = t < count ? D - c : 0;
+      const size_t n = (size_t)(c0 + (t < count ? t : 0)), at = (size_t)hk * D + (live > 0 ? c : 0);
+      rq[u].fetch(q + n * ldq + at, live, vec);
+      rk[u].fetch(k + n * ldk + at, live, vec);
+    }
+#pragma unroll
+    for (int u = 0; u < NVL; ++u) {
+      const int i = threadIdx.x + u * TH, t = i / (VT / 4), c = v0 + (i % (VT / 4)) * 4;
+      const int live = t < count ? V - c : 0;
+      rv[u].fetch(v + (size_t)(c0 + (t < count ? t : 0)) * ldv + (size_t)h * V + (live > 0 ? c : 0), live, vec);
+    }
+    if (threadIdx.x < count) {
+      rg = g[(size_t)(c0 + threadIdx.x) * H + h];
+      rb = beta[(size_t)(c0 + threadIdx.x) * H + h];
+    }
+  };
+  fetch(t_begin);
+  for (int c0 = t_begin; c0 < t_end; c0 += CH) {
+    const int count = min(CH, t_end - c0);
+    __syncthreads();  // the tokens before have been read
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      const int i = threadIdx.x + u * TH;
+      if (i >= CH * W / 4) continue;
+      *reinterpret_cast<float4*>(&sq[i / (W / 4)][(i % (W / 4)) * 4]) = rq[u].raw;
+      *reinterpret_cast<float4*>(&sk[i / (W / 4)][(i % (W / 4)) * 4]) = rk[u].raw;
+    }
+#pragma unroll
+    for (int u = 0; u < NVL; ++u) {
+      const int i = threadIdx.x + u * TH;
+      if (i < CH * VT / 4) *reinterpret_cast<float4*>(&sv[i / (VT / 4)][(i % (VT / 4)) * 4]) = rv[u].raw;
+    }
+    if (threadIdx.x < CH) {
+      sg[threadIdx.x] = rg;
+      sb[threadIdx.x] = rb;
+    }
+    __syncthreads();
+    if (c0 + CH < t_end) fetch(c0 + CH);
+#pragma unroll 2
+    for (int t = 0; t < count; ++t) {
+      float kk[16], part[NV][2] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(&sk[t][4 * (ks + KS * i)]);
+        kk[4 * i] = x.x; kk[4 * i + 1] = x.y; kk[4 * i + 2] = x.z; kk[4 * i + 3] = x.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int n = 0; n < NV; ++n) part[n][e & 1] = fmaf(s[n][4 * i + e], kk[4 * i + e], part[n][e & 1]);
+      }
+      const float gt = sg[t], bt = sb[t];
+      float u[NV];
+#pragma unroll
+      for (int n = 0; n < NV; ++n) u[n] = part[n][0] + part[n][1];
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+        for (int n = 0; n < NV && off < KS; ++n) u[n] += __shfl_xor_sync(0xffffffffu, u[n], off);
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int r = 0; r < 16; ++r) s[n][r] *= gt;
+#pragma unroll
+      for (int n = 0; n < NV; ++n) u[n] = bt * (sv[t][jl * NV + n] - gt * u[n]);
+      float acc[NV][2] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(&sq[t][4 * (ks + KS * i)]);
+        const float qq[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int n = 0; n < NV; ++n) {
+            s[n][4 * i + e] = fmaf(kk[4 * i + e], u[n], s[n][4 * i + e]);
+            acc[n][e & 1] = fmaf(s[n][4 * i + e], qq[e], acc[n][e & 1]);
+          }
+      }
+      float o[NV];
+#pragma unroll
+      for (int n = 0; n < NV; ++n) o[n] = acc[n][0] + acc[n][1];
+#pragma unroll
+      for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+        for (int n = 0; n < NV && off < KS; ++n) o[n] += __shfl_xor_sync(0xffffffffu, o[n], off);
+      if (ks == 0) {
+        float* dst = out + (size_t)(c0 + t) * ((size_t)H * V) + (size_t)h * V + j0;
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+          if (j0 + n < V) dst[n] = o[n];
+      }
+    }
+  }
+  if (!write) return;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    if (j0 + n >= V) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = 4 * (ks + KS * i);
+      float* dst = srow + (size_t)n * D + c;
+      if (whole && c + 3 < D) {
+        *reinterpret_cast<float4*>(dst) = make_float4(s[n][4 * i], s[n][4 * i + 1], s[n][4 * i + 2], s[n][4 * i + 3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (c + e < D) dst[e] = s[n][4 * i + e];
+      }
+    }
+  }
+}
+
+int launch_delta_walk(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, const float* beta,
+                      const float* g, float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out,
+                      int requests, int H, int rep, int D, int V, int write, cudaStream_t stream) {
+  if (requests <= 0 || H <= 0) return 0;
+  if (requests > 65535) return (int)cudaErrorInvalidValue;
+  const int vec = D % 4 == 0 && V % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && (uintptr_t)q % 16 == 0 &&
+                  (uintptr_t)k % 16 == 0 && (uintptr_t)v % 16 == 0;
+#define AKAS_DELTA(KS, NV)                                                                                                    \
+  return launch_ordinary(delta_walk_kernel<KS, NV>, dim3(H, requests, (V + kDeltaThreads / KS * NV - 1) / (kDeltaThreads / KS * NV)), \
+                         dim3(kDeltaThreads), 0, stream, q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, \
+                         H, rep, D, V, write, vec)
+  // One value channel a thread where the blocks that gives still have an SM each: a round of the walk is then shorter, one more
+  // block costs nothing. With more of them two channels share what a round reads of q and k. 16 heads, D = V = 128 (us, scan_kernel
+  // / one channel / two): a prompt of 2,048 tokens (128 blocks of one channel) 670 / 485 / 625, of 512 170 / 123 / 158, two of 1,337
+  // and 2,048 (256) 671 / 624 / 628, sixteen of 300 526 / 486 / 329, one token of 8 requests 8.5 / 6.9 / 5.4, of 64 47 / 36 / 28.5.
+  const bool alone = (long long)H * requests * ((V + kDeltaThreads / 8 - 1) / (kDeltaThreads / 8)) <= 148;
+  if (D <= 16) AKAS_DELTA(1, 2);
+  if (D <= 32) AKAS_DELTA(2, 2);
+  if (D <= 64) AKAS_DELTA(4, 2);
+  if (alone) AKAS_DELTA(8, 1);
+  AKAS_DELTA(8, 2);
+#undef AKAS_DELTA
 }
 
 // ------------------------------------------------------------------------------------------------ causal convolution
@@ -1151,6 +1337,9 @@ AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long
                              const int* slots, float* out, int tokens, int requests, int H, int G, int D, int V, int write,
                              cudaStream_t stream) {
   if (G <= 0 || H % G) return (int)cudaErrorInvalidValue;
+  if (D <= 128)
+    return launch_delta_walk(q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, requests, H, H / G, D, V,
+                             write, stream);
   return launch_scan<float, RULE_DELTA>(q, ldq, k, ldk, v, ldv, g, beta, state, slot_stride, cu_seqlens, slots, out, tokens,
                                   requests, H, H / G, D, V, 1.f, write, stream);
 }
