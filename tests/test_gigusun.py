@@ -350,6 +350,37 @@ def test_delta_scan_kernel(heads, kv_heads, dim, vdim):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dim,vdim", [(12, 20), (28, 36), (52, 33), (72, 40), (128, 128)])
+def test_delta_scan_of_many_requests(dim, vdim):
+    """Steps of enough requests for the walk that takes two value channels a thread, against the reference, and every request
+    alone (one channel a thread where the keys are over 64 channels) to the same bits: a channel's sums are the same chains."""
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(dim)
+    heads, kv_heads, lengths = 16, 8, [1, 17, 16, 0, 33, 2, 1, 5, 40, 3, 1, 31]
+    slots, n, gd = list(range(12)), sum(lengths), 8 * dim
+    y = torch.randn(n, 2 * gd + heads * vdim, generator=g).cuda()
+    y[:, : 2 * gd] *= dim ** -0.5
+    beta, decay = torch.rand(n, heads, generator=g).cuda(), (torch.rand(n, heads, generator=g) * 0.4 + 0.6).cuda()
+    state = (torch.randn(12, heads, vdim, dim, generator=g) * 0.3).cuda()
+    s_ref, s_got, s_one = state.clone(), state.clone(), state.clone()
+    cu, _, sl = _batch(lengths, slots, "cuda")
+    run = lambda ops, r, s, cu, sl: ops.delta_scan(y[r, :gd], y[r, gd : 2 * gd], y[r, 2 * gd :], beta[r], decay[r], s, cu, sl, heads, kv_heads, dim, vdim)
+    want, got = run(reference, slice(0, n), s_ref, cu, sl), run(cuda, slice(0, n), s_got, cu, sl)
+    _close(got, want, 3e-5, "delta o")
+    _close(s_got, s_ref, 3e-5, "delta state")
+    first = 0
+    for length, slot in zip(lengths, slots):
+        if length:
+            cu, _, sl = _batch([length], [slot], "cuda")
+            r = slice(first, first + length)
+            assert torch.equal(run(cuda, r, s_one, cu, sl), got[r])
+        first += length
+    assert torch.equal(s_one, s_got)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps", [2, 3, 4, 7])
 def test_causal_conv_silu_kernel(taps, dtype):
@@ -371,6 +402,21 @@ def test_causal_conv_silu_kernel(taps, dtype):
         got = cuda.causal_conv_silu(x, w, view(s_got), cu, seq, sl, write=write)
         _close(got, want, 1e-5, "conv")
         _close(s_got, s_ref, 1e-6, "conv state")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rank,out", [(64, 2048), (20, 2050), (7, 2500), (768, 2048), (1000, 2048)])
+def test_decay_gates_of_many_tokens(rank, out, dtype):
+    """Sixteen tokens a block where there are blocks enough give the bits of eight."""
+    from akas_b200.ops import cuda
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(rank)
+    low = torch.randn(603, rank, generator=g).to(dtype).cuda()
+    w, bias = (torch.randn(rank, out, generator=g) * rank ** -0.5).cuda(), torch.randn(out, generator=g).cuda()
+    whole = cuda.decay_gates(low, w, bias, 8.0)
+    assert torch.equal(whole, torch.cat([cuda.decay_gates(part, w, bias, 8.0) for part in low.split(67)]))
 
 
 @pytest.mark.gpu
