@@ -421,6 +421,31 @@ def test_decay_gates_of_many_tokens(rank, out, dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_causal_conv_silu_in_runs(dtype):
+    """Steps of many tokens run eight tokens a thread: requests that begin and end inside a run, steps shorter than the taps
+    reach, a padding token; the same chain of multiply-adds as the oracle's, in float32."""
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(3)
+    c, taps = 2052, 4
+    lengths, slots = [1, 2, 300, 0, 5, 3, 401], [3, 0, 1, -1, 2, 5, 4]
+    n = sum(lengths)
+    x = torch.randn(n, c + 4, generator=g).to(dtype).cuda()[:, 4:]
+    w = torch.randn(c, taps, generator=g).cuda()
+    state = torch.randn(6, (taps - 1) * c, generator=g).cuda().view(6, taps - 1, c)
+    cu, seq, sl = _batch(lengths, slots, "cuda")
+    s_ref, s_got = state.clone(), state.clone()
+    want = reference.causal_conv_silu(x, w, s_ref, cu, seq, sl)
+    _close(cuda.causal_conv_silu(x, w, s_got, cu, seq, sl), want, 1e-5, "conv")
+    _close(s_got, s_ref, 1e-6, "conv state")
+    padded = torch.cat([x, x[:6]])  # six tokens of no request behind them
+    got = cuda.causal_conv_silu(padded, w, state.clone(), cu, torch.cat([seq, seq.new_full((6,), -1)]), sl)
+    _close(got[:n], want, 1e-5, "conv, padded")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gates_norms_and_polynorm_kernels(dtype):
     from akas_b200.ops import cuda, reference
 
