@@ -446,6 +446,25 @@ def test_causal_conv_silu_in_runs(dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,vdim", [(1, 768), (1, 1024), (2, 260), (1, 516)])
+def test_gated_norm_of_few_long_rows_gives_the_bits_of_many(heads, vdim, dtype):
+    from akas_b200.ops import cuda
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(vdim)
+    n = 400
+    o = torch.randn(n, heads * vdim, generator=g).cuda()
+    w = torch.randn(vdim, generator=g).cuda()
+    gate = torch.randn(n, heads * vdim + 8, generator=g).to(dtype).cuda()[:, 8:]
+    for act in ("silu", "sigmoid"):
+        whole = cuda.gated_rmsnorm(o, w, 1e-5, gate, heads, vdim, dtype, gate_activation=act)
+        assert torch.equal(cuda.gated_rmsnorm(o[:9], w, 1e-5, gate[:9], heads, vdim, dtype, gate_activation=act), whole[:9])
+    plain = cuda.gated_rmsnorm(o, None, 1e-5, None, heads, vdim, dtype)
+    assert torch.equal(cuda.gated_rmsnorm(o[:9], None, 1e-5, None, heads, vdim, dtype), plain[:9])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gates_norms_and_polynorm_kernels(dtype):
     from akas_b200.ops import cuda, reference
 
