@@ -111,8 +111,9 @@ __global__ void qk_norm_store_kernel(const TI* __restrict__ q, long long ldq, co
 }
 
 // The same for head sizes that are multiples of 8 (at most 256), rotate-half pairs and a rotary width that is a multiple
-// of 16, everything on 16 bytes: a thread owns 8 neighbouring channels of a head (LPH threads, D / 8 rounded up to a
-// power of two, share one; those past D / 8 only shuffle, as do those past the last head) and reads its rotation partner's 8 channels itself; the
+// of 16, or neighbouring pairs and a multiple of 8, everything on 16 bytes: a thread owns 8 neighbouring channels of a head
+// (LPH threads, D / 8 rounded up to a power of two, share one; those past D / 8 only shuffle, as do those past the last head)
+// and holds its pairs itself or reads its rotation partner's 8 channels; the
 // threads behind the heads' copy the values. A token's heads are spread over gridDim.y blocks.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(128)
@@ -122,7 +123,7 @@ qk_norm_store8_kernel(const TI* __restrict__ q, long long ldq, const TI* __restr
                       const int* __restrict__ seq_of_token, const int* __restrict__ positions, int page_size, int H, int G, int D,
                       int V, int write, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                       const float* __restrict__ qb, const float* __restrict__ kb, const float* __restrict__ vb, int unit, int lph,
-                      float temp_coef, int temp_every) {
+                      float temp_coef, int temp_every, int interleaved) {
   const int n = blockIdx.x;
   const int req = seq_of_token[n];
   if (req < 0) return;
@@ -170,7 +171,18 @@ qk_norm_store8_kernel(const TI* __restrict__ q, long long ldq, const TI* __restr
     inv = inverse_rms();
     if (turns) weigh(e0, inv, x);
   }
-  if (cos_t != nullptr && turns && e0 < rot) {
+  if (cos_t != nullptr && turns && e0 < rot && interleaved) {
+    const int half = rot / 2;
+    const float4 c4 = *reinterpret_cast<const float4*>(cos_t + (size_t)n * half + e0 / 2);
+    const float4 s4 = *reinterpret_cast<const float4*>(sin_t + (size_t)n * half + e0 / 2);
+    const float c[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float u = x[2 * i], y = x[2 * i + 1];
+      x[2 * i] = fmaf(u, c[i], -y * sn[i]);
+      x[2 * i + 1] = fmaf(y, c[i], u * sn[i]);
+    }
+  } else if (cos_t != nullptr && turns && e0 < rot) {
     const int half = rot / 2;
     const bool low = e0 < half;
     const int p0 = low ? e0 + half : e0 - half, f0 = low ? e0 : e0 - half;
@@ -518,8 +530,10 @@ AKAS_API int akas_qk_norm_store(const void* q, long long ldq, const void* k, lon
   const uintptr_t bases = (uintptr_t)q | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)qw | (uintptr_t)kw |
                           (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)qb | (uintptr_t)kb | (uintptr_t)vb |
                           (write ? (uintptr_t)k | (uintptr_t)v : 0);
-  if (D % 8 == 0 && D <= 256 && V % 8 == 0 && (cos_t == nullptr || (!interleaved && rot % 16 == 0)) && bases % 16 == 0 && ldq % 8 == 0 &&
-      (!write || (ldk % 8 == 0 && ldv % 8 == 0))) {
+  // rows of whole 16-byte words, and pairs that lie in one thread's 8 channels or in two whole threads': 8 tokens of 12 + 2 heads
+  // of 64, neighbouring pairs, 5.3 us by the kernel of one channel a lane, 2.85 here
+  const bool pairs = cos_t == nullptr || (interleaved ? rot > 0 && rot <= D && rot % 8 == 0 : rot % 16 == 0);
+  if (D % 8 == 0 && D <= 256 && V % 8 == 0 && pairs && bases % 16 == 0 && ldq % 8 == 0 && (!write || (ldk % 8 == 0 && ldv % 8 == 0))) {
     int lph = 1;
     while (lph < D / 8) lph *= 2;
     const int threads = (write ? H + G : H) * lph + (write ? G * (V / 8) : 0);
@@ -528,7 +542,7 @@ AKAS_API int akas_qk_norm_store(const void* q, long long ldq, const void* k, lon
   return launch_ordinary(qk_norm_store8_kernel<TI, T>, grid, dim3(128), 0, stream, (const TI*)q, ldq, (const TI*)k, ldk,      \
                          (const TI*)v, ldv, qw, kw, eps, (T*)q_out, (T*)k_pool, (T*)v_pool, block_table, max_blocks,          \
                          seq_of_token, positions, page_size, H, G, D, V, write, cos_t, sin_t, rot, qb, kb, vb, unit, lph,     \
-                         temp_coef, temp_every)
+                         temp_coef, temp_every, interleaved)
     if (dtype == AKAS_F32) AKAS_STORE8(float, float);
     if (in_dtype == AKAS_F32) AKAS_STORE8(float, bf16);
     AKAS_STORE8(bf16, bf16);
