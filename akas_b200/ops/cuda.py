@@ -316,12 +316,15 @@ def _check(err: int, what: str, kernels: int = 1) -> None:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """The handle of torch's current stream on the current device (every launch goes there)."""
-    if _raw_stream is not None:  # the same value as below without building a Stream object per launch
-        return _raw_stream(torch.cuda.current_device())
+    if _raw_stream is not None and _current_device is not None:
+        # the same value as below without building a Stream object per launch (a tensor on the device exists by now, so
+        # the context does too)
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -516,14 +519,18 @@ def take_tokens(token_ids, source, previous):
                                                  token_ids.numel(), _stream()), "take_tokens")
 
 
-@_flushes
 def rmsnorm(x, weight, eps, zero_centered, out_dtype, rows=None):
-    c = x.shape[-1]
+    if _chain_open:  # (inline, not by the decorator: a mixed step calls this dozens of times)
+        chain_flush()
     _dense(x, "x")
-    lead = x.shape[:-1]
-    m = rows.numel() if rows is not None else x.numel() // c
-    out_shape = (m, c) if rows is not None else (*lead, c)
-    out = torch.empty(out_shape, dtype=out_dtype, device=x.device)
+    shape = x.shape
+    c = shape[-1]
+    if rows is not None:
+        m = rows.numel()
+        shape = (m, c)
+    else:
+        m = shape[0] if len(shape) == 2 else x.numel() // c
+    out = torch.empty(shape, dtype=out_dtype, device=x.device)
     _check(_fn("elementwise", "akas_rmsnorm")(_ptr(x), _ptr(weight), _ptr(out), _ptr(rows), m, c, float(eps),
                                              int(bool(zero_centered)), _code(x), _CODE[out_dtype], _stream()),
            "rmsnorm")
@@ -968,12 +975,13 @@ def gemm_rows_status() -> int:
     return int(_fn("gemm_rows", "akas_gemm_rows_status")())
 
 
-@_flushes
 def paired_product(x, w, swiglu_out: bool = False, out_dtype=None, residual=None, few_rows=True):
     """x [N, K] times w [O, K] transposed on pairs of SMs. bfloat16 out by default; float32 out with ``out_dtype``;
     added into ``residual`` (float32 [N, O]) when that is given; with ``swiglu_out`` w is the stacked [2F, K] gate and
     up matrices and the result is swiglu of the product, bfloat16 [N, F]. Up to 128 tokens go to ``rows_product``
     unless ``few_rows`` is False."""
+    if _chain_open:  # (inline, not by the decorator: a mixed step calls this dozens of times)
+        chain_flush()
     n, k = x.shape
     o = w.shape[0]
     out, epilogue = _tma_product("paired_product", x, w, swiglu_out, out_dtype, residual)
@@ -1190,9 +1198,10 @@ def _norm_place(q_weight, zero_centered, unit) -> int:
     return _UNIT_BEHIND if unit else int(bool(zero_centered))
 
 
-@_flushes
 def qk_norm_rope_store(qkv, heads, kv_heads, head_dim, q_weight, k_weight, eps, zero_centered, cos, sin,
                        k_pool, v_pool, block_table, seq_of_token, positions, page_size, unit=False):
+    if _chain_open:  # (inline, not by the decorator: a mixed step calls this dozens of times)
+        chain_flush()
     n = qkv.shape[0]
     _dense(qkv, "qkv")
     if qkv.shape[1] != (heads + 2 * kv_heads) * head_dim:
@@ -1399,8 +1408,9 @@ def _leading_single_tokens(ctx) -> int:
     return count
 
 
-@_flushes
 def paged_attention(q, k_pool, v_pool, block_table, seq_of_token, positions, scale, window, page_size, ctx=None):
+    if _chain_open:  # (inline, not by the decorator: a mixed step calls this dozens of times)
+        chain_flush()
     n = q.shape[0]
     kh, d = k_pool.shape[1], k_pool.shape[3]
     heads = q.shape[1] // d
