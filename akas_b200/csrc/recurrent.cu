@@ -4,9 +4,10 @@
 // step sizes and decays of the delta rule, the gated RMS norm of the read-out).
 //
 // Everything here is float32 arithmetic whatever the compute dtype; inputs that a matrix product wrote may be
-// bfloat16 and are widened on load. The recurrences run token by token in one fixed order per (request, head,
-// value channel), so a request's results do not depend on how its tokens were cut into steps or on what else
-// is in the batch.
+// bfloat16 and are widened on load. Token by token the recurrences run in one fixed order per (request, head, value
+// channel), so a request's results do not depend on how its tokens were cut into steps or on what else is in the
+// batch; in chunks (see each recurrence for when), chunk borders follow the portion's first token, so results differ
+// between ways of cutting a prompt by rounding.
 //
 // State layouts (one row per request slot; only the slot stride is free, so a state may be part of a wider
 // row): a matrix state is S^T, [heads, value_dim, key_dim] float32, so that the key channels a thread owns are
@@ -93,12 +94,17 @@ template <int KS> __device__ __forceinline__ float group_sum(float v) {
 
 constexpr int kChunk = 64;  // tokens of a chunk of the recurrences that run in chunks
 
+// Chunks of a request's `tokens` in this step; none where they are fewer than `from` (another kernel walks those).
+__device__ __forceinline__ int chunks_of(int tokens, int slot, int from) {
+  return slot < 0 || tokens < from ? 0 : (tokens + kChunk - 1) / kChunk;
+}
+
 // which (request, chunk of it) the block's chunk number is; false if there is none
-__device__ __forceinline__ bool find_chunk(const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int R, int id,
+__device__ __forceinline__ bool find_chunk(const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int R, int from, int id,
                                            int& req, int& first, int& len, int& index) {
   for (int r = 0; r < R; ++r) {
     const int b = cu_seqlens[r], e = cu_seqlens[r + 1];
-    const int chunks = slots[r] < 0 ? 0 : (e - b + kChunk - 1) / kChunk;
+    const int chunks = chunks_of(e - b, slots[r], from);
     if (id < chunks) {
       req = r; index = id; first = b + id * kChunk; len = min(kChunk, e - first);
       return true;
@@ -116,7 +122,7 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
             long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; DELTA: g [N, H] */,
             const float* __restrict__ beta /* DELTA: [N, H] */, float* __restrict__ state, long long slot_stride,
             const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ out, int H, int rep,
-            int D, int V, float q_scale, int write, int act) {
+            int D, int V, float q_scale, int write, int act, int below /* requests with this many tokens or more are not walked here */) {
   constexpr bool DELTA = RULE == RULE_DELTA, FIXED = RULE == RULE_FIXED, GATE = RULE == RULE_GATE;
   constexpr int VT = TH / KS;           // value channels of a block
   constexpr int ROW = KS * (R + kPad);  // floats of a padded shared row of key channels
@@ -129,7 +135,7 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   const int h = blockIdx.x;
   const int req = blockIdx.y, t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
   const int slot = slots[req];
-  if (slot < 0 || t_end <= t_begin) return;
+  if (slot < 0 || t_end <= t_begin || t_end - t_begin >= below) return;
   const int ks = threadIdx.x % KS, jl = threadIdx.x / KS;
   const int j = blockIdx.z * VT + jl;
   const bool live = j < V;
@@ -286,7 +292,7 @@ template <typename T, int RULE>
 int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v, long long ldv, const float* decay,
                 const float* beta, float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out,
                 int tokens, int requests, int H, int rep, int D, int V, float q_scale, int write, cudaStream_t stream,
-                int act = 0) {
+                int act = 0, int below = 0x7fffffff) {
   if (requests <= 0 || H <= 0) return 0;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (D > 1024) return (int)cudaErrorInvalidValue;
@@ -298,7 +304,7 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
   {                                                                                                                       \
     const dim3 grid(H, requests, (V + 256 / KS - 1) / (256 / KS));                                                           \
     return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
-                          decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act);       \
+                          decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act, below); \
   }
   if constexpr (RULE != RULE_DELTA) {  // (which walks such keys with delta_walk_kernel)
     if (D <= 8) AKAS_SCAN(8, 1, 16)
@@ -374,7 +380,7 @@ chunk_state_kernel(const T* __restrict__ k, long long ldk, const T* __restrict__
   float* sv = sk + kChunk * DP;      // [kChunk][kChunkVT], already times a^(len - 1 - s)
   float* pw = sv + kChunk * kChunkVT;  // [kChunk] powers of the decay
   int req, first, len, index;
-  if (!find_chunk(cu_seqlens, slots, R, blockIdx.x, req, first, len, index)) return;
+  if (!find_chunk(cu_seqlens, slots, R, 1, blockIdx.x, req, first, len, index)) return;
   const int h = blockIdx.y, v0 = blockIdx.z * kChunkVT;
   const double a = (double)decay[h];
   for (int i = threadIdx.x; i < kChunk; i += kChunkThreads) pw[i] = (float)pow(a, (double)i);
@@ -453,7 +459,7 @@ chunk_output_kernel(const T* __restrict__ q, long long ldq, const T* __restrict_
   float* sa = sv + kChunk * kChunkVT;    // [kChunk][kChunk] decayed scores, zero above the diagonal
   float* pw = sa + kChunk * kChunk;      // [kChunk + 1] powers of the decay
   int req, first, len, index;
-  if (!find_chunk(cu_seqlens, slots, R, blockIdx.x, req, first, len, index)) return;
+  if (!find_chunk(cu_seqlens, slots, R, 1, blockIdx.x, req, first, len, index)) return;
   const int h = blockIdx.y, v0 = blockIdx.z * kChunkVT;
   const double a = (double)decay[h];
   for (int i = threadIdx.x; i <= kChunk; i += kChunkThreads) pw[i] = (float)pow(a, (double)i);
@@ -611,7 +617,7 @@ walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ 
                   long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; GATE: the logits' bias [H * D] */,
                   const float* __restrict__ low /* GATE: the gates' lower bounds [H * D] */, const int* __restrict__ cu_seqlens,
                   const int* __restrict__ slots, float* __restrict__ out, int H, int D, int V, float q_scale,
-                  float* __restrict__ scratch, float* __restrict__ gates, int requests, int vec) {
+                  float* __restrict__ scratch, float* __restrict__ gates, int requests, int from, int vec) {
   static_assert(RULE == RULE_GLA || RULE == RULE_GATE, "a decay per key channel");
   constexpr int R = kWalkR, NV = kWalkNV, CH = kWalkTokens, TH = kWalkThreads;
   constexpr int VT = TH / KS * NV, W = KS * R, ROW = KS * (R + kPad);
@@ -623,7 +629,7 @@ walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ 
 
   const int h = blockIdx.x;
   int req, t_begin, len, index;
-  if (!find_chunk(cu_seqlens, slots, requests, blockIdx.y, req, t_begin, len, index)) return;
+  if (!find_chunk(cu_seqlens, slots, requests, from, blockIdx.y, req, t_begin, len, index)) return;
   const int t_end = t_begin + len;
   const int ks = threadIdx.x % KS, jl = threadIdx.x / KS, kk0 = ks * R;
   const int v0 = blockIdx.z * VT, j0 = v0 + jl * NV;
@@ -782,13 +788,13 @@ walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ 
 
 __global__ void gate_carry_kernel(const float* __restrict__ gates, float* __restrict__ state, long long slot_stride,
                                   const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ scratch,
-                                  int H, int D, int V, int write) {
+                                  int H, int D, int V, int from, int write) {
   const int req = blockIdx.x, h = blockIdx.y;
   const int slot = slots[req];
-  if (slot < 0) return;
+  const int chunks = chunks_of(cu_seqlens[req + 1] - cu_seqlens[req], slot, from);
+  if (chunks == 0) return;
   int base = 0;  // the number of the request's first chunk
-  for (int r = 0; r < req; ++r) base += slots[r] < 0 ? 0 : (cu_seqlens[r + 1] - cu_seqlens[r] + kChunk - 1) / kChunk;
-  const int chunks = (cu_seqlens[req + 1] - cu_seqlens[req] + kChunk - 1) / kChunk;
+  for (int r = 0; r < req; ++r) base += chunks_of(cu_seqlens[r + 1] - cu_seqlens[r], slots[r], from);
   float* srow = state + (size_t)slot * slot_stride + (size_t)h * V * D;
   for (int i = blockIdx.z * blockDim.x + threadIdx.x; i < V * D; i += gridDim.z * blockDim.x) {
     float s = srow[i];
@@ -808,14 +814,14 @@ __global__ void gate_carry_kernel(const float* __restrict__ gates, float* __rest
         }
       }
     }
-    if (write && chunks > 0) srow[i] = s;
+    if (write) srow[i] = s;
   }
 }
 
 template <typename T, int RULE>
 int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* v, long long ldv, const float* decay, const float* low,
                  float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out, float* scratch, int tokens,
-                 int requests, int H, int D, int V, float q_scale, int write, cudaStream_t stream) {
+                 int requests, int H, int D, int V, float q_scale, int from, int write, cudaStream_t stream) {
   const int chunks = (tokens + kChunk - 1) / kChunk + requests;  // at most: every request may end with a part of a chunk
   float* gates = scratch + (size_t)chunks * H * D * V;
   const size_t four = 4 * sizeof(T);
@@ -824,12 +830,12 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
 #define AKAS_WALK(KS, PART)                                                                                                  \
   launch_ordinary(walk_chunk_kernel<T, KS, RULE, PART>, dim3(H, chunks, (V + kWalkThreads / KS * kWalkNV - 1) / (kWalkThreads / KS * kWalkNV)), \
                   dim3(kWalkThreads), 0, stream, q, ldq, k, ldk, v, ldv, decay, low, cu_seqlens, slots, out, H, D, V, q_scale,   \
-                  scratch, gates, requests, vec)
+                  scratch, gates, requests, from, vec)
 #define AKAS_WALKS(PART) (D <= 16 ? AKAS_WALK(1, PART) : D <= 32 ? AKAS_WALK(2, PART) : D <= 64 ? AKAS_WALK(4, PART) : AKAS_WALK(8, PART))
   int err = AKAS_WALKS(1);
   if (err) return err;
   err = launch_ordinary(gate_carry_kernel, dim3(requests, H, min(64, (V * D + 255) / 256)), dim3(256), 0, stream, (const float*)gates,
-                        state, slot_stride, cu_seqlens, slots, scratch, H, D, V, write);
+                        state, slot_stride, cu_seqlens, slots, scratch, H, D, V, from, write);
   if (err) return err;
   return AKAS_WALKS(2);
 #undef AKAS_WALKS
@@ -1413,21 +1419,27 @@ AKAS_API int akas_gate_scan_chunked(const float* q, long long ldq, const float* 
   if (tokens <= 0 || requests <= 0 || H <= 0) return 0;
   if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr) return (int)cudaErrorInvalidValue;
   return launch_walks<float, RULE_GATE>(q, ldq, f, ldf, v, ldv, f_bias, lower, state, slot_stride, cu_seqlens, slots, out, scratch,
-                                        tokens, requests, H, D, V, 1.f, write, stream);
+                                        tokens, requests, H, D, V, 1.f, 1, write, stream);
 }
 
-// The gated linear attention of akas_gla_scan in chunks; scratch as for akas_gate_scan_chunked.
+// The gated linear attention of akas_gla_scan on bfloat16 rows, in chunks where a request brings at least `from` tokens and
+// token by token where it brings fewer: what a request gets does not hang on how many tokens its neighbours bring. scratch as
+// for akas_gate_scan_chunked. Float32 rows have no such entry: their results do not depend on how a prompt was cut, which no
+// chunk can promise.
 AKAS_API int akas_gla_scan_chunked(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                                    const float* alpha, float* state, long long slot_stride, const int* cu_seqlens, const int* slots,
-                                   float* out, float* scratch, int tokens, int requests, int H, int D, int V, float q_scale, int write,
-                                   int dtype, cudaStream_t stream) {
+                                   float* out, float* scratch, int from, int tokens, int requests, int H, int D, int V, float q_scale,
+                                   int write, cudaStream_t stream) {
   if (tokens <= 0 || requests <= 0 || H <= 0) return 0;
-  if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr) return (int)cudaErrorInvalidValue;
-  if (dtype == AKAS_F32)
-    return launch_walks<float, RULE_GLA>((const float*)q, ldq, (const float*)k, ldk, (const float*)v, ldv, alpha, nullptr, state,
-                                         slot_stride, cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, write, stream);
+  if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr || from < 1) return (int)cudaErrorInvalidValue;
+  if (requests > 1 && from > 1) {
+    const int err = launch_scan<bf16, RULE_GLA>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state,
+                                                slot_stride, cu_seqlens, slots, out, tokens, requests, H, 1, D, V, q_scale, write, stream,
+                                                0, from);
+    if (err) return err;
+  }
   return launch_walks<bf16, RULE_GLA>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state, slot_stride,
-                                      cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, write, stream);
+                                      cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, from, write, stream);
 }
 
 AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv,

@@ -73,7 +73,7 @@ _SIGNATURES = {
         "akas_gla_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
         "akas_gla_scan_chunked": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
-                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
+                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "akas_delta_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_causal_conv_silu": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
@@ -1523,8 +1523,9 @@ def decay_gates(low, w_up, bias, tau):
 
 @_flushes
 def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True, longest=None):
-    """In chunks (three kernels, see csrc/recurrent.cu) when some request of the step brings at least _GATE_CHUNKED_FROM
-    tokens (``longest``) and the key size allows, token by token otherwise."""
+    """bfloat16 rows: requests that bring at least _GATE_CHUNKED_FROM tokens in chunks (three kernels, see csrc/recurrent.cu;
+    ``longest`` says that the step holds one) if the key size allows, the others token by token. float32 rows: token by
+    token, so that a request's results do not depend on how its tokens were cut into steps."""
     n = q.shape[0]
     if q.dtype != k.dtype or q.dtype != v.dtype or alpha.dtype != torch.float32 or not alpha.is_contiguous():
         raise ValueError("gla_scan takes q, k, v of one dtype and a dense float32 alpha")
@@ -1532,14 +1533,16 @@ def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale
     sp, stride = _slot_rows(state, "state")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     head = (qp, ldq, kp, ldk, vp, ldv, _ptr(alpha), sp, stride, _ptr(cu_seqlens), _ptr(slots), _ptr(out))
-    tail = (n, slots.numel(), heads, dim, vdim, float(q_scale), int(bool(write)), _code(q), _stream())
-    if decay_scan_kernels == "auto" and longest is not None and longest >= _GATE_CHUNKED_FROM:
-        words = int(_fn("recurrent", "akas_gate_chunk_scratch")(n, slots.numel(), heads, dim, vdim))
+    requests = slots.numel()
+    tail = (n, requests, heads, dim, vdim, float(q_scale), int(bool(write)))
+    if decay_scan_kernels == "auto" and q.dtype == torch.bfloat16 and longest is not None and longest >= _GATE_CHUNKED_FROM:
+        words = int(_fn("recurrent", "akas_gate_chunk_scratch")(n, requests, heads, dim, vdim))
         if words:
             scratch = torch.empty(words, dtype=torch.float32, device=q.device)
-            _check(_fn("recurrent", "akas_gla_scan_chunked")(*head, _ptr(scratch), *tail), "gla_scan (chunks)", kernels=3)
+            _check(_fn("recurrent", "akas_gla_scan_chunked")(*head, _ptr(scratch), _GATE_CHUNKED_FROM, *tail, _stream()),
+                   "gla_scan (chunks)", kernels=4 if requests > 1 else 3)
             return out
-    _check(_fn("recurrent", "akas_gla_scan")(*head, *tail), "gla_scan")
+    _check(_fn("recurrent", "akas_gla_scan")(*head, *tail, _code(q), _stream()), "gla_scan")
     return out
 
 
@@ -1632,14 +1635,15 @@ def gated_rmsnorm(o, weight, eps, gate, heads, vdim, out_dtype, gate_activation=
     return out
 
 
-# How the recurrence with a constant decay runs: "auto" (default), in chunks (three kernels of float32 products, see
-# csrc/recurrent.cu) when some request of the step brings at least _CHUNKED_FROM tokens and the key size allows, token by
-# token otherwise; "tokens": token by token always.
+# How the recurrences with a decay run: "auto" (default), in chunks (see csrc/recurrent.cu) where the key size allows. The
+# constant decay's when some request of the step brings at least _CHUNKED_FROM tokens, the forget gates' when some request
+# brings at least _GATE_CHUNKED_FROM, and of bfloat16 rows of gated linear attention the requests that bring so many;
+# otherwise, and always with "tokens": token by token.
 decay_scan_kernels = os.environ.get("AKAS_B200_DECAY_SCAN", "auto")
 if decay_scan_kernels not in ("auto", "tokens"):
     raise ValueError(f"AKAS_B200_DECAY_SCAN must be auto or tokens, got {decay_scan_kernels!r}")
 _CHUNKED_FROM = 48
-_GATE_CHUNKED_FROM = 160  # the forget gates' recurrence walks every chunk twice: it pays from three chunks on
+_GATE_CHUNKED_FROM = 160  # the recurrences with a gate per key channel walk every chunk twice: that pays from three chunks on
 
 
 @_flushes

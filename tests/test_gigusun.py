@@ -291,28 +291,70 @@ def test_gla_scan_kernel(heads, dim, vdim, dtype):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,dim,vdim,pad", [(3, 20, 24, 3), (2, 72, 136, 0), (1, 8, 5, 3), (2, 128, 66, 4), (2, 64, 128, 0), (1, 16, 520, 0)])
 def test_gla_scan_in_chunks(heads, dim, vdim, pad, dtype):
-    """Portions around the edges of a chunk (64 tokens), rows that start on four elements and rows that do not, gates from
-    nearly closed to nearly open. The bounds are the token-by-token kernel's: both sum in float32, at most 300 tokens."""
+    """A portion in chunks beside shorter ones that are walked, lengths around the edges of a chunk (64 tokens) and of where
+    chunks begin, rows that start on four elements and rows that do not, gates from nearly closed to nearly open. The bounds
+    are the token-by-token kernel's: both sum in float32, at most 300 tokens."""
     from akas_b200.ops import cuda, reference
 
     cuda.require(["recurrent"])
     g = torch.Generator().manual_seed(heads * 1000 + dim)
-    lengths, slots = [300, 1, 0, 64, 65, 129], [2, 0, -1, 3, 1, 4]
+    lengths, slots = [300, 1, 0, 64, 65, 129, 192, 193, 159], [2, 0, -1, 3, 1, 4, 5, 6, 7]
     n = sum(lengths)
     proj = (torch.randn(n, 2 * heads * dim + heads * vdim + pad, generator=g) * 0.5).to(dtype).cuda()
     q, k, v = proj[:, : heads * dim], proj[:, heads * dim : 2 * heads * dim], proj[:, 2 * heads * dim : 2 * heads * dim + heads * vdim]
     alpha = torch.sigmoid(torch.randn(n, heads * dim, generator=g) * 4 + 3)
     alpha[torch.rand(n, heads * dim, generator=g) < 0.01] = 0.0  # a gate that closes altogether
     alpha = alpha.cuda()
-    state = (torch.randn(5, heads, vdim, dim, generator=g) * 0.3).cuda()
+    state = (torch.randn(8, heads, vdim, dim, generator=g) * 0.3).cuda()
     cu, _, sl = _batch(lengths, slots, "cuda")
     for write in (True, False):
         s_ref, s_got = state.clone(), state.clone()
         want = reference.gla_scan(q, k, v, alpha, s_ref, cu, sl, heads, dim, vdim, dim ** -0.5, write=write)
+        launches = cuda.launch_count
         got = cuda.gla_scan(q, k, v, alpha, s_got, cu, sl, heads, dim, vdim, dim ** -0.5, write=write, longest=300)
+        # two walks and the carry, and the walk of the short portions; float32 rows are walked token by token
+        assert cuda.launch_count - launches == (4 if dtype == torch.bfloat16 else 1)
         _close(got, want, 2e-5, "gla o")
         _close(s_got, s_ref, 2e-5, "gla state")
         assert write or torch.equal(s_got, state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (20, 24)])
+def test_gla_scan_of_a_request_does_not_depend_on_its_company(dim, vdim, dtype):
+    """Requests on both sides of the length from which portions run in chunks, together and alone: the same bits. In float32
+    the same bits too however a prompt was cut."""
+    from akas_b200.ops import cuda
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(dim)
+    edge, heads = cuda._GATE_CHUNKED_FROM, 3
+    lengths, slots = [1, edge, 20, edge - 1, 400, 1], [5, 0, 3, 1, 2, 4]
+    n, hd = sum(lengths), heads * dim
+    proj = (torch.randn(n, 2 * hd + heads * vdim, generator=g) * 0.5).to(dtype).cuda()
+    alpha = torch.sigmoid(torch.randn(n, hd, generator=g) * 2 + 3).cuda()
+    state = (torch.randn(6, heads, vdim, dim, generator=g) * 0.3).cuda()
+
+    def run(rows, s, lens, places):
+        cu, _, sl = _batch(lens, places, "cuda")
+        return cuda.gla_scan(proj[rows, :hd], proj[rows, hd : 2 * hd], proj[rows, 2 * hd :], alpha[rows], s, cu, sl, heads, dim, vdim,
+                             dim ** -0.5, longest=max(lens))
+
+    together, apart = state.clone(), state.clone()
+    want = run(slice(0, n), together, lengths, slots)
+    first = 0
+    for length, slot in zip(lengths, slots):
+        rows = slice(first, first + length)
+        assert torch.equal(run(rows, apart, [length], [slot]), want[rows]), length
+        first += length
+    assert torch.equal(apart, together)
+    if dtype == torch.float32:
+        cut, at = state.clone(), sum(lengths[:4])
+        for piece in (3, 200, edge, 400 - 203 - edge):
+            assert torch.equal(run(slice(at, at + piece), cut, [piece], [2]), want[at : at + piece]), piece
+            at += piece
+        assert torch.equal(cut[2], together[2])
 
 
 @pytest.mark.gpu
