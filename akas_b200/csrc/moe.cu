@@ -15,8 +15,8 @@
 // Experts, token by token (moe_gate_up, moe_down): act[pair] = silu(W_gate h) * (W_up h) for every (token, chosen
 // real expert) pair, then out[n] = sum over the token's chosen outputs of weight * (W_down act, or h for an identity
 // expert), added in the order of the choice. Every output is one warp's sum over the inner size in a fixed order, so
-// a token's result does not depend on what else the step holds. (bfloat16 steps of few pairs and large matrices take an
-// expert's rows once for all of its pairs: "experts, few pairs".) Weights of all experts are stacked: gate and up as
+// a token's result does not depend on what else the step holds. (bfloat16 steps of few pairs take an expert's rows once for
+// all of its pairs where a model's sizes suit that: "experts, few pairs".) Weights of all experts are stacked: gate and up as
 // [experts, 2 F, C] (gate rows first), down as [experts, C, F]. Where the weight multiplies the expert's INPUT
 // (out[n] = sum expert(w h)), moe_gate_up gets the weights and scales both of its float32 sums (W (w h) = w (W h))
 // before the activation, and moe_down gets none. Ungated experts (`plain`, an AKAS_PLAIN_* activation): the stack is
@@ -790,27 +790,41 @@ int allow_smem(K kernel, bool (&done)[64]) {
   return 0;
 }
 
-// Where the two below are the faster ones (us, pair by pair / here, caches cold). A launch of theirs starts about 3 us later (the
-// choice sorted out, the first rows' way), so gate and up want work: 19 M products of 4 pairs of 2,048 x 2,304 9.7 / 11.5, 21 M
-// (1,536 x 3,456) 12.3 / 10.1, 23 M of 8 pairs of 1,024 x 2,816 10.8 / 10.7, 41 M (1,280 x 2,560) 20.1 / 16.1. The down projection also
-// wants long rows, a copy being 65 ns at least (64 experts of 2,048 x 768, 64 pairs: 39.6 / 42.3), and channels enough for every
-// SM that the matrix's rows outnumber the activations (16 pairs of 1,280 x 1,280 12.4 / 14.4, of 768 x 3,072 13.8 / 16.3; of
-// 2,048 x 1,152 20.5 / 17.1, of 1,536 x 1,728 17.7 / 14.7), the work of a second block per SM where they are more than 16 a
-// block (2 pairs of 4,096 x 1,536 11.0 / 11.7, 8 of them 22.4 / 20.3).
-constexpr long long kStreamWork = 20000000;
-inline bool stream_down(int pairs, int C, int F) {
-  return C >= 1536 && F >= 1152 && (long long)pairs * C * F >= kStreamWork / 2 * ((C + 16 * 148 - 1) / (16 * 148));
+// Which models' experts the two below take. The lines go by a model's sizes alone, never by how many pairs a step holds, so that
+// a token's result has the same bits whatever its company, up to kFewPairs. Measured at 1 to 64 pairs of 16 experts, caches cold
+// (us, pair by pair / here):
+//   gate and up: two stages must fit beside the rows of the most tokens (rows stay whole in shared memory: C up to 1,192 where a
+//   token chooses one expert, 1,792 for two, 2,392 for four, 2,872 for eight). A launch of theirs starts 1 to 2 us later (the choice
+//   sorted out, the first rows' way), which one token's experts make up for from C = 1,280 on: four of 1,280 x 1,152 7.2 / 7.8 at
+//   one token, 18 / 14 at four, 29 / 17 at eight; 1,536 x 1,536 12.2 / 9.9, 26 / 20 and 41 / 26; of 1,024 x 1,152 6.6 / 7.3, 16 / 13
+//   and 24 / 16, of 768 x 1,152 5.4 / 7.2, 13 / 13 and 21 / 16, of 1,024 x 128 3 / 4, 5 / 5 and 6 / 6.
+//   down: a copy being 65 ns at least, rows want length and a token more than one expert: four of 1,024 x 960 13.1 / 7.1, 14 / 12
+//   and 22 / 15, of 1,536 x 1,152 11 / 7.8, 14 / 14 and 22 / 18; but of 1,536 x 768 8.4 / 7.3, 11 / 13 and 16 / 17; two of
+//   2,048 x 1,152 6.9 / 6.4, 12 / 11 and 17 / 14, of 1,536 x 1,152 6.6 / 6.1, 8.4 / 9.7 and 13 / 14; one of 2,048 x 1,536 4.8 / 6.0,
+//   8.6 / 8.5 and 12 / 11.
+constexpr int kFewStages = 2;
+inline size_t gate_up_row(int C) { return (size_t)(C + kPad) * sizeof(bf16); }
+inline bool streams_gate_up(int top, int C, int F, bool plain) {
+  return C >= 1024 && C % 32 == 0 && (long long)top * F * (plain ? 1 : 2) >= 2048 &&
+         (kFewStages * kTileRows + kFewPairs / top) * gate_up_row(C) <= kStreamSmem;
+}
+// The channels of a block of the down projection (as many as give every SM one, 16 at most), and a stage of its ring.
+inline int down_channels(int C, int sms) { return min(16, (C + sms - 1) / sms); }
+inline size_t down_stage(int channels, int F) { return (size_t)max(channels + 8, kTileRows) * (F + kPad) * sizeof(bf16); }
+inline bool streams_down(int top, int C, int F, int sms) {
+  const int channels = down_channels(C, sms);
+  return F % 32 == 0 && ((top >= 4 && C >= 1024 && F >= 960) || (top >= 2 && C >= 1792 && F >= 1152)) &&
+         kFewPairs * channels * sizeof(float) + kFewStages * down_stage(channels, F) <= kStreamSmem;
 }
 
-constexpr int kNotTaken = -1;  // the sizes do not fit: nothing was launched
 static_assert(kStreamSmem + sizeof(Chosen) + sizeof(Ring) + 256 <= 227 * 1024, "with the static arrays, what a block may have");
 
 template <bool PLAIN>
 int launch_gate_up_stream(const bf16* h, long long ldh, const bf16* w, const int* chosen, bf16* act, int pairs, int top, int C, int F,
                           int experts, const float* in_weights, int plain, cudaStream_t stream) {
-  const size_t row = (size_t)(C + kPad) * sizeof(bf16), stage = kTileRows * row, xs = (size_t)(pairs / top) * row;
+  const size_t stage = kTileRows * gate_up_row(C), xs = (size_t)(pairs / top) * gate_up_row(C);
   const int sms = sm_count();
-  if (sms <= 0 || xs + 3 * stage > kStreamSmem) return kNotTaken;
+  if (sms <= 0) return (int)cudaErrorInvalidDevice;
   const int stages = (int)min((size_t)kMostStages, (kStreamSmem - xs) / stage);
   static bool done[64] = {};
   const int err = allow_smem(moe_gate_up_stream_kernel<PLAIN>, done);
@@ -824,12 +838,9 @@ int launch_gate_up_stream(const bf16* h, long long ldh, const bf16* w, const int
 int launch_down_stream(const bf16* h, long long ldh, const bf16* w, const int* chosen, const float* weights, const bf16* act, float* out,
                        int pairs, int top, int C, int F, int experts, float* x, const float* a_res, const float* ls_a,
                        const float* ls_b, float mult, const float* shared, const float* shared_gate, long long ldsg,
-                       cudaStream_t stream) {
-  const int sms = sm_count();
-  if (sms <= 0) return kNotTaken;
-  const int channels = min(16, (C + sms - 1) / sms);
-  const size_t stage = (size_t)max(channels + 8, kTileRows) * (F + kPad) * sizeof(bf16), dots = (size_t)pairs * channels * sizeof(float);
-  if (dots + 2 * stage > kStreamSmem) return kNotTaken;
+                       int sms, cudaStream_t stream) {
+  const int channels = down_channels(C, sms);
+  const size_t stage = down_stage(channels, F), dots = (size_t)pairs * channels * sizeof(float);
   const int stages = (int)min((size_t)kMostStages, (kStreamSmem - dots) / stage);
   static bool done[64] = {};
   const int err = allow_smem(moe_down_stream_kernel, done);
@@ -881,21 +892,20 @@ AKAS_API int akas_moe_route(const void* h, long long ldh, const float* w, const 
                          chosen, weights, N, C, R, groups, keep, top, sigmoid, renorm, extra, extras, group_best, wscale);
 }
 
+// few: 0 keeps a step of few pairs on the kernels that walk pair by pair (both entries).
 AKAS_API int akas_moe_gate_up(const void* h, long long ldh, const void* w_gate_up, const int* chosen, void* act, int N,
-                              int top, int C, int F, int experts, int dtype, const float* in_weights, int plain, cudaStream_t stream) {
+                              int top, int C, int F, int experts, int dtype, const float* in_weights, int plain, int few, cudaStream_t stream) {
   if (N <= 0 || top <= 0 || experts <= 0) return 0;
   if (plain < AKAS_PLAIN_NONE || plain > AKAS_PLAIN_SILU) return (int)cudaErrorInvalidValue;
   const int pairs = N * top;
   // few pairs: every chosen expert's rows once through the tensor cores' older path (both sums of a pair, gate and up, end in
-  // one thread), where rows are whole steps of 32 channels and start on 16 bytes and there is enough to multiply
-  if (dtype == AKAS_BF16 && pairs <= kFewPairs && (long long)pairs * (plain ? F : 2 * F) * C >= kStreamWork && C % 32 == 0 &&
-      ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)w_gate_up % 16 == 0) {
-    const int err = plain ? launch_gate_up_stream<true>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
-                                                        experts, in_weights, plain, stream)
-                          : launch_gate_up_stream<false>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
-                                                         experts, in_weights, plain, stream);
-    if (err != kNotTaken) return err;
-  }
+  // one thread), where rows start on 16 bytes
+  if (few && dtype == AKAS_BF16 && (long long)N * top <= kFewPairs && streams_gate_up(top, C, F, plain != 0) && ldh % 8 == 0 &&
+      (uintptr_t)h % 16 == 0 && (uintptr_t)w_gate_up % 16 == 0)
+    return plain ? launch_gate_up_stream<true>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
+                                               experts, in_weights, plain, stream)
+                 : launch_gate_up_stream<false>((const bf16*)h, ldh, (const bf16*)w_gate_up, chosen, (bf16*)act, pairs, top, C, F,
+                                                experts, in_weights, plain, stream);
   // warps enough to fill the GPU when the pairs are few (a row of F per warp), fewer and longer-lived when they are many
   const dim3 grid(pairs, max(1, min((F + 7) / 8, pairs >= 4096 ? 2 : pairs >= 256 ? 16 : 256)));
   if (dtype == AKAS_F32)
@@ -908,20 +918,26 @@ AKAS_API int akas_moe_gate_up(const void* h, long long ldh, const void* w_gate_u
 AKAS_API int akas_moe_down(const void* h, long long ldh, const void* w_down, const int* chosen, const float* weights,
                            const void* act, float* out, int N, int top, int C, int F, int experts, int dtype, float* x,
                            const float* a_res, const float* ls_a, const float* ls_b, float mult, const float* shared,
-                           const float* shared_gate, long long ldsg, cudaStream_t stream) {
+                           const float* shared_gate, long long ldsg, int few, cudaStream_t stream) {
   if (N <= 0) return 0;
-  if (dtype == AKAS_BF16 && N * (long long)top <= kFewPairs && top > 0 && stream_down(N * top, C, F) && F % 32 == 0 &&
-      (uintptr_t)act % 16 == 0 && (uintptr_t)w_down % 16 == 0) {
-    const int err = launch_down_stream((const bf16*)h, ldh, (const bf16*)w_down, chosen, weights, (const bf16*)act, out, N * top, top, C, F,
-                                       experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg, stream);
-    if (err != kNotTaken) return err;
-  }
+  const int sms = sm_count();
+  if (few && dtype == AKAS_BF16 && top > 0 && (long long)N * top <= kFewPairs && sms > 0 && streams_down(top, C, F, sms) &&
+      (uintptr_t)act % 16 == 0 && (uintptr_t)w_down % 16 == 0)
+    return launch_down_stream((const bf16*)h, ldh, (const bf16*)w_down, chosen, weights, (const bf16*)act, out, N * top, top, C, F,
+                              experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg, sms, stream);
   const dim3 grid(N, max(1, min((C + 7) / 8, N >= 2048 ? 2 : N >= 64 ? 32 : 256)));
   if (dtype == AKAS_F32)
     return launch_ordinary(moe_down_kernel<float>, grid, dim3(256), 0, stream, (const float*)h, ldh, (const float*)w_down, chosen,
                            weights, (const float*)act, out, top, C, F, experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg);
   return launch_ordinary(moe_down_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)h, ldh, (const bf16*)w_down, chosen,
                          weights, (const bf16*)act, out, top, C, F, experts, x, a_res, ls_a, ls_b, mult, shared, shared_gate, ldsg);
+}
+
+// Whether the kernels for few pairs take these sizes (bfloat16): 1 for gate and up, 2 for the down projection, or both.
+AKAS_API int akas_moe_few_takes(int top, int C, int F, int plain) {
+  if (top <= 0 || top > kFewPairs || C <= 0 || F <= 0) return 0;
+  const int sms = sm_count();
+  return (streams_gate_up(top, C, F, plain != 0) ? 1 : 0) + (sms > 0 && streams_down(top, C, F, sms) ? 2 : 0);
 }
 
 // 0 unless a bounded wait of the kernels for few pairs has run out on the current device. Synchronises with the device.

@@ -62,11 +62,12 @@ _SIGNATURES = {
         "akas_moe_route": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p],
         "akas_moe_status": [],
+        "akas_moe_few_takes": [c_int, c_int, c_int, c_int],
         "akas_moe_gate_up": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-                             c_void_p, c_int, c_void_p],
+                             c_void_p, c_int, c_int, c_void_p],
         "akas_moe_down": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_longlong,
-                          c_void_p],
+                          c_int, c_void_p],
     },
     "recurrent": {
         "akas_decay_gates": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -1979,8 +1980,9 @@ def moe_route(h, w_router, correction, groups, keep, top, scoring="softmax", ren
 
 
 # Which kernels run the experts in bfloat16: "auto" (default), the grouped product on the tensor cores
-# (csrc/moe_grouped.cu) for steps of more than _MOE_SIMPLE_PAIRS (token, expert) pairs and sizes it takes, the
-# token-by-token kernels (csrc/moe.cu) otherwise; "simple": those for everything.
+# (csrc/moe_grouped.cu) for steps of more than _MOE_SIMPLE_PAIRS (token, expert) pairs and sizes it takes, the kernels of
+# csrc/moe.cu otherwise (a model's sizes choose between those that take an expert's rows once for all of its pairs and
+# those that walk pair by pair); "simple": pair by pair, everything.
 moe_kernels = os.environ.get("AKAS_B200_MOE", "auto")
 if moe_kernels not in ("auto", "simple"):
     raise ValueError(f"AKAS_B200_MOE must be auto or simple, got {moe_kernels!r}")
@@ -2073,12 +2075,13 @@ def moe_experts(h, w_gate_up, w_down, chosen, weights, update=None, weight_input
         return _moe_experts_grouped(h, w_gate_up, w_down, chosen, weights, update, weight_input, shared, activation)
     act = torch.empty((n * top, f), dtype=h.dtype, device=h.device)
     out = torch.empty((n, c), dtype=torch.float32, device=h.device) if update is None else update[0]
+    few = int(moe_kernels == "auto")
     _check(_fn("moe", "akas_moe_gate_up")(hp, ldh, _ptr(_dense(w_gate_up, "w_gate_up")), _ptr(chosen), _ptr(act), n, top, c, f,
                                          experts, _code(h), _ptr(weights) if weight_input else None,
-                                         _READOUT_PLAIN[activation] if activation is not None else 0, _stream()), "moe_gate_up")
+                                         _READOUT_PLAIN[activation] if activation is not None else 0, few, _stream()), "moe_gate_up")
     _check(_fn("moe", "akas_moe_down")(hp, ldh, _ptr(_dense(w_down, "w_down")), _ptr(chosen), None if weight_input else _ptr(weights),
                                       _ptr(act), _ptr(out), n, top, c, f, experts, _code(h), *_update_args(update, n, c),
-                                      *_shared_args(shared, n, c), _stream()), "moe_down")
+                                      *_shared_args(shared, n, c), few, _stream()), "moe_down")
     return out
 
 

@@ -533,16 +533,22 @@ def test_route_of_few_tokens_gives_the_bits_of_many(outputs, count, keep, top, c
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("outputs,experts,top,c,f", [(16, 14, 4, 1536, 1728), (20, 17, 3, 2080, 1152), (6, 5, 2, 2304, 1160), (70, 64, 1, 1536, 1152), (8, 8, 8, 1568, 1184),
-                                                   (6, 5, 4, 4100, 1568), (6, 6, 2, 32, 32)])
+@pytest.mark.parametrize("outputs,experts,top,c,f,takes", [
+    (16, 14, 4, 1536, 1728, (3, 3)), (20, 17, 3, 2080, 1152, (3, 3)), (6, 5, 2, 2304, 1160, (0, 0)), (70, 64, 1, 1536, 1152, (0, 0)),
+    (8, 8, 8, 1568, 1184, (3, 3)), (6, 5, 4, 4100, 1568, (2, 2)), (6, 6, 2, 32, 32, (0, 0)),
+    (16, 14, 4, 1024, 1732, (1, 1)),  # the last tile of hidden channels is not whole (tiles of 8, ungated of 16)
+    (9, 9, 1, 1184, 1056, (1, 0)), (12, 10, 4, 2368, 992, (3, 3)), (8, 8, 8, 2848, 960, (3, 3)), (5, 5, 2, 1792, 1152, (3, 3)),
+    (5, 5, 2, 1824, 1152, (2, 2))])  # widths on both sides of what two stages leave room for
 @pytest.mark.parametrize("options", [dict(), dict(weight_input=True), dict(activation="relu2")], ids=["silu", "weighted", "relu2"])
-def test_experts_of_few_pairs(outputs, experts, top, c, f, options):
-    """bfloat16 steps of one to 64 (token, expert) pairs against the kernels that walk pair by pair (more pairs take those here),
-    with an expert that many tokens chose and outputs that are no experts; a token's results do not depend on its company. The
-    kernels' sums differ in order alone, so an activation can round to the neighbouring bfloat16 (2^-8 of itself at most)."""
+def test_experts_of_few_pairs(outputs, experts, top, c, f, takes, options):
+    """bfloat16 steps of one to 64 (token, expert) pairs against the kernels that walk pair by pair, with an expert that many
+    tokens chose and outputs that are no experts; ``takes``: which of the two products (1: gate and up, 2: down) run on the kernels
+    for few pairs, gated and not. A token's results do not depend on its company. The kernels' sums differ in order alone, so an
+    activation can round to the neighbouring bfloat16 (2^-8 of itself at most)."""
     from akas_b200.ops import cuda
 
     cuda.require(["moe"])
+    assert cuda._fn("moe", "akas_moe_few_takes")(top, c, f, int("activation" in options)) == takes["activation" in options]
     g = torch.Generator().manual_seed(outputs * 100 + c)
     n = 64 // top + 1
     h = torch.randn(n, c, generator=g).to(torch.bfloat16).cuda()
@@ -583,8 +589,9 @@ def test_experts_of_few_pairs(outputs, experts, top, c, f, options):
         rounded = 4e-6 * (1 + updated[:rows].abs() + x0[:rows].abs() + (la * a0[:rows]).abs() + (lb * whole[:rows]).abs())
         assert ((residual - updated[:rows]).abs() <= 0.7 * lb.abs() * 2.0 ** -8 * size[:rows] + rounded).all()
         results.append((got, residual))
-    rows = results[1][0].shape[0]  # (one row may be below the work that the kernels are for)
-    assert torch.equal(results[1][0], results[0][0][:rows]) and torch.equal(results[1][1], results[0][1][:rows])
+    for got, residual in results[1:]:
+        rows = got.shape[0]
+        assert torch.equal(got, results[0][0][:rows]) and torch.equal(residual, results[0][1][:rows])
 
 
 @pytest.mark.gpu
