@@ -339,7 +339,8 @@ sgemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
 }
 
 // Operands whose rows do not start on 16 bytes (K no multiple of 4, or an odd base): tiles BM x BN x 16 through registers,
-// stored k-major, a thread a TM x TN part.
+// stored k-major, a thread a TM x TN part. A thread fetches four neighbouring k of a row (one k a thread, 16 threads a row,
+// stored down a column into two banks: 1,024 x 4,606 with one row 684 us, 293 so).
 template <int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 sgemm_any_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
@@ -358,13 +359,17 @@ sgemm_any_kernel(const float* __restrict__ x, const float* __restrict__ w, float
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
   for (int k0 = 0; k0 < K; k0 += kBK) {
-    for (int i = tid; i < BM * kBK; i += NT) {
-      const int r = i / kBK, c = i % kBK;
-      As[c][r] = row0 + r < N && k0 + c < K ? x[(size_t)(row0 + r) * K + k0 + c] : 0.f;
+    for (int i = tid; i < BM * (kBK / 4); i += NT) {
+      const int r = i / (kBK / 4), c = (i % (kBK / 4)) * 4;
+      const float* p = x + (size_t)(row0 + r) * K + k0 + c;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) As[c + j][r] = row0 + r < N && k0 + c + j < K ? p[j] : 0.f;
     }
-    for (int i = tid; i < BN * kBK; i += NT) {
-      const int r = i / kBK, c = i % kBK;
-      Bs[c][r] = col0 + r < O && k0 + c < K ? w[(size_t)(col0 + r) * K + k0 + c] : 0.f;
+    for (int i = tid; i < BN * (kBK / 4); i += NT) {
+      const int r = i / (kBK / 4), c = (i % (kBK / 4)) * 4;
+      const float* p = w + (size_t)(col0 + r) * K + k0 + c;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Bs[c + j][r] = col0 + r < O && k0 + c + j < K ? p[j] : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -431,13 +436,20 @@ int launch_few(const float* x, const float* w, float* y, const float* residual, 
 //   64 x 64 tiles up to 511 rows: 1,024 x 1,024 with 128 rows 38 (185), 300 rows 39 (185); 9,216 x 1,024 with 300 rows 141 (276;
 //     128 x 64 tiles 147). Tiles of 128 x 64 from there on: 9,216 x 1,024 with 723 rows 281 (524; 64 x 64 tiles 322), with
 //     2,048 rows 732 (1,056): 53 TFLOP/s. Up to 32 rows against a wide w, 32 x 32 tiles: 16,384 x 2,048 135 (197; 64 x 64 181).
+//   rows off 16 bytes: 16 x 64 tiles up to 16 rows (4,096 x 1,022 with 16 rows 66; 32 x 64 tiles of one k a thread 174), 32 x 64 up to
+//     64 (with 17 rows 80), 128 x 128 from there on (with 300 rows 230, with 2,048 595; 32 x 64 tiles 853).
 AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* residual, int N, int O, int K,
                         cudaStream_t stream) {
   if (N <= 0 || O <= 0) return 0;
   if (K <= 0) return (int)cudaErrorInvalidValue;
   const bool rows_on_16_bytes = (K % 4 == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0);
   if (!rows_on_16_bytes) {
-    sgemm_any_kernel<32, 64, 2, 4><<<dim3((O + 63) / 64, (N + 31) / 32), 256, 0, stream>>>(x, w, y, residual, N, O, K);
+    if (N > 64)
+      sgemm_any_kernel<128, 128, 8, 8><<<dim3((O + 127) / 128, (N + 127) / 128), 256, 0, stream>>>(x, w, y, residual, N, O, K);
+    else if (N > 16)
+      sgemm_any_kernel<32, 64, 2, 4><<<dim3((O + 63) / 64, (N + 31) / 32), 256, 0, stream>>>(x, w, y, residual, N, O, K);
+    else
+      sgemm_any_kernel<16, 64, 1, 4><<<dim3((O + 63) / 64, 1), 256, 0, stream>>>(x, w, y, residual, N, O, K);
     return launch_status();
   }
   const bool wide = O >= 8192;

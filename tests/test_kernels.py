@@ -119,6 +119,25 @@ def test_linear_float32_every_kernel_gives_the_same_bits(ops, k, o):
         assert torch.equal(cuda.linear(x[:n], w, residual=res[:n].clone()), added[:n]), n
 
 
+@pytest.mark.parametrize("k,o", [(70, 130), (33, 300), (5, 64)])
+def test_linear_float32_rows_off_16_bytes(ops, k, o):
+    """An inner size that is no multiple of 4: every tile shape (up to 16, up to 64 and more rows) gives a row the same bits."""
+    cuda, _ = ops
+    x, w, res = _rand((300, k), torch.float32, 14), _rand((o, k), torch.float32, 15), _rand((300, o), torch.float32, 16)
+    want, added = cuda.linear(x, w), cuda.linear(x, w, residual=res.clone())
+    _close(want, x.double() @ w.double().T, torch.float32, "product")
+    for n in (1, 16, 17, 64, 65, 129):
+        assert torch.equal(cuda.linear(x[:n], w), want[:n]), n
+        assert torch.equal(cuda.linear(x[:n], w, residual=res[:n].clone()), added[:n]), n
+
+
+def test_linear_float32_of_millions_of_rows_off_16_bytes(ops):
+    """More rows than 65,535 tiles of 32 hold."""
+    cuda, _ = ops
+    x, w = _rand((65535 * 32 + 70, 2), torch.float32, 17), _rand((3, 2), torch.float32, 18)
+    _close(cuda.linear(x, w), x.double() @ w.double().T, torch.float32, "product")
+
+
 @pytest.mark.parametrize("n,k,o", [(1, 64, 50), (17, 104, 37), (70, 56, 130), (300, 96, 192), (8, 2048, 321)])
 def test_linear_bfloat16(ops, n, k, o):
     cuda, ref = ops
