@@ -296,7 +296,8 @@ sgemm_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
     for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&tile[buffer][load_row + 8 * j][load_k]) = next[j];
   };
 
-  chain_release();
+  // (No early release: the next launch's blocks would take the places of this one's that have not begun yet. 8,192 x 1,024 with
+  // 16 rows, launch after launch: 41 us with it, 24 so.)
   fetch(0);  // weights: no kernel writes them
   chain_wait();
   int buffer = 0;
@@ -411,17 +412,7 @@ int launch_tile(const float* x, const float* w, float* y, const float* residual,
 template <int TOK, int STAGES>
 int launch_few(const float* x, const float* w, float* y, const float* residual, int N, int O, int K, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (kFewRows + 4 * TOK) * kFewPitch * sizeof(float);
-  static_assert(smem <= 227 * 1024, "the ring fits a block");
-  if (smem > 48 * 1024) {
-    static bool configured[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
-    if (!configured[device]) {
-      const cudaError_t e = cudaFuncSetAttribute(sgemm_few_kernel<TOK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return (int)e;
-      configured[device] = true;
-    }
-  }
+  static_assert(smem <= 48 * 1024, "the ring fits what a block has without asking");
   return launch_chained(sgemm_few_kernel<TOK, STAGES>, dim3((O + kFewRows - 1) / kFewRows), dim3(32), smem, stream, x, w, y, residual, N, O, K);
 }
 
@@ -431,8 +422,13 @@ int launch_few(const float* x, const float* w, float* y, const float* residual, 
 //
 // Which kernel, from times on a B200 (us; the kernels before were 128 x 128 tiles from 65 rows on, 32 x 64 tiles from 17, and
 // sgemm_wide_kernel up to 16 rows):
-//   up to 4 rows, a warp per 8 rows of w: w of 1,024 x 4,608 18.5 (58.6 before), 9,216 x 1,024 16.2 (17.4), 65,536 x 1,024 72
-//     (79). Eight rows: 30.6 (67), 30 (21), 109 (89), so from 5 rows on a wide w stays with the kernel of 32 rows a block.
+//   up to 4 rows, a warp per 8 rows of w: one row against 1,024 x 4,608 17 (53 before), 8,192 x 1,024 12 (15), 65,536 x 1,024 66
+//     (72); four rows 18 (57), 14 (16), 83 (76).
+//   5 to 16 rows: the same against a narrow w, a block per 32 rows of a wide one. Five rows (narrow / wide): 4,096 x 1,024 14 / 16,
+//     5,120 x 1,024 18 / 17, 6,144 x 2,048 35 / 32, 16,384 x 2,048 71 / 53; sixteen: 2,048 x 2,048 29 / 35, 3,072 x 2,048 37 / 35,
+//     4,096 x 1,024 24 / 18, 6,144 x 2,048 55 / 45.
+//   17 rows (32 x 64 tiles before): 512 x 512 18 (28), 1,024 x 1,024 35 (54), 4,096 x 1,024 47 (79); 64 rows 19 (29), 37 (55), 48 (76);
+//     65 rows (128 x 128 before) 19 (88), 37 (172), 61 (211).
 //   64 x 64 tiles up to 511 rows: 1,024 x 1,024 with 128 rows 38 (185), 300 rows 39 (185); 9,216 x 1,024 with 300 rows 141 (276;
 //     128 x 64 tiles 147). Tiles of 128 x 64 from there on: 9,216 x 1,024 with 723 rows 281 (524; 64 x 64 tiles 322), with
 //     2,048 rows 732 (1,056): 53 TFLOP/s. Up to 32 rows against a wide w, 32 x 32 tiles: 16,384 x 2,048 135 (197; 64 x 64 181).
@@ -452,7 +448,7 @@ AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* r
       sgemm_any_kernel<16, 64, 1, 4><<<dim3((O + 63) / 64, 1), 256, 0, stream>>>(x, w, y, residual, N, O, K);
     return launch_status();
   }
-  const bool wide = O >= 8192;
+  const bool wide = O >= (N > 16 ? 8192 : N > 8 ? 4096 : 5120);
   if (N <= 4) return launch_few<1, 12>(x, w, y, residual, N, O, K, stream);
   if (N <= 16 && wide) {
     const dim3 grid((O + 31) / 32);

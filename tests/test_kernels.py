@@ -105,7 +105,7 @@ def test_linear_float32_rows_do_not_depend_on_the_batch(ops):
             assert torch.equal(cuda.linear(x[rows].contiguous(), w, residual=res[rows].clone()), added[rows])
 
 
-@pytest.mark.parametrize("k,o", [(68, 8200), (132, 257), (1024, 72), (16, 65)])
+@pytest.mark.parametrize("k,o", [(68, 8200), (132, 257), (1024, 72), (16, 65), (68, 5124), (36, 4100)])
 def test_linear_float32_every_kernel_gives_the_same_bits(ops, k, o):
     """Row counts on both sides of every line between the float32 product's kernels (4, 8, 16, 32, 511 rows; a wide w and a
     narrow one; remainders of tiles and of stages), against the kernel for operands whose rows do not start on 16 bytes."""
