@@ -1227,9 +1227,9 @@ def kv_store(k, v, k_pool, v_pool, block_table, seq_of_token, positions, page_si
                                        _code(k_pool), _stream()), "kv_store")
 
 
-# Which kernel runs attention over prompt portions in bfloat16: "mma" (the mma.sync kernel, 64-query tiles),
-# "tcgen05" (the tensor-memory kernel, 128-query tiles, where it takes the sizes: head size 64, page size a multiple
-# of 64) or "auto": the tensor-memory kernel when the step's requests mostly bring more than 64 tokens. Measured on
+# Which kernel runs attention over prompt portions in bfloat16 (the general attention's with a sink and no other option
+# too, where "tcgen05" means "auto"): "mma" (the mma.sync kernels, 64-query tiles), "tcgen05" (the tensor-memory kernel,
+# 128-query tiles, where it takes the sizes: head size 64, page size a multiple of 64) or "auto": the tensor-memory kernel when the step's requests mostly bring more than 64 tokens. Measured on
 # the 1.2B shape: 222 against 182 TFLOP/s at 2,048 tokens, 392 against 220 at 8,192 (mma.sync peaks at 550 here).
 prompt_attention = os.environ.get("AKAS_B200_PROMPT_ATTENTION", "auto")
 if prompt_attention not in ("auto", "tcgen05", "mma"):
@@ -1808,8 +1808,9 @@ def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, s
         if launches and all(0 < tiles <= 65535 for _, _, tiles, _ in launches):
             for start, requests, tiles, packed in launches:
                 # A sink at most beside the plain softmax, and prompts of more than 64 tokens: the tensor-memory kernel of the
-                # plain attention (its rule for the tiles; 12 heads, 2,048 tokens: see attention_prefill_tc.cu)
-                if (not packed and not softcap and r1 is None and gate is None and blocks is None and not (window and keep_first)
+                # plain attention (its rule for the tiles and its switch; 12 heads, one prompt of 2,048 tokens: 32 us against 87).
+                # It takes a row's maximum before the scale, so the scale must be positive.
+                if (not packed and prompt_attention != "mma" and scale > 0 and not softcap and r1 is None and gate is None and blocks is None and not (window and keep_first)
                         and d == 64 and vd == 64 and vpitch == 64 and page_size % 64 == 0
                         and 0 < sum(-(-c // 128) for c in lens[start:]) <= 0.9 * tiles):
                     err = _fn("attention_prefill_tc", "akas_prefill_attention_tc_sinks")(

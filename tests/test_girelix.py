@@ -650,7 +650,7 @@ def test_routed_experts_kernels(outputs, experts, count, keep, top, c, f, dtype)
 @pytest.mark.parametrize("lengths,starts,heads,kv_heads,page,window,sink", [
     ([129, 300, 65], [0, 77, 301], 6, 2, 64, None, "learned"), ([1, 128, 257], [150, 0, 63], 4, 4, 128, None, "unit"),
     ([200, 1, 66], [5, 9, 190], 3, 1, 64, 100, "learned"), ([130], [0], 2, 1, 192, 64, "none")])
-def test_sinks_on_the_tensor_memory_kernel(lengths, starts, heads, kv_heads, page, window, sink):
+def test_sinks_on_the_tensor_memory_kernel(lengths, starts, heads, kv_heads, page, window, sink, monkeypatch):
     """Head size 64 and portions of more than 64 tokens: the tensor-memory kernel with a sink per head, a unit sink or none,
     under a window, a request's single token in front, rows of the caller's pitch and a scale. A sink of 20 leaves a row
     almost nothing, one of -20 everything. The bound is that of the kernel's plain calls (bfloat16 weights and values)."""
@@ -677,10 +677,53 @@ def test_sinks_on_the_tensor_memory_kernel(lengths, starts, heads, kv_heads, pag
     want = reference.attention_general(q, *args, sinks=sinks, out_scale=1.2)
     wide = torch.zeros(n, heads * dim + 16, dtype=torch.bfloat16, device="cuda")
     view = wide[:, 8 : 8 + heads * dim]
+    entries = _entries(cuda, monkeypatch)
     cuda.attention_general(q, *args, ctx, sinks=sinks, out=view, out_scale=1.2)
+    assert ("akas_prefill_attention_tc_sinks", 0) in entries
     _close(view, want, 1e-2, "sinks")
     assert float(wide[:, :8].abs().max()) == 0.0 and float(wide[:, 8 + heads * dim :].abs().max()) == 0.0
     assert cuda.prefill_attention_tc_status() == 0
+
+
+def _entries(cuda, monkeypatch):
+    """The C entries that are called from here on, with what they return."""
+    entries, real = [], cuda._fn
+
+    def entry(lib, name):
+        fn = real(lib, name)
+
+        def call(*args):
+            entries.append((name, fn(*args)))
+            return entries[-1][1]
+
+        return call
+
+    monkeypatch.setattr(cuda, "_fn", entry)
+    return entries
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale,switch,tensor_memory", [(0.3, "auto", True), (0.3, "mma", False), (0.0, "auto", False), (-0.3, "auto", False)])
+def test_sinks_leave_other_scales_to_the_general_kernel(scale, switch, tensor_memory, monkeypatch):
+    """The tensor-memory kernel takes a row's maximum before the scale: a scale that is not positive stays with the kernel
+    that scales first, and so does everything where AKAS_B200_PROMPT_ATTENTION says "mma"."""
+    from types import SimpleNamespace
+
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["attention_general", "attention_general_tc", "attention_prefill_tc"])
+    g = torch.Generator().manual_seed(5)
+    k_pool, v_pool = (torch.randn(4, 1, 64, 64, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    q = (torch.randn(250, 128, generator=g) * 0.5).to(torch.bfloat16).cuda()
+    cu, seq, _ = _batch([250], [0], "cuda")
+    table, pos, sinks = torch.arange(4).int().view(1, 4).cuda(), torch.arange(250).int().cuda(), torch.tensor([0.5, -1.0]).cuda()
+    ctx = SimpleNamespace(query_lens=(250,), decode_only=False, cu_seqlens=cu, max_context=250)
+    args = (k_pool, v_pool, table, seq, pos, scale, None, 0, 0.0, None, None, False, None, 64)
+    monkeypatch.setattr(cuda, "prompt_attention", switch)
+    entries = _entries(cuda, monkeypatch)
+    got = cuda.attention_general(q, *args, ctx, sinks=sinks)
+    assert [name for name, _ in entries if "tc_takes" not in name] == ["akas_prefill_attention_tc_sinks" if tensor_memory else "akas_attention_general_tc"]
+    _close(got, reference.attention_general(q, *args, sinks=sinks), 1e-2, "sinks")
 
 
 @pytest.mark.gpu
