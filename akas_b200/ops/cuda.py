@@ -1741,6 +1741,15 @@ if general_attention not in ("mma", "plain"):
 general_splits = os.environ.get("AKAS_B200_GENERAL_SPLITS", "1") != "0"  # 0: a decoding request's keys are never cut into parts
 
 
+def _short_walks(lens, max_context) -> bool:
+    """Whether most tokens of these portions see few keys: no request of the step reaches further back than the longest
+    portion, and a token's portion has at most 192 tokens on average. A half-filled 128-query tile of the tensor-memory
+    kernel then costs more than the 64-query tiles of the mma.sync kernel (12 heads, us, tensor memory / mma.sync: one
+    prompt of 100 tokens 9.1 / 7.8, sixteen 15.1 / 10.3, sixteen of 192 24.1 / 19.0, of 256 26.6 / 27.4, one of 200 10.4 /
+    12.2, sixty of 100 and one of 500 64 / 38; behind 500 tokens of the past sixteen of 70 26.6 / 32.6)."""
+    return max_context <= max(lens) and sum(c * c for c in lens) <= 192 * sum(lens)
+
+
 @_flushes
 def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, scale, window, keep_first, softcap,
                       r1, r2, sink, gate, page_size, ctx=None, sinks=None, out=None, out_scale=1.0, values_in_keys=0,
@@ -1812,7 +1821,8 @@ def attention_general(q, k_pool, v_pool, block_table, seq_of_token, positions, s
                 # It takes a row's maximum before the scale, so the scale must be positive.
                 if (not packed and prompt_attention != "mma" and scale > 0 and not softcap and r1 is None and gate is None and blocks is None and not (window and keep_first)
                         and d == 64 and vd == 64 and vpitch == 64 and page_size % 64 == 0
-                        and 0 < sum(-(-c // 128) for c in lens[start:]) <= 0.9 * tiles):
+                        and 0 < sum(-(-c // 128) for c in lens[start:]) <= 0.9 * tiles
+                        and not _short_walks(lens[start:], getattr(ctx, "max_context", 0) or 0)):
                     err = _fn("attention_prefill_tc", "akas_prefill_attention_tc_sinks")(
                         _ptr(q), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0] * k_pool.shape[1] * k_pool.shape[2],
                         _ptr(block_table[start:]), block_table.shape[1], _ptr(ctx.cu_seqlens[start:]), _ptr(positions), op,

@@ -726,6 +726,15 @@ def test_sinks_leave_other_scales_to_the_general_kernel(scale, switch, tensor_me
     _close(got, reference.attention_general(q, *args, sinks=sinks), 1e-2, "sinks")
 
 
+@pytest.mark.parametrize("lengths,max_context,short", [
+    ([192], 192, True), ([193], 193, False), ([100] * 4, 100, True), ([100] * 4, 101, False), ([70] * 15 + [500], 500, False),
+    ([100] * 60 + [500], 500, True), ([2048], 2048, False), ([65], 0, True)])
+def test_which_portions_are_short(lengths, max_context, short):
+    from akas_b200.ops import cuda
+
+    assert cuda._short_walks(lengths, max_context) is short
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,dim,rot,page", [(6, 2, 24, 16, 8), (4, 4, 16, 16, 16), (3, 1, 20, 6, 4), (36, 2, 8, 0, 64),
