@@ -116,13 +116,15 @@ __device__ __forceinline__ bool find_chunk(const int* __restrict__ cu_seqlens, c
 
 enum { RULE_GLA = 0, RULE_DELTA = 1, RULE_FIXED = 2, RULE_GATE = 3 };
 
-template <typename T, int R, int KS, int CH, int TH, int RULE>
+// SHORT: requests with `below` tokens or more are another kernel's. (Compile-time: with the comparison in every instance the
+// float32 GLA walk of 64 keys got 80 registers instead of 95, three blocks an SM, and its chain 7 % longer.)
+template <typename T, int R, int KS, int CH, int TH, int RULE, bool SHORT>
 __global__ void __launch_bounds__(TH)
 scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk, const T* __restrict__ v,
             long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; DELTA: g [N, H] */,
             const float* __restrict__ beta /* DELTA: [N, H] */, float* __restrict__ state, long long slot_stride,
             const int* __restrict__ cu_seqlens, const int* __restrict__ slots, float* __restrict__ out, int H, int rep,
-            int D, int V, float q_scale, int write, int act, int below /* requests with this many tokens or more are not walked here */) {
+            int D, int V, float q_scale, int write, int act, int below) {
   constexpr bool DELTA = RULE == RULE_DELTA, FIXED = RULE == RULE_FIXED, GATE = RULE == RULE_GATE;
   constexpr int VT = TH / KS;           // value channels of a block
   constexpr int ROW = KS * (R + kPad);  // floats of a padded shared row of key channels
@@ -135,7 +137,8 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   const int h = blockIdx.x;
   const int req = blockIdx.y, t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
   const int slot = slots[req];
-  if (slot < 0 || t_end <= t_begin || t_end - t_begin >= below) return;
+  if (slot < 0 || t_end <= t_begin) return;
+  if (SHORT && t_end - t_begin >= below) return;
   const int ks = threadIdx.x % KS, jl = threadIdx.x / KS;
   const int j = blockIdx.z * VT + jl;
   const bool live = j < V;
@@ -288,11 +291,11 @@ scan_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, lon
   }
 }
 
-template <typename T, int RULE>
+template <typename T, int RULE, bool SHORT = false>
 int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v, long long ldv, const float* decay,
                 const float* beta, float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out,
                 int tokens, int requests, int H, int rep, int D, int V, float q_scale, int write, cudaStream_t stream,
-                int act = 0, int below = 0x7fffffff) {
+                int act = 0, int below = 0) {
   if (requests <= 0 || H <= 0) return 0;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (D > 1024) return (int)cudaErrorInvalidValue;
@@ -303,7 +306,7 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
 #define AKAS_SCAN(R, KS, CH)                                                                                              \
   {                                                                                                                       \
     const dim3 grid(H, requests, (V + 256 / KS - 1) / (256 / KS));                                                           \
-    return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
+    return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE, SHORT>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
                           decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act, below); \
   }
   if constexpr (RULE != RULE_DELTA) {  // (which walks such keys with delta_walk_kernel)
@@ -313,6 +316,7 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
     if (D <= 64) AKAS_SCAN(16, 4, 16)
     if (D <= 128) AKAS_SCAN(16, 8, 16)
   }
+  if constexpr (SHORT) return (int)cudaErrorInvalidValue;  // (larger keys do not run in chunks)
   if (D <= 256) AKAS_SCAN(16, 16, 8)
   if (D <= 512) AKAS_SCAN(16, 32, 4)
   AKAS_SCAN(32, 32, 2)
@@ -1433,9 +1437,9 @@ AKAS_API int akas_gla_scan_chunked(const void* q, long long ldq, const void* k, 
   if (tokens <= 0 || requests <= 0 || H <= 0) return 0;
   if (akas_gate_chunk_scratch(tokens, requests, H, D, V) == 0 || scratch == nullptr || from < 1) return (int)cudaErrorInvalidValue;
   if (requests > 1 && from > 1) {
-    const int err = launch_scan<bf16, RULE_GLA>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state,
-                                                slot_stride, cu_seqlens, slots, out, tokens, requests, H, 1, D, V, q_scale, write, stream,
-                                                0, from);
+    const int err = launch_scan<bf16, RULE_GLA, true>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state,
+                                                      slot_stride, cu_seqlens, slots, out, tokens, requests, H, 1, D, V, q_scale, write,
+                                                      stream, 0, from);
     if (err) return err;
   }
   return launch_walks<bf16, RULE_GLA>((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, alpha, nullptr, state, slot_stride,
