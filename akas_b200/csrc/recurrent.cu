@@ -309,10 +309,10 @@ int launch_scan(const T* q, long long ldq, const T* k, long long ldk, const T* v
     return launch_ordinary(scan_kernel<T, R, KS, CH, 256, RULE, SHORT>, grid, dim3(256), 0, stream, q, ldq, k, ldk, v, ldv,   \
                           decay, beta, state, slot_stride, cu_seqlens, slots, out, H, rep, D, V, q_scale, write, act, below); \
   }
+  if (D <= 8) AKAS_SCAN(8, 1, 16)
+  if (D <= 16) AKAS_SCAN(8, 2, 16)
+  if (D <= 32) AKAS_SCAN(8, 4, 16)
   if constexpr (RULE != RULE_DELTA) {  // (which walks such keys with delta_walk_kernel)
-    if (D <= 8) AKAS_SCAN(8, 1, 16)
-    if (D <= 16) AKAS_SCAN(8, 2, 16)
-    if (D <= 32) AKAS_SCAN(8, 4, 16)
     if (D <= 64) AKAS_SCAN(16, 4, 16)
     if (D <= 128) AKAS_SCAN(16, 8, 16)
   }
@@ -846,9 +846,9 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
 #undef AKAS_WALK
 }
 
-// ------------------------------------------------------------------------------------------------ delta rule, small keys
+// ------------------------------------------------------------------------------------------------ delta rule, 33 to 128 keys
 //
-// The delta rule of scan_kernel for keys of up to 128 channels. A token's u waits for the sums over the keys, and the next
+// The delta rule of scan_kernel for keys of 33 to 128 channels. A token's u waits for the sums over the keys, and the next
 // token's sums for its u: a walk is a chain of such rounds, so what a round holds beside its arithmetic is what costs.
 // A thread owns 16 key channels of NV value channels (see the launch); the decay is applied after the sums (S^T k of the state as it stands,
 // times g) and to the state while the lanes' sums meet; the read-out's sums are nobody's input and run under the next
@@ -1022,8 +1022,6 @@ int launch_delta_walk(const float* q, long long ldq, const float* k, long long l
   // / one channel / two): a prompt of 2,048 tokens (128 blocks of one channel) 670 / 485 / 625, of 512 170 / 123 / 158, two of 1,337
   // and 2,048 (256) 671 / 624 / 628, sixteen of 300 526 / 486 / 329, one token of 8 requests 8.5 / 6.9 / 5.4, of 64 47 / 36 / 28.5.
   const bool alone = (long long)H * requests * ((V + kDeltaThreads / 8 - 1) / (kDeltaThreads / 8)) <= 148;
-  if (D <= 16) AKAS_DELTA(1, 2);
-  if (D <= 32) AKAS_DELTA(2, 2);
   if (D <= 64) AKAS_DELTA(4, 2);
   if (alone) AKAS_DELTA(8, 1);
   AKAS_DELTA(8, 2);
@@ -1451,7 +1449,9 @@ AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long
                              const int* slots, float* out, int tokens, int requests, int H, int G, int D, int V, int write,
                              cudaStream_t stream) {
   if (G <= 0 || H % G) return (int)cudaErrorInvalidValue;
-  if (D <= 128)
+  // (keys of up to 32 channels leave the walk's threads two lanes a value channel to share the sums with: 8 heads of 32 x 64, a
+  // prompt of 2,048 tokens, 508 us against 432 of scan_kernel; 4 of 16 x 16, 256 requests of one token, 9.0 against 6.1)
+  if (D > 32 && D <= 128)
     return launch_delta_walk(q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, requests, H, H / G, D, V,
                              write, stream);
   return launch_scan<float, RULE_DELTA>(q, ldq, k, ldk, v, ldv, g, beta, state, slot_stride, cu_seqlens, slots, out, tokens,
