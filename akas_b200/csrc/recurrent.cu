@@ -868,12 +868,14 @@ delta_walk_kernel(const float* __restrict__ q, long long ldq, const float* __res
   __shared__ __align__(16) float sk[CH][W];
   __shared__ __align__(16) float sv[CH][VT];
   __shared__ float sg[CH], sb[CH];
-  const int h = blockIdx.x, req = blockIdx.y, hk = h / rep;
+  // The last request's blocks first: a step's single tokens stand in front of its prompts, whose long walks then begin on empty
+  // SMs, one on each (16 heads, a prompt of 2,048 behind 15 single tokens: in the requests' order 815 us).
+  const int h = blockIdx.x, req = gridDim.z - 1 - blockIdx.z, hk = h / rep;
   const int t_begin = cu_seqlens[req], t_end = cu_seqlens[req + 1];
   const int slot = slots[req];
   if (slot < 0 || t_end <= t_begin) return;
   const int ks = threadIdx.x % KS, jl = threadIdx.x / KS;
-  const int v0 = blockIdx.z * VT, j0 = v0 + jl * NV;
+  const int v0 = blockIdx.y * VT, j0 = v0 + jl * NV;
 
   float s[NV][16];
   float* srow = state + (size_t)slot * slot_stride + ((size_t)h * V + j0) * D;
@@ -1008,20 +1010,24 @@ delta_walk_kernel(const float* __restrict__ q, long long ldq, const float* __res
 
 int launch_delta_walk(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, const float* beta,
                       const float* g, float* state, long long slot_stride, const int* cu_seqlens, const int* slots, float* out,
-                      int requests, int H, int rep, int D, int V, int write, cudaStream_t stream) {
+                      int tokens, int longest, int requests, int H, int rep, int D, int V, int write, cudaStream_t stream) {
   if (requests <= 0 || H <= 0) return 0;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   const int vec = D % 4 == 0 && V % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && (uintptr_t)q % 16 == 0 &&
                   (uintptr_t)k % 16 == 0 && (uintptr_t)v % 16 == 0;
 #define AKAS_DELTA(KS, NV)                                                                                                    \
-  return launch_ordinary(delta_walk_kernel<KS, NV>, dim3(H, requests, (V + kDeltaThreads / KS * NV - 1) / (kDeltaThreads / KS * NV)), \
+  return launch_ordinary(delta_walk_kernel<KS, NV>, dim3(H, (V + kDeltaThreads / KS * NV - 1) / (kDeltaThreads / KS * NV), requests), \
                          dim3(kDeltaThreads), 0, stream, q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, \
                          H, rep, D, V, write, vec)
   // One value channel a thread where the blocks that gives still have an SM each: a round of the walk is then shorter, one more
   // block costs nothing. With more of them two channels share what a round reads of q and k. 16 heads, D = V = 128 (us, scan_kernel
   // / one channel / two): a prompt of 2,048 tokens (128 blocks of one channel) 670 / 485 / 625, of 512 170 / 123 / 158, two of 1,337
   // and 2,048 (256) 671 / 624 / 628, sixteen of 300 526 / 486 / 329, one token of 8 requests 8.5 / 6.9 / 5.4, of 64 47 / 36 / 28.5.
-  const bool alone = (long long)H * requests * ((V + kDeltaThreads / 8 - 1) / (kDeltaThreads / 8)) <= 148;
+  // A request counts there by its share of the longest portion (`longest`; 0: not known, every request counts whole): the blocks of
+  // short ones are gone when the long walk is still at its beginning (a prompt of 2,048 behind 15 single tokens, 8 heads: 865 /
+  // 485 / 627; 16 heads 680 / 621 / 626).
+  const long long blocks = (long long)H * ((V + kDeltaThreads / 8 - 1) / (kDeltaThreads / 8));
+  const bool alone = longest > 0 ? blocks * tokens <= 148LL * longest : blocks * requests <= 148;
   if (D <= 64) AKAS_DELTA(4, 2);
   if (alone) AKAS_DELTA(8, 1);
   AKAS_DELTA(8, 2);
@@ -1444,16 +1450,17 @@ AKAS_API int akas_gla_scan_chunked(const void* q, long long ldq, const void* k, 
                                       cu_seqlens, slots, out, scratch, tokens, requests, H, D, V, q_scale, from, write, stream);
 }
 
+// longest: the most tokens that a request brings in this step, where the caller knows it (0: it does not).
 AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv,
                              const float* beta, const float* g, float* state, long long slot_stride, const int* cu_seqlens,
-                             const int* slots, float* out, int tokens, int requests, int H, int G, int D, int V, int write,
+                             const int* slots, float* out, int tokens, int longest, int requests, int H, int G, int D, int V, int write,
                              cudaStream_t stream) {
   if (G <= 0 || H % G) return (int)cudaErrorInvalidValue;
   // (keys of up to 32 channels leave the walk's threads two lanes a value channel to share the sums with: 8 heads of 32 x 64, a
   // prompt of 2,048 tokens, 508 us against 432 of scan_kernel; 4 of 16 x 16, 256 requests of one token, 9.0 against 6.1)
   if (D > 32 && D <= 128)
-    return launch_delta_walk(q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, requests, H, H / G, D, V,
-                             write, stream);
+    return launch_delta_walk(q, ldq, k, ldk, v, ldv, beta, g, state, slot_stride, cu_seqlens, slots, out, tokens, longest, requests, H, H / G,
+                             D, V, write, stream);
   return launch_scan<float, RULE_DELTA>(q, ldq, k, ldk, v, ldv, g, beta, state, slot_stride, cu_seqlens, slots, out, tokens,
                                   requests, H, H / G, D, V, 1.f, write, stream);
 }

@@ -76,7 +76,7 @@ _SIGNATURES = {
         "akas_gla_scan_chunked": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
                                   c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "akas_delta_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
-                            c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                            c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_causal_conv_silu": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_delta_prep": [c_void_p, c_longlong, c_int, c_int, c_float, c_float, c_void_p, c_longlong, c_void_p, c_longlong,
@@ -1602,7 +1602,9 @@ def delta_prep(y, kv_heads, dim, q_scale, unit_eps, b, a, a_log, dt_bias):
 
 
 @_flushes
-def delta_scan(q, k, v, beta, g, state, cu_seqlens, slots, heads, kv_heads, dim, vdim, write=True):
+def delta_scan(q, k, v, beta, g, state, cu_seqlens, slots, heads, kv_heads, dim, vdim, write=True, longest=None):
+    """``longest``: the most tokens a request brings in this step, where the caller knows it (it chooses how a walk is split
+    over threads; the results are the same bits)."""
     n = q.shape[0]
     if any(t.dtype != torch.float32 for t in (q, k, v, beta, g)) or not beta.is_contiguous() or not g.is_contiguous():
         raise ValueError("delta_scan takes float32 inputs")
@@ -1610,8 +1612,8 @@ def delta_scan(q, k, v, beta, g, state, cu_seqlens, slots, heads, kv_heads, dim,
     sp, stride = _slot_rows(state, "state")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     _check(_fn("recurrent", "akas_delta_scan")(qp, ldq, kp, ldk, vp, ldv, _ptr(beta), _ptr(g), sp, stride, _ptr(cu_seqlens),
-                                              _ptr(slots), _ptr(out), n, slots.numel(), heads, kv_heads, dim, vdim,
-                                              int(bool(write)), _stream()), "delta_scan")
+                                              _ptr(slots), _ptr(out), n, int(longest or 0), slots.numel(), heads, kv_heads, dim,
+                                              vdim, int(bool(write)), _stream()), "delta_scan")
     return out
 
 

@@ -433,7 +433,7 @@ def delta_prep(y, kv_heads, dim, q_scale, unit_eps, b, a, a_log, dt_bias):
     return beta, g.to(torch.float32)
 
 
-def delta_scan(q, k, v, beta, g, state, cu_seqlens, slots, heads, kv_heads, dim, vdim, write=True):
+def delta_scan(q, k, v, beta, g, state, cu_seqlens, slots, heads, kv_heads, dim, vdim, write=True, longest=None):
     """Per request and head, token by token: S <- g_t S; u = beta_t (v_t - S^T k_t); S <- S + k_t u^T; o_t = S^T q_t.
     q, k [N, kv_heads * dim] (head h reads q/k head h // (heads / kv_heads)), v [N, heads * vdim] -> o float32."""
     n = q.shape[0]

@@ -275,7 +275,8 @@ class GatedDelta(Mixer):
         beta, g = ops.delta_prep(y, s.num_kv_heads, s.key_dim, s.key_dim ** -0.5, s.unit_eps, proj[:, ch : ch + h],
                                  proj[:, ch + h : ch + 2 * h], self.a_log, self.dt_bias)
         o = ops.delta_scan(y[:, :gd], y[:, gd : 2 * gd], y[:, 2 * gd :], beta, g, matrix_state, ctx.cu_seqlens, ctx.slots,
-                           h, s.num_kv_heads, s.key_dim, s.value_dim, write=write)
+                           h, s.num_kv_heads, s.key_dim, s.value_dim, write=write,
+                           longest=getattr(ctx, "max_query_len", None))
         out = ops.gated_rmsnorm(o, self.norm, s.norm_eps, proj[:, ch + 2 * h : ch + 2 * h + hv], h, s.value_dim, self.rt.dtype)
         return project(self.rt, out, self.w_out, residual=residual)
 

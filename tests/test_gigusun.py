@@ -423,6 +423,32 @@ def test_delta_scan_of_many_requests(dim, vdim):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (72, 40)])
+def test_delta_scan_of_a_portion_beside_single_tokens(dim, vdim):
+    """Whether the caller says how long the longest portion is decides between one and two value channels a thread: the same
+    bits, and those of the reference's sums."""
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(dim)
+    heads, lengths = 8, [1] * 15 + [64]
+    n, gd = sum(lengths), heads * dim
+    y = torch.randn(n, 2 * gd + heads * vdim, generator=g).cuda()
+    y[:, : 2 * gd] *= dim ** -0.5
+    beta, decay = torch.rand(n, heads, generator=g).cuda(), (torch.rand(n, heads, generator=g) * 0.4 + 0.6).cuda()
+    state = (torch.randn(16, heads, vdim, dim, generator=g) * 0.3).cuda()
+    cu, _, sl = _batch(lengths, list(range(15, -1, -1)), "cuda")
+    args = (y[:, :gd], y[:, gd : 2 * gd], y[:, 2 * gd :], beta, decay)
+    states = [state.clone() for _ in range(3)]
+    want = reference.delta_scan(*args, states[0], cu, sl, heads, heads, dim, vdim)
+    one = cuda.delta_scan(*args, states[1], cu, sl, heads, heads, dim, vdim, longest=64)
+    two = cuda.delta_scan(*args, states[2], cu, sl, heads, heads, dim, vdim)
+    assert torch.equal(one, two) and torch.equal(states[1], states[2])
+    _close(one, want, 3e-5, "delta o")
+    _close(states[1], states[0], 3e-5, "delta state")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps", [2, 3, 4, 7])
 def test_causal_conv_silu_kernel(taps, dtype):
