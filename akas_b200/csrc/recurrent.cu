@@ -587,7 +587,10 @@ int launch_chunks(const T* q, long long ldq, const T* k, long long ldk, const T*
 // shared memory keeps up: a thread owns 16 key channels of FOUR value channels, 64 elements of state, and reads a token's
 // q, k and gate of its key channels once for all four. KS neighbouring lanes hold a value channel's D key channels and
 // exchange halves of their four sums until each holds one (the order of the additions is that of scan_kernel). A block's
-// 128 threads cover 512 / KS value channels of one (head, chunk).
+// 128 threads cover 512 / KS value channels of one (head, chunk), or 64 threads half of that where a head has no more and the
+// chunks are enough for three blocks to two SMs: half of the 128 would only help to fetch, which fewer blocks are glad of. 8 heads
+// of 64 x 64 (us, 128 / 64 threads): bfloat16 GLA, sixteen prompts of 300 132 / 77, 64 of 200 357 / 211, one of 512 36 / 36; the
+// forget gate 141 / 110, 369 / 279 and, whose gates a thread works out while it fetches, 47 / 55.
 constexpr int kWalkThreads = 128, kWalkR = 16, kWalkNV = 4, kWalkTokens = 16;
 
 // Four neighbouring elements as they are in memory; `live` of them exist, the others are zero. Where the rows do not start
@@ -615,15 +618,15 @@ template <> struct Four<bf16> {
   }
 };
 
-template <typename T, int KS, int RULE, int PART>
-__global__ void __launch_bounds__(kWalkThreads)
+template <typename T, int KS, int RULE, int PART, int TH>
+__global__ void __launch_bounds__(TH)
 walk_chunk_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk, const T* __restrict__ v,
                   long long ldv, const float* __restrict__ decay /* GLA: alpha [N, H * D]; GATE: the logits' bias [H * D] */,
                   const float* __restrict__ low /* GATE: the gates' lower bounds [H * D] */, const int* __restrict__ cu_seqlens,
                   const int* __restrict__ slots, float* __restrict__ out, int H, int D, int V, float q_scale,
                   float* __restrict__ scratch, float* __restrict__ gates, int requests, int from, int vec) {
   static_assert(RULE == RULE_GLA || RULE == RULE_GATE, "a decay per key channel");
-  constexpr int R = kWalkR, NV = kWalkNV, CH = kWalkTokens, TH = kWalkThreads;
+  constexpr int R = kWalkR, NV = kWalkNV, CH = kWalkTokens;
   constexpr int VT = TH / KS * NV, W = KS * R, ROW = KS * (R + kPad);
   constexpr int NQ = (CH * W / 4 + TH - 1) / TH, NVL = CH * VT / 4 / TH;
   __shared__ __align__(16) float sq[PART == 1 ? 1 : CH][ROW];
@@ -831,10 +834,11 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
   const size_t four = 4 * sizeof(T);
   const int vec = D % 4 == 0 && V % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && (uintptr_t)q % four == 0 &&
                   (uintptr_t)k % four == 0 && (uintptr_t)v % four == 0 && (RULE != RULE_GLA || (uintptr_t)decay % 16 == 0);
-#define AKAS_WALK(KS, PART)                                                                                                  \
-  launch_ordinary(walk_chunk_kernel<T, KS, RULE, PART>, dim3(H, chunks, (V + kWalkThreads / KS * kWalkNV - 1) / (kWalkThreads / KS * kWalkNV)), \
-                  dim3(kWalkThreads), 0, stream, q, ldq, k, ldk, v, ldv, decay, low, cu_seqlens, slots, out, H, D, V, q_scale,   \
-                  scratch, gates, requests, from, vec)
+#define AKAS_WALK_TH(KS, PART, TH)                                                                                              \
+  launch_ordinary(walk_chunk_kernel<T, KS, RULE, PART, TH>, dim3(H, chunks, (V + TH / KS * kWalkNV - 1) / (TH / KS * kWalkNV)), dim3(TH), 0, \
+                  stream, q, ldq, k, ldk, v, ldv, decay, low, cu_seqlens, slots, out, H, D, V, q_scale, scratch, gates, requests, from, vec)
+  const bool many = 2LL * H * chunks >= 3LL * 148;
+#define AKAS_WALK(KS, PART) (many && V <= kWalkThreads / 2 / KS * kWalkNV ? AKAS_WALK_TH(KS, PART, kWalkThreads / 2) : AKAS_WALK_TH(KS, PART, kWalkThreads))
 #define AKAS_WALKS(PART) (D <= 16 ? AKAS_WALK(1, PART) : D <= 32 ? AKAS_WALK(2, PART) : D <= 64 ? AKAS_WALK(4, PART) : AKAS_WALK(8, PART))
   int err = AKAS_WALKS(1);
   if (err) return err;
@@ -844,6 +848,7 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
   return AKAS_WALKS(2);
 #undef AKAS_WALKS
 #undef AKAS_WALK
+#undef AKAS_WALK_TH
 }
 
 // ------------------------------------------------------------------------------------------------ delta rule, 33 to 128 keys

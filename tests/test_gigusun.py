@@ -289,7 +289,7 @@ def test_gla_scan_kernel(heads, dim, vdim, dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("heads,dim,vdim,pad", [(3, 20, 24, 3), (2, 72, 136, 0), (1, 8, 5, 3), (2, 128, 66, 4), (2, 64, 128, 0), (1, 16, 520, 0)])
+@pytest.mark.parametrize("heads,dim,vdim,pad", [(3, 20, 24, 3), (2, 72, 136, 0), (1, 8, 5, 3), (2, 128, 66, 4), (2, 64, 128, 0), (1, 16, 520, 0), (2, 100, 32, 0), (24, 64, 64, 4), (24, 100, 32, 0), (16, 20, 24, 3)])
 def test_gla_scan_in_chunks(heads, dim, vdim, pad, dtype):
     """A portion in chunks beside shorter ones that are walked, lengths around the edges of a chunk (64 tokens) and of where
     chunks begin, rows that start on four elements and rows that do not, gates from nearly closed to nearly open. The bounds
@@ -321,15 +321,15 @@ def test_gla_scan_in_chunks(heads, dim, vdim, pad, dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("dim,vdim", [(64, 128), (20, 24)])
-def test_gla_scan_of_a_request_does_not_depend_on_its_company(dim, vdim, dtype):
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 64, 128), (3, 20, 24), (24, 64, 64)])  # the last: 64 threads a block in company, 128 alone
+def test_gla_scan_of_a_request_does_not_depend_on_its_company(heads, dim, vdim, dtype):
     """Requests on both sides of the length from which portions run in chunks, together and alone: the same bits. In float32
     the same bits too however a prompt was cut."""
     from akas_b200.ops import cuda
 
     cuda.require(["recurrent"])
     g = torch.Generator().manual_seed(dim)
-    edge, heads = cuda._GATE_CHUNKED_FROM, 3
+    edge = cuda._GATE_CHUNKED_FROM
     lengths, slots = [1, edge, 20, edge - 1, 400, 1], [5, 0, 3, 1, 2, 4]
     n, hd = sum(lengths), heads * dim
     proj = (torch.randn(n, 2 * hd + heads * vdim, generator=g) * 0.5).to(dtype).cuda()

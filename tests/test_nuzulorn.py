@@ -994,7 +994,8 @@ def test_linear_distance_penalty_kernel(heads, kv_heads, dim, vdim, page, window
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("heads,dim,vdim", [(3, 12, 10), (1, 5, 33), (2, 20, 36), (4, 64, 128), (2, 128, 128), (2, 128, 40), (1, 8, 300), (2, 200, 24), (1, 600, 8), (1, 1024, 3)])
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 12, 10), (1, 5, 33), (2, 20, 36), (4, 64, 128), (2, 128, 128), (2, 128, 40), (1, 8, 300), (2, 200, 24), (1, 600, 8), (1, 1024, 3),
+                                             (24, 64, 64), (24, 100, 32), (24, 20, 30), (24, 12, 40)])  # chunks enough for blocks of 64 threads
 def test_forget_gates_that_write_kernel(heads, dim, vdim):
     """Token by token and in chunks against the plain statement: requests of unequal length, gates that are nearly shut,
     nearly open and in between, states carried in and out, a slot that stays untouched."""
