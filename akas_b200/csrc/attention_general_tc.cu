@@ -77,7 +77,7 @@ __device__ __forceinline__ float gate_of(const Options& opt, size_t token, int h
 
 constexpr int kTableBefore = 128, kTableAfter = 192;  // entries of the penalty table on either side of the window's distances
 
-template <int DKP, int DVP>  // head sizes rounded up to multiples of 32
+template <int DKP, int DVP, bool WHOLE>  // head sizes rounded up to multiples of 32; pages of whole tiles (see below)
 __global__ void __launch_bounds__(WARPS * 32, (DKP + DVP <= 192) ? 3 : 2)
 general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool,
                        const int* __restrict__ block_table, int max_blocks, const int* __restrict__ cu_seqlens,
@@ -152,11 +152,11 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
 
   // A page that holds whole tiles (its size a multiple of 64) is looked up once per tile, an iteration before the tile's
   // copies are issued; the copies then only step through it. (A look-up and a division per 16-byte copy, in front of
-  // every tile's products, took longer than the products.)
-  const bool whole_pages = page_size % BK == 0;
+  // every tile's products, took longer than the products. Other pages have a kernel without this: with both in one, theirs
+  // were up to 10 % slower.)
   auto page_of = [&](int i) {
     const int kt = tile_of(i);
-    return whole_pages && kt >= 0 ? block_table[(size_t)r * max_blocks + kt * BK / page_size] : -1;
+    return WHOLE && kt >= 0 ? block_table[(size_t)r * max_blocks + kt * BK / page_size] : -1;
   };
   auto load_tile = [&](int kt, int stage, int tile_page) {
     bf16* ks_ = k_s + stage * BK * KSTRIDE;
@@ -181,7 +181,7 @@ general_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
       cp_async_commit();
       return;
     }
-    if (whole_pages) {
+    if constexpr (WHOLE) {
       const size_t base = tile_page >= 0 ? ((size_t)tile_page * KH + kvh) * page_size + kt * BK % page_size : 0;
       const bf16* kp = k_pool + base * D;
       const bf16* vp = v_pool + base * opt.vpitch;
@@ -710,8 +710,9 @@ int launch(const void* q, const void* k_pool, const void* v_pool, const int* blo
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
   if (!configured[device]) {
-    const cudaError_t e = cudaFuncSetAttribute(general_prefill_kernel<DKP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               tiles_bytes + (kTableMost + kTableBefore + kTableAfter) * (int)sizeof(float));
+    constexpr int most = tiles_bytes + (kTableMost + kTableBefore + kTableAfter) * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(general_prefill_kernel<DKP, DVP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(general_prefill_kernel<DKP, DVP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return (int)e;
     const cudaError_t d = cudaFuncSetAttribute(general_decode_kernel<DKP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize, tiles_bytes);
     if (d != cudaSuccess) return (int)d;
@@ -721,9 +722,10 @@ int launch(const void* q, const void* k_pool, const void* v_pool, const int* blo
       ? launch_ordinary(general_decode_kernel<DKP, DVP>, dim3(KH, R, splits), dim3(WARPS * 32), (size_t)tiles_bytes, stream, (const bf16*)q,
                         (const bf16*)k_pool, (const bf16*)v_pool, block_table, max_blocks, cu_seqlens, positions, (bf16*)out, opt,
                         page_size, H, KH, D, V, partial, splits)
-      : launch_ordinary(general_prefill_kernel<DKP, DVP>, dim3(packed ? KH : H, tiles, splits), dim3(WARPS * 32), (size_t)smem,
-                                  stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, block_table, max_blocks,
-                                  cu_seqlens, positions, (bf16*)out, opt, page_size, H, KH, D, V, R, packed, table, partial, splits);
+      : launch_ordinary(page_size % BK == 0 ? general_prefill_kernel<DKP, DVP, true> : general_prefill_kernel<DKP, DVP, false>,
+                        dim3(packed ? KH : H, tiles, splits), dim3(WARPS * 32), (size_t)smem, stream, (const bf16*)q,
+                        (const bf16*)k_pool, (const bf16*)v_pool, block_table, max_blocks, cu_seqlens, positions, (bf16*)out, opt,
+                        page_size, H, KH, D, V, R, packed, table, partial, splits);
   if (err || splits <= 1) return err;
   return launch_ordinary(general_merge_kernel, dim3(R, H), dim3(V >= 128 ? 128 : 64), 0, stream, (const float*)partial, cu_seqlens,
                          (bf16*)out, opt, H, V, splits);
