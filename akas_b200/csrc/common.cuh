@@ -171,6 +171,15 @@ static inline int launch_ordinary(void (*kernel)(Params...), dim3 grid, dim3 blo
   return (int)cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
+// The SMs of the current device (0 where there is none), for rules that count blocks.
+static inline int sm_count() {
+  static int sms[64] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
+  if (sms[device] == 0) cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
+  return sms[device];
+}
+
 inline bool chained_launches_enabled() {
   static const bool enabled = [] {
     const char* v = getenv("AKAS_B200_CHAINED_LAUNCHES");

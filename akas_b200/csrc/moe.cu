@@ -275,7 +275,7 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
 // the rows' trips per token weigh as much. bfloat16 rows, us, the kernel above / this one: 16 outputs of 1,536 at 1, 8 and 296 tokens
 // 11.3 / 5.9, 12.3 / 6.1 and 12.3 / 6.7; 256 of 2,048 110 / 36, 111 / 37 and 104 / 42; at 512 tokens 12.3 / 11.6 and 104 / 82, but
 // 8 outputs of 512 7.3 / 10.0 (at 296 7.3 / 5.8).
-constexpr int kRouteFewOutputs = 16, kRouteFewMost = 296;
+constexpr int kRouteFewOutputs = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(kRouteTokens * 32)
@@ -770,14 +770,7 @@ moe_down_stream_kernel(const bf16* __restrict__ h, long long ldh, const bf16* __
   }
 }
 
-// The SMs of the current device, or 0; and the shared-memory limit of a kernel raised once per device.
-int sm_count() {
-  static int sms[64] = {};
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
-  if (sms[device] == 0) cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
-  return sms[device];
-}
+// The shared-memory limit of a kernel, raised once per device.
 template <typename K>
 int allow_smem(K kernel, bool (&done)[64]) {
   int device = 0;
@@ -862,7 +855,7 @@ AKAS_API int akas_moe_route(const void* h, long long ldh, const float* w, const 
     return (int)cudaErrorInvalidValue;
   const size_t elem = dtype == AKAS_F32 ? 4 : 2;
   const size_t few_smem = sizeof(float) * (2 * (size_t)(R + extra) + groups + kRouteTokens * kRouteFewOutputs);
-  if (N <= kRouteFewMost && C % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)w % 16 == 0 &&
+  if (N <= 2 * sm_count() && C % 4 == 0 && ldh % 4 == 0 && (uintptr_t)h % (4 * elem) == 0 && (uintptr_t)w % 16 == 0 &&
       few_smem <= 48 * 1024) {
     if (dtype == AKAS_F32)
       return launch_ordinary(moe_route_few_kernel<float>, dim3(N), dim3(kRouteTokens * 32), few_smem, stream, (const float*)h, ldh, w,

@@ -837,7 +837,7 @@ int launch_walks(const T* q, long long ldq, const T* k, long long ldk, const T* 
 #define AKAS_WALK_TH(KS, PART, TH)                                                                                              \
   launch_ordinary(walk_chunk_kernel<T, KS, RULE, PART, TH>, dim3(H, chunks, (V + TH / KS * kWalkNV - 1) / (TH / KS * kWalkNV)), dim3(TH), 0, \
                   stream, q, ldq, k, ldk, v, ldv, decay, low, cu_seqlens, slots, out, H, D, V, q_scale, scratch, gates, requests, from, vec)
-  const bool many = 2LL * H * chunks >= 3LL * 148;
+  const bool many = 2LL * H * chunks >= 3LL * sm_count();
 #define AKAS_WALK(KS, PART) (many && V <= kWalkThreads / 2 / KS * kWalkNV ? AKAS_WALK_TH(KS, PART, kWalkThreads / 2) : AKAS_WALK_TH(KS, PART, kWalkThreads))
 #define AKAS_WALKS(PART) (D <= 16 ? AKAS_WALK(1, PART) : D <= 32 ? AKAS_WALK(2, PART) : D <= 64 ? AKAS_WALK(4, PART) : AKAS_WALK(8, PART))
   int err = AKAS_WALKS(1);
@@ -1032,7 +1032,8 @@ int launch_delta_walk(const float* q, long long ldq, const float* k, long long l
   // short ones are gone when the long walk is still at its beginning (a prompt of 2,048 behind 15 single tokens, 8 heads: 865 /
   // 485 / 627; 16 heads 680 / 621 / 626).
   const long long blocks = (long long)H * ((V + kDeltaThreads / 8 - 1) / (kDeltaThreads / 8));
-  const bool alone = longest > 0 ? blocks * tokens <= 148LL * longest : blocks * requests <= 148;
+  const long long sms = sm_count();
+  const bool alone = longest > 0 ? blocks * tokens <= sms * longest : blocks * requests <= sms;
   if (D <= 64) AKAS_DELTA(4, 2);
   if (alone) AKAS_DELTA(8, 1);
   AKAS_DELTA(8, 2);
@@ -1351,7 +1352,7 @@ AKAS_API int akas_decay_gates(const void* low, long long ld, const float* w, con
   // eight tokens a block; sixteen, which read the matrix half as often, where that leaves enough blocks
   const size_t row = (size_t)R * sizeof(float);
   if (8 * row > 48 * 1024) return (int)cudaErrorInvalidValue;
-  const bool wide = 16 * row <= 48 * 1024 && (long long)((N + 15) / 16) * ((O + 127) / 128) >= 592;
+  const bool wide = 16 * row <= 48 * 1024 && (long long)((N + 15) / 16) * ((O + 127) / 128) >= 4 * sm_count();
   const int tokens = wide ? 16 : 8;
   const dim3 grid((N + tokens - 1) / tokens, min((O + 127) / 128, 64));
 #define AKAS_GATES(T, TOKENS)                                                                                                     \
@@ -1483,7 +1484,7 @@ AKAS_API int akas_causal_conv_silu(const void* x, long long ldx, const float* ta
   // runs of 8 tokens a thread where the step holds enough of them for two blocks an SM: 1,024 channels of 1,184 tokens (296 blocks)
   // 13.4 -> 6.2 us, 4,096 of 296 13.7 -> 6.2; with a token a thread 1,024 of 148 take 3.9, 2,048 of 148 5.4
   const dim3 runs((N + kConvRun - 1) / kConvRun, (C / 4 + 127) / 128);
-  const bool run = four && L == 4 && (uintptr_t)taps % 16 == 0 && (long long)runs.x * runs.y >= 296 && runs.y <= 65535;
+  const bool run = four && L == 4 && (uintptr_t)taps % 16 == 0 && (long long)runs.x * runs.y >= 2 * sm_count() && runs.y <= 65535;
   int err = run ? (dtype == AKAS_F32
       ? launch_ordinary(causal_conv_silu_run_kernel<float>, runs, dim3(128), 0, stream, (const float*)x, ldx, taps, old, slot_stride,
                         cu_seqlens, seq_of_token, slots, y, N, C)
@@ -1530,7 +1531,7 @@ AKAS_API int akas_gated_rmsnorm(const float* o, const float* w, float eps, const
                          sigmoid, out_scale, ldo)
   const size_t ge = gate_dtype == AKAS_F32 ? 4 : 2, oe = out_dtype == AKAS_F32 ? 4 : 2;
   // (the vector path's conditions, and rows enough to go round the SMs twice at most)
-  if (items <= 296 && V > 256 && V <= 1024 && V % 4 == 0 && ldg % 4 == 0 && ldo % 4 == 0 && ge == oe && (uintptr_t)gate % (4 * ge) == 0 &&
+  if (items <= 2 * sm_count() && V > 256 && V <= 1024 && V % 4 == 0 && ldg % 4 == 0 && ldo % 4 == 0 && ge == oe && (uintptr_t)gate % (4 * ge) == 0 &&
       (uintptr_t)out % (4 * oe) == 0) {
     if (ge == 4)
       return launch_ordinary(gated_rmsnorm_wide_kernel<float, float>, dim3((int)items), dim3(256), 0, stream, o, w, eps, (const float*)gate,
