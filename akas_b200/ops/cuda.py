@@ -1522,6 +1522,17 @@ def decay_gates(low, w_up, bias, tau):
     return out
 
 
+def _scratch(words: int, device) -> Optional[torch.Tensor]:
+    """A recurrence's float32 scratch for its chunks, or None where it has none or the device has no room for it: the caller
+    then walks token by token, which needs none."""
+    if not words:
+        return None
+    try:
+        return torch.empty(words, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 @_flushes
 def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale, write=True, longest=None):
     """bfloat16 rows: requests that bring at least _GATE_CHUNKED_FROM tokens in chunks (three kernels, see csrc/recurrent.cu;
@@ -1537,9 +1548,8 @@ def gla_scan(q, k, v, alpha, state, cu_seqlens, slots, heads, dim, vdim, q_scale
     requests = slots.numel()
     tail = (n, requests, heads, dim, vdim, float(q_scale), int(bool(write)))
     if decay_scan_kernels == "auto" and q.dtype == torch.bfloat16 and longest is not None and longest >= _GATE_CHUNKED_FROM:
-        words = int(_fn("recurrent", "akas_gate_chunk_scratch")(n, requests, heads, dim, vdim))
-        if words:
-            scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        scratch = _scratch(int(_fn("recurrent", "akas_gate_chunk_scratch")(n, requests, heads, dim, vdim)), q.device)
+        if scratch is not None:
             _check(_fn("recurrent", "akas_gla_scan_chunked")(*head, _ptr(scratch), _GATE_CHUNKED_FROM, *tail, _stream()),
                    "gla_scan (chunks)", kernels=4 if requests > 1 else 3)
             return out
@@ -1561,9 +1571,8 @@ def hgrn2_scan(q, f, v, f_bias, lower, state, cu_seqlens, slots, heads, dim, vdi
     head = (qp, ldq, fp, ldf, vp, ldv, _ptr(f_bias), _ptr(lower), sp, stride, _ptr(cu_seqlens), _ptr(slots), _ptr(out))
     tail = (n, slots.numel(), heads, dim, vdim, int(bool(write)), _stream())
     if decay_scan_kernels == "auto" and longest is not None and longest >= _GATE_CHUNKED_FROM:
-        words = int(_fn("recurrent", "akas_gate_chunk_scratch")(n, slots.numel(), heads, dim, vdim))
-        if words:
-            scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        scratch = _scratch(int(_fn("recurrent", "akas_gate_chunk_scratch")(n, slots.numel(), heads, dim, vdim)), q.device)
+        if scratch is not None:
             _check(_fn("recurrent", "akas_gate_scan_chunked")(*head, _ptr(scratch), *tail), "hgrn2_scan (chunks)", kernels=3)
             return out
     _check(_fn("recurrent", "akas_gate_scan")(*head, *tail), "hgrn2_scan")
@@ -1661,9 +1670,8 @@ def decay_scan(q, k, v, decay, state, cu_seqlens, slots, heads, dim, vdim, q_sca
     sp, stride = _slot_rows(state, "state")
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     if decay_scan_kernels == "auto" and longest is not None and longest >= _CHUNKED_FROM:
-        words = int(_fn("recurrent", "akas_decay_chunk_scratch")(n, slots.numel(), heads, dim, vdim))
-        if words:
-            scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        scratch = _scratch(int(_fn("recurrent", "akas_decay_chunk_scratch")(n, slots.numel(), heads, dim, vdim)), q.device)
+        if scratch is not None:
             _check(_fn("recurrent", "akas_decay_scan_chunked")(
                 qp, ldq, kp, ldk, vp, ldv, _ptr(decay), sp, stride, _ptr(cu_seqlens), _ptr(slots), _ptr(out), _ptr(scratch), n,
                 slots.numel(), heads, dim, vdim, float(q_scale), int(activation == "silu"), int(bool(write)), _code(q), _stream()),

@@ -358,6 +358,36 @@ def test_gla_scan_of_a_request_does_not_depend_on_its_company(heads, dim, vdim, 
 
 
 @pytest.mark.gpu
+def test_gla_scan_without_room_for_its_chunks(monkeypatch):
+    """Where the device has no room for the chunks' scratch, a long portion is walked token by token, which needs none."""
+    from akas_b200.ops import cuda, reference
+
+    cuda.require(["recurrent"])
+    g = torch.Generator().manual_seed(3)
+    proj = (torch.randn(300, 256, generator=g) * 0.5).to(torch.bfloat16).cuda()
+    alpha, state = torch.sigmoid(torch.randn(300, 64, generator=g) + 3).cuda(), (torch.randn(1, 1, 128, 64, generator=g) * 0.3).cuda()
+    cu, _, sl = _batch([300], [0], "cuda")
+    args = (proj[:, :64], proj[:, 64:128], proj[:, 128:], alpha)
+    s_ref, s_got = state.clone(), state.clone()
+    want = reference.gla_scan(*args, s_ref, cu, sl, 1, 64, 128, 0.125)
+    words = int(cuda._fn("recurrent", "akas_gate_chunk_scratch")(300, 1, 1, 64, 128))
+    empty, refused = torch.empty, []
+
+    def full(*size, **kw):  # a device with room for the results, but not for the scratch
+        if size == (words,):
+            refused.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", full)
+    got = cuda.gla_scan(*args, s_got, cu, sl, 1, 64, 128, 0.125, longest=300)
+    monkeypatch.undo()
+    assert refused
+    _close(got, want, 2e-5, "gla o")
+    _close(s_got, s_ref, 2e-5, "gla state")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 4, 16, 12), (6, 2, 40, 20), (2, 1, 136, 72), (1, 1, 7, 3), (2, 2, 300, 33)])
 def test_delta_scan_kernel(heads, kv_heads, dim, vdim):
     from akas_b200.ops import cuda, reference
