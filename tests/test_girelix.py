@@ -516,20 +516,25 @@ def test_gated_norm_options_and_scaled_add_kernels(dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("outputs,count,keep,top,c", [(16, 4, 2, 4, 1536), (20, 1, 1, 3, 2056), (6, 2, 1, 2, 264), (3, 1, 1, 1, 24)])
+@pytest.mark.parametrize("options", [dict(), dict(scoring="sigmoid"), dict(scoring="sigmoid", plain=True, renormalize=False, weight_scale=2.5),
+                                     dict(extra=1), dict(extra=2, group_best=2), dict(scoring="sigmoid", group_best=2, plain=True)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_route_of_few_tokens_gives_the_bits_of_many(outputs, count, keep, top, c, dtype):
-    """A block per token where the tokens are few, four tokens a block where they are many: one order of sums, the same bits."""
+def test_route_of_few_tokens_gives_the_bits_of_many(outputs, count, keep, top, c, options, dtype):
+    """A block per token where the tokens are few, eight tokens a block where they are many: one order of sums, the same bits,
+    with every way of scoring and choosing (``plain``: without a correction)."""
     from akas_b200.ops import cuda
 
     cuda.require(["moe"])
     g = torch.Generator().manual_seed(outputs * 100 + c)
+    options = dict(options)
+    plain, extra = options.pop("plain", False), options.get("extra", 0)
     h = torch.randn(700, c, generator=g).to(dtype).cuda()
-    w = (torch.randn(outputs, c, generator=g) * (3.0 / c ** 0.5)).cuda()
-    correction = (torch.randn(outputs, generator=g) * 0.2).cuda()
-    chosen, weights = cuda.moe_route(h, w, correction, count, keep, top)
-    for rows in (1, 37, 296):
-        few_c, few_w = cuda.moe_route(h[:rows], w, correction, count, keep, top)
-        assert torch.equal(few_c, chosen[:rows]) and torch.equal(few_w, weights[:rows])
+    w = (torch.randn(outputs + extra, c, generator=g) * (3.0 / c ** 0.5)).cuda()
+    correction = None if plain else (torch.randn(outputs, generator=g) * 0.2).cuda()
+    many = cuda.moe_route(h, w, correction, count, keep, top, **options)
+    for rows in (1, 37, 2 * cuda._sm_count()):
+        few = cuda.moe_route(h[:rows], w, correction, count, keep, top, **options)
+        assert len(few) == (3 if extra else 2) and all(torch.equal(a, b[:rows]) for a, b in zip(few, many))
 
 
 @pytest.mark.gpu
