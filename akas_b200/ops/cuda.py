@@ -860,7 +860,12 @@ def _skinny_takes(m: int, o: int, k: int, mode: int) -> bool:
 
 
 _SKINNY_ROWS = 16
-_SKINNY_CUT_ROWS = 8  # 2,048 x 12,288: 13.2 us against 17.0 of the weight-streaming kernel; 9 to 16 tokens, in two groups: 21.7
+# Up to 8 tokens and an inner size too long for a block: cut along K, against the kernels of more than 16 tokens (us, bfloat16 /
+# accumulating read-out, there / here). The C rule (akas_skinny_gemm_takes) refuses widths whose row tiles and parts do not fit the
+# clusters the GPU holds at once (at 6,144 channels for inner sizes up to 16,384, at 3,072 beyond); below that it was never slower: 64 x 10,240
+# 18 / 5.5 and 9 / 5.4, 2,048 x 12,288 22 / 14.5 and 17.6 / 13, 4,096 x 10,240 21 / 20.7 and 22 / 20.5, 1,536 x 32,768 53 / 25 and
+# 24.5 / 24.6, 2,048 x 32,768 53 / 31 and 33 / 31. 9 to 16 tokens, in two groups: 2,048 x 12,288 17.0 / 21.7.
+_SKINNY_CUT_ROWS = 8
 # Which kernels run the products of more than 16 tokens (prompt portions, mixed steps, large decode batches). "own"
 # (default; "auto" and "tcgen05" mean the same): the hand-written tcgen05 kernels everywhere: the kernel for pairs of
 # SMs (gemm_pair.cu, TMA-written read-outs) for every product whose output rows TMA can write, the one-block kernel
