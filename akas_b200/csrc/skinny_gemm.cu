@@ -22,6 +22,18 @@
 // meet in shared memory (a barrier of the consumer warps only).
 //
 // The producer starts before the kernel waits for its predecessor (weights depend on nothing).
+//
+// What bounds it. With 8 tokens and wide matrices, DRAM. With one token or small matrices (2 to 20 MB, a rate at which
+// DRAM is done in 1 to 3 us) the chain of latencies from the predecessor's end to this kernel's: 0.6 us until the wait
+// returns, activations into shared memory, first stage, products, the warps' sums, the store. Most of that was time to issue
+// instructions that a block runs once, not time in memory, so: no divisions in the prologue, only the rows that exist are staged,
+// the stages' barriers are looked at once before anything else is, one barrier a tile, the norm's factor without IEEE
+// root and division and ahead of the loop, what a read-out adds to asked for ahead by cp.async (into registers the
+// compiler waits for it in front of the loop), and partial sums sent to a peer block word by word, counted on its
+// mbarrier, instead of stores, a barrier, a fence and an arrival. Measured, four products and a convolution a layer, 16
+// layers as a captured graph: 367 -> 284 us at width 1,024 and one token, 583 -> 519 at 2,048, 621 -> 614 with 8
+// tokens; a product of 1,024 x 1,024 whose weights lie in the L2, launch to launch, 3.08 -> 2.20 us.
+//
 // Every wait on an mbarrier is bounded: a wait that runs out sets a status flag that the host can read
 // (akas_skinny_gemm_status), everyone stops waiting and the block runs to its end; results of such a launch
 // are not valid.
@@ -44,7 +56,7 @@
 // are a third of what a block fetches, and they leave room for one block per SM only. Such a product is cut
 // along K as well: the `ksplit` blocks of a thread-block cluster take one part of K each for the same row
 // tiles, keep their sums in shared memory, and at the end send them to the cluster's first block
-// (st.shared::cluster, one arrival per block on its mbarrier), which adds the parts in rank order and writes
+// (st.async, counted in bytes on its mbarrier), which adds the parts in rank order and writes
 // the result. Not for the SwiGLU read-out.
 // Needs K % 64 == 0. Results do not depend on what else runs; summation order is fixed.
 #include <cuda.h>
@@ -62,6 +74,7 @@ using namespace akas;
 namespace {
 
 constexpr int CONSUMERS = 8, KC = 512, STAGES = 4;
+constexpr int kBulkRows = 2;  // bfloat16 activations of at least this many tokens come by bulk copies
 constexpr int MAX_KSPLIT = 8, SPLIT_TILES = 4;  // parts of K; row tiles a cluster may take when K is cut
 constexpr int STAGE_BYTES = 16 * KC * 2;  // one box of [8 groups of k][16 rows][128 bytes], or (SwiGLU) two of 8 rows
 constexpr int THREADS = (CONSUMERS + 1) * 32;
@@ -89,6 +102,17 @@ struct ConvTail {
   const float* in_alpha;    // in_mode 2: the norm's slope, one number
 };
 
+// How the launch is cut, in the form that costs a block no division (a division by a run-time number is a few hundred
+// cycles of a prologue that nothing hides where the block could not be resident early).
+struct Cut {
+  int ksplit_log2, groups_log2;  // parts of K and token groups: powers of two
+  int rounds;                    // row tiles of the busiest block; every other one has as many or one less
+  int two_sums;                  // whether two tiles' partial sums have places of their own (else one place, and a barrier more a tile)
+  float inv_k;                   // 1 / K, for the norm's mean
+};
+
+template <int N> struct Rows { static constexpr int value = N; };  // a number of token rows that code is made for
+
 __device__ int g_skinny_status = 0;  // 0, or the code of a wait that ran out (1: a full stage, 2: an empty stage)
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -101,8 +125,15 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Waits for the phase of the given parity to complete; false if the bounded wait ran out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_done(uint64_t* bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return done;
+}
+// Waits for the phase of the given parity to complete, or for another thread's wait to run out (`lost`); false if this one does.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, const volatile int* lost) {
   const unsigned addr = smem_u32(bar);
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
     unsigned done;
@@ -110,6 +141,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done) : "r"(addr), "r"(parity), "r"(200u) : "memory");
     if (done) return true;
+    if (*lost) return true;
   }
   return false;
 }
@@ -117,6 +149,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
 __device__ __forceinline__ void tma_load_box(void* smem_dst, const CUtensorMap* map, int row, int group, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                ::"r"(smem_u32(smem_dst)), "l"(map), "r"(0), "r"(row), "r"(group), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* smem_dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS * 32) : "memory"); }
 
@@ -130,8 +166,14 @@ __device__ __forceinline__ unsigned peer_address(const void* local, unsigned ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(local)), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void peer_store(unsigned address, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
+// 4 bytes from global memory into shared memory, behind the thread's back.
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+// A word into another block of the cluster; its 4 bytes are counted on that block's mbarrier when they have arrived.
+__device__ __forceinline__ void peer_store(unsigned address, float v, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+               ::"r"(address), "r"(__float_as_uint(v)), "r"(bar) : "memory");
 }
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, unsigned parity) {
   const unsigned addr = smem_u32(bar);
@@ -144,47 +186,59 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, unsigned parity
   }
   return false;
 }
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// 1 / sqrt(x): the unit's estimate and one Newton step, right to an ulp like the two IEEE operations, which take several
+// hundred cycles in a block that runs them once; those are left for what the step does not take.
+__device__ __forceinline__ float inverse_root(float x) {
+  if (!(x > 1e-30f && x < 1e30f)) return 1.f / sqrtf(x);
+  const float r = rsqrtf(x);
+  return r * fmaf(-0.5f * x * r, r, 1.5f);
 }
 
 template <int NT, int IN, int OUT, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 2)
 skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __restrict__ x_, const int* __restrict__ rows,
                    const float* __restrict__ norm_w, float eps, int zero_centered, void* __restrict__ y_, int M, int O,
-                   int K, int num_tiles, int ksplit, int groups, const ConvTail tail) {
+                   int K, int num_tiles, const Cut cut, const ConvTail tail) {
   constexpr int STAGES = Ring<OUT>::DEPTH, STAGE_BYTES = Ring<OUT>::BYTES, RT = Ring<OUT>::ROWS;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);  // [STAGES][STAGE_BYTES]
-  float* red = reinterpret_cast<float*>(ring + STAGES * STAGE_BYTES);   // [CONSUMERS][NT][RT][8]: partial sums
+  const int ksplit = 1 << cut.ksplit_log2;
+  // [one or two places][CONSUMERS][NT][RT][8]: partial sums
+  float* red = reinterpret_cast<float*>(ring + STAGES * STAGE_BYTES);
+  constexpr int RED = CONSUMERS * NT * RT * 8;
   // ksplit > 1: this block's sums of its row tiles, then (first block only) the other blocks' sums and sums of x^2
-  float* part = red + CONSUMERS * NT * RT * 8;                           // [SPLIT_TILES][NT * 128]
+  float* part = red + (cut.two_sums ? 2 * RED : RED);                    // [SPLIT_TILES][NT * 128]
   float* peer = part + (ksplit > 1 ? SPLIT_TILES * NT * 128 : 0);        // [ksplit - 1][SPLIT_TILES][NT * 128]
   float* peer_ss = peer + (ksplit > 1 ? (ksplit - 1) * SPLIT_TILES * NT * 128 : 0);  // [ksplit - 1][NT * 8]
   bf16* xs = reinterpret_cast<bf16*>(peer_ss + (ksplit > 1 ? (ksplit - 1) * NT * 8 : 0));  // [NT * 8][XS]: activations
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], gathered;
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], gathered, rows_bar;
   __shared__ float ss_s[CONSUMERS][NT * 8];  // sums of x^2 per token, one part per consumer warp (added in warp order)
-  __shared__ int slot_s[NT * 8];  // convolution read-out: the state row of each token's request, or -1
+  // what the read-out adds to or convolves, on its way while the products run: the residual stream's values, or the state rows
+  constexpr int TAPS = 4, AHEAD = OUT == OUT_CONV ? (TAPS - 1) * NT * 64 : OUT == OUT_ACC ? NT * 128 : 1;
+  __shared__ float ahead_s[AHEAD];
   __shared__ int abort_s;  // set by the first wait that runs out; from then on nobody waits on an mbarrier
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int F = O / 2;  // swiglu only: O is the stacked height 2F
   const int all_chunks = (K + KC - 1) / KC;
   // this block's part of K: chunks [chunk0, chunk0 + chunks) of all_chunks, k from k0 on
   const int rank = ksplit > 1 ? (int)cluster_rank() : 0;
-  const int chunk0 = all_chunks * rank / ksplit, chunks = all_chunks * (rank + 1) / ksplit - chunk0;
+  const int chunk0 = all_chunks * rank >> cut.ksplit_log2, chunks = (all_chunks * (rank + 1) >> cut.ksplit_log2) - chunk0;
   const int k0 = chunk0 * KC, k_len = min(K, (chunk0 + chunks) * KC) - k0;
-  const int XS = ((all_chunks + ksplit - 1) / ksplit) * KC + 32;
+  const int XS = ((all_chunks + ksplit - 1) >> cut.ksplit_log2) * KC + 32;
   // Token groups (9 to 16 tokens on the kernel for 8): every row tile is the work of `groups` blocks (clusters), one per
   // group of NT * 8 tokens, that run side by side and read the same weights, the second one mostly from the L2. A
   // block's group is fixed (the host makes the number of clusters a multiple of `groups`); from here on it sees only
   // its own tokens.
   // (GROUPED is a template argument so that the kernel for a single group keeps its registers: with the group's offsets
   // computed in every instance the staging of the normed rows spilled)
-  const int item0 = (int)blockIdx.x / ksplit, item_step = (int)gridDim.x / ksplit;  // of this block's cluster
-  const int first_tile = GROUPED ? item0 / groups : item0, tile_step = GROUPED ? item_step / groups : item_step;
+  const int item0 = (int)blockIdx.x >> cut.ksplit_log2, item_step = (int)gridDim.x >> cut.ksplit_log2;  // of this block's cluster
+  const int first_tile = GROUPED ? item0 >> cut.groups_log2 : item0, tile_step = GROUPED ? item_step >> cut.groups_log2 : item_step;
   const int* token_request = tail.seq_of_token;
   if (GROUPED) {
-    const int m0 = (item0 % groups) * NT * 8;
+    const int m0 = (item0 & ((1 << cut.groups_log2) - 1)) * NT * 8;
     if (rows) rows += m0;
     else x_ = IN != IN_BF16 ? (const void*)((const float*)x_ + (size_t)m0 * K) : (const void*)((const bf16*)x_ + (size_t)m0 * K);
     const size_t width = OUT == OUT_SWIGLU ? O / 2 : OUT == OUT_CONV ? O / 3 : O;
@@ -192,30 +246,60 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
     if (OUT == OUT_CONV) token_request += m0;
     M = max(0, min(M - m0, NT * 8));
   }
-  const int my_tiles = first_tile < num_tiles ? (num_tiles - first_tile + tile_step - 1) / tile_step : 0;
+  const int my_tiles = first_tile + (cut.rounds - 1) * tile_step < num_tiles ? cut.rounds : cut.rounds - 1;
   const int items = my_tiles * chunks;  // this block's work: the chunks of its row tiles, in order
 
-  if (tid == 0) {
+  // A bounded wait. When one runs out the launch is lost (the status flag says so), but every thread keeps
+  // following the same path through the barriers, so the block still ends.
+  auto wait_for = [&](uint64_t* bar, unsigned parity, int code) {
+    if (mbar_done(bar, parity)) return;
+    if (!mbar_wait(bar, parity, (const volatile int*)&abort_s)) {
+      *(volatile int*)&abort_s = 1;
+      if (lane == 0) atomicExch(&g_skinny_status, code);
+    }
+  };
+  // Stage n of the block's work, chunk `chunk` of row tile `tile`, on its way into the ring.
+  auto load_stage = [&](int s, int tile, int chunk) {
+    unsigned char* dst = ring + (size_t)s * STAGE_BYTES;
+    mbar_expect_tx(&full_bar[s], STAGE_BYTES);  // rows or k past the matrix arrive as zeros and count too
+    // An instruction that starts a TMA copy costs the issuing thread some 300 cycles whatever the copy holds, so
+    // the boxes are as large as they can be: 16 rows x 512 k (16 KB), or two of 8 rows for SwiGLU's two halves (8 gate
+    // rows and the 8 up rows under them).
+    // (SwiGLU as a run of stages over 16 gate rows and then one over 16 up rows, one box a stage, measured
+    // slower here: 0.926 against 0.898 ms a decode step of the 1.2B shape.)
+    const int group = (chunk0 + chunk) * (KC / 64);
+    if (OUT == OUT_CONV) {  // 8 rows each of the projection's B, C and x parts, C = O / 3 rows apart
+      for (int h = 0; h < 3; ++h)
+        tma_load_box(dst + h * (STAGE_BYTES / 3), &map_w, h * (O / 3) + tile * 8, group, &full_bar[s]);
+    } else if (OUT == OUT_SWIGLU) {
+      tma_load_box(dst, &map_w, tile * 8, group, &full_bar[s]);
+      tma_load_box(dst + STAGE_BYTES / 2, &map_w, F + tile * 8, group, &full_bar[s]);
+    } else {
+      tma_load_box(dst, &map_w, tile * 16, group, &full_bar[s]);
+    }
+  };
+  if (tid == CONSUMERS * 32) {  // by the thread that uses them first
     abort_s = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], CONSUMERS);
     }
-    mbar_init(&gathered, ksplit > 1 ? (unsigned)(ksplit - 1) : 1u);
+    mbar_init(&gathered, 1);
+    mbar_init(&rows_bar, 1);
+    if (IN == IN_BF16 && M >= kBulkRows) mbar_expect_tx(&rows_bar, (unsigned)(M * k_len * 2));
+    // the first block of a cluster waits for the others' words: sums of its tiles' rows for M tokens, and of x^2
+    if (ksplit > 1 && rank == 0) mbar_expect_tx(&gathered, (unsigned)((ksplit - 1) * M * (my_tiles * 16 + (IN == IN_NORM ? 1 : 0)) * 4));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
-  if (ksplit > 1) cluster_meet();  // the first block's barrier exists before a peer arrives on it
+  // (the producer's warp tells the others that the barriers exist and goes on to its first loads)
+  if (warp == CONSUMERS) {
+    __syncwarp();
+    asm volatile("bar.arrive 2, %0;" ::"n"(THREADS) : "memory");
+  } else {
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+  }
+  if (ksplit > 1) cluster_arrive();  // (waited for in front of the first word to a peer: its barrier exists by then)
   chain_release();
-  // A bounded wait. When one runs out the launch is lost (the status flag says so), but every thread keeps
-  // following the same path through the barriers, so the block still ends.
-  auto wait_for = [&](uint64_t* bar, unsigned parity, int code) {
-    if (*(volatile int*)&abort_s) return;
-    if (!mbar_wait(bar, parity)) {
-      *(volatile int*)&abort_s = 1;
-      if (lane == 0) atomicExch(&g_skinny_status, code);
-    }
-  };
 
   if (warp == CONSUMERS) {
     // ---------------------------------------------------------------- producer: one thread, one box per stage (SwiGLU: two)
@@ -223,50 +307,61 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
       int tile = first_tile, chunk = 0;
       for (int n = 0; n < items; ++n) {
         const int s = n % STAGES;
-        if (n >= STAGES) wait_for(&empty_bar[s], ((n / STAGES) & 1) ^ 1, 2);
-        if (*(volatile int*)&abort_s) break;  // no more copies
-        // rows 0-7 and 8-15 of the tile: 16 consecutive weight rows, or 8 gate rows and the 8 up rows under them
-        const int row_lo = OUT == OUT_SWIGLU ? tile * 8 : tile * 16;
-        const int row_hi = OUT == OUT_SWIGLU ? F + tile * 8 : tile * 16 + 8;
-        unsigned char* dst = ring + (size_t)s * STAGE_BYTES;
-        mbar_expect_tx(&full_bar[s], STAGE_BYTES);  // rows or k past the matrix arrive as zeros and count too
-        // An instruction that starts a TMA copy costs the issuing thread some 300 cycles whatever the copy holds, so
-        // the boxes are as large as they can be: 16 rows x 512 k (16 KB), or two of 8 rows for SwiGLU's two halves.
-        // (SwiGLU as a run of stages over 16 gate rows and then one over 16 up rows, one box a stage, measured
-        // slower here: 0.926 against 0.898 ms a decode step of the 1.2B shape.)
-        if (OUT == OUT_CONV) {  // 8 rows each of the projection's B, C and x parts, C = O / 3 rows apart
-          for (int h = 0; h < 3; ++h)
-            tma_load_box(dst + h * (STAGE_BYTES / 3), &map_w, h * (O / 3) + tile * 8, (chunk0 + chunk) * (KC / 64), &full_bar[s]);
-        } else if (OUT == OUT_SWIGLU) {
-          tma_load_box(dst, &map_w, row_lo, (chunk0 + chunk) * (KC / 64), &full_bar[s]);
-          tma_load_box(dst + STAGE_BYTES / 2, &map_w, row_hi, (chunk0 + chunk) * (KC / 64), &full_bar[s]);
-        } else {
-          tma_load_box(dst, &map_w, row_lo, (chunk0 + chunk) * (KC / 64), &full_bar[s]);
+        if (n >= STAGES) {
+          wait_for(&empty_bar[s], ((n / STAGES) & 1) ^ 1, 2);
+          if (*(volatile int*)&abort_s) break;  // no more copies
         }
+        load_stage(s, tile, chunk);
         if (++chunk == chunks) { chunk = 0; tile += tile_step; }
       }
     }
+    __syncwarp();
+    if (ksplit > 1) { cluster_wait(); cluster_arrive(); }
     // Copies may still be in flight: the block must not exit before they have landed. The consumers wait for
     // every stage they read; the producer stays until they are through (the block-wide barrier below).
   } else {
     // ---------------------------------------------------------------- consumers
     const int g = lane >> 2, t = lane & 3;
-    if (OUT == OUT_CONV && tid < NT * 8) {
-      // which request a token belongs to and where its state lies is what the host wrote for this step: looked up while
-      // the kernel ahead is still at work, not once per tile in the read-out (two loads, one after the other)
-      const int r = tid < M ? token_request[tid] : -1;
-      slot_s[tid] = r >= 0 ? tail.slots[r] : -1;
+    constexpr bool BOXES8 = OUT == OUT_SWIGLU || OUT == OUT_CONV;  // boxes of 8 rows: a group of 64 k is 1 KB
+    // This thread's (row, token) pair of a tile's read-out.
+    constexpr int per_tile = BOXES8 ? 64 : 128;  // pairs per n-block
+    static_assert(2 * 128 <= CONSUMERS * 32, "a thread reads out at most one (row, token) pair of a tile");
+    const int out_m = 8 * (tid / per_tile) + tid % 8, out_row = (tid % per_tile) / 8;
+    const bool reads_out = tid < NT * per_tile && out_m < M;
+    // which request this thread's token belongs to and where its state lies is what the host wrote for this step: asked
+    // for while the kernel ahead is still at work (two loads, one after the other), and not looked at before the
+    // activations are in shared memory
+    int my_slot = -1;
+    if (OUT == OUT_CONV) {
+      const int r = token_request[min(out_m, max(M, 1) - 1)];
+      my_slot = tail.slots[max(r, 0)];
+      if (r < 0) my_slot = -1;
     }
+    // the convolution's taps and bias of this thread's channel, up to 4 taps (longer ones are read where they are used)
+    float taps_r[TAPS] = {0.f, 0.f, 0.f, 0.f}, bias_r = 0.f;
+    auto fetch_taps = [&](int tile) {
+      const int c = min(tile * 8 + out_row, O / 3 - 1);
+#pragma unroll
+      for (int l = 0; l < TAPS; ++l) taps_r[l] = tail.taps[(size_t)c * tail.L + min(l, tail.L - 1)];
+      if (tail.bias) bias_r = tail.bias[c];
+    };
+    if (OUT == OUT_CONV) fetch_taps(first_tile);
+    // the rows of tokens that do not exist: the products' columns for them must be numbers, and nobody reads them
+    if (IN != IN_DYT)
+      for (int i = (IN == IN_BF16 ? M : M <= 1 ? 1 : M <= 4 ? 4 : NT * 8) * XS + tid * 8; i < NT * 8 * XS; i += CONSUMERS * 32 * 8) *reinterpret_cast<uint4*>(xs + i) = make_uint4(0u, 0u, 0u, 0u);
     if (IN == IN_BF16) {
       chain_wait();  // from here on the kernel reads what its predecessor wrote
-#pragma unroll
-      for (int m = 0; m < NT * 8; ++m) {  // all copies in flight together
-        const size_t src = m < M ? (size_t)(rows ? rows[m] : m) : 0;
+      // One row: 16-byte loads, which are back sooner than a bulk copy. Several: a warp a row, one copy each (8 rows of
+      // 2,048: 627 -> 613 us a pass over 64 products against 16-byte loads through registers).
+      if (M >= kBulkRows) {
+        for (int m = warp; m < M; m += CONSUMERS)
+          if (lane == 0) bulk_copy(xs + (size_t)m * XS, (const bf16*)x_ + (size_t)(rows ? rows[m] : m) * K + k0, k_len * 2, &rows_bar);
+        wait_for(&rows_bar, 0, 4);
+      } else if (M > 0) {
+        const bf16* src = (const bf16*)x_ + (size_t)(rows ? rows[0] : 0) * K + k0;
         for (int col = tid * 8; col < k_len; col += CONSUMERS * 32 * 8)
-          cp_async16(xs + (size_t)m * XS + col, (const bf16*)x_ + src * K + k0 + col, m < M ? 16 : 0);
+          *reinterpret_cast<uint4*>(xs + col) = *reinterpret_cast<const uint4*>(src + col);
       }
-      cp_async_commit();
-      cp_async_wait<0>();
     } else if (IN == IN_DYT) {
       // float32 residual rows -> bf16(tanh(alpha x) * w + b), element by element: a norm without sums. A warp takes
       // 128-float blocks of k for every token, as below; the weights and shifts are fetched before the wait.
@@ -308,23 +403,23 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
         wv[p] = k < k_len ? *reinterpret_cast<const float4*>(norm_w + k0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       chain_wait();  // from here on the kernel reads what its predecessor wrote
-#pragma unroll 1
-      for (int half = 0; half < NT; ++half) {  // 8 tokens at a time
-        float ss[8];
+      auto stage_rows = [&](auto most, int m0) {  // tokens m0 .. m0 + R - 1
+        constexpr int R = decltype(most)::value;
+        float ss[R];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss[i] = 0.f;
+        for (int i = 0; i < R; ++i) ss[i] = 0.f;
         for (int b0 = warp; b0 < kblocks; b0 += CONSUMERS * PER) {
-          if (b0 != warp || half > 0) {
+          if (b0 != warp || m0 > 0) {
 #pragma unroll
             for (int p = 0; p < PER; ++p) {
               const int k = (b0 + CONSUMERS * p) * 128 + lane * 4;
               wv[p] = k < k_len ? *reinterpret_cast<const float4*>(norm_w + k0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
-          float4 v[PER][8];
+          float4 v[PER][R];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int m = half * 8 + i;
+          for (int i = 0; i < R; ++i) {
+            const int m = m0 + i;
             const float* src = (const float*)x_ + (size_t)(m < M ? (rows ? rows[m] : m) : 0) * K + k0;
 #pragma unroll
             for (int p = 0; p < PER; ++p) {
@@ -338,21 +433,27 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
             float4 w = wv[p];
             if (zero_centered) { w.x += 1.f; w.y += 1.f; w.z += 1.f; w.w += 1.f; }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < R; ++i) {
               const float4 a = v[p][i];
               ss[i] = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss[i]))));
               uint2 packed;
               packed.x = pack_bf16(a.x * w.x, a.y * w.y);
               packed.y = pack_bf16(a.z * w.z, a.w * w.w);
-              if (k < k_len) *reinterpret_cast<uint2*>(xs + (size_t)(half * 8 + i) * XS + k) = packed;
+              if (k < k_len) *reinterpret_cast<uint2*>(xs + (size_t)(m0 + i) * XS + k) = packed;
             }
           }
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < R; ++i) {
           const float total = warp_sum(ss[i]);
-          if (lane == 0) ss_s[warp][half * 8 + i] = total;
+          if (lane == 0) ss_s[warp][m0 + i] = total;
         }
+      };
+      if (M <= 1) stage_rows(Rows<1>(), 0);
+      else if (M <= 4) stage_rows(Rows<4>(), 0);
+      else {
+#pragma unroll 1
+        for (int half = 0; half < NT; ++half) stage_rows(Rows<8>(), half * 8);
       }
     }
     consumer_barrier();  // the activations are in shared memory for every consumer warp
@@ -366,104 +467,114 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
     // Where this thread's 16 bytes of weight rows g and g + 8 lie inside a stage: group of 64 k, row, and the 16-byte
     // unit (slice & 1) * 4 + t XOR g of the 128-byte swizzle. One box holds 16 rows to a group of k, SwiGLU's two boxes
     // 8 rows each. A warp multiplies 64 of a chunk's 512 k: slices 2 * warp and 2 * warp + 1 of 32 k.
-    constexpr bool BOXES8 = OUT == OUT_SWIGLU || OUT == OUT_CONV;  // boxes of 8 rows: a group of 64 k is 1 KB
     constexpr int kg_stride = BOXES8 ? 1024 : 2048;
     constexpr int hi_off = OUT == OUT_CONV ? STAGE_BYTES / 3 : OUT == OUT_SWIGLU ? STAGE_BYTES / 2 : 1024;
-    float acc[NT][4], acc_x[OUT == OUT_CONV ? NT : 1][4];  // acc_x: the convolution's x rows (rows g; rows g + 8 unused)
+    float acc[NT][4], acc2[NT][4], acc_x[OUT == OUT_CONV ? NT : 1][4];  // acc_x: the convolution's x rows (rows g; rows g + 8 unused)
 #pragma unroll
-    for (int j = 0; j < NT; ++j) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
+    for (int j = 0; j < NT; ++j)
+      for (int e = 0; e < 4; ++e) acc[j][e] = acc2[j][e] = 0.f;
 #pragma unroll
     for (int j = 0; j < (OUT == OUT_CONV ? NT : 1); ++j) { acc_x[j][0] = acc_x[j][1] = acc_x[j][2] = acc_x[j][3] = 0.f; }
     int tile = first_tile, c = 0, tiles_done = 0;
+    // What this thread's pair of a tile's read-out needs beside the sums is fetched before the loop over the stages: the norm's factor of the token, and the first tile's values in global memory (the residual stream's, or
+    // the convolution's state, up to 4 taps; longer ones are read where they are used).
+    float inv = 1.f;
+    if (IN == IN_NORM && ksplit == 1 && reads_out) inv = inverse_root(fmaf(sum_sq(out_m), cut.inv_k, eps));
+    // (into shared memory: loads into registers would have to be waited for in front of the loop)
+    const int safe_m = min(out_m, max(M, 1) - 1);
+    auto fetch_ahead = [&](int tile) {
+      if (OUT == OUT_ACC && ksplit == 1 && tid < NT * per_tile)
+        cp_async4(&ahead_s[tid], (const float*)y_ + (size_t)safe_m * O + min(tile * 16 + out_row, O - 1));
+      if (OUT == OUT_CONV && tid < NT * per_tile) {
+        const int C = O / 3;
+        const float* hist = tail.state + (size_t)max(my_slot, 0) * (tail.L - 1) * C + min(tile * 8 + out_row, C - 1);
+#pragma unroll
+        for (int l = 0; l < TAPS - 1; ++l) cp_async4(&ahead_s[l * NT * 64 + tid], hist + (size_t)min(l, tail.L - 2) * C);
+      }
+      if (OUT == OUT_ACC || OUT == OUT_CONV) cp_async_commit();
+    };
+    if (items > 0) fetch_ahead(first_tile);
+    // K cut into parts: the blocks behind the first one send it their sums of x^2, and a tile's sums as soon as they have met (every word is counted on the first block's mbarrier, so that neither
+    // a barrier nor a fence stands between a sum and its way).
+    unsigned peer_part = 0, peer_bar = 0;
+    if (ksplit > 1 && !BOXES8) {
+      cluster_wait();  // the first block's barrier exists
+      if (rank > 0) {
+        peer_part = peer_address(peer, 0) + (unsigned)((rank - 1) * SPLIT_TILES * NT * 128 * 4);
+        peer_bar = peer_address(&gathered, 0);
+        if (IN == IN_NORM && tid < M) peer_store(peer_address(peer_ss, 0) + (unsigned)(((rank - 1) * NT * 8 + tid) * 4), sum_sq(tid), peer_bar);
+      }
+    }
     for (int n = 0; n < items; ++n) {
       const int s = n % STAGES;
       wait_for(&full_bar[s], (n / STAGES) & 1, 1);
+      // all of the stage's reads, then the products in two chains
+      uint4 a_lo[2], a_hi[2], a_x[2], b[2][NT];
 #pragma unroll
       for (int i2 = 0; i2 < 2; ++i2) {
         const int k = c * KC + warp * 64 + i2 * 32 + 8 * t;  // this thread's 8 consecutive k, counted from k0
-        if (k < k_len) {
-          const unsigned char* st = ring + (size_t)s * STAGE_BYTES + warp * kg_stride + g * 128 + (((i2 * 4 + t) ^ g) << 4);
-          const uint4 a_lo = *reinterpret_cast<const uint4*>(st);
-          const uint4 a_hi = *reinterpret_cast<const uint4*>(st + hi_off);
-          const uint32_t a1[4] = {a_lo.x, a_hi.x, a_lo.y, a_hi.y};  // first k-step: this thread's k 0..3
-          const uint32_t a2[4] = {a_lo.z, a_hi.z, a_lo.w, a_hi.w};  // second k-step: its k 4..7
-          uint4 a_x = make_uint4(0u, 0u, 0u, 0u);
-          if (OUT == OUT_CONV) a_x = *reinterpret_cast<const uint4*>(st + 2 * hi_off);
-          const uint32_t x1[4] = {a_x.x, 0u, a_x.y, 0u}, x2[4] = {a_x.z, 0u, a_x.w, 0u};
+        const unsigned char* st = ring + (size_t)s * STAGE_BYTES + warp * kg_stride + g * 128 + (((i2 * 4 + t) ^ g) << 4);
+        a_lo[i2] = *reinterpret_cast<const uint4*>(st);
+        a_hi[i2] = *reinterpret_cast<const uint4*>(st + hi_off);
+        if (OUT == OUT_CONV) a_x[i2] = *reinterpret_cast<const uint4*>(st + 2 * hi_off);
 #pragma unroll
-          for (int j = 0; j < NT; ++j) {
-            const uint4 b = *reinterpret_cast<const uint4*>(xs + (size_t)(8 * j + g) * XS + k);
-            mma_bf16(acc[j], a1, b.x, b.y);
-            mma_bf16(acc[j], a2, b.z, b.w);
-            if (OUT == OUT_CONV) {
-              mma_bf16(acc_x[j], x1, b.x, b.y);
-              mma_bf16(acc_x[j], x2, b.z, b.w);
-            }
-          }
-        }
+        for (int j = 0; j < NT; ++j)  // (k past the end: zeros, as the weights there are)
+          b[i2][j] = k < k_len ? *reinterpret_cast<const uint4*>(xs + (size_t)(8 * j + g) * XS + k) : make_uint4(0u, 0u, 0u, 0u);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[s]);  // this warp has read the stage
+#pragma unroll
+      for (int i2 = 0; i2 < 2; ++i2) {
+        const uint32_t a1[4] = {a_lo[i2].x, a_hi[i2].x, a_lo[i2].y, a_hi[i2].y};  // first k-step: this thread's k 0..3
+        const uint32_t a2[4] = {a_lo[i2].z, a_hi[i2].z, a_lo[i2].w, a_hi[i2].w};  // second k-step: its k 4..7
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          mma_bf16(acc[j], a1, b[i2][j].x, b[i2][j].y);
+          mma_bf16(acc2[j], a2, b[i2][j].z, b[i2][j].w);
+          if (OUT == OUT_CONV) {
+            const uint32_t x1[4] = {a_x[i2].x, 0u, a_x[i2].y, 0u}, x2[4] = {a_x[i2].z, 0u, a_x[i2].w, 0u};
+            mma_bf16(acc_x[j], x1, b[i2][j].x, b[i2][j].y);
+            mma_bf16(acc_x[j], x2, b[i2][j].z, b[i2][j].w);
+          }
+        }
+      }
       if (++c < chunks) continue;
 
-      // the row tile is complete: the consumer warps' partial sums meet in shared memory, then the epilogue
+      // the row tile is complete: the consumer warps' partial sums meet in shared memory, then the epilogue. Where the
+      // tiles' sums take two places in turn one barrier a tile is enough: who writes the third tile's has passed the second
+      // one's barrier, and with it whoever reads the first one's.
+      float* sums = red + (cut.two_sums ? (tiles_done & 1) * RED : 0);
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        float* r0 = red + (((size_t)warp * NT + j) * RT + g) * 8 + 2 * t;
-        r0[0] = acc[j][0];
-        r0[1] = acc[j][1];
-        r0[64] = acc[j][2];  // row g + 8
-        r0[65] = acc[j][3];
-        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        float* r0 = sums + (((size_t)warp * NT + j) * RT + g) * 8 + 2 * t;
+        *reinterpret_cast<float2*>(r0) = make_float2(acc[j][0] + acc2[j][0], acc[j][1] + acc2[j][1]);
+        *reinterpret_cast<float2*>(r0 + 64) = make_float2(acc[j][2] + acc2[j][2], acc[j][3] + acc2[j][3]);  // row g + 8
+        for (int e = 0; e < 4; ++e) acc[j][e] = acc2[j][e] = 0.f;
         if (OUT == OUT_CONV) {
           r0[128] = acc_x[j][0];  // row g + 16: the x part
           r0[129] = acc_x[j][1];
           acc_x[j][0] = acc_x[j][1] = acc_x[j][2] = acc_x[j][3] = 0.f;
         }
       }
-      constexpr int per_tile = BOXES8 ? 64 : 128;  // (row, token) pairs per n-block
-      static_assert(2 * 128 <= CONSUMERS * 32, "a thread reads out at most one (row, token) pair of a tile");
-      float before = 0.f;  // the residual stream's value, on its way while the sums meet
-      if (OUT == OUT_ACC && ksplit == 1 && tid < NT * per_tile) {
-        const int m = 8 * (tid / per_tile) + tid % 8, o = tile * 16 + (tid % per_tile) / 8;
-        if (m < M && o < O) before = ((const float*)y_)[(size_t)m * O + o];
-      }
-      // The convolution's taps, bias and state rows of this thread's (channel, token), likewise (up to 4 taps; longer
-      // ones are read where they are used).
-      constexpr int TAPS = 4;
-      float taps_r[TAPS] = {0.f, 0.f, 0.f, 0.f}, hist_r[TAPS - 1] = {0.f, 0.f, 0.f}, bias_r = 0.f;
-      if (OUT == OUT_CONV && tail.L <= TAPS && tid < NT * per_tile) {
-        const int m = 8 * (tid / per_tile) + tid % 8, C = O / 3, c = tile * 8 + (tid % per_tile) / 8;
-        const int slot = m < M ? slot_s[m] : -1;
-        if (slot >= 0 && c < C) {
-          const float* hist = tail.state + (size_t)slot * (tail.L - 1) * C + c;
-#pragma unroll
-          for (int l = 0; l < TAPS; ++l) {
-            if (l < tail.L) taps_r[l] = tail.taps[(size_t)c * tail.L + l];
-            if (l < tail.L - 1) hist_r[l] = hist[(size_t)l * C];
-          }
-          if (tail.bias) bias_r = tail.bias[c];
-        }
-      }
       consumer_barrier();
-      for (int i = tid; i < NT * per_tile; i += CONSUMERS * 32) {
-        const int j = i / per_tile, row = (i % per_tile) / 8, tok = i % 8;
-        const int m = 8 * j + tok;
-        if (m >= M) continue;
+      // (one pass: the loop only gives `continue` its meaning)
+      if (OUT == OUT_ACC || OUT == OUT_CONV) cp_async_wait<0>();
+      for (bool once = reads_out; once; once = false) {
+        const int j = tid / per_tile, row = out_row, tok = tid % 8, m = out_m, i = tid;
         float v = 0.f, u = 0.f, xv = 0.f;
 #pragma unroll
         for (int w = 0; w < CONSUMERS; ++w) {
-          const float* r0 = red + (((size_t)w * NT + j) * RT + row) * 8 + tok;
+          const float* r0 = sums + (((size_t)w * NT + j) * RT + row) * 8 + tok;
           v += r0[0];
           if (BOXES8) u += r0[64];
           if (OUT == OUT_CONV) xv += r0[128];
         }
         if (ksplit > 1) {  // a part of K: kept until the parts meet
-          part[tiles_done * NT * 128 + i] = v;
+          if (rank > 0) peer_store(peer_part + (unsigned)((tiles_done * NT * 128 + i) * 4), v, peer_bar);
+          else part[tiles_done * NT * 128 + i] = v;  // (read again by this thread)
           continue;
         }
         if (IN == IN_NORM) {
-          const float inv = 1.f / sqrtf(sum_sq(m) / (float)K + eps);
           v *= inv;
           u *= inv;
           xv *= inv;
@@ -472,7 +583,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
           // v, u, xv: the B, C and x parts of channel c for token m, rounded as the projection's own read-out would
           const int C = O / 3, c = tile * 8 + row, L = tail.L;
           if (c >= C) continue;
-          const int slot = slot_s[m];
+          const int slot = my_slot;
           bf16* out = (bf16*)y_ + (size_t)m * C + c;
           if (slot < 0) {
             *out = __float2bfloat16_rn(0.f);
@@ -482,12 +593,13 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
           const float uu = bq * xq;
           float* hist = tail.state + (size_t)slot * (L - 1) * C + c;
           float sum = 0.f;
-          if (L <= TAPS) {  // (everything is in registers already)
+          if (L <= TAPS) {  // (everything is here already)
 #pragma unroll
             for (int l = 0; l < TAPS - 1; ++l) {
               if (l < L - 1) {
-                sum = fmaf(hist_r[l], taps_r[l], sum);
-                if (l > 0 && tail.write) hist[(size_t)(l - 1) * C] = hist_r[l];
+                const float h = ahead_s[l * NT * 64 + tid];
+                sum = fmaf(h, taps_r[l], sum);
+                if (l > 0 && tail.write) hist[(size_t)(l - 1) * C] = h;
               }
             }
             float last = taps_r[0];
@@ -521,65 +633,51 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
           if (OUT != OUT_BF16 && tail.bias != nullptr) v += tail.bias[o];
           if (OUT == OUT_BF16) ((bf16*)y_)[at] = __float2bfloat16_rn(plain_activation_fast(v, tail.L));
           else if (OUT == OUT_F32) ((float*)y_)[at] = v;
-          else ((float*)y_)[at] = before + v;
+          else ((float*)y_)[at] = ahead_s[tid] + v;
         }
       }
-      consumer_barrier();  // `red` is free again before the next tile's sums are written
       c = 0;
       tile += tile_step;
       ++tiles_done;
+      if (n + 1 < items) {
+        fetch_ahead(tile);
+        if (OUT == OUT_CONV) fetch_taps(tile);
+      }
+      if (!cut.two_sums) consumer_barrier();  // `red` is free again for the next tile (and `part` complete before it is read)
     }
 
-    if (ksplit > 1 && !BOXES8) {
+    __syncwarp();
+    if (ksplit > 1) cluster_arrive();  // (a peer has sent its words by now)
+    if (ksplit > 1 && !BOXES8 && rank == 0) {
       // ---------------------------------------------------------------- the parts of K meet in the first block
-      const int count = my_tiles * NT * 128;
-      if (rank > 0) {
-        const unsigned to = peer_address(peer, 0) + (unsigned)((rank - 1) * SPLIT_TILES * NT * 128 * 4);
-        for (int i = tid; i < count; i += CONSUMERS * 32) peer_store(to + (unsigned)i * 4u, part[i]);
-        if (IN == IN_NORM && tid < NT * 8) peer_store(peer_address(peer_ss, 0) + (unsigned)(((rank - 1) * NT * 8 + tid) * 4), sum_sq(tid));
-        consumer_barrier();  // all of this block's sums are on their way; one thread tells the first block
-        if (tid == 0) {
-          asm volatile("fence.acq_rel.cluster;" ::: "memory");
-          asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_address(&gathered, 0)) : "memory");
-        }
-      } else {
-        constexpr int MOST = (SPLIT_TILES * NT * 128 + CONSUMERS * 32 - 1) / (CONSUMERS * 32);  // pairs a thread writes
-        float before[MOST];  // the residual stream's values, fetched while the other parts are on their way
+      float before_split[SPLIT_TILES] = {};  // the residual stream's values, asked for while the other parts are on their way
+      if (OUT == OUT_ACC) {
 #pragma unroll
-        for (int n = 0; n < MOST; ++n) {
-          before[n] = 0.f;
-          const int i = tid + n * CONSUMERS * 32;
-          if (OUT == OUT_ACC && i < count) {
-            const int tl = i / (NT * 128), e = i % (NT * 128);
-            const int m = 8 * (e / 128) + e % 8, o = (first_tile + tl * tile_step) * 16 + (e % 128) / 8;
-            if (m < M && o < O) before[n] = ((const float*)y_)[(size_t)m * O + o];
-          }
+        for (int tl = 0; tl < SPLIT_TILES; ++tl)
+          before_split[tl] = ((const float*)y_)[(size_t)safe_m * O + min((first_tile + tl * tile_step) * 16 + out_row, O - 1)];
+      }
+      if (!*(volatile int*)&abort_s && !mbar_wait_cluster(&gathered, 0)) {
+        *(volatile int*)&abort_s = 1;
+        if (lane == 0) atomicExch(&g_skinny_status, 3);
+      }
+      if (reads_out && !*(volatile int*)&abort_s) {
+        float ss = IN == IN_NORM ? sum_sq(out_m) : 0.f;
+        if (IN == IN_NORM) {
+          for (int r = 0; r < ksplit - 1; ++r) ss += peer_ss[r * NT * 8 + out_m];  // in rank order, like the sums below
+          inv = inverse_root(fmaf(ss, cut.inv_k, eps));
         }
-        if (!*(volatile int*)&abort_s && !mbar_wait_cluster(&gathered, 0)) {
-          *(volatile int*)&abort_s = 1;
-          if (lane == 0) atomicExch(&g_skinny_status, 3);
-        }
-        if (!*(volatile int*)&abort_s) {
 #pragma unroll
-          for (int n = 0; n < MOST; ++n) {
-            const int i = tid + n * CONSUMERS * 32;
-            if (i >= count) continue;
-            const int tl = i / (NT * 128), e = i % (NT * 128);
-            const int j = e / 128, row = (e % 128) / 8, tok = e % 8;
-            const int m = 8 * j + tok, o = (first_tile + tl * tile_step) * 16 + row;
-            if (m >= M || o >= O) continue;
-            float v = part[i], ss = IN == IN_NORM ? sum_sq(m) : 0.f;
-            for (int r = 0; r < ksplit - 1; ++r) {  // in rank order
-              v += peer[(r * SPLIT_TILES + tl) * NT * 128 + e];
-              if (IN == IN_NORM) ss += peer_ss[r * NT * 8 + m];
-            }
-            if (IN == IN_NORM) v *= 1.f / sqrtf(ss / (float)K + eps);
-            const size_t at = (size_t)m * O + o;
-            if (OUT != OUT_BF16 && tail.bias != nullptr) v += tail.bias[o];
-            if (OUT == OUT_BF16) ((bf16*)y_)[at] = __float2bfloat16_rn(plain_activation_fast(v, tail.L));
-            else if (OUT == OUT_F32) ((float*)y_)[at] = v;
-            else ((float*)y_)[at] = before[n] + v;
-          }
+        for (int tl = 0; tl < SPLIT_TILES; ++tl) {
+          const int o = (first_tile + tl * tile_step) * 16 + out_row;
+          if (tl >= my_tiles || o >= O) break;
+          float v = part[tl * NT * 128 + tid];
+          for (int r = 0; r < ksplit - 1; ++r) v += peer[(r * SPLIT_TILES + tl) * NT * 128 + tid];
+          if (IN == IN_NORM) v *= inv;
+          const size_t at = (size_t)out_m * O + o;
+          if (OUT != OUT_BF16 && tail.bias != nullptr) v += tail.bias[o];
+          if (OUT == OUT_BF16) ((bf16*)y_)[at] = __float2bfloat16_rn(plain_activation_fast(v, tail.L));
+          else if (OUT == OUT_F32) ((float*)y_)[at] = v;
+          else ((float*)y_)[at] = before_split[tl] + v;
         }
       }
     }
@@ -588,7 +686,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const void* __rest
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // a lost launch: give copies still in flight time to land
   }
   __syncthreads();  // nobody leaves while a copy into this block's shared memory may be in flight
-  if (ksplit > 1) cluster_meet();  // nor while a peer may still write its sums there
+  if (ksplit > 1) cluster_wait();  // nor while a peer may still write its sums there
 }
 
 // ------------------------------------------------------------------------------------------------ host side
@@ -635,21 +733,22 @@ int weight_map(CUtensorMap* out, const void* w, int O, int K, int box_rows) {
   return 0;
 }
 
-constexpr int kMaxSmemBytes = 226 * 1024;  // the block also has a few hundred bytes of static shared memory
+constexpr int kMaxSmemBytes = 226 * 1024;  // the block also has up to 1.3 KB of static shared memory
+constexpr int kSmBytes = 228 * 1024, kBesideSmem = 1024 + 1152;  // an SM's; what a block takes beside the dynamic part, at 8 tokens
 
 // Shared memory of a block with `ksplit` parts of K: alignment slack, the ring, the consumers' partial sums, the
 // parts' meeting place, and the activations of this block's part of K.
 template <int NT, int OUTM>
-int block_smem(int K, int ksplit) {
+int block_smem(int K, int ksplit, int places = 1) {
   const int chunks = (K + KC - 1) / KC, part_k = (chunks + ksplit - 1) / ksplit * KC;
-  int bytes = 1024 + Ring<OUTM>::DEPTH * Ring<OUTM>::BYTES + CONSUMERS * NT * Ring<OUTM>::ROWS * 8 * (int)sizeof(float) +
+  int bytes = 1024 + Ring<OUTM>::DEPTH * Ring<OUTM>::BYTES + places * CONSUMERS * NT * Ring<OUTM>::ROWS * 8 * (int)sizeof(float) +
               NT * 8 * (part_k + 32) * (int)sizeof(bf16);
   if (ksplit > 1) bytes += (ksplit * SPLIT_TILES * NT * 128 + (ksplit - 1) * NT * 8) * (int)sizeof(float);
   return bytes;
 }
 
 struct SplitPlan {
-  int ksplit, grid, smem;
+  int ksplit, grid, smem, rounds, two_sums;
 };
 
 // How a product is cut; not 0 where no cut fits (the whole K, or a part of it, does not fit a block's shared memory, or a
@@ -669,9 +768,14 @@ int plan_for(SplitPlan& plan, int num_tiles, int K, int groups) {
   {
     std::lock_guard<std::mutex> lock(mutex);
     if (sms_of[device] == 0) {
-      cudaError_t e = cudaFuncSetAttribute(skinny_gemm_kernel<NT, IN, OUTM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(skinny_gemm_kernel<NT, IN, OUTM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes);
+      auto allow = [](auto kernel) {  // all that a block may have beside its static part
+        cudaFuncAttributes has;
+        cudaError_t e = cudaFuncGetAttributes(&has, kernel);
+        const int most = min(kMaxSmemBytes, 227 * 1024 - (int)has.sharedSizeBytes);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      };
+      cudaError_t e = allow(skinny_gemm_kernel<NT, IN, OUTM, false>);
+      if (e == cudaSuccess) e = allow(skinny_gemm_kernel<NT, IN, OUTM, true>);
       if (e != cudaSuccess) return (int)e;
       cudaDeviceGetAttribute(&sms_of[device], cudaDevAttrMultiProcessorCount, device);
     }
@@ -688,13 +792,16 @@ int plan_for(SplitPlan& plan, int num_tiles, int K, int groups) {
       // (nothing cut).
       const int chunks = (K + KC - 1) / KC;
       long long best = -1;
-      plan = SplitPlan{1, 0, 0};
+      plan = SplitPlan{1, 0, 0, 0, 0};
       for (int ksplit = 1; ksplit <= MAX_KSPLIT; ksplit *= 2) {
         if (ksplit > 1 && (UNCUT || ksplit > chunks)) break;
         const int smem = block_smem<NT, OUTM>(K, ksplit);
         if (smem > kMaxSmemBytes) continue;
         static const int per_sm_cap = [] { const char* v = getenv("AKAS_B200_SKINNY_PER_SM"); return v ? atoi(v) : 3; }();
-        const int per_sm = max(1, min(per_sm_cap, kMaxSmemBytes / (smem + 1024)));
+        const int per_sm = max(1, min(per_sm_cap, kSmBytes / (smem + kBesideSmem)));
+        // two places for the tiles' sums where K is whole and they cost no SM a block
+        const int wider = block_smem<NT, OUTM>(K, ksplit, 2);
+        const int two_sums = ksplit == 1 && wider <= kMaxSmemBytes - 2048 && max(1, min(per_sm_cap, kSmBytes / (wider + kBesideSmem))) == per_sm;
         int clusters = sms * per_sm / ksplit;
         if (ksplit > 1) {
           const auto room_key = std::make_tuple(device, ksplit, smem);
@@ -732,7 +839,7 @@ int plan_for(SplitPlan& plan, int num_tiles, int K, int groups) {
         if (ksplit > 1) fetched += (long long)part_cost * ksplit;
         if (best < 0 || fetched < best) {
           best = fetched;
-          plan = SplitPlan{ksplit, blocks, smem};
+          plan = SplitPlan{ksplit, blocks, two_sums ? wider : smem, rounds, two_sums};
         }
       }
       if (best < 0) return (int)cudaErrorInvalidValue;
@@ -776,7 +883,8 @@ int launch_one(int num_tiles, const void* x, const int* rows, const float* norm_
   }
   config.attrs = attribute;
   config.numAttrs = n;
-  return (int)cudaLaunchKernelEx(&config, kernel, map, x, rows, norm_w, eps, zero_centered, y, M, O, K, num_tiles, plan.ksplit, groups, tail);
+  const Cut cut{plan.ksplit == 1 ? 0 : plan.ksplit == 2 ? 1 : plan.ksplit == 4 ? 2 : 3, groups > 1 ? 1 : 0, plan.rounds, plan.two_sums, 1.f / (float)K};
+  return (int)cudaLaunchKernelEx(&config, kernel, map, x, rows, norm_w, eps, zero_centered, y, M, O, K, num_tiles, cut, tail);
 }
 
 template <int NT, int IN>

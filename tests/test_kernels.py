@@ -196,6 +196,27 @@ def test_skinny_products_for_few_tokens(ops, m, k, o, monkeypatch):
     assert cuda.skinny_status() == 0  # no bounded wait inside the kernel ran out
 
 
+@pytest.mark.parametrize("m", [1, 2, 4, 5, 7])
+@pytest.mark.parametrize("k,o", [(512, 20008), (1088, 9999), (4096, 520), (8192, 264)])
+def test_skinny_products_by_rows_and_tiles(ops, m, k, o):
+    """One row, several rows by a copy each, numbers of rows that have code of their own behind a norm; several row tiles a
+    block, whose sums take turns in shared memory; K cut over a cluster, with and without the norm. A row of infinities
+    beside the others stays in its own row."""
+    cuda, ref = ops
+    x, w = _rand((m, k), torch.bfloat16, 51), _rand((o, k), torch.bfloat16, 52, 0.05)
+    if m > 2:
+        x[1] = float("inf")
+    keep = [i for i in range(m) if m <= 2 or i != 1]
+    want = x.double()[keep] @ w.double().T
+    res = _rand((m, o), torch.float32, 53)
+    _close(cuda.linear(x, w, out_dtype=torch.float32)[keep], want, torch.float32, "f32 out", k)
+    _close(cuda.linear(x, w, residual=res.clone())[keep], res.double()[keep] + want, torch.float32, "accumulate", k)
+    h, nw = _rand((m, k), torch.float32, 54, 3.0), _rand((k,), torch.float32, 55) + 1
+    _close(cuda.norm_linear(h, nw, 1e-6, False, w, torch.float32), ref.norm_linear(h, nw, 1e-6, False, w, torch.float32), torch.bfloat16,
+           "norm + product")
+    assert cuda.skinny_status() == 0
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 17, 40, 64, 128])
 @pytest.mark.parametrize("k,o", [(64, 50), (192, 320), (2048, 37), (8192, 64), (96, 40), (2048, 1000), (1024, 2048),
                                  (520, 3000), (256, 20000)])
