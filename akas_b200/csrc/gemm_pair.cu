@@ -21,18 +21,28 @@
 //            the stage's "empty" barrier of BOTH blocks (multicast commit: a commit to both blocks costs the issuing
 //            thread about as much as four products, hence two steps of K per stage); after a tile's last stage it
 //            commits to both blocks' "accumulator full" barrier.
-//   warps 2-5 read-out, in both blocks: each warp owns the 32 accumulator lanes (token rows) of its sub-partition
-//            of its own block's tensor memory. A lane holds a token row, so storing from registers would touch 32
-//            rows per instruction; instead the warp reads 32 columns with tcgen05.ld, writes them into a staging
-//            tile in shared memory in the swizzle that TMA expects (no bank conflicts), and one lane hands the tile
-//            (32 rows x 128 or 64 bytes) to TMA, which writes whole rows and clips at the matrix's edges:
-//              BF16    y bfloat16 [M, N]          a TMA store of 32 x 64 channels
-//              ACC     y float32 [M, N] +=        a TMA reduce-add of 32 x 32 channels: the residual stream is added
+//   warps 2-9 read-out, in both blocks: two groups of four warps, a warp of each for the 32 accumulator lanes (token
+//            rows) of a sub-partition of its own block's tensor memory. A lane holds a token row, so storing from
+//            registers would touch 32 rows per instruction; instead a group reads 32 or 64 columns with tcgen05.ld,
+//            writes them into a staging tile in shared memory in the swizzle that TMA expects (no bank conflicts), and
+//            one thread hands the tile (128 rows x 128 or 64 bytes) to TMA, which writes whole rows and clips at the
+//            matrix's edges (a copy per warp and 32 rows was four times as many copies, each some 300 cycles):
+//              BF16    y bfloat16 [M, N]          a TMA store of 128 x 64 channels
+//              ACC     y float32 [M, N] +=        a TMA reduce-add of 128 x 32 channels: the residual stream is added
 //                                                 to in the L2, no SM reads it
-//              F32     y float32 [M, N]           a TMA store of 32 x 32 channels
-//              SWIGLU  y bfloat16 [M, F]          silu(gate) * up of 32 channels, a TMA store of 32 x 32
-//            Two staging tiles per warp: the next is filled while TMA reads the last. The warp then arrives on the
+//              F32     y float32 [M, N]           a TMA store of 128 x 32 channels
+//              SWIGLU  y bfloat16 [M, F]          silu(gate) * up of 32 channels, a TMA store of 128 x 32
+//            The groups take a tile's columns in turn, each with a staging tile of its own; the block's last tile uses
+//            the ring, which nobody needs any more, so that no store is waited for. The warps then arrive on the
 //            leader's "accumulator empty" barrier (the peer through the cluster's shared memory window).
+// Weights. The tensor cores' warp of the block that issues nothing asks the L2 for the pair's weights, whole rows, as soon
+// as the kernel runs (219 -> 211 us a layer of four products at 2,048 tokens and width 2,048, the read-out above included).
+// Parts of K (SPLIT, ACC and F32 only). A product with few tiles and a long K leaves most pairs idle and the others walking
+// their stages (some 1,100 cycles each with four in flight). There a cluster is 2 to 4 pairs that take a part of K each of one
+// tile of 128 channels. When all have run, every block sends the sums of the 32-column units that it does not finish to
+// the block of the same rows that does (16 KB copies between shared memories, counted on the receiver's mbarrier), which
+// adds the parts in their order and reads out: sums do not depend on timing. [768 x 4608] . [1024 x 4608]^T 26.5 -> 18.7
+// us, 512 rows 26.3 -> 16.4; the meeting takes 4.5 us, so a K of 1,024 (9.8 us) stays whole.
 // For SWIGLU the leader stages the tile's BN/2 gate rows and the peer the BN/2 up rows under them of the stacked
 // [2F, K] matrix, so columns 0..BN/2-1 of an accumulator are gate and the rest up, in both blocks.
 // No load is multicast. Every wait on an mbarrier is bounded (akas_gemm_pair_status); the cluster meets before any
@@ -48,15 +58,18 @@ namespace {
 
 constexpr int BM = 128;    // token rows a block stages; a pair's tile has 256
 constexpr int STEPS = 2;    // 64-wide steps of K in a stage
-constexpr int THREADS = 192;
-constexpr int STAGING = 4096;  // bytes of one staging tile: 32 rows x 128 bytes
+constexpr int READERS = 8;  // read-out warps: two per sub-partition of tensor memory, each for every second staging tile
+constexpr int THREADS = 64 + READERS * 32;
+constexpr int STAGING = 16384;  // bytes of one staging tile: the block's 128 token rows x 128 bytes
+constexpr int MAX_PARTS = 4;   // parts of K: pairs of one cluster (SPLIT)
+constexpr int SPLIT_BN = 128;  // channels of a tile whose K is cut
 enum { EPI_BF16 = 0, EPI_ACC = 1, EPI_SWIGLU = 2, EPI_F32 = 3 };
 
 template <int BN> struct Shape {
   static constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, HALF_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGE_BYTES = STEPS * HALF_BYTES;  // x of both steps of K, then W of both steps
   static constexpr int STAGES = BN >= 192 ? 3 : 4;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 8 * STAGING + 1024;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 2 * STAGING + 1024;
   static constexpr int TMEM_COLS = BN > 128 ? 512 : 2 * BN;  // two accumulators of BN columns, a power of two
 };
 
@@ -76,8 +89,12 @@ __device__ __forceinline__ unsigned peer_address(const void* local, unsigned ran
 __device__ __forceinline__ void mbar_arrive_at(unsigned cluster_address) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Bytes of this block's shared memory into another block's of the cluster, counted there on an mbarrier.
+__device__ __forceinline__ void copy_to_peer(unsigned peer_dst, const void* src, unsigned bytes, unsigned peer_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(peer_dst), "r"(smem_u32(src)), "r"(bytes), "r"(peer_bar) : "memory");
 }
 // A tile load into this block's shared memory whose bytes are counted on a barrier given by its address in the
 // cluster's window (the leader's). Not a multicast: one destination.
@@ -100,15 +117,16 @@ __device__ __forceinline__ void umma_pair(unsigned tmem_d, uint64_t a_desc, uint
       ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Arrives, once the products issued so far have run, on the barrier at this offset in both blocks of the pair.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, unsigned leader) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
+               ::"r"(smem_u32(bar)), "h"((unsigned short)(3u << leader)) : "memory");
 }
-template <int BN, int EPI, bool WIDE>
+// SPLIT: the cluster is `parts` pairs of blocks that take a part of K each of ONE tile; see "Parts of K" above.
+template <int BN, int EPI, bool WIDE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_y, int M, int N, int K, int F, const float* __restrict__ bias,
-                 int act) {
+                 int act, int parts, const __nv_bfloat16* __restrict__ w) {
   // N: channels of the product (for SWIGLU the stacked height 2F); a tile covers BN of them (SWIGLU: BN/2 gate
   // rows f0.. and BN/2 up rows F + f0..).
   using S = Shape<BN>;
@@ -116,21 +134,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;  // output columns a tile yields
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
-  unsigned char* staging = smem + STAGES * STAGE_BYTES;  // [4 warps][2][STAGING], 1,024-byte aligned
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+  unsigned char* staging = smem + STAGES * STAGE_BYTES;  // [2 groups of read-out warps][STAGING], 1,024-byte aligned
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2], gathered;
   __shared__ unsigned tmem_base_s;
   __shared__ int abort_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const unsigned rank = cluster_rank();
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  // this block's number in its pair, its pair's part of K, and the cluster rank of the pair's leader
+  const unsigned crank = cluster_rank(), rank = crank & 1u, part = SPLIT ? crank >> 1 : 0u, leader = SPLIT ? crank & ~1u : 0u;
+  const int pair = SPLIT ? (int)blockIdx.x / (2 * parts) : (int)blockIdx.x >> 1, pairs = SPLIT ? (int)gridDim.x / (2 * parts) : (int)gridDim.x >> 1;
   const int out_cols = EPI == EPI_SWIGLU ? F : N;
   const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (out_cols + TILE_N - 1) / TILE_N;
   const int tiles = tiles_m * tiles_n, k_blocks = (K + BK - 1) / BK;
+  const int all_stages = (k_blocks + STEPS - 1) / STEPS;  // stages of a tile, and those of this pair's part of K
+  const int stage0 = SPLIT ? all_stages * (int)part / parts : 0, stage1 = SPLIT ? all_stages * ((int)part + 1) / parts : all_stages;
+  constexpr int UNITS = BN / 32;  // SPLIT: a tile's sums are exchanged by 32 columns; unit u is finished by part u % parts
+  const int my_units = SPLIT ? (UNITS - (int)part + parts - 1) / parts : 0;
 
   if (tid == 0) {
     abort_s = 0;
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }  // four warps of each block
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * READERS); }  // the read-out warps of both blocks
+    mbar_init(&gathered, 1);
+    if (SPLIT) mbar_expect_tx(&gathered, (unsigned)((parts - 1) * my_units * STAGING));  // the other parts' sums of this block's units
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // tensor memory of both SMs: two accumulators of BN float32 columns, 128 lanes in each block
@@ -139,7 +164,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  cluster_meet();  // the peer's barriers exist and its tensor memory is allocated before anything arrives there
+  cluster_arrive();
+  cluster_wait();  // the peers' barriers exist and their tensor memory is allocated before anything arrives there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem_base = tmem_base_s;
   chain_release();  // (programmatic dependent launch) the next kernel on the stream may set itself up beside this one
@@ -157,39 +183,68 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (lane == 0) {
       // The ring's first filling asks for the weights at once (no kernel writes them) and for the token rows only when
       // the kernel before this one on the stream is done; from then on a stage's two copies go out together.
-      const int per_tile = (k_blocks + STEPS - 1) / STEPS;  // stages of a tile
+      const int per_tile = stage1 - stage0;
       const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
       const int total = my_tiles * per_tile, head = total < STAGES ? total : STAGES;
-      auto load = [&](int i, bool weights, bool rows) {
-        const int tile = pair + (i / per_tile) * pairs, kb = (i % per_tile) * STEPS, s = i % STAGES;
-        const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM, n0 = (tile % tiles_n) * TILE_N;
+      // the next stage, walked without divisions: its tile's rows and channels, its steps of K
+      struct Place { int tile, stage, m0, w_row; };
+      auto place_tile = [&](Place& at) {
+        at.m0 = (at.tile / tiles_n) * 2 * BM + (int)rank * BM;
+        const int n0 = (at.tile % tiles_n) * TILE_N;
         // this block's half of the tile's channels: rows of W
-        const int w_row = EPI == EPI_SWIGLU ? (rank == 0 ? n0 : F + n0) : n0 + (int)rank * (BN / 2);
+        at.w_row = EPI == EPI_SWIGLU ? (rank == 0 ? n0 : F + n0) : n0 + (int)rank * (BN / 2);
+      };
+      auto next_stage = [&](Place& at) {
+        if (++at.stage == stage1) { at.stage = stage0; at.tile += pairs; place_tile(at); }
+      };
+      auto load = [&](int s, const Place& at, bool weights, bool rows) {
+        const int kb = at.stage * STEPS;
         unsigned char* a = smem + (size_t)s * STAGE_BYTES;
-        const unsigned leader_full = peer_address(&full_bar[s], 0);
+        const unsigned leader_full = peer_address(&full_bar[s], leader);
         if (weights && rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);  // the bytes of both blocks
         if (WIDE) {  // K is a multiple of 64: both steps of K in one copy per operand (groups past K: zeros)
-          if (rows) tma_load_3d_for(a, &map_x, m0, kb, leader_full);
-          if (weights) tma_load_3d_for(a + STEPS * A_BYTES, &map_w, w_row, kb, leader_full);
+          if (rows) tma_load_3d_for(a, &map_x, at.m0, kb, leader_full);
+          if (weights) tma_load_3d_for(a + STEPS * A_BYTES, &map_w, at.w_row, kb, leader_full);
         } else {
 #pragma unroll
           for (int h = 0; h < STEPS; ++h) {  // a step past the end of K is filled with zeros
-            if (rows) tma_load_2d_for(a + h * A_BYTES, &map_x, (kb + h) * BK, m0, leader_full);
-            if (weights) tma_load_2d_for(a + STEPS * A_BYTES + h * S::B_BYTES, &map_w, (kb + h) * BK, w_row, leader_full);
+            if (rows) tma_load_2d_for(a + h * A_BYTES, &map_x, (kb + h) * BK, at.m0, leader_full);
+            if (weights) tma_load_2d_for(a + STEPS * A_BYTES + h * S::B_BYTES, &map_w, (kb + h) * BK, at.w_row, leader_full);
           }
         }
       };
-      for (int i = 0; i < head; ++i) load(i, true, false);
+      Place first{pair, stage0, 0, 0};
+      place_tile(first);
+      Place at = first;
+      for (int i = 0; i < head; ++i) { load(i, at, true, false); next_stage(at); }
       chain_wait();
-      for (int i = 0; i < head; ++i) load(i, false, true);
+      at = first;
+      for (int i = 0; i < head; ++i) { load(i, at, false, true); next_stage(at); }
+      int s = head % STAGES;
       for (int i = head; i < total; ++i) {
-        wait_for(&empty_bar[i % STAGES], ((i / STAGES) & 1) ^ 1, 1);
+        wait_for(&empty_bar[s], ((i / STAGES) & 1) ^ 1, 1);
         if (*(volatile int*)&abort_s) break;
-        load(i, true, true);
+        load(s, at, true, true);
+        next_stage(at);
+        if (++s == STAGES) s = 0;
       }
     }
+    if (SPLIT) { __syncwarp(); cluster_arrive(); cluster_wait(); }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ tensor cores (the leader issues for the pair)
+    if (rank == 1) {
+      // The other block's warp asks the L2 for the weights of the pair's tiles, whole rows at a time, as soon as the kernel
+      // runs: with the ring's stages alone, what is in flight does not cover DRAM's latency where few pairs work. Where
+      // several pairs read the same channels, the first row tile's does it.
+      for (int tile = pair; tile < tiles_n; tile += pairs) {
+        const int n0 = tile * TILE_N, from = stage0 * STEPS * BK, upto = min(K, stage1 * STEPS * BK);
+        for (int r = lane; r < BN; r += 32) {
+          const int row = EPI != EPI_SWIGLU ? n0 + r : r < TILE_N ? n0 + r : F + n0 + r - TILE_N;
+          if (n0 + (EPI != EPI_SWIGLU ? r : r % TILE_N) < out_cols && upto > from)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)row * K + from), "r"((upto - from) * 2) : "memory");
+        }
+      }
+    }
     if (lane == 0 && rank == 0) {
       // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 256 over the pair
       constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(2 * BM >> 4) << 24);
@@ -199,7 +254,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         wait_for(&acc_empty[acc], ((t >> 1) & 1) ^ 1, 2);  // both blocks' read-outs have drained this accumulator
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned d = tmem_base + acc * BN;
-        for (int kb = 0; kb < k_blocks; kb += STEPS, ++it) {
+        for (int kb = stage0 * STEPS; kb < (SPLIT ? stage1 * STEPS : k_blocks); kb += STEPS, ++it) {
           const int s = it % STAGES;
           wait_for(&full_bar[s], (it / STAGES) & 1, 2);
           if (*(volatile int*)&abort_s) break;
@@ -212,38 +267,97 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; ++k)  // 32 bytes further along the swizzled row per step
               umma_pair(d, a_desc + (uint64_t)(k * UMMA_K * 2 >> 4), b_desc + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
-                        (kb | h | k) != 0 ? 1u : 0u);
+                        ((kb - stage0 * STEPS) | h | k) != 0 ? 1u : 0u);
           }
-          umma_commit_pair(&empty_bar[s]);  // the stage is free in both blocks once these products have read it
+          umma_commit_pair(&empty_bar[s], leader);  // the stage is free in both blocks once these products have read it
         }
         if (*(volatile int*)&abort_s) break;
-        umma_commit_pair(&acc_full[acc]);  // the tile's sums are complete, in both blocks
+        umma_commit_pair(&acc_full[acc], leader);  // the tile's sums are complete, in both blocks
       }
     }
+    if (SPLIT) { __syncwarp(); cluster_arrive(); cluster_wait(); }
   } else {
-    // ------------------------------------------------------------------ read-out: warps 2..5 (both blocks)
+    // ------------------------------------------------------------------ read-out: warps 2..9 (both blocks)
     const int sub = warp & 3;  // the tensor-memory sub-partition (32 lanes) this warp may read
-    unsigned char* stage_of_warp = staging + (size_t)sub * 2 * STAGING;
-    unsigned t = 0, stores = 0;
+    const int turn = (warp - 2) >> 2;  // which of the two warps of the sub-partition: the groups take staging tiles in turn
+    const bool hands_over = warp == 2 + 4 * turn && lane == 0;  // this thread hands its group's tiles to TMA
+    auto group_meet = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + turn) : "memory"); };
+    unsigned t = 0;
+    bool pending = false;  // a store that may still read this group's place in `staging`
     chain_wait();  // what the read-out adds to is an earlier kernel's
     for (int tile = pair; tile < tiles; tile += pairs, ++t) {
       const unsigned acc = t & 1;
       const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM, n0 = (tile % tiles_n) * TILE_N;
-      wait_for(&acc_full[acc], (t >> 1) & 1, 3);
-      if (*(volatile int*)&abort_s) break;
+      wait_for(&acc_full[acc], (t >> 1) & 1, 3);  // (a lost launch goes on without waiting: the groups' barriers stay in step)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int row0 = m0 + sub * 32;  // this warp's 32 token rows; lane l holds row0 + l
       const unsigned taddr = tmem_base + acc * BN + ((unsigned)(sub * 32) << 16);
       constexpr int COLS = EPI == EPI_BF16 ? 64 : 32;  // output columns per staging tile
+      if (SPLIT) {
+        // Parts of K. All of the cluster's products have run when it has met (every read-out warp has seen its pair's sums
+        // complete), so the rings are free: one part of a block's ring takes the others' sums of the units that it
+        // finishes, another holds its own sums on their way.
+        cluster_arrive();
+        cluster_wait();
+        // [part][the owner's unit] tiles of 128 x 32 come in (parts times units of one owner: at most 6 for 4 units in 2, 3
+        // or 4 parts), [unit] go out
+        constexpr int INCOMING = 6 * STAGING;
+        static_assert(!SPLIT || (UNITS == 4 && INCOMING + UNITS * STAGING <= STAGES * STAGE_BYTES), "the ring holds the exchange");
+        int sent = 0;
 #pragma unroll 1
-      for (int c = 0; c < TILE_N; c += COLS, ++stores) {
-        if (n0 + c >= out_cols || row0 >= M) break;  // nothing of this warp's rows or of these columns is inside
-        unsigned char* buf = stage_of_warp + (stores & 1) * STAGING;
-        if (lane == 0) bulk_wait_read<1>();  // the store before last has read this tile
-        __syncwarp();
+        for (int u = 0; u < UNITS; ++u) {
+          if (u % parts == (int)part || (sent++ & 1) != turn) continue;
+          float v[32];
+          tmem_load32(taddr + u * 32, v);
+          unsigned char* out = smem + INCOMING + (size_t)u * STAGING;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<float4*>(out + sub * 4096 + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          fence_async_smem();
+          group_meet();
+          if (hands_over) {
+            const unsigned to = (unsigned)(u % parts) * 2 + rank;
+            copy_to_peer(peer_address(smem + (size_t)((int)part * ((UNITS + parts - 1) / parts) + u / parts) * STAGING, to), out, STAGING,
+                         peer_address(&gathered, to));
+          }
+        }
+        wait_for(&gathered, 0, 4);
+        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+      }
+      // The block's last tile: nothing reads or writes the ring any more (all its products have run), so every staging tile has a
+      // place of its own there and nobody waits for a store to have read the one before it.
+      const bool roomy = !SPLIT && tile + pairs >= tiles;
+      if (pending && roomy) pending = false;
+#pragma unroll 1
+      for (int n = 0; n * COLS < TILE_N; ++n) {
+        const int c = n * COLS;
+        if (n0 + c >= out_cols || m0 >= M) break;  // nothing of this block's rows or of these columns is inside
+        if (SPLIT ? n % parts != (int)part || ((n / parts) & 1) != turn : (n & 1) != turn) continue;
+        unsigned char* tile_buf = roomy ? smem + (size_t)n * STAGING : staging + (size_t)turn * STAGING;
+        unsigned char* buf = tile_buf + sub * (EPI == EPI_SWIGLU ? 2048 : 4096);  // this warp's 32 rows of it
+        if (pending) {
+          if (hands_over) bulk_wait_read<0>();  // the store before has read this tile
+          group_meet();
+        }
+        pending = !roomy;
         if (EPI == EPI_ACC || EPI == EPI_F32) {
           float v[32];
           tmem_load32(taddr + c, v);
+          if (SPLIT) {  // the parts in their order, this one's in its place
+            float sum[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+            for (int from = 0; from < parts; ++from) {
+              const unsigned char* in = smem + (size_t)(from * ((UNITS + parts - 1) / parts) + n / parts) * STAGING + sub * 4096;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                if (from != (int)part) o = *reinterpret_cast<const float4*>(in + lane * 128 + ((j ^ (lane & 7)) << 4));
+                sum[4 * j] += o.x; sum[4 * j + 1] += o.y; sum[4 * j + 2] += o.z; sum[4 * j + 3] += o.w;
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = sum[i];
+          }
           if (bias != nullptr) {  // one number per output channel, added before anything is written
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += n0 + c + i < N ? bias[n0 + c + i] : 0.f;
@@ -254,9 +368,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             *reinterpret_cast<float4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) =
                 make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           fence_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (EPI == EPI_ACC) tma_add_2d(&map_y, buf, n0 + c, row0); else tma_store_2d(&map_y, buf, n0 + c, row0);
+          group_meet();
+          if (hands_over) {
+            if (EPI == EPI_ACC) tma_add_2d(&map_y, tile_buf, n0 + c, m0); else tma_store_2d(&map_y, tile_buf, n0 + c, m0);
             bulk_commit();
           }
         } else if (EPI == EPI_BF16) {
@@ -278,8 +392,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             *reinterpret_cast<uint4*>(buf + lane * 128 + (((j + 4) ^ (lane & 7)) << 4)) = p;
           }
           fence_async_smem();
-          __syncwarp();
-          if (lane == 0) { tma_store_2d(&map_y, buf, n0 + c, row0); bulk_commit(); }
+          group_meet();
+          if (hands_over) { tma_store_2d(&map_y, tile_buf, n0 + c, m0); bulk_commit(); }
         } else {
           float v[32], u[32];
           tmem_load32(taddr + c, v);
@@ -303,28 +417,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             *reinterpret_cast<uint4*>(buf + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = o;
           }
           fence_async_smem();
-          __syncwarp();
-          if (lane == 0) { tma_store_2d(&map_y, buf, n0 + c, row0); bulk_commit(); }
+          group_meet();
+          if (hands_over) { tma_store_2d(&map_y, tile_buf, n0 + c, m0); bulk_commit(); }
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) {  // the leader's tensor-core thread waits for all eight warps
         if (rank == 0) mbar_arrive(&acc_empty[acc]);
-        else mbar_arrive_at(peer_address(&acc_empty[acc], 0));
+        else mbar_arrive_at(peer_address(&acc_empty[acc], leader));
       }
     }
-    if (lane == 0) bulk_wait_all();  // what this warp handed to TMA has been written before the block may leave
-    __syncwarp();
   }
 
-  // wind down: everyone meets, the pair meets, then the allocating warps free tensor memory
+  // wind down: the cluster meets, then the allocating warps free tensor memory
   if (*(volatile int*)&abort_s) {
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // a lost launch: let copies and products in flight finish
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  cluster_meet();
+  __syncwarp();
+  cluster_arrive();  // (counts every thread: this block's warps need no barrier of their own)
+  if (warp == 2 || warp == 6) {  // TMA has read what the groups handed to it
+    if (lane == 0) bulk_wait_read<0>();
+  }
+  __syncwarp();
+  cluster_wait();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::TMEM_COLS));
@@ -366,34 +483,45 @@ int cached_wide_map(CUtensorMap* out, const void* base, int rows, int K, int box
   return 0;
 }
 
-template <int BN, int EPI, bool WIDE>
-int launch(const void* x, const void* w, void* y, int M, int N, int K, const float* bias, int act, cudaStream_t stream) {
+// The clusters of 2 * parts blocks that the device holds at once.
+template <int BN, int EPI, bool WIDE, bool SPLIT>
+int cluster_room(int& out, int parts) {
   constexpr int smem = Shape<BN>::SMEM;
-  static int pairs_room[64] = {};
+  static int room_of[64][MAX_PARTS + 1] = {};
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
-  if (pairs_room[device] == 0) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<BN, EPI, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (room_of[device][parts] == 0) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<BN, EPI, WIDE, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaLaunchConfig_t probe = {};
-    probe.gridDim = dim3(sms & ~1);
+    probe.gridDim = dim3(sms / (2 * parts) * (2 * parts));
     probe.blockDim = dim3(THREADS);
     probe.dynamicSmemBytes = smem;
     cudaLaunchAttribute attribute[1];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = 2;
+    attribute[0].val.clusterDim.x = 2 * parts;
     attribute[0].val.clusterDim.y = 1;
     attribute[0].val.clusterDim.z = 1;
     probe.attrs = attribute;
     probe.numAttrs = 1;
     int room = 0;
-    e = cudaOccupancyMaxActiveClusters(&room, gemm_pair_kernel<BN, EPI, WIDE>, &probe);
+    e = cudaOccupancyMaxActiveClusters(&room, gemm_pair_kernel<BN, EPI, WIDE, SPLIT>, &probe);
     if (e != cudaSuccess) return (int)e;
     if (room < 1) return (int)cudaErrorInvalidConfiguration;
-    pairs_room[device] = room < sms / 2 ? room : sms / 2;
+    room_of[device][parts] = room < sms / (2 * parts) ? room : sms / (2 * parts);
   }
+  out = room_of[device][parts];
+  return 0;
+}
+
+template <int BN, int EPI, bool WIDE, bool SPLIT>
+int launch(const void* x, const void* w, void* y, int M, int N, int K, const float* bias, int act, int parts, cudaStream_t stream) {
+  constexpr int smem = Shape<BN>::SMEM;
+  int room = 0;
+  const int roomy = cluster_room<BN, EPI, WIDE, SPLIT>(room, parts);
+  if (roomy) return roomy;
   const int F = N / 2;
   const int out_cols = EPI == EPI_SWIGLU ? F : N, tile_n = EPI == EPI_SWIGLU ? BN / 2 : BN;
   CUtensorMap map_x, map_w, map_y;
@@ -401,26 +529,27 @@ int launch(const void* x, const void* w, void* y, int M, int N, int K, const flo
   if (err) return err;
   err = WIDE ? cached_wide_map(&map_w, w, N, K, BN / 2, true) : cached_map(&map_w, w, N, K, BN / 2, true);
   if (err) return err;
-  err = EPI == EPI_ACC || EPI == EPI_F32 ? make_store_map(&map_y, y, M, out_cols, 4, 32)
-                                         : make_store_map(&map_y, y, M, out_cols, 2, EPI == EPI_BF16 ? 64 : 32);
+  err = EPI == EPI_ACC || EPI == EPI_F32 ? make_store_map(&map_y, y, M, out_cols, 4, 32, BM)
+                                         : make_store_map(&map_y, y, M, out_cols, 2, EPI == EPI_BF16 ? 64 : 32, BM);
   if (err) return err;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((out_cols + tile_n - 1) / tile_n);
-  const int pairs = tiles < pairs_room[device] ? tiles : pairs_room[device];
+  if (SPLIT && tiles > room) return (int)cudaErrorInvalidValue;  // (a cluster takes one tile)
+  const int pairs = tiles < room ? tiles : room;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(2 * pairs);
+  config.gridDim = dim3(2 * parts * pairs);
   config.blockDim = dim3(THREADS);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = 2;
+  attribute[0].val.clusterDim.x = 2 * parts;
   attribute[0].val.clusterDim.y = 1;
   attribute[0].val.clusterDim.z = 1;
   attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = chained_launches_enabled() ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&config, gemm_pair_kernel<BN, EPI, WIDE>, map_x, map_w, map_y, M, N, K, F, bias, act);
+  const cudaError_t e = cudaLaunchKernelEx(&config, gemm_pair_kernel<BN, EPI, WIDE, SPLIT>, map_x, map_w, map_y, M, N, K, F, bias, act, parts, (const __nv_bfloat16*)w);
   return e != cudaSuccess ? (int)e : launch_status();
 }
 
@@ -435,8 +564,7 @@ int launch_width(const void* x, const void* w, void* y, int M, int N, int K, con
   const long long rows = (M + 2 * BM - 1) / (2 * BM);
   const int out_cols = EPI == EPI_SWIGLU ? N / 2 : N;
   const int unit = EPI == EPI_SWIGLU ? 2 : 1;  // a SwiGLU tile of BN stacked rows yields BN / 2 channels
-  int device = 0, sms = 148;
-  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  const int sms = sm_count();
   const long long pairs = sms / 2 > 0 ? sms / 2 : 1;
   int best = 256;
   long long best_cost = -1;
@@ -446,8 +574,30 @@ int launch_width(const void* x, const void* w, void* y, int M, int N, int K, con
     const long long cost = rounds * stage;
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
   }
+  // Parts of K where a tile's stages are many and the tiles are few: `parts` pairs of SMs take a part each of one tile. A
+  // stage then takes some 1,100 cycles (four stages in flight, 2.3 us from asking for one to its products' end), and the
+  // parts' meeting some 8,500.
+  if constexpr (EPI == EPI_ACC || EPI == EPI_F32) {
+    const long long stages = (K + BK * STEPS - 1) / (BK * STEPS), tiles = rows * ((out_cols + SPLIT_BN - 1) / SPLIT_BN);
+    const long long whole = best_cost / (1048ll * best / 256 > 700 ? 1048ll * best / 256 : 700) * stages * (1048ll * best / 256 > 1100 ? 1048ll * best / 256 : 1100);
+    int parts = 1;
+    long long cost = whole;
+    for (int p = 2; p <= MAX_PARTS; ++p) {
+      if (p > stages || tiles * p > pairs) break;
+      const long long c = (stages + p - 1) / p * 1100 + 8500;
+      if (c >= cost) continue;
+      int room = 0;
+      if ((K % 64 == 0 ? cluster_room<SPLIT_BN, EPI, true, true>(room, p) : cluster_room<SPLIT_BN, EPI, false, true>(room, p)) == 0 && tiles <= room) {
+        cost = c;
+        parts = p;
+      }
+    }
+    if (parts > 1)
+      return K % 64 == 0 ? launch<SPLIT_BN, EPI, true, true>(x, w, y, M, N, K, bias, act, parts, stream)
+                         : launch<SPLIT_BN, EPI, false, true>(x, w, y, M, N, K, bias, act, parts, stream);
+  }
 #define AKAS_PAIR_WIDTH(BN_) \
-  case BN_: return K % 64 == 0 ? launch<BN_, EPI, true>(x, w, y, M, N, K, bias, act, stream) : launch<BN_, EPI, false>(x, w, y, M, N, K, bias, act, stream);
+  case BN_: return K % 64 == 0 ? launch<BN_, EPI, true, false>(x, w, y, M, N, K, bias, act, 1, stream) : launch<BN_, EPI, false, false>(x, w, y, M, N, K, bias, act, 1, stream);
   switch (best) {
     AKAS_PAIR_WIDTH(256) AKAS_PAIR_WIDTH(192) AKAS_PAIR_WIDTH(128) AKAS_PAIR_WIDTH(64)
   }

@@ -163,13 +163,13 @@ inline int cached_map(CUtensorMap* out, const void* base, int rows, int K, int b
 }
 
 // A tensor map of a row-major matrix [rows, cols] of 2- or 4-byte elements for the read-out's staging tiles:
-// boxes of 32 rows x box_cols (128 or 64 bytes), in the swizzle of that width.
-inline int make_store_map(CUtensorMap* map, void* base, int rows, int cols, int elem_bytes, int box_cols) {
+// boxes of box_rows x box_cols (128 or 64 bytes), in the swizzle of that width.
+inline int make_store_map(CUtensorMap* map, void* base, int rows, int cols, int elem_bytes, int box_cols, int box_rows = 32) {
   EncodeTiled fn = encode_tiled();
   if (!fn) return 3001;
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)box_cols, 32};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1, 1};
   const CUresult r = fn(map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims,
                         strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -294,6 +294,23 @@ def test_products_on_pairs_of_sms(ops, m, k, o):
     assert cuda.gemm_pair_status() == 0
 
 
+@pytest.mark.parametrize("m,k,o", [(512, 4608, 1024), (768, 4608, 1020), (130, 8192, 256), (257, 3080, 132), (1024, 6912, 1536),
+                                   (200, 4104, 64), (600, 16384, 512)])
+def test_products_on_pairs_of_sms_with_k_in_parts(ops, m, k, o):
+    """Few tiles and a long inner size: 2 to 4 pairs of SMs take a part of K each and add the parts in a fixed order. Ragged
+    rows, channels and steps of K; the same bits every time."""
+    cuda, _ = ops
+    x, w = _rand((m, k), torch.bfloat16, 61), _rand((o, k), torch.bfloat16, 62, 0.05)
+    want = x.double() @ w.double().T
+    _close(cuda.paired_product(x, w, out_dtype=torch.float32), want, torch.float32, "f32 out", k)
+    h0 = _rand((m, o), torch.float32, 63, 2.0)
+    first = cuda.paired_product(x, w, residual=h0.clone())
+    _close(first, h0.double() + want, torch.float32, "added into the residual stream", k)
+    for _ in range(3):
+        assert torch.equal(cuda.paired_product(x, w, residual=h0.clone()), first)
+    assert cuda.gemm_pair_status() == 0
+
+
 @pytest.mark.parametrize("m,k,o", [(17, 64, 48), (64, 2048, 6144), (33, 264, 520), (128, 8192, 2048), (100, 200, 2056),
                                    (64, 2048, 65536), (20, 1024, 40), (96, 704, 1160), (48, 128, 40000), (64, 8192, 2048),
                                    (33, 4096, 1000), (70, 6912, 1536)])
