@@ -82,11 +82,13 @@ class BatchLayout:
         self.size = off
 
 
-def fill_batch(host: np.ndarray, layout: BatchLayout, entries: Sequence[StepEntry], cache, pad_to: int = 0, tokens=None):
+def fill_batch(host: np.ndarray, layout: BatchLayout, entries: Sequence[StepEntry], cache, pad_to: int = 0, tokens=None, gap=(0, 0)):
     """Writes the arrays of ``entries`` into ``host`` (int32) at ``layout``'s offsets.
 
     ``pad_to``: for a decode-only step, the bucket size; padding tokens get request -1.
     ``tokens``: the entries' token ids as arrays, if the caller has them already.
+    ``gap``: (entries, count): behind the first ``entries`` entries stand ``count`` padding requests of one token each
+    (request -1), so that what follows starts at the same request and token whatever the number of entries in front.
     Returns (max_query_len, max_context).
     """
     n, r = layout.n, layout.r
@@ -115,6 +117,22 @@ def fill_batch(host: np.ndarray, layout: BatchLayout, entries: Sequence[StepEntr
         cu[:live] = first[:live]
         slots[:live] = np.fromiter((cache.slot(e.request) for e in entries), dtype=np.int64, count=live)
         src[:at] = -1
+        row = np.arange(live, dtype=np.int64)  # the request's row in slots and block tables
+        if gap[1]:
+            front, more = gap
+            split = int(first[front])
+            for array, empty in ((tok, 0), (pos, 0), (seq, -1), (src, -1)):
+                array[split + more : at + more] = array[split:at].copy()
+                array[split : split + more] = empty
+            seq[split + more : at + more] += more
+            slots[front + more : live + more] = slots[front:live].copy()
+            slots[front : front + more] = -1
+            cu[front + more : live + more] = cu[front:live].copy() + more
+            cu[front : front + more] = split + np.arange(more)
+            row[front:] += more
+            first[front:] += more
+            at += more
+            live += more
         for i, e in enumerate(entries):
             if e.source >= 0:
                 if counts[i] != 1:
@@ -125,12 +143,12 @@ def fill_batch(host: np.ndarray, layout: BatchLayout, entries: Sequence[StepEntr
         for g, (offset, max_blocks) in enumerate(zip(layout.tables, layout.table_widths)):
             table = host[offset : offset + live * max_blocks].reshape(live, max_blocks)
             table[:] = -1
-            for i, e in enumerate(entries):
+            for i, e in zip(row.tolist(), entries):
                 blocks = cache.blocks(e.request, g)
                 table[i, : len(blocks)] = blocks
         max_q = int(counts.max())
         max_ctx = int((starts + counts).max())
-    cu[len(entries)] = at
+    cu[live] = at
     if pad_to:
         tok[at:n] = 0
         src[at:n] = -1

@@ -33,6 +33,11 @@ _DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 _GRAPH_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
 _TOKEN_ROUNDING = 256
 _SHAPE_REPEATS, _SHAPE_GRAPHS = 3, 4  # a step shape is captured when it comes the third time; at most four are kept
+# Steps that mix decoded tokens with prompt portions, up to this many rows, run as captured graphs per bucket of (rows, decoded
+# requests, portions): enqueueing such a step kernel by kernel takes the host 1.9 ms at 16 layers, the GPU 1.4 (640 rows of
+# the 350m shape). Above, the GPU takes longer than the host, and a graph would hold its activations for good. A bucket
+# is captured when it comes the second time; at most sixteen are kept, which share their activations' memory.
+_MIXED_ROWS, _MIXED_REPEATS, _MIXED_GRAPHS, _MIXED_SINGLES, _MIXED_PORTIONS = 1024, 2, 16, 8, (1, 2, 4, 8)
 
 
 def default_ops(device: torch.device, dtype: torch.dtype, parts=()):
@@ -88,6 +93,12 @@ class ModelRunner:
         self._graphs: Dict[int, "_DecodeGraph"] = {}
         self._shape_graphs: Dict[tuple, "_DecodeGraph"] = {}
         self._shape_counts: Dict[tuple, int] = {}
+        self._mixed_graphs: Dict[tuple, "_MixedGraph"] = {}
+        self._mixed_counts: Dict[tuple, int] = {}
+        self._mixed_pool = None
+        blocks = self.model.blocks
+        self._mixed = (self.device.type == "cuda" and self.dtype == torch.bfloat16 and spec.bigram is None and all(
+            getattr(b.mixer, "bounded", False) and (b.ffn is None or getattr(b.ffn, "bounded", False)) for b in blocks))
         self.steps = 0
         self.kernels_per_decode_step: Dict[int, int] = {}  # bucket -> kernels inside its captured graph
 
@@ -178,6 +189,8 @@ class ModelRunner:
         all_wanted = all(list(e.want) == [0] for e in entries)
         graphs = self.config.cuda_graphs and self.device.type == "cuda"
         repeated = self._repeated_shape(entries) if graphs and not (decode_only and all_wanted) else None
+        if repeated is None and graphs and self._mixed and not decode_only:
+            repeated = self._mixed_bucket(entries)
         if decode_only and all_wanted and graphs:
             logits = self._decode_graph_step(entries, arrays, previous)
         elif repeated is not None:
@@ -261,6 +274,32 @@ class ModelRunner:
         graph = self._shape_graphs[key] = _DecodeGraph(self, 0, lengths=key[0], wanted=key[1])
         return graph
 
+    def _mixed_bucket(self, entries):
+        """The captured graph for steps of this one's bucket, once that has come _MIXED_REPEATS times; else None. The decoded
+        tokens at the front are padded to a multiple of 8 requests, the portions behind them to 1, 2, 4 or 8 requests and
+        to whole rows of 256."""
+        singles = 0
+        while len(entries[singles].tokens) == 1:  # (not a step of single tokens only)
+            singles += 1
+        portions = next((p for p in _MIXED_PORTIONS if p >= len(entries) - singles), 0)
+        if not portions:
+            return None
+        rows = -(-singles // _MIXED_SINGLES) * _MIXED_SINGLES + sum(len(e.tokens) for e in entries[singles:])
+        if not _TOKEN_ROUNDING < rows <= _MIXED_ROWS:
+            return None
+        singles = -(-singles // _MIXED_SINGLES) * _MIXED_SINGLES
+        wanted = sum(len(e.want) for e in entries)
+        if wanted > singles + portions:
+            return None
+        key = (-(-rows // _TOKEN_ROUNDING) * _TOKEN_ROUNDING, singles, portions, singles + portions if wanted else 0)
+        graph = self._mixed_graphs.get(key)
+        if graph is None:
+            seen = self._mixed_counts[key] = self._mixed_counts.get(key, 0) + 1
+            if seen < _MIXED_REPEATS or len(self._mixed_graphs) >= _MIXED_GRAPHS:
+                return None
+            graph = self._mixed_graphs[key] = _MixedGraph(self, *key)
+        return graph
+
     def decode_capacity(self, count: int) -> int:
         """The number of rows that a step of ``count`` decoded tokens runs at: the bucket of its captured graph."""
         if not (self.config.cuda_graphs and self.device.type == "cuda"):
@@ -328,6 +367,7 @@ class _DecodeGraph:
         self.dev = torch.zeros(self.layout.size, dtype=torch.int32, device=runner.device)
         self.graph = None
         self.logits = None
+        self.pool = None  # a memory pool shared with other graphs, if any
 
     def _fill(self, entries, arrays=None):
         host = self.ring.take()
@@ -349,11 +389,8 @@ class _DecodeGraph:
             # Warm-up and capture run on a batch of padding only: they must leave pages and state alone.
             # The context's host-side sizes are upper bounds so that the captured launches fit every replay.
             self._fill([])
-            if self.lengths is None:
-                ctx = runner._context(self.dev, self.layout, 1, runner.config.context, True, [1] * self.bucket)
-            else:
-                ctx = runner._context(self.dev, self.layout, max(self.lengths), runner.config.context,
-                                      all(n == 1 for n in self.lengths), self.lengths)
+            lengths = [1] * self.bucket if self.lengths is None else self.lengths
+            ctx = runner._context(self.dev, self.layout, max(lengths), runner.config.context, all(n == 1 for n in lengths), lengths)
             ctx.memo["captured"] = True
             stream = torch.cuda.Stream(device=runner.device)
             stream.wait_stream(torch.cuda.current_stream(runner.device))
@@ -372,7 +409,7 @@ class _DecodeGraph:
             collecting = gc.isenabled()
             gc.disable()
             try:
-                with torch.cuda.graph(graph):
+                with torch.cuda.graph(graph, pool=self.pool):
                     self.logits = runner.model.forward(ctx, runner.cache.views)
             finally:
                 if collecting:
@@ -391,3 +428,35 @@ class _DecodeGraph:
                                    self.dev[lay.token_src : lay.token_src + lay.n], previous)
         self.graph.replay()
         return self.logits[: len(entries)] if self.lengths is None else self.logits
+
+
+class _MixedGraph(_DecodeGraph):
+    """One captured step of ``singles`` requests of one token each, then ``portions`` requests that bring any numbers of
+    tokens, ``rows`` token rows in all; every place may be padding."""
+
+    def __init__(self, runner: ModelRunner, rows: int, singles: int, portions: int, wanted: int):
+        # The lengths it is captured with: no portions of these rows have more tiles of 64 or 128 queries.
+        lengths = (1,) * singles + (64,) * (portions - 1) + (rows - singles,)
+        super().__init__(runner, 0, lengths=lengths, wanted=wanted)
+        self.singles = singles
+        self.layout = BatchLayout(rows, singles + portions, wanted, runner.cache.table_widths)
+        self.ring = _Pinned(self.layout.size, runner.device)
+        self.dev = torch.zeros(self.layout.size, dtype=torch.int32, device=runner.device)
+        if runner._mixed_pool is None:
+            runner._mixed_pool = torch.cuda.graph_pool_handle()
+        self.pool = runner._mixed_pool
+
+    def _fill(self, entries, arrays=None):
+        host, lay = self.ring.take(), self.layout
+        array, front = host.numpy(), 0
+        while front < len(entries) and len(entries[front].tokens) == 1:
+            front += 1
+        wanted = sum(len(e.want) for e in entries)
+        array[lay.logit_rows + wanted : lay.logit_rows + max(lay.m, 1)] = 0
+        fill_batch(array, lay, entries, self.runner.cache, pad_to=lay.n, tokens=arrays,
+                   gap=(front, self.singles - front) if entries else (0, 0))
+        self.dev.copy_(host, non_blocking=True)
+        self.ring.copied()
+
+    def run(self, entries, arrays=None, previous=None):
+        return super().run(entries, arrays, previous)[: sum(len(e.want) for e in entries)]

@@ -158,6 +158,10 @@ class Attention(Mixer):
             self.q_norm.weight = get(self._n("q_norm.weight"))
             self.k_norm.weight = get(self._n("k_norm.weight"))
 
+    @property
+    def bounded(self):
+        return not self.general and (self.position is None or hasattr(self.position, "tables"))
+
     def cache(self):
         s = self.spec
         if not self.own_kv:

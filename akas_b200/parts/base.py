@@ -265,6 +265,10 @@ class Part:
     # loading); a part that leaves this False is asked for its result and the block adds it.
     takes_residual_scale = False
     residual_scale = 1.0
+    # True: the part launches the same kernels with the same sizes for every step of as many rows, requests and leading
+    # single tokens, whatever the requests' lengths are (it reads those on the device, and sizes its grids from upper
+    # bounds), so that one captured step serves all of them.
+    bounded = False
 
     def __init__(self, spec, runtime: Runtime):
         self.spec = spec

@@ -20,6 +20,7 @@ ACTIVATIONS = ("gelu_tanh", "silu")
 class GatedMLP(FeedForward):
     takes_normed = True
     chain_safe = True
+    bounded = True
 
     def __init__(self, spec, runtime):
         super().__init__(spec, runtime)

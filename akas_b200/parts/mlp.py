@@ -33,6 +33,7 @@ def project_activated(rt, x, w_up, activation):
 class MLP(FeedForward):
     takes_normed = True
     chain_safe = True
+    bounded = True
     takes_out_dtype = True
 
     def __init__(self, spec, runtime):

@@ -25,6 +25,7 @@ from .base import Mixer, Normed, Param, StateSpec, project, register_mixer, rena
 class ShortConv(Mixer):
     takes_normed = True
     chain_safe = True
+    bounded = True
 
     @classmethod
     def kernels(cls, spec):

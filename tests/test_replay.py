@@ -275,3 +275,78 @@ def test_timed_operations_change_nothing_and_account_for_the_step(tmp_path):
     assert abs(sum(row["share"] for row in rows.values()) - 1.0) < 1e-6
     timed.clear()
     assert timed.table() == []
+
+
+def test_padding_requests_between_entries():
+    """``fill_batch`` with a gap: the entries behind it stand where they would stand behind that many more requests of one token,
+    which are padding in every array."""
+    from akas_b200.engine.batch import BatchLayout, StepEntry, fill_batch
+
+    class Cache:
+        def length(self, r):
+            return 10 * r
+
+        def slot(self, r):
+            return r + 5
+
+        def blocks(self, r, g):
+            return [r + 1] * (r % 3 + 1)
+
+    entries = [StepEntry(0, [9], (0,)), StepEntry(1, [8], (0,)), StepEntry(2, [1, 2, 3, 4], (3,)), StepEntry(3, [7, 6], ())]
+    lay = BatchLayout(16, 8, 8, (4,))
+    host = np.full(lay.size, -77, dtype=np.int32)
+    assert fill_batch(host, lay, entries, Cache(), pad_to=16, gap=(2, 2)) == (4, 32)
+    part = lambda at, n: host[at : at + n].tolist()  # noqa: E731
+    assert part(lay.token_ids, 16) == [9, 8, 0, 0, 1, 2, 3, 4, 7, 6] + [0] * 6
+    assert part(lay.positions, 16) == [0, 10, 0, 0, 20, 21, 22, 23, 30, 31] + [0] * 6
+    assert part(lay.seq_of_token, 16) == [0, 1, -1, -1, 4, 4, 4, 4, 5, 5] + [-1] * 6
+    assert part(lay.token_src, 16) == [-1] * 16
+    assert part(lay.cu_seqlens, 9) == [0, 1, 2, 3, 4, 8, 10, 10, 10]
+    assert part(lay.slots, 8) == [5, 6, -1, -1, 7, 8, -1, -1]
+    assert part(lay.logit_rows, 3) == [0, 1, 7]
+    table = host[lay.tables[0] : lay.tables[0] + 32].reshape(8, 4).tolist()
+    assert table == [[1, -1, -1, -1], [2, 2, -1, -1], [-1] * 4, [-1] * 4, [3, 3, 3, -1], [4, -1, -1, -1], [-1] * 4, [-1] * 4]
+
+
+@pytest.mark.gpu
+def test_captured_mixed_steps_agree_with_the_plain_model(tmp_path):
+    """Steps that mix decoded tokens with prompt portions, captured per bucket of rows, decoded requests and portions: any
+    number of decoded requests from none to more than a bucket, one to four portions of any lengths, steps that want no logits."""
+    from akas_b200.config import EngineConfig
+    from akas_b200.engine.batch import StepEntry
+    from akas_b200.engine.runner import ModelRunner
+
+    folder = tiny.make_folder(tiny.CONFIGS["c"], seed=13, dtype="bfloat16", folder=tmp_path / "c")
+    cfg, w = plain.load_folder(folder)
+    lengths = [500, 290, 310, 77, 150, 333, 301, 64, 65, 700, 290, 40, 300]
+    texts = dict(enumerate(tiny.prompts(cfg["vocab_size"], [n + 14 for n in lengths], seed=8)))
+    want = {r: plain.forward(cfg, w, toks).numpy() for r, toks in texts.items()}
+    r = ModelRunner(folder, EngineConfig(dtype="bfloat16", device="cuda:0", page_size=64, max_tokens=16 * 768,
+                                         max_requests=16, context=768, cuda_graphs=True))
+    for _ in range(3):
+        at = {q: 0 for q in texts}
+        got = {q: {} for q in texts}
+        while any(at[q] < len(texts[q]) for q in texts):
+            room, entries = 300, []
+            for q in sorted(texts, key=lambda q: at[q] < lengths[q]):  # decoded requests in front
+                n = 1 if at[q] >= lengths[q] else min(room, lengths[q] - at[q])
+                if at[q] < len(texts[q]) and n:
+                    room -= n if n > 1 else 0
+                    ends = at[q] + n >= lengths[q]
+                    entries.append(StepEntry(q, texts[q][at[q] : at[q] + n], (n - 1,) if ends else ()))
+            logits = r.step(entries).cpu().numpy()
+            assert len(logits) == sum(len(e.want) for e in entries)
+            row = 0
+            for e in entries:
+                at[e.request] += len(e.tokens)
+                if e.want:
+                    got[e.request][at[e.request] - 1] = logits[row]
+                    row += 1
+        for q in texts:
+            r.release(q)
+            places = sorted(got[q])
+            assert places == list(range(lengths[q] - 1, len(texts[q])))
+            have, ref = np.stack([got[q][p] for p in places]), want[q][places]
+            err, l2 = traces.worst(have, ref)
+            assert err <= 2 * BF16["c"][0] and l2 <= 1.5 * BF16["c"][1], (q, err, l2)  # (of 15 rows, not of a whole request)
+    assert len(r._mixed_graphs) >= 3 and all(g.graph is not None for g in r._mixed_graphs.values())
