@@ -5,7 +5,8 @@
 // the tile shape and however many rows the launch has, so a row's result does not depend on what
 // else is in the batch (bitwise). Both operands are contiguous along K.
 //
-// Four kernels: pipelined tiles for more than 16 rows; a warp per 8 rows of w, or a block per 32 of a wide w, for fewer,
+// Five kernels: two with tiles for more than 16 rows, of packed multiply-adds where an SM gets several large tiles, fed by
+// cp.async where the tiles are few; a warp per 8 rows of w, or a block per 32 of a wide w, for fewer,
 // which stream w once; and a plain tiled kernel for operands whose rows do not start on 16 bytes. kreasof-ai/akas's plain float32
 // `linear` is a per-row tree reduction (src/akas/ops/linear/kernel.py:403-447).
 #include "common.cuh"
@@ -166,6 +167,123 @@ sgemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, floa
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         if (gc + e < O) y[place + e] = residual ? residual[place + e] + v[e] : v[e];
+    }
+  }
+}
+
+// Tiles of BM x BN outputs for products that leave an SM few tiles. The kernel above loses the most there: a warp a scheduler,
+// one stage of loads ahead (512 cycles at 64 x 64, less than DRAM takes) and a transposition behind them. Here STAGES stages of
+// BK of K come by cp.async and stay as they lie in memory, K along a row, rows BK + 4 floats apart: the next stages are on their way while one is multiplied, through no register and no transposition. A warp
+// owns 4 TM x 8 TN outputs, lane (ty, tx) of 4 x 8 the rows ty + 4 i and columns tx + 8 j of them: four k of a row are one
+// 16-byte load, and the eight rows of w that a warp reads at once lie in different banks.
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+struct PipeTile {
+  static constexpr int NT = (BM / (4 * TM)) * (BN / (8 * TN)) * 32, PITCH = BK + 4, STAGE = (BM + BN) * PITCH;
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float);
+};
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+__global__ void __launch_bounds__((PipeTile<BM, BN, TM, TN, BK, STAGES>::NT))
+sgemm_pipe_kernel(const float* __restrict__ x, const float* __restrict__ w, float* y, const float* residual, int N, int O, int K) {
+  using P = PipeTile<BM, BN, TM, TN, BK, STAGES>;
+  constexpr int NT = P::NT, PITCH = P::PITCH, PER = BK / 4;          // 16-byte pieces of a row in a stage
+  constexpr int CA = BM * PER / NT, CB = BN * PER / NT;              // copies of a stage per thread
+  static_assert(CA * NT == BM * PER && CB * NT == BN * PER, "whole copies");
+  extern __shared__ __align__(16) float ring[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = lane >> 3, tx = lane & 7;
+  const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+  const int wm = (warp / (BN / (8 * TN))) * 4 * TM + ty, wn = (warp % (BN / (8 * TN))) * 8 * TN + tx;
+  const int lr = tid / PER, lc = (tid % PER) * 4;
+  auto issue_w = [&](int stage, int k0) {
+    float* to = ring + stage * P::STAGE + BM * PITCH;
+#pragma unroll
+    for (int i = 0; i < CB; ++i) {
+      const int r = lr + i * (NT / PER);
+      const bool live = col0 + r < O && k0 + lc < K;
+      copy16(to + r * PITCH + lc, live ? w + (size_t)(col0 + r) * K + k0 + lc : w, live);
+    }
+  };
+  auto issue_x = [&](int stage, int k0) {
+    float* to = ring + stage * P::STAGE;
+#pragma unroll
+    for (int i = 0; i < CA; ++i) {
+      const int r = lr + i * (NT / PER);
+      const bool live = row0 + r < N && k0 + lc < K;
+      copy16(to + r * PITCH + lc, live ? x + (size_t)(row0 + r) * K + k0 + lc : x, live);
+    }
+  };
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+
+  const int steps = (K + BK - 1) / BK;
+  chain_release();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) issue_w(s, s * BK);  // weights: no kernel writes them
+  chain_wait();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    issue_x(s, s * BK);
+    copies_commit();
+  }
+  int at = 0, to = STAGES - 1;
+  for (int step = 0; step < steps; ++step) {
+    copies_wait<STAGES - 2>();
+    __syncthreads();  // the stage has landed for every thread, and the one before it has been read
+    const int ahead = (step + STAGES - 1) * BK;
+    if (ahead < K) {
+      issue_w(to, ahead);
+      issue_x(to, ahead);
+    }
+    copies_commit();
+    const float* as = ring + at * P::STAGE + wm * PITCH;
+    const float* bs = ring + at * P::STAGE + (BM + wn) * PITCH;
+    float4 a[2][TM], b[2][TN];
+    auto load = [&](int slot, int k) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[slot][i] = *reinterpret_cast<const float4*>(as + 4 * i * PITCH + k);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[slot][j] = *reinterpret_cast<const float4*>(bs + 8 * j * PITCH + k);
+    };
+    constexpr bool AHEAD = TM * TN <= 32;  // the next four k's operands are loaded while these are multiplied
+    if (AHEAD) load(0, 0);
+#pragma unroll
+    for (int u = 0; u < BK / 4; ++u) {
+      const int slot = AHEAD ? u & 1 : 0;
+      if (!AHEAD) load(0, 4 * u);
+      else if (u + 1 < BK / 4) load(slot ^ 1, 4 * (u + 1));
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[slot][i].x, b[slot][j].x, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[slot][i].y, b[slot][j].y, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[slot][i].z, b[slot][j].z, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[slot][i].w, b[slot][j].w, acc[i][j]);
+    }
+    at = at + 1 == STAGES ? 0 : at + 1;
+    to = to + 1 == STAGES ? 0 : to + 1;
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gr = row0 + wm + 4 * i;
+    if (gr >= N) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int gc = col0 + wn + 8 * j;
+      if (gc >= O) continue;
+      const size_t place = (size_t)gr * O + gc;
+      y[place] = residual ? residual[place] + acc[i][j] : acc[i][j];
     }
   }
 }
@@ -409,6 +527,23 @@ int launch_tile(const float* x, const float* w, float* y, const float* residual,
                         residual, N, O, K);
 }
 
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+int launch_pipe(const float* x, const float* w, float* y, const float* residual, int N, int O, int K, cudaStream_t stream) {
+  using P = PipeTile<BM, BN, TM, TN, BK, STAGES>;
+  auto kernel = sgemm_pipe_kernel<BM, BN, TM, TN, BK, STAGES>;
+  if constexpr (P::SMEM > 48 * 1024) {
+    static bool allowed[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
+    if (!allowed[device]) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM);
+      if (e != cudaSuccess) return (int)e;
+      allowed[device] = true;
+    }
+  }
+  return launch_chained(kernel, dim3((O + BN - 1) / BN, (N + BM - 1) / BM), dim3(P::NT), P::SMEM, stream, x, w, y, residual, N, O, K);
+}
+
 template <int TOK, int STAGES>
 int launch_few(const float* x, const float* w, float* y, const float* residual, int N, int O, int K, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (kFewRows + 4 * TOK) * kFewPitch * sizeof(float);
@@ -427,11 +562,13 @@ int launch_few(const float* x, const float* w, float* y, const float* residual, 
 //   5 to 16 rows: the same against a narrow w, a block per 32 rows of a wide one. Five rows (narrow / wide): 4,096 x 1,024 14 / 16,
 //     5,120 x 1,024 18 / 17, 6,144 x 2,048 35 / 32, 16,384 x 2,048 71 / 53; sixteen: 2,048 x 2,048 29 / 35, 3,072 x 2,048 37 / 35,
 //     4,096 x 1,024 24 / 18, 6,144 x 2,048 55 / 45.
-//   17 rows (32 x 64 tiles before): 512 x 512 18 (28), 1,024 x 1,024 35 (54), 4,096 x 1,024 47 (79); 64 rows 19 (29), 37 (55), 48 (76);
-//     65 rows (128 x 128 before) 19 (88), 37 (172), 61 (211).
-//   64 x 64 tiles up to 511 rows: 1,024 x 1,024 with 128 rows 38 (185), 300 rows 39 (185); 9,216 x 1,024 with 300 rows 141 (276;
-//     128 x 64 tiles 147). Tiles of 128 x 64 from there on: 9,216 x 1,024 with 723 rows 281 (524; 64 x 64 tiles 322), with
-//     2,048 rows 732 (1,056): 53 TFLOP/s. Up to 32 rows against a wide w, 32 x 32 tiles: 16,384 x 2,048 135 (197; 64 x 64 181).
+//   17 rows and more, x 1,024 of K unless said (128 x 64 tiles of packed multiply-adds / 64 x 64 / 64 x 32 / 32 x 32 of 4 x 4 a thread /
+//     of 4 x 2, all fed by cp.async but the first; before: 64 x 64 tiles of the first kernel up to 511 rows, 128 x 64 from there on):
+//     40 rows x 1,024 57 / 38 / 27 / 22 / 18.5 (before 38), K 4,608 254 / 160 / 113 / 93 / 75 (212); 100 x 1,024 of K 4,608 260 / 160 /
+//     114 / 95 / 85 (196); 300 x 2,048 80 / 70 / 67 / 52 / 60 (72); 722 x 1,024 76 / 76 / 67 / 52 / 60 (76), of K 4,608 321 / 333 / 287 / 218
+//     / 257 (321); 722 x 3,072 142 / 115 / 133 / 132 / 149 (142); 722 x 9,216 282 / 333 / 384 / 366 / 431 (282); 2,048 x 1,024 142 / 116 / 117
+//     / 127 / 140 (142), x 9,216 734 / 869 / 996 / 988 / 1,184 (734): 53 TFLOP/s.
+//     The rule below is these times by the tiles of the busiest SM.
 //   rows off 16 bytes: 16 x 64 tiles up to 16 rows (4,096 x 1,022 with 16 rows 66; 32 x 64 tiles of one k a thread 174), 32 x 64 up to
 //     64 (with 17 rows 80), 128 x 128 from there on (with 300 rows 230, with 2,048 595; 32 x 64 tiles 853).
 AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* residual, int N, int O, int K,
@@ -448,7 +585,7 @@ AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* r
       sgemm_any_kernel<16, 64, 1, 4><<<dim3((O + 63) / 64, 1), 256, 0, stream>>>(x, w, y, residual, N, O, K);
     return launch_status();
   }
-  const bool wide = O >= (N > 16 ? 8192 : N > 8 ? 4096 : 5120);
+  const bool wide = O >= (N > 8 ? 4096 : 5120);
   if (N <= 4) return launch_few<1, 12>(x, w, y, residual, N, O, K, stream);
   if (N <= 16 && wide) {
     const dim3 grid((O + 31) / 32);
@@ -457,7 +594,21 @@ AKAS_API int akas_sgemm(const float* x, const float* w, float* y, const float* r
   }
   if (N <= 8) return launch_few<2, 4>(x, w, y, residual, N, O, K, stream);
   if (N <= 16) return launch_few<4, 4>(x, w, y, residual, N, O, K, stream);
-  if (N <= 32 && wide) return launch_tile<32, 32, 8, 4>(x, w, y, residual, N, O, K, stream);
-  if (N < 512) return launch_tile<64, 64, 8, 4>(x, w, y, residual, N, O, K, stream);
-  return launch_tile<128, 64, 8, 8>(x, w, y, residual, N, O, K, stream);
+  // us per 1,024 of K, by the number of tiles that the busiest SM gets (times above): the smaller the tile, the more evenly the SMs
+  // are filled; the larger, the fewer operands are read per multiply-add
+  const long long sms = max(1, sm_count());
+  auto busiest = [&](int bm, int bn) { return ((long long)((N + bm - 1) / bm) * ((O + bn - 1) / bn) + sms - 1) / sms; };
+  const long long large = busiest(128, 64), middle = busiest(64, 64), narrow = busiest(64, 32), small = busiest(32, 32);
+  const double times[5] = {46. * large + (large == 1 ? 20. : large == 2 ? 80. : 12.), middle <= 3 ? 38. * middle : 28.5 * middle, 15. + 15. * narrow,
+                           17. + 8. * small, small == 1 ? 19. : 1e30};
+  int best = 0;
+  for (int i = 1; i < 5; ++i)
+    if (times[i] < times[best] && (N + (i < 3 ? 63 : 31)) / (i < 3 ? 64 : 32) <= 65535) best = i;  // (rows of tiles are a grid's y)
+  switch (best) {
+    case 0: return launch_tile<128, 64, 8, 8>(x, w, y, residual, N, O, K, stream);
+    case 1: return launch_pipe<64, 64, 8, 4, 32, 3>(x, w, y, residual, N, O, K, stream);
+    case 2: return launch_pipe<64, 32, 4, 4, 32, 4>(x, w, y, residual, N, O, K, stream);
+    case 3: return launch_pipe<32, 32, 4, 4, 32, 4>(x, w, y, residual, N, O, K, stream);
+    default: return launch_pipe<32, 32, 4, 2, 32, 4>(x, w, y, residual, N, O, K, stream);
+  }
 }

@@ -119,6 +119,20 @@ def test_linear_float32_every_kernel_gives_the_same_bits(ops, k, o):
         assert torch.equal(cuda.linear(x[:n], w, residual=res[:n].clone()), added[:n]), n
 
 
+@pytest.mark.parametrize("n,k,o", [(40, 1000, 1020), (100, 132, 2048), (100, 68, 3072), (722, 36, 1024), (721, 100, 3071), (700, 20, 9216),
+                                   (2300000, 4, 3)])
+def test_linear_float32_tiles_by_the_tiles_of_an_sm(ops, n, k, o):
+    """Sizes that each kind of tiles takes on a B200 (and more rows than tiles of 32 can be numbered), against the kernel for operands
+    off 16 bytes: the same bits, remainders of tiles and stages included."""
+    cuda, _ = ops
+    x, w = _rand((n, k), torch.float32, 71), _rand((o, k), torch.float32, 72)
+    odd = torch.empty(o * k + 1, device=w.device)[1:].view(o, k).copy_(w)
+    assert torch.equal(cuda.linear(x, w), cuda.linear(x, odd))
+    if n < 1000:
+        res = _rand((n, o), torch.float32, 73)
+        assert torch.equal(cuda.linear(x, w, residual=res.clone()), cuda.linear(x, odd, residual=res.clone()))
+
+
 @pytest.mark.parametrize("k,o", [(70, 130), (33, 300), (5, 64)])
 def test_linear_float32_rows_off_16_bytes(ops, k, o):
     """An inner size that is no multiple of 4: every tile shape (up to 16, up to 64 and more rows) gives a row the same bits."""
