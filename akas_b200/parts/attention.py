@@ -160,7 +160,7 @@ class Attention(Mixer):
 
     @property
     def bounded(self):
-        return not self.general and (self.position is None or hasattr(self.position, "tables"))
+        return not self.pool and (self.position is None or hasattr(self.position, "tables"))
 
     def cache(self):
         s = self.spec

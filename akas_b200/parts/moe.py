@@ -25,6 +25,7 @@ from .mlp import ACTIVATIONS, project_activated
 
 class RoutedExperts(FeedForward):
     chain_safe = True
+    bounded = True
     takes_out_dtype = True
     takes_residual_scale = True
 

@@ -72,6 +72,10 @@ class ParallelMixer(Mixer):
             else:
                 part.w_in = None
 
+    @property
+    def bounded(self):
+        return all(part.bounded for _, part, _ in self.branches)
+
     def cache(self):
         return tuple(part.cache() for _, part, _ in self.branches)
 

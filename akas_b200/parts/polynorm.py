@@ -18,6 +18,7 @@ from .base import FeedForward, Param, project, register_ffn, renamed
 class PolyNormMLP(FeedForward):
     takes_normed = True
     chain_safe = True
+    bounded = True
 
     def __init__(self, spec, runtime):
         super().__init__(spec, runtime)

@@ -31,6 +31,7 @@ from .base import Mixer, Param, StateSpec, project, register_mixer, renamed, sta
 class GatedLinearAttention(Mixer):
     takes_normed = True
     chain_safe = True
+    bounded = True
 
     @classmethod
     def kernels(cls, spec):
@@ -93,6 +94,7 @@ class GatedLinearAttention(Mixer):
 class DecayedLinearAttention(Mixer):
     takes_normed = True
     chain_safe = True
+    bounded = True
     takes_out_dtype = True
 
     @classmethod
@@ -212,6 +214,7 @@ class HGRN2(Mixer):
 class GatedDelta(Mixer):
     takes_normed = True
     chain_safe = True
+    bounded = True
 
     @classmethod
     def kernels(cls, spec):

@@ -247,6 +247,27 @@ def test_long_decoding(dtype, tmp_path):
         assert bad is None, (i, bad, traces.worst(np.stack(rows[i]), want))
 
 
+@pytest.mark.gpu
+def test_captured_mixed_steps(tmp_path):
+    """Decoded tokens beside prompt portions as captured steps per bucket (matrix states, causal convolutions and windowed attention
+    among padding requests in every place), against whole passes of the plain model."""
+    from akas_b200 import EngineConfig
+    from akas_b200.engine.runner import ModelRunner
+
+    config = CONFIGS["mix"]
+    folder, w = make_folder(config, seed=71, folder=tmp_path / "mixed")
+    lengths = dict(enumerate([400, 280, 10, 300, 77, 290, 65, 333, 5]))
+    texts = dict(enumerate(prompts(config["vocab"], [n + 12 for n in lengths.values()], seed=3)))
+    runner = ModelRunner(folder, EngineConfig(dtype="bfloat16", device="cuda:0", page_size=8, max_requests=9, context=448, max_tokens=9 * 448))
+    for _ in range(3):
+        got = traces.beside(runner, texts, lengths, 300)
+        for r, toks in texts.items():
+            want = plain.forward(config, w, toks).numpy()[lengths[r] - 1 :]
+            bad = traces.first_bad(got[r], want, TOL["bfloat16"])
+            assert bad is None, (r, bad, traces.worst(got[r], want))
+    assert len(runner._mixed_graphs) >= 3
+
+
 # --------------------------------------------------------------------------- the kernels one by one
 
 

@@ -436,6 +436,25 @@ def test_long_decoding(dtype, tmp_path):
     compare({i: np.stack(r) for i, r in enumerate(rows)}, want, dtype, f"long decoding/{dtype}")
 
 
+@pytest.mark.gpu
+def test_captured_mixed_steps(tmp_path):
+    """Decoded tokens beside prompt portions as captured steps per bucket (mixers side by side and experts among padding requests in
+    every place), against whole passes of the plain model."""
+    from akas_b200 import EngineConfig
+    from akas_b200.engine.runner import ModelRunner
+
+    config = CONFIGS["odd"]
+    folder, w = make_folder(config, seed=71, folder=tmp_path / "mixed")
+    lengths = dict(enumerate([400, 280, 10, 300, 77, 290, 65, 333, 5]))
+    texts = dict(enumerate(prompts(config["vocab"], [n + 12 for n in lengths.values()], seed=3)))
+    runner = ModelRunner(folder, EngineConfig(dtype="bfloat16", device="cuda:0", page_size=16, max_requests=9, context=448, max_tokens=9 * 448))
+    want = {r: oracle(config, w, toks) for r, toks in texts.items()}
+    want = {r: (logits[lengths[r] - 1 :], held[lengths[r] - 1 :]) for r, (logits, held) in want.items()}
+    for _ in range(3):
+        compare(traces.beside(runner, texts, lengths, 300), want, "bfloat16", "mixed steps, captured")
+    assert len(runner._mixed_graphs) >= 3
+
+
 # --------------------------------------------------------------------------- the kernels one by one
 
 

@@ -313,7 +313,6 @@ def test_captured_mixed_steps_agree_with_the_plain_model(tmp_path):
     """Steps that mix decoded tokens with prompt portions, captured per bucket of rows, decoded requests and portions: any
     number of decoded requests from none to more than a bucket, one to four portions of any lengths, steps that want no logits."""
     from akas_b200.config import EngineConfig
-    from akas_b200.engine.batch import StepEntry
     from akas_b200.engine.runner import ModelRunner
 
     folder = tiny.make_folder(tiny.CONFIGS["c"], seed=13, dtype="bfloat16", folder=tmp_path / "c")
@@ -324,29 +323,8 @@ def test_captured_mixed_steps_agree_with_the_plain_model(tmp_path):
     r = ModelRunner(folder, EngineConfig(dtype="bfloat16", device="cuda:0", page_size=64, max_tokens=16 * 768,
                                          max_requests=16, context=768, cuda_graphs=True))
     for _ in range(3):
-        at = {q: 0 for q in texts}
-        got = {q: {} for q in texts}
-        while any(at[q] < len(texts[q]) for q in texts):
-            room, entries = 300, []
-            for q in sorted(texts, key=lambda q: at[q] < lengths[q]):  # decoded requests in front
-                n = 1 if at[q] >= lengths[q] else min(room, lengths[q] - at[q])
-                if at[q] < len(texts[q]) and n:
-                    room -= n if n > 1 else 0
-                    ends = at[q] + n >= lengths[q]
-                    entries.append(StepEntry(q, texts[q][at[q] : at[q] + n], (n - 1,) if ends else ()))
-            logits = r.step(entries).cpu().numpy()
-            assert len(logits) == sum(len(e.want) for e in entries)
-            row = 0
-            for e in entries:
-                at[e.request] += len(e.tokens)
-                if e.want:
-                    got[e.request][at[e.request] - 1] = logits[row]
-                    row += 1
+        got = traces.beside(r, texts, dict(enumerate(lengths)), 300)
         for q in texts:
-            r.release(q)
-            places = sorted(got[q])
-            assert places == list(range(lengths[q] - 1, len(texts[q])))
-            have, ref = np.stack([got[q][p] for p in places]), want[q][places]
-            err, l2 = traces.worst(have, ref)
+            err, l2 = traces.worst(got[q], want[q][lengths[q] - 1 :])
             assert err <= 2 * BF16["c"][0] and l2 <= 1.5 * BF16["c"][1], (q, err, l2)  # (of 15 rows, not of a whole request)
     assert len(r._mixed_graphs) >= 3 and all(g.graph is not None for g in r._mixed_graphs.values())

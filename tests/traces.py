@@ -121,3 +121,28 @@ def first_bad(got, want, tol):
     err = np.abs(np.asarray(got, np.float64) - np.asarray(want, np.float64)).max(axis=-1) / scale
     bad = np.nonzero(err > tol)[0]
     return int(bad[0]) if len(bad) else None
+
+
+def beside(runner, texts, lengths, room):
+    """Runs every text through the runner, its first ``lengths[r]`` tokens as a prompt in portions and the rest one by one, decoded
+    requests in front and at most ``room`` prompt tokens a step: {request: logits of its last prompt token and all behind it}."""
+    from akas_b200 import StepEntry
+
+    at, got = {r: 0 for r in texts}, {r: [] for r in texts}
+    while any(at[r] < len(texts[r]) for r in texts):
+        left, entries = room, []
+        for r in sorted(texts, key=lambda r: at[r] < lengths[r]):
+            n = 1 if at[r] >= lengths[r] else min(left, lengths[r] - at[r])
+            if at[r] < len(texts[r]) and n:
+                left -= n if at[r] < lengths[r] else 0
+                entries.append(StepEntry(r, texts[r][at[r] : at[r] + n], (n - 1,) if at[r] + n >= lengths[r] else ()))
+        logits, row = runner.step(entries).float().cpu().numpy(), 0
+        assert len(logits) == sum(len(e.want) for e in entries)
+        for e in entries:
+            at[e.request] += len(e.tokens)
+            if e.want:
+                got[e.request].append(logits[row])
+                row += 1
+    for r in texts:
+        runner.release(r)
+    return {r: np.stack(rows) for r, rows in got.items()}
