@@ -80,9 +80,12 @@ def _parallel(block, h, ctx, cache, write):
     if block.ffn is None and block.mixer_scale is None and block.spec.residual_multiplier == 1.0:
         return block.mixer.forward(_normed(block.mixer_norm, block.mixer, h), ctx, cache, residual=h, write=write)
     n = block.mixer_norm.forward(h)
+    # (the router of a captured decode step reads n beside the mixer)
+    routed = block.ffn.route_beside(n, ctx) if hasattr(block.ffn, "route_beside") else None
     a = _float32_result(block.mixer, n, ctx, cache, residual=None, write=write)
     if hasattr(block.ffn, "forward_update"):  # the feed-forward's last kernel does the block's update itself
-        return block.ffn.forward_update(n, ctx, h, a, block.mixer_scale, block.ffn_scale, block.spec.residual_multiplier)
+        more = {} if routed is None else dict(routed=routed)
+        return block.ffn.forward_update(n, ctx, h, a, block.mixer_scale, block.ffn_scale, block.spec.residual_multiplier, **more)
     b = None if block.ffn is None else _float32_result(block.ffn, n, ctx, residual=None)
     return block.mixer.rt.ops.scaled_add(h, a, block.mixer_scale, b, block.ffn_scale, block.spec.residual_multiplier)
 

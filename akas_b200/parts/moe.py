@@ -117,9 +117,21 @@ class RoutedExperts(FeedForward):
                                weight_scale=self.weight_scale)
         return routed if self.shared_gate else (*routed, None)
 
-    def _experts(self, x, update=None):
+    def route_beside(self, x, ctx):
+        """The router's answers for ``forward_update``, computed beside what the block runs in between; None where nothing runs
+        beside anything."""
+        side = self.rt.beside(ctx)
+        if side is None:
+            return None
+        side.wait_stream(torch.cuda.current_stream(self.rt.device))
+        with torch.cuda.stream(side):
+            return self._route(x)
+
+    def _experts(self, x, update=None, routed=None):
         ops = self.rt.ops
-        chosen, weights, gate = self._route(x)
+        if routed is not None:
+            torch.cuda.current_stream(self.rt.device).wait_stream(self.rt._side)
+        chosen, weights, gate = self._route(x) if routed is None else routed
         more = {}
         if self.weight_input:
             more["weight_input"] = True
@@ -135,10 +147,10 @@ class RoutedExperts(FeedForward):
             more["shared"] = (project(self.rt, act, self.w_shared_down, out_dtype=torch.float32), gate)
         return ops.moe_experts(x, self.w_gate_up, self.w_down, chosen, weights, update=update, **more)
 
-    def forward_update(self, x, ctx, h, a, scale_a, scale_b, mult):
+    def forward_update(self, x, ctx, h, a, scale_a, scale_b, mult, routed=None):
         """h += mult * (scale_a * a + scale_b * experts(x)) in place on the float32 residual stream h, by the experts' last
         kernel: what a block whose sublayers' results meet the stream in one sum asks for."""
-        return self._experts(x, update=(h, a, scale_a, scale_b, mult))
+        return self._experts(x, update=(h, a, scale_a, scale_b, mult), routed=routed)
 
     def forward(self, x, ctx, residual=None, out_dtype=None):
         if residual is not None:  # added by the experts' last kernel

@@ -83,8 +83,21 @@ class ParallelMixer(Mixer):
         proj = project(self.rt, x, self.w_in)
         make = torch.zeros if self.padded else torch.empty
         acts = make((proj.shape[0], self.w_out.shape[1]), dtype=self.rt.dtype, device=proj.device)
-        for (_, part, scale), (a, b), (oa, ob), view in zip(self.branches, self.in_spans, self.out_spans, cache):
+        side = self.rt.beside(ctx) if len(self.branches) > 1 else None
+        work = list(zip(self.branches, self.in_spans, self.out_spans, cache))
+        if side is not None:
+            # A captured decode step: the kernels of a branch are a few blocks that wait for memory, so the branches behind the
+            # first run beside it. proj and acts outlive both (the streams meet before they are given back).
+            current = torch.cuda.current_stream(self.rt.device)
+            side.wait_stream(current)
+            with torch.cuda.stream(side):
+                for (_, part, scale), (a, b), (oa, ob), view in work[1:]:
+                    part.core(proj[:, a:b], ctx, view, write, out=acts[:, oa:ob], out_scale=scale)
+            work = work[:1]
+        for (_, part, scale), (a, b), (oa, ob), view in work:
             part.core(proj[:, a:b], ctx, view, write, out=acts[:, oa:ob], out_scale=scale)
+        if side is not None:
+            current.wait_stream(side)
         return project(self.rt, acts, self.w_out, out_dtype=out_dtype, residual=residual)
 
 
