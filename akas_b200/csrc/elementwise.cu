@@ -575,13 +575,33 @@ AKAS_API int akas_round_rows(const float* x, void* out, long long ldo, int N, in
 // PolyNorm of rows: out = a N(z) + b N(z^2) + c N(z^3) + e with N(x) = x / sqrt(mean(x^2) + eps) over the row and
 // the powers taken element by element; coeffs = (a, b, c, e). One block per row; powers and sums are float32. VEC: the
 // row's width is a multiple of 8 and rows start on 16 bytes, so 8 elements move at a time.
-template <typename TI, typename TO, bool VEC>
+// KEEP: up to this many groups of 8 elements per thread stay in registers between the sums and the result (rows of up to
+// 8 KEEP blockDim elements are read once).
+template <typename TI, typename TO, bool VEC, int KEEP>
 __global__ void polynorm_kernel(const TI* __restrict__ z, const float* __restrict__ coeffs, float eps,
                                 TO* __restrict__ out, int F) {
   __shared__ float scratch[3][32];
   const TI* row = z + (size_t)blockIdx.x * F;
   float s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  if (VEC) {
+  float held[KEEP > 0 ? KEEP : 1][8];
+  if (KEEP > 0) {
+#pragma unroll
+    for (int u = 0; u < KEEP; ++u) {
+      const int c = (u * blockDim.x + threadIdx.x) * 8;
+      if (c < F) load8(row + c, held[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < KEEP; ++u) {
+      if ((u * blockDim.x + threadIdx.x) * 8 >= F) break;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = held[u][e], x2 = x * x, x3 = x2 * x;
+        s1 = fmaf(x, x, s1);
+        s2 = fmaf(x2, x2, s2);
+        s3 = fmaf(x3, x3, s3);
+      }
+    }
+  } else if (VEC) {
     for (int c = threadIdx.x * 8; c < F; c += blockDim.x * 8) {
       float x[8];
       load8(row + c, x);
@@ -614,7 +634,20 @@ __global__ void polynorm_kernel(const TI* __restrict__ z, const float* __restric
   const float i3 = coeffs[2] / sqrtf(s3 / (float)F + eps);
   const float e0 = coeffs[3];
   TO* dst = out + (size_t)blockIdx.x * F;
-  if (VEC) {
+  if (KEEP > 0) {
+#pragma unroll
+    for (int u = 0; u < KEEP; ++u) {
+      const int c = (u * blockDim.x + threadIdx.x) * 8;
+      if (c >= F) break;
+      float y[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = held[u][e], x2 = x * x;
+        y[e] = fmaf(x, i1, fmaf(x2, i2, fmaf(x2 * x, i3, e0)));
+      }
+      store8(dst + c, y);
+    }
+  } else if (VEC) {
     for (int c = threadIdx.x * 8; c < F; c += blockDim.x * 8) {
       float x[8], y[8];
       load8(row + c, x);
@@ -640,8 +673,9 @@ AKAS_API int akas_polynorm(const void* z, const float* coeffs, float eps, void* 
   const bool vec = F % 8 == 0 && (uintptr_t)z % 16 == 0 && (uintptr_t)out % 16 == 0;
 #define AKAS_POLY(TI, TO)                                                                                              \
   {                                                                                                                    \
-    if (vec) return launch_ordinary(polynorm_kernel<TI, TO, true>, dim3(N), dim3(threads), 0, stream, (const TI*)z, coeffs, eps, (TO*)out, F);  \
-    return launch_ordinary(polynorm_kernel<TI, TO, false>, dim3(N), dim3(threads), 0, stream, (const TI*)z, coeffs, eps, (TO*)out, F);          \
+    if (vec && F <= 24 * threads) return launch_ordinary(polynorm_kernel<TI, TO, true, 3>, dim3(N), dim3(threads), 0, stream, (const TI*)z, coeffs, eps, (TO*)out, F); \
+    if (vec) return launch_ordinary(polynorm_kernel<TI, TO, true, 0>, dim3(N), dim3(threads), 0, stream, (const TI*)z, coeffs, eps, (TO*)out, F);  \
+    return launch_ordinary(polynorm_kernel<TI, TO, false, 0>, dim3(N), dim3(threads), 0, stream, (const TI*)z, coeffs, eps, (TO*)out, F);          \
   }
   if (in_dtype == AKAS_F32 && out_dtype == AKAS_F32) AKAS_POLY(float, float)
   else if (in_dtype == AKAS_F32) AKAS_POLY(float, bf16)

@@ -45,6 +45,20 @@ decay_gates_kernel(const T* __restrict__ low, long long ld, const float* __restr
     // load comes from DRAM, took 15 us for a rank of 64
     int r = 0;
     if (R % 4 == 0) {
+      if constexpr (TOKENS == 1)  // (a step of few tokens, where the trips are most of the time: 64 at once)
+        for (; r + 64 <= R; r += 64) {
+          float wv[64];
+#pragma unroll
+          for (int j = 0; j < 64; ++j) wv[j] = w[(size_t)(r + j) * O + o];
+#pragma unroll
+          for (int t = 0; t < TOKENS; ++t)
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) {
+              const float4 x = *reinterpret_cast<const float4*>(rows + t * R + r + j);
+              acc[t] = fmaf(x.x, wv[j], acc[t]); acc[t] = fmaf(x.y, wv[j + 1], acc[t]);
+              acc[t] = fmaf(x.z, wv[j + 2], acc[t]); acc[t] = fmaf(x.w, wv[j + 3], acc[t]);
+            }
+        }
       for (; r + 16 <= R; r += 16) {
         float wv[16];
 #pragma unroll
@@ -1080,9 +1094,11 @@ __device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
   v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
 }
 
-template <typename T>
+// WRITE: every request brings one token at most, and whoever has computed a token's channels moves their state on: one launch
+// instead of two.
+template <typename T, bool WRITE>
 __global__ void causal_conv_silu4_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ taps,
-                                         const float* __restrict__ state, long long slot_stride,
+                                         float* state, long long slot_stride,
                                          const int* __restrict__ cu_seqlens, const int* __restrict__ seq_of_token,
                                          const int* __restrict__ slots, float* __restrict__ y, int C, int L) {
   const int n = blockIdx.x;
@@ -1092,7 +1108,7 @@ __global__ void causal_conv_silu4_kernel(const T* __restrict__ x, long long ldx,
   if (slot < 0) return;
   const int first = cu_seqlens[req];
   const int i = n - first;
-  const float* st = state + (size_t)slot * slot_stride;
+  float* st = state + (size_t)slot * slot_stride;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4; c < C; c += gridDim.y * blockDim.x * 4) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < L; ++j) {
@@ -1105,6 +1121,14 @@ __global__ void causal_conv_silu4_kernel(const T* __restrict__ x, long long ldx,
     }
     *reinterpret_cast<float4*>(y + (size_t)n * C + c) =
         make_float4(acc[0] * sigmoid_f(acc[0]), acc[1] * sigmoid_f(acc[1]), acc[2] * sigmoid_f(acc[2]), acc[3] * sigmoid_f(acc[3]));
+    if (WRITE) {
+      for (int j = 0; j < L - 1; ++j) {
+        float in[4];
+        if (j + 1 < L - 1) load4(st + (size_t)(j + 1) * C + c, in);
+        else load4(x + (size_t)n * ldx + c, in);
+        *reinterpret_cast<float4*>(st + (size_t)j * C + c) = make_float4(in[0], in[1], in[2], in[3]);
+      }
+    }
   }
 }
 
@@ -1349,18 +1373,22 @@ gated_rmsnorm_wide_kernel(const float* __restrict__ o, const float* __restrict__
 AKAS_API int akas_decay_gates(const void* low, long long ld, const float* w, const float* bias, float* out, int N, int O,
                               int R, float tau, int dtype, cudaStream_t stream) {
   if (N <= 0 || O <= 0) return 0;
-  // eight tokens a block; sixteen, which read the matrix half as often, where that leaves enough blocks
+  // Eight tokens a block; sixteen, which read the matrix half as often, where that leaves enough blocks; one in a step of at most
+  // 16 tokens, whose few blocks would else form every token's chain and gate one after the other (8 tokens, 1,024 outputs, rank
+  // 64: 5.5 us; eight a block 9.8).
   const size_t row = (size_t)R * sizeof(float);
   if (8 * row > 48 * 1024) return (int)cudaErrorInvalidValue;
   const bool wide = 16 * row <= 48 * 1024 && (long long)((N + 15) / 16) * ((O + 127) / 128) >= 4 * sm_count();
-  const int tokens = wide ? 16 : 8;
+  const int tokens = wide ? 16 : N <= 16 ? 1 : 8;
   const dim3 grid((N + tokens - 1) / tokens, min((O + 127) / 128, 64));
 #define AKAS_GATES(T, TOKENS)                                                                                                     \
   return launch_ordinary(decay_gates_kernel<T, TOKENS>, grid, dim3(128), TOKENS * row, stream, (const T*)low, ld, w, bias, out, N, O, R, \
                          1.f / tau)
   if (dtype == AKAS_F32 && wide) AKAS_GATES(float, 16);
+  if (dtype == AKAS_F32 && tokens == 1) AKAS_GATES(float, 1);
   if (dtype == AKAS_F32) AKAS_GATES(float, 8);
   if (wide) AKAS_GATES(bf16, 16);
+  if (tokens == 1) AKAS_GATES(bf16, 1);
   AKAS_GATES(bf16, 8);
 #undef AKAS_GATES
 }
@@ -1473,7 +1501,8 @@ AKAS_API int akas_delta_scan(const float* q, long long ldq, const float* k, long
 
 AKAS_API int akas_causal_conv_silu(const void* x, long long ldx, const float* taps, float* state, long long slot_stride,
                                    const int* cu_seqlens, const int* seq_of_token, const int* slots, float* y, int N,
-                                   int requests, int C, int L, int write, int dtype, cudaStream_t stream) {
+                                   int requests, int C, int L, int write, int longest, int dtype, cudaStream_t stream) {
+  // longest: the most tokens that a request brings, where the caller knows it (0: it does not)
   if (N <= 0 || C <= 0) return 0;
   const dim3 grid(N, min((C + 255) / 256, 32));
   const float* old = state;
@@ -1485,15 +1514,22 @@ AKAS_API int akas_causal_conv_silu(const void* x, long long ldx, const float* ta
   // 13.4 -> 6.2 us, 4,096 of 296 13.7 -> 6.2; with a token a thread 1,024 of 148 take 3.9, 2,048 of 148 5.4
   const dim3 runs((N + kConvRun - 1) / kConvRun, (C / 4 + 127) / 128);
   const bool run = four && L == 4 && (uintptr_t)taps % 16 == 0 && (long long)runs.x * runs.y >= 2 * sm_count() && runs.y <= 65535;
+  if (longest == 1 && write && four && !run && L > 1) {  // every token's own thread moves the state on
+    if (dtype == AKAS_F32)
+      return launch_ordinary(causal_conv_silu4_kernel<float, true>, grid4, dim3(128), 0, stream, (const float*)x, ldx, taps, state,
+                             slot_stride, cu_seqlens, seq_of_token, slots, y, C, L);
+    return launch_ordinary(causal_conv_silu4_kernel<bf16, true>, grid4, dim3(128), 0, stream, (const bf16*)x, ldx, taps, state, slot_stride,
+                           cu_seqlens, seq_of_token, slots, y, C, L);
+  }
   int err = run ? (dtype == AKAS_F32
       ? launch_ordinary(causal_conv_silu_run_kernel<float>, runs, dim3(128), 0, stream, (const float*)x, ldx, taps, old, slot_stride,
                         cu_seqlens, seq_of_token, slots, y, N, C)
       : launch_ordinary(causal_conv_silu_run_kernel<bf16>, runs, dim3(128), 0, stream, (const bf16*)x, ldx, taps, old, slot_stride,
                         cu_seqlens, seq_of_token, slots, y, N, C))
       : four ? (dtype == AKAS_F32
-      ? launch_ordinary(causal_conv_silu4_kernel<float>, grid4, dim3(128), 0, stream, (const float*)x, ldx, taps, old, slot_stride,
+      ? launch_ordinary(causal_conv_silu4_kernel<float, false>, grid4, dim3(128), 0, stream, (const float*)x, ldx, taps, state, slot_stride,
                         cu_seqlens, seq_of_token, slots, y, C, L)
-      : launch_ordinary(causal_conv_silu4_kernel<bf16>, grid4, dim3(128), 0, stream, (const bf16*)x, ldx, taps, old, slot_stride,
+      : launch_ordinary(causal_conv_silu4_kernel<bf16, false>, grid4, dim3(128), 0, stream, (const bf16*)x, ldx, taps, state, slot_stride,
                         cu_seqlens, seq_of_token, slots, y, C, L))
       : dtype == AKAS_F32
       ? launch_ordinary(causal_conv_silu_kernel<float>, grid, dim3(256), 0, stream, (const float*)x, ldx, taps, old, slot_stride,

@@ -78,7 +78,7 @@ _SIGNATURES = {
         "akas_delta_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_causal_conv_silu": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
-                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "akas_delta_prep": [c_void_p, c_longlong, c_int, c_int, c_float, c_float, c_void_p, c_longlong, c_void_p, c_longlong,
                             c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "akas_gated_rmsnorm": [c_void_p, c_void_p, c_float, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -1585,7 +1585,9 @@ def hgrn2_scan(q, f, v, f_bias, lower, state, cu_seqlens, slots, heads, dim, vdi
 
 
 @_flushes
-def causal_conv_silu(x, taps, state, cu_seqlens, seq_of_token, slots, write=True):
+def causal_conv_silu(x, taps, state, cu_seqlens, seq_of_token, slots, write=True, longest=None):
+    """``longest``: the most tokens a request brings in this step, where the caller knows it (where that is one, the kernel that
+    convolves moves the state on too)."""
     n, c = x.shape
     l = taps.shape[1]
     if taps.dtype != torch.float32 or taps.shape[0] != c or not taps.is_contiguous():
@@ -1594,8 +1596,8 @@ def causal_conv_silu(x, taps, state, cu_seqlens, seq_of_token, slots, write=True
     sp, stride = _slot_rows(state, "state")
     y = torch.empty((n, c), dtype=torch.float32, device=x.device)
     _check(_fn("recurrent", "akas_causal_conv_silu")(xp, ldx, _ptr(taps), sp, stride, _ptr(cu_seqlens), _ptr(seq_of_token),
-                                                    _ptr(slots), _ptr(y), n, slots.numel(), c, l, int(bool(write)), _code(x),
-                                                    _stream()), "causal_conv_silu", kernels=2 if write else 1)
+                                                    _ptr(slots), _ptr(y), n, slots.numel(), c, l, int(bool(write)), int(longest or 0),
+                                                    _code(x), _stream()), "causal_conv_silu", kernels=2 if write and longest != 1 else 1)
     return y
 
 

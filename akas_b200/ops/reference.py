@@ -401,7 +401,7 @@ def hgrn2_scan(q, f, v, f_bias, lower, state, cu_seqlens, slots, heads, dim, vdi
     return o.reshape(n, heads * vdim)
 
 
-def causal_conv_silu(x, taps, state, cu_seqlens, seq_of_token, slots, write=True):
+def causal_conv_silu(x, taps, state, cu_seqlens, seq_of_token, slots, write=True, longest=None):
     """silu of a causal depthwise convolution over each request's tokens: y_t = silu(sum_j taps[:, j] x_(t - L + 1 + j)),
     inputs before the step's first token from ``state`` (zero at a request's start). x [N, C] -> float32 [N, C]."""
     n, c = x.shape

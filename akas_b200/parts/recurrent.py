@@ -274,7 +274,8 @@ class GatedDelta(Mixer):
         matrix_state = cache.state[:, :matrix_words].view(slots, h, s.value_dim, s.key_dim)
         conv_state = cache.state[:, matrix_words : matrix_words + (s.conv_kernel - 1) * ch].view(slots, s.conv_kernel - 1, ch)
         proj = project(self.rt, x, self.w_in)
-        y = ops.causal_conv_silu(proj[:, :ch], self.taps, conv_state, ctx.cu_seqlens, ctx.seq_of_token, ctx.slots, write=write)
+        y = ops.causal_conv_silu(proj[:, :ch], self.taps, conv_state, ctx.cu_seqlens, ctx.seq_of_token, ctx.slots, write=write,
+                                 longest=getattr(ctx, "max_query_len", None))
         beta, g = ops.delta_prep(y, s.num_kv_heads, s.key_dim, s.key_dim ** -0.5, s.unit_eps, proj[:, ch : ch + h],
                                  proj[:, ch + h : ch + 2 * h], self.a_log, self.dt_bias)
         o = ops.delta_scan(y[:, :gd], y[:, gd : 2 * gd], y[:, 2 * gd :], beta, g, matrix_state, ctx.cu_seqlens, ctx.slots,

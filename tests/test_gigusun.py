@@ -248,6 +248,29 @@ def test_long_decoding(dtype, tmp_path):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("channels,taps", [(2048, 4), (12, 2), (1028, 5), (64, 3)])
+def test_convolution_of_single_tokens_moves_the_state_on(channels, taps):
+    """A step in which no request brings more than one token, said so: one kernel convolves and shifts the states, padding left
+    alone, to the same bits as the two kernels."""
+    from akas_b200.ops import cuda
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    lengths, slots = [1, 1, 0, 1, 1], [3, 0, -1, 6, -1]
+    cu, seq, sl = _batch(lengths, slots, "cuda:0")
+    x = torch.randn((len(seq), channels), device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn((channels, taps), device="cuda", generator=g)
+    state = torch.randn((8, taps - 1, channels), device="cuda", generator=g)
+    two, one = state.clone(), state.clone()
+    live = [i for i, r in enumerate(seq.tolist()) if slots[r] >= 0]
+    want = cuda.causal_conv_silu(x, w, two, cu, seq, sl)
+    got = cuda.causal_conv_silu(x, w, one, cu, seq, sl, longest=1)
+    assert torch.equal(got[live], want[live]) and torch.equal(one, two) and not torch.equal(one, state)
+    untouched = state.clone()
+    cuda.causal_conv_silu(x, w, untouched, cu, seq, sl, write=False, longest=1)
+    assert torch.equal(untouched, state)
+
+
+@pytest.mark.gpu
 def test_captured_mixed_steps(tmp_path):
     """Decoded tokens beside prompt portions as captured steps per bucket (matrix states, causal convolutions and windowed attention
     among padding requests in every place), against whole passes of the plain model."""
