@@ -158,16 +158,18 @@ class Runtime:
     ops: Any
     _side: Any = None
 
-    def beside(self, ctx):
-        """The stream for kernels of a captured decode step that may run beside the step's own stream, or None (any other step:
+    def beside(self, ctx, lane: int = 0):
+        """The stream (one per lane) for kernels of a captured decode step that may run beside the step's own stream, or None (any other step:
         its kernels fill the GPU, or the host enqueues them one by one). Whoever uses it lets it wait for the current stream
         first and lets the current stream wait for it before anything it reads, writes or has allocated there is touched
         or given back."""
         if not (ctx.decode_only and ctx.memo.get("captured")) or self.device.type != "cuda":
             return None
         if self._side is None:
-            self._side = torch.cuda.Stream(device=self.device)
-        return self._side
+            self._side = {}
+        if lane not in self._side:
+            self._side[lane] = torch.cuda.Stream(device=self.device)
+        return self._side[lane]
 
 
 class Normed:

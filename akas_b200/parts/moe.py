@@ -120,7 +120,7 @@ class RoutedExperts(FeedForward):
     def route_beside(self, x, ctx):
         """The router's answers for ``forward_update``, computed beside what the block runs in between; None where nothing runs
         beside anything."""
-        side = self.rt.beside(ctx)
+        side = self.rt.beside(ctx, 1)  # (not the mixer's branches' lane: they need not wait for the router)
         if side is None:
             return None
         side.wait_stream(torch.cuda.current_stream(self.rt.device))
@@ -130,7 +130,7 @@ class RoutedExperts(FeedForward):
     def _experts(self, x, update=None, routed=None):
         ops = self.rt.ops
         if routed is not None:
-            torch.cuda.current_stream(self.rt.device).wait_stream(self.rt._side)
+            torch.cuda.current_stream(self.rt.device).wait_stream(self.rt._side[1])
         chosen, weights, gate = self._route(x) if routed is None else routed
         more = {}
         if self.weight_input:
