@@ -50,6 +50,9 @@ class StepContext:
     max_context: int  # largest position + 1 in the batch
     decode_only: bool  # every request brings exactly one token
     query_lens: Tuple[int, ...] = ()  # how many tokens each request brings, known on the host (a kernel sizes its grid from it)
+    # Whether the pages hold every earlier token's keys and values since before the step's first kernel (the runner's steps: a copy
+    # from the host, which waits for the step before, stands in front of them)
+    earlier_keys_settled: bool = False
     memo: Dict = field(default_factory=dict)  # per-step results shared between layers (rotary tables)
 
     def block_table(self, group: int) -> torch.Tensor:

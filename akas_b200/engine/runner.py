@@ -139,6 +139,7 @@ class ModelRunner:
             max_context=max_ctx,
             decode_only=decode_only,
             query_lens=tuple(query_lens),
+            earlier_keys_settled=True,
         )
 
     # ------------------------------------------------------------------ the step

@@ -1391,8 +1391,9 @@ def qkv_decode_attention(qkv, heads, kv_heads, head_dim, q_weight, k_weight, eps
     if splits > 1:
         part_o = torch.empty((n, heads, splits, head_dim), dtype=torch.float32, device=qkv.device)
         part_ml = torch.empty((n, heads, splits, 2), dtype=torch.float32, device=qkv.device)
+    settled = 2 if not walks and getattr(ctx, "earlier_keys_settled", False) else 0
     prep = (_ptr(qkv), _ptr(q_weight), _ptr(k_weight), float(eps), _norm_place(q_weight, zero_centered, unit), _ptr(cos), _ptr(sin), rotary,
-            int(bool(write)), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0], _ptr(block_table), block_table.shape[1],
+            int(bool(write)) + settled, _ptr(k_pool), _ptr(v_pool), k_pool.shape[0], _ptr(block_table), block_table.shape[1],
             _ptr(seq_of_token), _ptr(positions), _ptr(out), _ptr(part_o), _ptr(part_ml), float(scale), win, page_size, n,
             heads, kv_heads, head_dim, splits, _stream())
     if walks:
