@@ -35,8 +35,6 @@
 //            The groups take a tile's columns in turn, each with a staging tile of its own; the block's last tile uses
 //            the ring, which nobody needs any more, so that no store is waited for. The warps then arrive on the
 //            leader's "accumulator empty" barrier (the peer through the cluster's shared memory window).
-// Weights. The tensor cores' warp of the block that issues nothing asks the L2 for the pair's weights, whole rows, as soon
-// as the kernel runs (219 -> 211 us a layer of four products at 2,048 tokens and width 2,048, the read-out above included).
 // Parts of K (SPLIT, ACC and F32 only). A product with few tiles and a long K leaves most pairs idle and the others walking
 // their stages (some 1,100 cycles each with four in flight). There a cluster is 2 to 4 pairs that take a part of K each of one
 // tile of 128 channels. When all have run, every block sends the sums of the 32-column units that it does not finish to
@@ -126,7 +124,7 @@ template <int BN, int EPI, bool WIDE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_y, int M, int N, int K, int F, const float* __restrict__ bias,
-                 int act, int parts, const __nv_bfloat16* __restrict__ w) {
+                 int act, int parts) {
   // N: channels of the product (for SWIGLU the stacked height 2F); a tile covers BN of them (SWIGLU: BN/2 gate
   // rows f0.. and BN/2 up rows F + f0..).
   using S = Shape<BN>;
@@ -232,19 +230,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (SPLIT) { __syncwarp(); cluster_arrive(); cluster_wait(); }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ tensor cores (the leader issues for the pair)
-    if (rank == 1) {
-      // The other block's warp asks the L2 for the weights of the pair's tiles, whole rows at a time, as soon as the kernel
-      // runs: with the ring's stages alone, what is in flight does not cover DRAM's latency where few pairs work. Where
-      // several pairs read the same channels, the first row tile's does it.
-      for (int tile = pair; tile < tiles_n; tile += pairs) {
-        const int n0 = tile * TILE_N, from = stage0 * STEPS * BK, upto = min(K, stage1 * STEPS * BK);
-        for (int r = lane; r < BN; r += 32) {
-          const int row = EPI != EPI_SWIGLU ? n0 + r : r < TILE_N ? n0 + r : F + n0 + r - TILE_N;
-          if (n0 + (EPI != EPI_SWIGLU ? r : r % TILE_N) < out_cols && upto > from)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)row * K + from), "r"((upto - from) * 2) : "memory");
-        }
-      }
-    }
     if (lane == 0 && rank == 0) {
       // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 256 over the pair
       constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(2 * BM >> 4) << 24);
@@ -549,7 +534,7 @@ int launch(const void* x, const void* w, void* y, int M, int N, int K, const flo
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = chained_launches_enabled() ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&config, gemm_pair_kernel<BN, EPI, WIDE, SPLIT>, map_x, map_w, map_y, M, N, K, F, bias, act, parts, (const __nv_bfloat16*)w);
+  const cudaError_t e = cudaLaunchKernelEx(&config, gemm_pair_kernel<BN, EPI, WIDE, SPLIT>, map_x, map_w, map_y, M, N, K, F, bias, act, parts);
   return e != cudaSuccess ? (int)e : launch_status();
 }
 
