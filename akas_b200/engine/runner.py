@@ -8,9 +8,10 @@ the scheduler and trace replay all go through it.
 kreasof-ai/akas's counterpart is ``Executor`` with ``Batch.prepare/run``
 (src/akas/execution/executor.py:360-374, src/akas/execution/batch.py:21-134): one
 captured CUDA graph per compiled ``rows x chunk`` geometry, prefill and decode in
-separate launches. Here any mix runs eagerly, and steps that only decode replay a
+separate launches. Here any mix is one step; steps that only decode replay a
 CUDA graph captured per batch-size bucket (the reference's device for decode
-latency too: src/akas/execution/forward.py:41-45).
+latency too: src/akas/execution/forward.py:41-45), mixed steps of up to a
+thousand rows one per bucket of rows and requests, and the rest runs eagerly.
 """
 
 from __future__ import annotations
